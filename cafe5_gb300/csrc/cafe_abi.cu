@@ -17,7 +17,6 @@
 #include <functional>
 #include <numeric>
 #include <random>
-#include <unordered_set>
 
 #include "runtime.h"
 
@@ -327,6 +326,14 @@ void build_plan(TreeHost& T) {
             if (!T.children[c].empty()) free_slots.push_back(T.slot[c]);
     }
     T.n_slots = n_slots;
+    std::vector<int> h(n, 0);
+    T.height.assign(order.size(), 0);
+    T.internal_index.assign(n, -1);
+    for (size_t ii = 0; ii < order.size(); ++ii) {
+        for (int c : T.children[order[ii]]) h[order[ii]] = std::max(h[order[ii]], h[c] + 1);
+        T.height[ii] = h[order[ii]];
+        T.internal_index[order[ii]] = (int)ii;
+    }
 }
 
 int upload_plan(cafe_ctx* C, TreeHost& T) {
@@ -356,19 +363,21 @@ int upload_plan(cafe_ctx* C, TreeHost& T) {
     return CAFE_OK;
 }
 
+// The S-bin of a family with largest count mx.
+int bin_width(int mx) {
+    const int need = (int)std::ceil(1.2 * mx) + 20 + 1;
+    for (int i = 0; i < kNumDefaultBins; ++i)
+        if (kDefaultBins[i] >= need) return kDefaultBins[i];
+    return kDefaultBins[kNumDefaultBins - 1];
+}
+
 int compute_bins(cafe_ctx* C, FamSet& S) {
     BinPlan& B = S.bins;
     const int64_t F = S.F;
     std::vector<int> wf(F), rf(F);
     for (int64_t f = 0; f < F; ++f) {
         const int mx = S.max_count[f];
-        const int need = (int)std::ceil(1.2 * mx) + 20 + 1;
-        int w = kDefaultBins[kNumDefaultBins - 1];
-        for (int i = 0; i < kNumDefaultBins; ++i)
-            if (kDefaultBins[i] >= need) {
-                w = kDefaultBins[i];
-                break;
-            }
+        const int w = bin_width(mx);
         wf[f] = w;
         const int Sf = w - 1;
         rf[f] = std::min(Sf, std::max(30, (int)std::rint(mx * 1.25)));
@@ -400,6 +409,119 @@ int compute_bins(cafe_ctx* C, FamSet& S) {
     return CAFE_OK;
 }
 
+// A device buffer of one call, stream-ordered.
+struct TempBuf {
+    void* p = nullptr;
+    cudaStream_t s;
+    explicit TempBuf(cudaStream_t st) : s(st) {}
+    ~TempBuf() {
+        if (p) cudaFreeAsync(p, s);
+    }
+    cudaError_t get(size_t n) { return cudaMallocAsync(&p, std::max<size_t>(n, 256), s); }
+    template <class T> T* as() const { return static_cast<T*>(p); }
+};
+
+// The distinct patterns of every subtree, for families grouped as in `first`
+// / `count` over perm: built on the device, one launch per tree level.
+int build_patterns(cafe_ctx* C, const TreeHost& T, FamSet& S, const int64_t* d_perm, const std::vector<int64_t>& first,
+                   const std::vector<int64_t>& count, const std::vector<int>& max_count, PatternPlan& P) {
+    const int64_t F = S.F;
+    const int ni = (int)T.internal.size(), ng = (int)first.size();
+    P.n_groups = ng;
+    P.n_internal = ni;
+    P.group_first = first;
+    P.group_count = count;
+    P.group_max = max_count;
+    P.rows.assign((size_t)ng * ni, 0);
+    P.child_off.assign((size_t)ng * ni, 0);
+    if (!F) return CAFE_OK;
+    CK(cudaDeviceSynchronize(), "patterns");      // the counts and the order are on the device, and no call in flight reads the old plan
+    if (ng > kMaxGroups) return fail(C, CAFE_ERR_INVALID, "%d family groups", ng);
+    const cudaStream_t st = C->ws[0]->stream_hi;
+    int64_t slots = 1024;
+    while (slots < 2 * F) slots *= 2;
+    int max_h = 0;
+    for (int h : T.height) max_h = std::max(max_h, h);
+    std::vector<std::vector<int32_t>> level(max_h + 1);
+    size_t widest = 1;
+    for (int ii = 0; ii + 1 < ni; ++ii) level[T.height[ii]].push_back(ii);     // (the root, last, keeps a row per family)
+    for (auto& l : level) widest = std::max(widest, l.size());
+    // the insertion tables take at most about 1 GB at a time
+    const size_t batch = std::max<size_t>(1, std::min(widest, ((size_t)1 << 30) / (slots * sizeof(int32_t))));
+    std::vector<int32_t> ints = T.internal_index;
+    for (auto& l : level) ints.insert(ints.end(), l.begin(), l.end());
+    TempBuf d_ints(st), d_rep(st), d_num(st), d_base(st), d_tab(st), d_off(st);
+    CK(d_ints.get(ints.size() * sizeof(int32_t)), "patterns");
+    CK(d_rep.get((size_t)ni * F * sizeof(int32_t)), "patterns");
+    CK(d_num.get((size_t)ni * F * sizeof(int32_t)), "patterns");
+    CK(d_base.get((size_t)ni * (ng + 1) * sizeof(int32_t)), "patterns");
+    CK(d_tab.get(batch * slots * sizeof(int32_t)), "patterns");
+    CK(cudaMemcpyAsync(d_ints.p, ints.data(), ints.size() * sizeof(int32_t), cudaMemcpyHostToDevice, st), "patterns");
+    PatBuildArgs a;
+    std::memset(&a, 0, sizeof a);
+    a.plan = T.plan;
+    a.counts = S.d_counts.as<int32_t>();
+    a.perm = d_perm;
+    a.node_ii = d_ints.as<int32_t>();
+    a.F = F;
+    a.n_groups = ng;
+    int64_t n_flags = 0;
+    for (int g = 0; g < ng; ++g) {
+        a.group_first[g] = first[g];
+        a.group_max[g] = max_count[g];
+        a.flag_off[g] = n_flags;
+        n_flags += (int64_t)T.n_leaves * (max_count[g] + 1);
+    }
+    TempBuf d_flags(st);
+    CK(d_flags.get((size_t)n_flags), "patterns");
+    CK(cudaMemsetAsync(d_flags.p, 0, (size_t)n_flags, st), "patterns");
+    CK(launch_pat_counts(a, d_flags.as<uint8_t>(), st), "patterns");
+    a.rep = d_rep.as<int32_t>();
+    a.num = d_num.as<int32_t>();
+    a.base = d_base.as<int32_t>();
+    const int32_t* d_nodes = d_ints.as<int32_t>() + T.n_nodes;
+    for (auto& l : level) {
+        for (size_t b = 0; b < l.size(); b += batch)
+            CK(launch_pat_insert(a, d_nodes + b, (int)std::min(batch, l.size() - b), d_tab.as<int32_t>(), slots, st),
+               "patterns");
+        d_nodes += l.size();
+    }
+    CK(launch_pat_number(a, st), "patterns");
+    std::vector<int32_t> base((size_t)ni * (ng + 1));
+    std::vector<uint8_t> flags((size_t)n_flags);
+    CK(cudaMemcpyAsync(flags.data(), d_flags.p, flags.size(), cudaMemcpyDeviceToHost, st), "patterns");
+    CK(cudaMemcpyAsync(base.data(), d_base.p, base.size() * sizeof(int32_t), cudaMemcpyDeviceToHost, st), "patterns");
+    CK(cudaStreamSynchronize(st), "patterns");
+    int64_t off = 0;
+    for (int g = 0; g < ng; ++g)
+        for (int ii = 0; ii < ni; ++ii) {
+            const bool root = T.internal[ii] == T.root;
+            const int64_t r = root ? count[g] : base[(size_t)ii * (ng + 1) + g + 1] - base[(size_t)ii * (ng + 1) + g];
+            P.rows[(size_t)g * ni + ii] = r;
+            P.child_off[(size_t)g * ni + ii] = off;
+            off += r * (T.cstart[ii + 1] - T.cstart[ii]);
+        }
+    CK(P.d_child.reserve(std::max<int64_t>(off, 1) * sizeof(int32_t)), "patterns");
+    CK(d_off.get(P.child_off.size() * sizeof(int64_t)), "patterns");
+    CK(cudaMemcpyAsync(d_off.p, P.child_off.data(), P.child_off.size() * sizeof(int64_t), cudaMemcpyHostToDevice, st),
+       "patterns");
+    std::vector<int32_t> used;
+    P.leaf_off.clear();
+    for (int g = 0; g < ng; ++g)
+        for (int c = 0; c < T.n_leaves; ++c) {
+            P.leaf_off.push_back((int64_t)used.size());
+            const uint8_t* f = flags.data() + a.flag_off[g] + (size_t)c * (max_count[g] + 1);
+            for (int n = 0; n <= max_count[g]; ++n)
+                if (f[n]) used.push_back(n);
+        }
+    P.leaf_off.push_back((int64_t)used.size());
+    CK(P.d_counts.reserve(used.size() * sizeof(int32_t)), "patterns");
+    CK(cudaMemcpyAsync(P.d_counts.p, used.data(), used.size() * sizeof(int32_t), cudaMemcpyHostToDevice, st), "patterns");
+    CK(launch_pat_write(a, d_off.as<int64_t>(), P.d_child.as<int32_t>(), st), "patterns");
+    CK(cudaStreamSynchronize(st), "patterns");
+    return CAFE_OK;
+}
+
 int prepare_set(cafe_ctx* C, FamSet& S) {
     const int64_t F = S.F;
     const int nl = S.n_leaves;
@@ -409,42 +531,27 @@ int prepare_set(cafe_ctx* C, FamSet& S) {
         for (int c = 0; c < nl; ++c) m = std::max(m, S.h_counts[f * nl + c]);
         S.max_count[f] = m;
     }
-    // dedupe (build_reference_list, src/base_model.cpp:27-51), hashed
-    std::vector<int64_t> ref(F);
-    std::unordered_map<uint64_t, std::vector<int64_t>> buckets;
-    S.unique.clear();
-    for (int64_t f = 0; f < F; ++f) {
-        const int32_t* row = &S.h_counts[f * nl];
-        uint64_t h = 1469598103934665603ull;
-        for (int c = 0; c < nl; ++c) h = (h ^ (uint32_t)row[c]) * 1099511628211ull;
-        auto& b = buckets[h];
-        int64_t found = -1;
-        for (int64_t g : b)
-            if (std::memcmp(&S.h_counts[g * nl], row, sizeof(int32_t) * nl) == 0) {
-                found = g;
-                break;
-            }
-        if (found < 0) {
-            b.push_back(f);
-            S.unique.push_back(f);
-            ref[f] = f;
-        } else {
-            ref[f] = found;
-        }
-    }
+    // (families with equal counts are found subtree by subtree, below)
     std::vector<int64_t> ident(F);
     std::iota(ident.begin(), ident.end(), 0);
-    const size_t nb = std::max<int64_t>(F, 1) * sizeof(int64_t);
-    CK(S.d_ref.reserve(nb), "families");
-    CK(S.d_identity.reserve(nb), "families");
-    CK(S.d_unique.reserve(nb), "families");
-    if (F) {
-        CK(cudaMemcpy(S.d_ref.p, ref.data(), F * sizeof(int64_t), cudaMemcpyHostToDevice), "families");
-        CK(cudaMemcpy(S.d_identity.p, ident.data(), F * sizeof(int64_t), cudaMemcpyHostToDevice), "families");
-        CK(cudaMemcpy(S.d_unique.p, S.unique.data(), S.unique.size() * sizeof(int64_t), cudaMemcpyHostToDevice),
-           "families");
+    CK(S.d_identity.reserve(std::max<int64_t>(F, 1) * sizeof(int64_t)), "families");
+    if (F) CK(cudaMemcpy(S.d_identity.p, ident.data(), F * sizeof(int64_t), cudaMemcpyHostToDevice), "families");
+    int rc = compute_bins(C, S);
+    if (rc) return rc;
+    const TreeHost& T = *C->trees.find(S.tree_id)->second;
+    // largest count of each bin (bins follow the counts) and of the set
+    std::vector<int> bin_max(S.bins.widths.size(), 0);
+    int all_max = 0;
+    for (int64_t f = 0; f < F; ++f) {
+        const int m = S.max_count[f];
+        const size_t b = std::lower_bound(S.bins.widths.begin(), S.bins.widths.end(), bin_width(m)) - S.bins.widths.begin();
+        bin_max[b] = std::max(bin_max[b], m);
+        all_max = std::max(all_max, m);
     }
-    return compute_bins(C, S);
+    rc = build_patterns(C, T, S, S.bins.d_perm.as<int64_t>(), S.bins.bin_first, S.bins.bin_count, bin_max, S.pat_bins);
+    if (!rc)
+        rc = build_patterns(C, T, S, S.d_identity.as<int64_t>(), {0}, {F}, {all_max}, S.pat_all);
+    return rc;
 }
 
 // Matrix cache: look up or schedule (size, lambda, t). Caller holds C->mu.
@@ -672,7 +779,8 @@ struct ScoreInfo {
     bool scaled = false;
     size_t footprint = 0;
     int64_t n_fallback = 0;
-    const int32_t* d_tail = nullptr;   // tensor-core pass: [status, fallback families, fallback tiles]
+    const int32_t* d_tail = nullptr;   // [status, fallback families, fallback tiles]
+    bool tail_counts = true;           // the tail's counts are set (tensor-core pass)
 };
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -782,8 +890,8 @@ int stage_cat_probs(cafe_ctx* C, Workspace& ws, const cafe_request* R, int K, in
 
 // Per-family lnL and the total of every candidate, then +inf / NaN for
 // the candidates rejected before pruning.
-int finish_batch(cafe_ctx* C, Workspace& ws, const ScoreInfo* info, bool gamma, bool scaled, const int64_t* d_ref,
-                 const int32_t* d_status, double* d_fam, double* d_total) {
+int finish_batch(cafe_ctx* C, Workspace& ws, const ScoreInfo* info, bool gamma, bool scaled, const int32_t* d_status,
+                 double* d_fam, double* d_total) {
     const int64_t F = info->F;
     const int NB = info->B;
     FinishArgs fa;
@@ -794,7 +902,6 @@ int finish_batch(cafe_ctx* C, Workspace& ws, const ScoreInfo* info, bool gamma, 
     fa.model = gamma ? 1 : 0;
     fa.scaled = scaled ? 1 : 0;
     fa.cat = ws.cat.as<double>();
-    fa.ref = d_ref;
     fa.family_lnl = d_fam;
     fa.total = d_total;
     fa.n_failed = ws.nfail.as<int32_t>();
@@ -825,129 +932,6 @@ int finish_batch(cafe_ctx* C, Workspace& ws, const ScoreInfo* info, bool gamma, 
     return CAFE_OK;
 }
 
-// Launch k_prune64 (per-node rescaled FP64) for the given 32-family tiles.
-int launch_fp64_tiles(cafe_ctx* C, Workspace& ws, const cafe_request* R, TreeHost& T, FamSet& S, int K,
-                      const std::vector<PruneTile>& tiles, DevBuf& d_tiles, PinnedBuf& h_tiles, const int64_t* d_perm,
-                      int W, int msize, double* out, int prof_kind) {
-    if (tiles.empty()) return CAFE_OK;
-    const int n = (int)tiles.size();
-    CK(h_tiles.reserve(n * sizeof(PruneTile)), "tiles");
-    CK(d_tiles.reserve(n * sizeof(PruneTile)), "tiles");
-    std::memcpy(h_tiles.p, tiles.data(), n * sizeof(PruneTile));
-    CK(op_h2d(ws, d_tiles.p, h_tiles.p, n * sizeof(PruneTile), ws.stream), "tiles");
-    const int n_ctas = std::max(1, std::min(n, C->n_ctas));
-    const int64_t per_cta = (int64_t)T.n_slots * W * 32;
-    CK(ws.scratch.reserve((size_t)n_ctas * per_cta * sizeof(double)), "scratch");
-    Prune64Args a;
-    std::memset(&a, 0, sizeof a);
-    a.plan = T.plan;
-    a.tiles = d_tiles.as<PruneTile>();
-    a.n_tiles = n;
-    a.counts = S.d_counts.as<int32_t>();
-    a.perm = d_perm;
-    a.mats = ws.mats.as<const double*>();
-    a.ld_mat = msize;
-    a.prior = C->d_prior.as<double>();
-    a.n_prior = (int)C->prior.size();
-    a.err = R->use_error_model ? C->d_err.as<double>() : nullptr;
-    a.err_rows = C->err_rows;
-    a.err_ndev = C->err_ndev;
-    a.fam_R = S.bins.d_famR.as<int32_t>();
-    a.scratch = ws.scratch.as<double>();
-    a.scratch_per_cta = per_cta;
-    a.scaled = 1;
-    a.model = R->model == CAFE_MODEL_GAMMA ? 1 : 0;
-    a.out = out;
-    a.K = K;
-    a.cat_probs = ws.catp.as<double>();
-    a.tile_families = 32;
-    a.W = W;
-    const bool prof = ws.sync;
-    cudaEvent_t ev;
-    if (prof) C->prof.begin(prof_kind, ws.stream, &ev);
-    CK(op_launch(ws, 3, [&] { return launch_prune64(a, n_ctas, ws.stream); }, a, n_ctas, ws.stream), "prune fp64");
-    if (prof) C->prof.end(prof_kind, ws.stream, ev);
-    return CAFE_OK;
-}
-
-// Bins walked one family per thread-block cluster (k_prune64_cl): those whose
-// 32-family tiles of one candidate would occupy less than half of the SMs.
-// The choice depends on the family set and the category count only, so a
-// candidate gets the same bits alone and in a batch. The cluster gives each
-// CTA at least 64 rows of the bin.
-int fp64_cluster_size(int w) { return w >= 512 ? 8 : w >= 256 ? 4 : w >= 128 ? 2 : 1; }
-
-bool fp64_cluster_bin(const cafe_ctx* C, const TreeHost& T, int64_t count, int K, int w) {
-    return count > 0 && ((count + 31) / 32) * (int64_t)K * 2 < C->sm_count &&
-           prune64_cluster_smem(T.n_slots, w) <= prune64_cluster_max_smem();
-}
-
-// One tile per family of bin b for every category index in `active`.
-void add_cluster_tiles(std::vector<PruneTile>& out, const BinPlan& B, size_t b, const std::vector<int32_t>& active) {
-    const int w = B.widths[b];
-    for (int k : active)
-        for (int64_t i = 0; i < B.bin_count[b]; ++i) {
-            PruneTile t{};
-            t.first = (int)(B.bin_first[b] + i);
-            t.count = 1;
-            t.k = k;
-            t.S = w - 1;
-            t.R = w - 1;
-            out.push_back(t);
-        }
-}
-
-// Launch the one-family-per-cluster FP64 walk over `tiles` (grouped by bin,
-// bins ascending): one launch per bin, sized by the bin's width.
-int launch_fp64_cluster(cafe_ctx* C, Workspace& ws, const cafe_request* R, TreeHost& T, FamSet& S, int K,
-                        const std::vector<PruneTile>& tiles, const int64_t* d_perm, const int32_t* d_famR, int msize,
-                        bool scaled, double* out, cudaStream_t st, int prof_kind) {
-    if (tiles.empty()) return CAFE_OK;
-    const size_t n = tiles.size();
-    CK(ws.h_tiles_cl.reserve(n * sizeof(PruneTile)), "tiles");
-    CK(ws.tiles_cl.reserve(n * sizeof(PruneTile)), "tiles");
-    std::memcpy(ws.h_tiles_cl.p, tiles.data(), n * sizeof(PruneTile));
-    CK(op_h2d(ws, ws.tiles_cl.p, ws.h_tiles_cl.p, n * sizeof(PruneTile), st), "tiles");
-    Prune64Args a;
-    std::memset(&a, 0, sizeof a);
-    a.plan = T.plan;
-    a.counts = S.d_counts.as<int32_t>();
-    a.perm = d_perm;
-    a.mats = ws.mats.as<const double*>();
-    a.ld_mat = msize;
-    a.prior = C->d_prior.as<double>();
-    a.n_prior = (int)C->prior.size();
-    a.err = R->use_error_model ? C->d_err.as<double>() : nullptr;
-    a.err_rows = C->err_rows;
-    a.err_ndev = C->err_ndev;
-    a.fam_R = d_famR;
-    a.scaled = scaled ? 1 : 0;
-    a.model = R->model == CAFE_MODEL_GAMMA ? 1 : 0;
-    a.out = out;
-    a.K = K;
-    a.cat_probs = ws.catp.as<double>();
-    a.tile_families = 1;
-    const bool prof = ws.sync;
-    cudaEvent_t ev;
-    if (prof) C->prof.begin(prof_kind, st, &ev);
-    for (size_t i = 0; i < n;) {
-        size_t j = i;
-        while (j < n && tiles[j].S == tiles[i].S) ++j;
-        Prune64Args b;
-        std::memcpy(&b, &a, sizeof b);   // padding included: the bytes are a graph signature
-        b.tiles = ws.tiles_cl.as<PruneTile>() + i;
-        b.n_tiles = (int)(j - i);
-        b.W = std::max(tiles[i].S + 1, tiles[i].R);
-        const int cl = fp64_cluster_size(b.W);
-        const int n_cl = (int)std::min<int64_t>((int64_t)(j - i), (int64_t)C->sm_count * 8);
-        CK(op_launch(ws, 8, [&] { return launch_prune64_cluster(b, cl, n_cl, st); }, b, cl, n_cl, st),
-           "prune fp64 (cluster)");
-        i = j;
-    }
-    if (prof) C->prof.end(prof_kind, st, ev);
-    return CAFE_OK;
-}
-
 // Algorithmic flops of one family of a tile (the roofline basis), by the
 // tile's (S, R) and error-model use.
 double family_flops(const TreeHost& T, int S, int R, bool err) {
@@ -962,6 +946,234 @@ double family_flops(const TreeHost& T, int S, int R, bool err) {
         per += (double)(nch - 1) * rows;
     }
     return per;
+}
+
+// ---- FP64 over distinct rows (k_pat64)
+
+// A group of families with a common state bound: vectors of S + 1 states,
+// root sizes 1..R.
+struct PatGroup {
+    int g;      // group of the plan
+    int S, R;
+};
+
+// Width class of a group: how many rows' vectors share a CTA's shared
+// memory. -1 when not even eight fit (the tile walk k_prune64 takes such
+// vectors from global memory).
+int pat64_lp(int S) { return (S + 1 + 31) / 32 * 32 + 2; }
+int pat64_class(const PatGroup& q) {
+    const int lp = pat64_lp(q.S);
+    if (!pat64_bufs(lp, q.R)) return -1;
+    return lp <= 66 ? 0 : lp <= 194 ? 1 : lp <= 514 ? 2 : 3;
+}
+
+// Prunes the plan's listed groups for every active combination (d_active:
+// their indices on the device) into out [F][K]. One launch per width class;
+// with `fork` the classes run side by side on the auxiliary streams.
+// Returns through d_status a word the kernel sets when a bounded wait gave
+// up; the caller zeroes it first.
+int launch_pat64_groups(cafe_ctx* C, Workspace& ws, const cafe_request* R, const TreeHost& T, const PatternPlan& P, const int64_t* d_perm, const int32_t* d_famR, const std::vector<PatGroup>& groups, int n_active,
+                        const int32_t* d_active, int K, int msize, bool scaled, double* out, int32_t* d_status, bool fork,
+                        int prof_kind) {
+    constexpr int NC = Workspace::kPatClasses;
+    const int ni = P.n_internal;
+    struct Class {
+        std::vector<PatGroup> groups;
+        std::vector<Pat64Node> nodes;
+        std::vector<int32_t> cdesc;
+        int s_run = 1, lp = 0, max_R = 0, units = 0, n_bufs = 1, group = 1, n_slots = 1, n_ctas = 1;
+        int64_t slot_doubles = 0, slot_rows = 0;
+        size_t o_nodes = 0, o_cdesc = 0, o_done = 0;
+    } cls[NC];
+    for (const PatGroup& q : groups) {
+        const int c = pat64_class(q);
+        if (c < 0) return fail(C, CAFE_ERR_INVALID, "vectors of %d states", q.S + 1);
+        if (P.group_count[q.g] > 0) cls[c].groups.push_back(q);
+    }
+    int levels = 1;
+    for (int h : T.height) levels = std::max(levels, h);
+    size_t blob = 0, ctr = NC * sizeof(unsigned long long);
+    for (int c = 0; c < NC; ++c) {
+        Class& X = cls[c];
+        if (X.groups.empty()) continue;
+        for (const PatGroup& q : X.groups) {
+            X.lp = std::max(X.lp, pat64_lp(q.S));
+            X.max_R = std::max(X.max_R, q.R);
+        }
+        X.n_bufs = pat64_bufs(X.lp, X.max_R);
+        // State tiles of a unit: about 20,000 to 40,000 products where a tree
+        // level has few units (1,000 families of 12 taxa at 171 states: 0.26 ms
+        // with one tile, 0.38 with four), four tiles where it keeps 24 units per
+        // SM anyway (10,000 families of 24 taxa, K = 4: 7.3 with one, 6.5 with
+        // four)
+        const int TP = kPat64Rows, TS = kPat64States;
+        int64_t units1 = 0;
+        for (const PatGroup& q : X.groups)
+            for (int ii = 0; ii + 1 < ni; ++ii) units1 += (P.row_count(q.g, ii) + TP - 1) / TP * ((q.S + TS) / TS);
+        X.s_run = std::max(1, std::min(4, 40000 / (TP * TS * (X.lp - 2))));
+        int64_t most = 0;
+        for (const PatGroup& q : X.groups) most = std::max(most, P.group_count[q.g]);
+        if (most <= 4) X.s_run = 4;      // (such units put eight times the work on a lane)
+        if (units1 * n_active >= (int64_t)24 * C->sm_count * levels) X.s_run = 4;
+        // nodes by height (children before parents, wide groups first); leaves
+        // come first, a row per count
+        std::stable_sort(X.groups.begin(), X.groups.end(), [](const PatGroup& a, const PatGroup& b) { return a.S > b.S; });
+        const int nn = T.n_nodes;
+        const int half = R->use_error_model ? (C->err_ndev - 1) / 2 : 0;
+        std::vector<int> at((size_t)X.groups.size() * nn, -1);
+        auto add = [&](size_t gi, int v, int64_t rows, int64_t cidx) {
+            const PatGroup& q = X.groups[gi];
+            Pat64Node nd;
+            std::memset(&nd, 0, sizeof nd);
+            nd.cidx = cidx;
+            nd.perm0 = P.group_first[q.g];
+            nd.rows = (int32_t)rows;
+            nd.node = v;
+            nd.nch = (int32_t)T.children[v].size();
+            nd.S = q.S;
+            nd.R = q.R;
+            nd.child0 = (int32_t)X.cdesc.size();
+            for (int c : T.children[v]) X.cdesc.push_back(at[gi * nn + c]);
+            nd.unit0 = X.units;
+            if (v == T.root) {
+                nd.n_units = (nd.rows + kPat64RootRows - 1) / kPat64RootRows;
+            } else {
+                // a child of the root gives factors for root sizes up to R
+                nd.s_cnt = T.parent[v] == T.root ? std::max(q.R, q.S) + 1 : q.S + 1;
+                nd.pitch = (nd.s_cnt + 1) & ~1;
+                nd.s_tiles = nd.nch ? ((nd.s_cnt + TS - 1) / TS + X.s_run - 1) / X.s_run : 1;
+                if (!nd.nch) {
+                    const size_t at_leaf = (size_t)q.g * T.n_leaves + T.leaf_col[v];
+                    nd.cidx = P.leaf_off[at_leaf];
+                    nd.n_list = (int32_t)(P.leaf_off[at_leaf + 1] - nd.cidx);
+                }
+                nd.n_units = ((nd.nch ? nd.rows : nd.n_list) + TP - 1) / TP * nd.s_tiles;
+                nd.tab = X.slot_doubles;
+                nd.erow0 = (int32_t)X.slot_rows;
+                X.slot_doubles += (int64_t)nd.rows * nd.pitch;
+                X.slot_rows += nd.nch ? nd.rows : 0;
+            }
+            X.units += nd.n_units;
+            at[gi * nn + v] = (int)X.nodes.size();
+            X.nodes.push_back(nd);
+        };
+        for (size_t gi = 0; gi < X.groups.size(); ++gi) {
+            // counts past the states (and the error model's reach) have a zero factor
+            const PatGroup& q = X.groups[gi];
+            const int64_t rows = std::min<int64_t>(P.group_max[q.g], (int64_t)q.S + half + 1) + 1;
+            for (int v = 0; v < nn; ++v)
+                if (T.leaf_col[v] >= 0) add(gi, v, rows, 0);
+        }
+        for (int h = 1; h <= levels; ++h)
+            for (size_t gi = 0; gi < X.groups.size(); ++gi)
+                for (int ii = 0; ii < ni; ++ii)
+                    if (T.height[ii] == h) {
+                        const int g = X.groups[gi].g;
+                        add(gi, T.internal[ii], P.row_count(g, ii), P.child_off[(size_t)g * ni + ii]);
+                    }
+        for (size_t gi = 0; gi < X.groups.size(); ++gi)
+            for (int v = 0; v < nn; ++v) X.nodes[at[gi * nn + v]].root = at[gi * nn + T.root];
+        // combinations interleaved until a level has about eight units per SM;
+        // tables for twice as many, within 2 GB
+        const int64_t want = ((int64_t)8 * C->sm_count * levels + X.units - 1) / std::max(1, X.units);
+        X.group = (int)std::max<int64_t>(1, std::min<int64_t>(n_active, want));
+        const int64_t fit = std::max<int64_t>(1, ((int64_t)2 << 30) / std::max<int64_t>(1, X.slot_doubles * 8));
+        X.group = (int)std::min<int64_t>(X.group, fit);
+        X.n_slots = (int)std::min<int64_t>(n_active, std::max<int64_t>(X.group, std::min<int64_t>(fit, 2 * X.group)));
+        X.n_ctas = (int)std::min<int64_t>((int64_t)X.units * n_active,
+                                          (int64_t)C->sm_count *
+                                              pat64_ctas_per_sm(X.n_bufs * pat64_buf_doubles(X.lp, X.max_R) * sizeof(double)));
+        CK(ws.pat_table[c].reserve((size_t)X.n_slots * X.slot_doubles * sizeof(double)), "factor tables");
+        CK(ws.pat_expo[c].reserve((size_t)X.n_slots * X.slot_rows * sizeof(int32_t)), "factor tables");
+        X.o_nodes = blob;
+        blob += X.nodes.size() * sizeof(Pat64Node);
+        X.o_cdesc = blob;
+        blob += (X.cdesc.size() * sizeof(int32_t) + 15) & ~(size_t)15;
+        X.o_done = ctr;
+        ctr += X.nodes.size() * n_active * sizeof(int32_t);
+    }
+    if (!blob) return CAFE_OK;
+    CK(ws.h_pat_desc.reserve(blob), "pattern nodes");
+    CK(ws.pat_desc.reserve(blob), "pattern nodes");
+    CK(ws.pat_ctr.reserve(ctr), "pattern counters");
+    char* h = ws.h_pat_desc.as<char>();
+    std::memset(h, 0, blob);
+    int n_cls = 0;
+    for (const Class& X : cls) {
+        if (X.groups.empty()) continue;
+        std::memcpy(h + X.o_nodes, X.nodes.data(), X.nodes.size() * sizeof(Pat64Node));
+        std::memcpy(h + X.o_cdesc, X.cdesc.data(), X.cdesc.size() * sizeof(int32_t));
+        ++n_cls;
+    }
+    CK(op_h2d(ws, ws.pat_desc.p, h, blob, ws.stream), "pattern nodes");
+    CK(op_memset(ws, ws.pat_ctr.p, 0, ctr, ws.stream), "pattern counters");
+    Pat64Args a;
+    std::memset(&a, 0, sizeof a);
+    a.plan = T.plan;
+    a.active = d_active;
+    a.n_active = n_active;
+    a.status = d_status;
+    a.child = P.d_child.as<int32_t>();
+    a.leaf_counts = P.d_counts.as<int32_t>();
+    a.perm = d_perm;
+    a.mats = ws.mats.as<const double*>();
+    a.ld_mat = msize;
+    a.prior = C->d_prior.as<double>();
+    a.n_prior = (int)C->prior.size();
+    a.err = R->use_error_model ? C->d_err.as<double>() : nullptr;
+    a.err_rows = C->err_rows;
+    a.err_ndev = C->err_ndev;
+    a.fam_R = d_famR;
+    a.scaled = scaled ? 1 : 0;
+    a.model = R->model == CAFE_MODEL_GAMMA ? 1 : 0;
+    a.out = out;
+    a.K = K;
+    a.cat_probs = ws.catp.as<double>();
+    const bool prof = ws.sync;
+    cudaEvent_t ev;
+    if (prof) {
+        C->prof.begin(prof_kind, ws.stream, &ev);
+        for (const PatGroup& q : groups)
+            C->prof.acc.prune_flops += (prof_kind == 1) * family_flops(T, q.S, q.R, R->use_error_model) *
+                                       (double)P.group_count[q.g] * n_active;
+    }
+    const bool forked = fork && n_cls > 1;
+    if (forked) {
+        CK(op_record(ws, ws.ev_fork, ws.stream), "fork");
+        for (int c = 0; c < NC; ++c) CK(op_wait(ws, ws.aux[c], ws.ev_fork), "fork");
+    }
+    for (int c = NC - 1; c >= 0; --c) {      // the widest vectors (the longest units) first
+        const Class& X = cls[c];
+        if (X.groups.empty()) continue;
+        Pat64Args b;
+        std::memcpy(&b, &a, sizeof b);       // padding included: the bytes are a graph signature
+        const char* d = ws.pat_desc.as<char>();
+        b.nodes = reinterpret_cast<const Pat64Node*>(d + X.o_nodes);
+        b.cdesc = reinterpret_cast<const int32_t*>(d + X.o_cdesc);
+        b.n_desc = (int)X.nodes.size();
+        b.units = X.units;
+        b.s_run = X.s_run;
+        b.n_bufs = X.n_bufs;
+        b.buf_doubles = pat64_buf_doubles(X.lp, X.max_R);
+        b.group = X.group;
+        b.n_slots = X.n_slots;
+        b.slot_doubles = X.slot_doubles;
+        b.slot_rows = X.slot_rows;
+        b.table = ws.pat_table[c].as<double>();
+        b.expo = ws.pat_expo[c].as<int32_t>();
+        b.next = ws.pat_ctr.as<unsigned long long>() + c;
+        b.done = reinterpret_cast<int32_t*>(ws.pat_ctr.as<char>() + X.o_done);
+        const cudaStream_t st = forked ? ws.aux[c] : ws.stream;
+        CK(op_launch(ws, 3, [&] { return launch_pat64(b, X.n_ctas, st); }, b, X.n_ctas, st),
+           "prune fp64");
+    }
+    if (forked)
+        for (int c = 0; c < NC; ++c) {
+            CK(op_record(ws, ws.ev_join[c], ws.aux[c]), "join");
+            CK(op_wait(ws, ws.stream, ws.ev_join[c]), "join");
+        }
+    if (prof) C->prof.end(prof_kind, ws.stream, ev);
+    return CAFE_OK;
 }
 
 double tiles_flops(const TreeHost& T, const std::vector<PruneTile>& tiles, bool err) {
@@ -1084,44 +1296,39 @@ int enqueue_mixed(cafe_ctx* C, Workspace& ws, const cafe_request* R, TreeHost& T
     uint8_t* d_term = ws.term_flags.as<uint8_t>();
     CK(op_memset(ws, ws.term_flags.p, 0, (size_t)std::max<int64_t>(F, 1) * K, ws.stream), "term flags");
 
-    // tiles: 128 families (tensor cores) or 32 families (FP64, wide bins)
+    // tiles: 128 families (tensor cores)
     // grouped by bin (bins ascend in width), so each bin's tiles are contiguous
-    std::vector<PruneTile> tc_tiles, wide_tiles;
-    std::vector<PruneTile>& cl_tiles = ws.cl_tile_vec;
-    cl_tiles.clear();
+    std::vector<PruneTile> tc_tiles;
+    std::vector<PatGroup> wide;      // bins past the tensor cores' width
     for (size_t b = 0; b < B.widths.size(); ++b) {
-        if (B.widths[b] > kTcMaxW && fp64_cluster_bin(C, T, B.bin_count[b], KC, B.widths[b])) {
-            add_cluster_tiles(cl_tiles, B, b, active);
+        const int w = B.widths[b];
+        if (w > kTcMaxW) {
+            wide.push_back(PatGroup{(int)b, w - 1, w - 1});
             continue;
         }
         for (int k : active) {
-            const int w = B.widths[b];
-            const int step = w <= kTcMaxW ? 128 : 32;
-            for (int64_t i = 0; i < B.bin_count[b]; i += step) {
+            for (int64_t i = 0; i < B.bin_count[b]; i += 128) {
                 PruneTile t{};
                 t.first = (int)(B.bin_first[b] + i);
-                t.count = (int)std::min<int64_t>(step, B.bin_count[b] - i);
+                t.count = (int)std::min<int64_t>(128, B.bin_count[b] - i);
                 t.k = k;
                 t.S = w - 1;
                 t.R = w - 1;
-                (w <= kTcMaxW ? tc_tiles : wide_tiles).push_back(t);
+                tc_tiles.push_back(t);
             }
         }
     }
     const bool prof = ws.sync;
     cudaEvent_t ev;
-    // FP64 bins (wider than the tensor-core tiles): 32-family tiles, or one
-    // family per cluster where a bin is sparse; beside the tensor-core bins
-    // when those fork onto the auxiliary streams (profiled calls: after them)
+    // FP64 bins (wider than the tensor-core tiles), beside the tensor-core
+    // bins when those fork onto the auxiliary streams (profiled calls: after
+    // them)
     bool wide_done = false;
     auto launch_wide = [&]() -> int {
         wide_done = true;
-        int rc = launch_fp64_tiles(C, ws, R, T, S, K, wide_tiles, ws.tiles64, ws.h_tiles64, B.d_perm.as<int64_t>(),
-                                   msize, msize, ws.cat.as<double>(), 3);
-        if (!rc)
-            rc = launch_fp64_cluster(C, ws, R, T, S, K, cl_tiles, B.d_perm.as<int64_t>(), B.d_famR.as<int32_t>(),
-                                     msize, true, ws.cat.as<double>(), ws.stream, 3);
-        return rc;
+        return launch_pat64_groups(C, ws, R, T, S.pat_bins, B.d_perm.as<int64_t>(), B.d_famR.as<int32_t>(), wide,
+                                   (int)active.size(), ws.catids.as<int32_t>(), K, msize, true, ws.cat.as<double>(), d_status,
+                                   false, 3);
     };
     if (!tc_tiles.empty()) {
         const size_t fl = (size_t)n_mat * Wm * Wm;
@@ -1461,7 +1668,7 @@ int enqueue_mixed(cafe_ctx* C, Workspace& ws, const cafe_request* R, TreeHost& T
         info->d_tail = d_status;     // [status, fallback families, fallback tiles]
     }
 
-    return finish_batch(C, ws, info, gamma, true, nullptr, tc_tiles.empty() ? nullptr : d_status, d_fam, d_total);
+    return finish_batch(C, ws, info, gamma, true, d_status, d_fam, d_total);
 }
 
 // The pruning phase of a mixed-precision request as a CUDA graph. A dry
@@ -1697,6 +1904,11 @@ int enqueue_score(cafe_ctx* C, Workspace& ws, const cafe_request* Rs, int NB, do
     for (int b : wait_chunks) CK(cudaStreamWaitEvent(ws.stream, C->batch_events[b], 0), "event");
     if (C->prof.on) C->prof.acc.host_keys_ms += host_ms_since(t_keys);
     CK(ws.cat.reserve((size_t)std::max<int64_t>(F, 1) * CT * sizeof(double)), "category buffer");
+    CK(ws.catids.reserve(active.size() * sizeof(int32_t)), "categories");
+    CK(ws.h_catids.reserve(active.size() * sizeof(int32_t)), "categories");
+    std::memcpy(ws.h_catids.p, active.data(), active.size() * sizeof(int32_t));
+    CK(cudaMemcpyAsync(ws.catids.p, ws.h_catids.p, active.size() * sizeof(int32_t), cudaMemcpyHostToDevice, ws.stream),
+       "categories");
     if (R->precision == CAFE_PREC_MIXED_TF32X3) {
         // polytomies stay on the FP64 path, and so do error models wider than
         // the +-kMaxErrHalf deviations the transposed leaf rows fold in;
@@ -1704,12 +1916,6 @@ int enqueue_score(cafe_ctx* C, Workspace& ws, const cafe_request* Rs, int NB, do
         // is exactly zero through one ends there)
         const bool to_fp64 = T.max_children > 2 || (R->use_error_model && C->err_ndev > 2 * kMaxErrHalf + 1);
         if (!to_fp64) {
-            CK(ws.catids.reserve(active.size() * sizeof(int32_t)), "categories");
-            CK(ws.h_catids.reserve(active.size() * sizeof(int32_t)), "categories");
-            std::memcpy(ws.h_catids.p, active.data(), active.size() * sizeof(int32_t));
-            CK(cudaMemcpyAsync(ws.catids.p, ws.h_catids.p, active.size() * sizeof(int32_t), cudaMemcpyHostToDevice,
-                               ws.stream),
-               "categories");
             const auto t_plan = std::chrono::steady_clock::now();
             const int rcm = enqueue_mixed_graph(C, ws, Rs, T, S, K, CT, active, hm, d_fam, d_total, info);
             if (C->prof.on) C->prof.acc.host_plan_ms += host_ms_since(t_plan);
@@ -1718,68 +1924,60 @@ int enqueue_score(cafe_ctx* C, Workspace& ws, const cafe_request* Rs, int NB, do
         info->n_fallback = F;
     }
 
-    // tiles
-    std::vector<PruneTile>& tiles = ws.tile_vec;
-    tiles.clear();
-    std::vector<PruneTile>& cl_tiles = ws.cl_tile_vec;
-    cl_tiles.clear();
-    const int TFm = 32;
-    const int64_t* d_perm;
-    const int32_t* d_famR = nullptr;
-    const bool dedupe = R->dedupe && !gamma && ref_mode;
+    // FP64: every family at the reference's global bounds, or by S-bin
+    std::vector<PatGroup> groups;
     if (ref_mode) {
-        const int64_t nf = dedupe ? (int64_t)S.unique.size() : F;
-        d_perm = dedupe ? S.d_unique.as<int64_t>() : S.d_identity.as<int64_t>();
-        // few families: one per cluster (the same bits as the tile walk)
-        const bool cl = fp64_cluster_bin(C, T, nf, K, W);
-        for (int c : active)
-            for (int64_t i = 0; i < nf; i += cl ? 1 : TFm) {
-                PruneTile t{};
-                t.first = (int)i;
-                t.count = cl ? 1 : (int)std::min<int64_t>(TFm, nf - i);
-                t.k = c;
-                t.S = Sg;
-                t.R = Rg;
-                (cl ? cl_tiles : tiles).push_back(t);
-            }
+        groups.push_back(PatGroup{0, Sg, Rg});
     } else {
-        d_perm = S.bins.d_perm.as<int64_t>();
-        d_famR = S.bins.d_famR.as<int32_t>();
         for (size_t b = 0; b < S.bins.widths.size(); ++b)
-            if (fp64_cluster_bin(C, T, S.bins.bin_count[b], K, S.bins.widths[b]))
-                add_cluster_tiles(cl_tiles, S.bins, b, active);
-        for (int c : active)
-            for (size_t b = 0; b < S.bins.widths.size(); ++b) {
-                if (fp64_cluster_bin(C, T, S.bins.bin_count[b], K, S.bins.widths[b])) continue;
-                for (int64_t i = 0; i < S.bins.bin_count[b]; i += TFm) {
-                    PruneTile t{};
-                    t.first = (int)(S.bins.bin_first[b] + i);
-                    t.count = (int)std::min<int64_t>(TFm, S.bins.bin_count[b] - i);
-                    t.k = c;
-                    t.S = S.bins.widths[b] - 1;
-                    t.R = S.bins.widths[b] - 1;
-                    tiles.push_back(t);
-                }
-            }
+            groups.push_back(PatGroup{(int)b, S.bins.widths[b] - 1, S.bins.widths[b] - 1});
     }
-    const int n_tiles = (int)tiles.size();
-    CK(ws.h_tiles.reserve(std::max(n_tiles, 1) * sizeof(PruneTile)), "tiles");
-    CK(ws.tiles.reserve(std::max(n_tiles, 1) * sizeof(PruneTile)), "tiles");
-    std::memcpy(ws.h_tiles.p, tiles.data(), n_tiles * sizeof(PruneTile));
-
-    const int n_ctas = std::max(1, std::min(n_tiles, C->n_ctas));
-    const int64_t per_cta = (int64_t)T.n_slots * W * TFm;
-    CK(ws.scratch.reserve((size_t)n_ctas * per_cta * sizeof(double)), "scratch");
-    info->footprint = (size_t)n_ctas * per_cta * sizeof(double) + (size_t)F * CT * sizeof(double);
-
-    CK(cudaMemcpyAsync(ws.tiles.p, ws.h_tiles.p, n_tiles * sizeof(PruneTile), cudaMemcpyHostToDevice, ws.stream),
-       "tiles");
+    const int64_t* d_perm = ref_mode ? S.d_identity.as<int64_t>() : S.bins.d_perm.as<int64_t>();
+    const int32_t* d_famR = ref_mode ? nullptr : S.bins.d_famR.as<int32_t>();
     CK(cudaMemcpyAsync(ws.mats.p, hm, (size_t)CT * T.n_nodes * sizeof(double*), cudaMemcpyHostToDevice, ws.stream),
        "mats");
     if (gamma && !scaled) CK(launch_fill(ws.cat.as<double>(), F * CT, 0.0, ws.stream), "fill");
     rc = stage_cat_probs(C, ws, Rs, K, NB);
     if (rc) return rc;
+    CK(ws.flags.reserve(64), "status");
+    int32_t* d_status = ws.flags.as<int32_t>();
+    CK(cudaMemsetAsync(d_status, 0, 64, ws.stream), "status");
+    bool fits = true;
+    for (const PatGroup& q : groups) fits &= pat64_class(q) >= 0;
+    if (fits) {
+        rc = launch_pat64_groups(C, ws, Rs, T, ref_mode ? S.pat_all : S.pat_bins, d_perm, d_famR, groups,
+                                 (int)active.size(), ws.catids.as<int32_t>(), CT, msize, scaled, ws.cat.as<double>(),
+                                 d_status, true, 1);
+        if (rc) return rc;
+        info->d_tail = d_status;
+        info->tail_counts = false;
+        return finish_batch(C, ws, info, gamma, scaled, d_status, d_fam, d_total);
+    }
 
+    // vectors too long for shared memory (global bounds in the thousands):
+    // 32-family tiles walked up the tree, vectors in global memory
+    std::vector<PruneTile>& tiles = ws.tile_vec;
+    tiles.clear();
+    const int TFm = 32;
+    for (int c : active)
+        for (int64_t i = 0; i < F; i += TFm) {
+            PruneTile t{};
+            t.first = (int)i;
+            t.count = (int)std::min<int64_t>(TFm, F - i);
+            t.k = c;
+            t.S = Sg;
+            t.R = Rg;
+            tiles.push_back(t);
+        }
+    const int n_tiles = (int)tiles.size();
+    CK(ws.h_tiles.reserve(std::max(n_tiles, 1) * sizeof(PruneTile)), "tiles");
+    CK(ws.tiles.reserve(std::max(n_tiles, 1) * sizeof(PruneTile)), "tiles");
+    std::memcpy(ws.h_tiles.p, tiles.data(), n_tiles * sizeof(PruneTile));
+    const int n_ctas = std::max(1, std::min(n_tiles, C->n_ctas));
+    const int64_t per_cta = (int64_t)T.n_slots * W * TFm;
+    CK(ws.scratch.reserve((size_t)n_ctas * per_cta * sizeof(double)), "scratch");
+    CK(cudaMemcpyAsync(ws.tiles.p, ws.h_tiles.p, n_tiles * sizeof(PruneTile), cudaMemcpyHostToDevice, ws.stream),
+       "tiles");
     Prune64Args a{};
     a.plan = T.plan;
     a.tiles = ws.tiles.as<PruneTile>();
@@ -1793,7 +1991,6 @@ int enqueue_score(cafe_ctx* C, Workspace& ws, const cafe_request* Rs, int NB, do
     a.err = R->use_error_model ? C->d_err.as<double>() : nullptr;
     a.err_rows = C->err_rows;
     a.err_ndev = C->err_ndev;
-    a.fam_R = d_famR;
     a.scratch = ws.scratch.as<double>();
     a.scratch_per_cta = per_cta;
     a.scaled = scaled ? 1 : 0;
@@ -1811,11 +2008,7 @@ int enqueue_score(cafe_ctx* C, Workspace& ws, const cafe_request* Rs, int NB, do
     }
     CK(launch_prune64(a, n_ctas, ws.stream), "prune");
     if (prof) C->prof.end(1, ws.stream, ev);
-    if (prof) C->prof.acc.prune_flops += tiles_flops(T, cl_tiles, R->use_error_model);
-    rc = launch_fp64_cluster(C, ws, R, T, S, CT, cl_tiles, d_perm, d_famR, msize, scaled, ws.cat.as<double>(),
-                             ws.stream, 1);
-    if (rc) return rc;
-    return finish_batch(C, ws, info, gamma, scaled, dedupe ? S.d_ref.as<int64_t>() : nullptr, nullptr, d_fam, d_total);
+    return finish_batch(C, ws, info, gamma, scaled, nullptr, d_fam, d_total);
 }
 
 bool small_request(const cafe_ctx* C, const cafe_request* R, int NB, int64_t F) {
@@ -1900,8 +2093,8 @@ int score_complete(cafe_ctx* C, Workspace& ws, const cafe_request* R, int NB, ca
     int64_t n_fb = info.n_fallback;
     if (info.d_tail) {
         const int32_t* tail = ws.h_tail.as<int32_t>();
-        if (tail[0]) return fail(C, CAFE_ERR_TIMEOUT, "tensor-core pruning gave up waiting (status %d)", tail[0]);
-        n_fb = tail[1];
+        if (tail[0]) return fail(C, CAFE_ERR_TIMEOUT, "pruning gave up waiting (status %d)", tail[0]);
+        if (info.tail_counts) n_fb = tail[1];
     }
     const bool gamma = R->model == CAFE_MODEL_GAMMA;
     for (int b = 0; b < NB; ++b) {
@@ -2762,7 +2955,7 @@ int cafe_ctx_create(const cafe_config* cfg, cafe_ctx** out) {
     cudaDeviceProp prop;
     cudaGetDeviceProperties(&prop, dev);
     C->sm_count = prop.multiProcessorCount;
-    if (tc_kernels_init() != cudaSuccess || prune64_cluster_init() != cudaSuccess || pvalue_kernels_init() != cudaSuccess ||
+    if (tc_kernels_init() != cudaSuccess || pat64_init() != cudaSuccess || pvalue_kernels_init() != cudaSuccess ||
         cudaEventCreateWithFlags(&C->gate, cudaEventDisableTiming) != cudaSuccess) {
         delete C;
         return CAFE_ERR_CUDA;

@@ -67,6 +67,99 @@ cudaError_t launch_matrix_build(const MatrixJob* d_jobs, int n_jobs, int max_siz
 // One-time per-device kernel attributes (shared-memory limits).
 cudaError_t tc_kernels_init();
 
+// ---- distinct count patterns per subtree (k_patterns.cu) ----
+constexpr int kMaxGroups = 16;
+struct PatBuildArgs {
+    TreePlan plan;
+    const int32_t* counts;       // [F][n_leaves]
+    const int64_t* perm;         // [F] family of each item (group order)
+    const int32_t* node_ii;      // [n_nodes] post-order index of an internal node, -1 for leaves
+    int64_t F;
+    int n_groups;
+    int64_t group_first[kMaxGroups];
+    int group_max[kMaxGroups];   // largest count of a group
+    int64_t flag_off[kMaxGroups];   // its first entry in the flags of launch_pat_counts
+    int32_t* rep;                // [n_internal][F] the item that represents an item's key at a node
+    int32_t* num;                // [n_internal][F] representatives before an item
+    int32_t* base;               // [n_internal][n_groups + 1] num at each group's first item; then the total
+};
+// nodes: post-order indices of one level; the table holds n_nodes x slots
+// (a power of two, at least 2 F) entries
+cudaError_t launch_pat_insert(const PatBuildArgs& a, const int32_t* d_nodes, int n_nodes, int32_t* table, int64_t slots,
+                              cudaStream_t s);
+// flags: [leaf][group_max + 1] per group, zeroed in; 1 where the count occurs
+cudaError_t launch_pat_counts(const PatBuildArgs& a, uint8_t* flags, cudaStream_t s);
+cudaError_t launch_pat_number(const PatBuildArgs& a, cudaStream_t s);
+// child_off [n_groups][n_internal]: first child index of a (group, node) in `child`
+cudaError_t launch_pat_write(const PatBuildArgs& a, const int64_t* d_child_off, int32_t* d_child, cudaStream_t s);
+
+// ---- FP64 pruning over distinct rows (k_pat64.cu) ----
+// One node of one group. An internal node's `rows` distinct vectors become
+// factor rows F[row][s] = sum_j M[s][j] L[row][j] (s < s_cnt) in the
+// combination's table; a leaf's rows are the factors of counts 0.. (the last
+// row stands for all larger counts; only counts that occur are filled in);
+// the root's rows are the group's families.
+struct Pat64Node {
+    int64_t tab;                 // first element of the node's factor rows in a combination's table
+    int64_t cidx;                // first of its rows' child indices; a leaf: of its counts in `leaf_counts`
+    int64_t perm0;               // root: first item of the group
+    int32_t unit0, n_units;      // its work units in a combination's list
+    int32_t rows;
+    int32_t n_list;              // a leaf's counts
+    int32_t node, nch;           // tree node, its children (0: a leaf)
+    int32_t S;                   // the group's states 0..S
+    int32_t s_cnt, pitch;        // factor entries per row, row pitch
+    int32_t s_tiles;             // state tiles of a row tile
+    int32_t erow0;               // first entry of its rows in the exponent table
+    int32_t child0;              // its children in cdesc
+    int32_t root;                // the group's root (index of its Pat64Node)
+    int32_t R;                   // root rows: root sizes 1..R
+};
+struct Pat64Args {
+    TreePlan plan;
+    const Pat64Node* nodes;      // [n_desc] by height, so children come first
+    const int32_t* cdesc;        // per node and child: the child's Pat64Node
+    int n_desc;
+    int units;                   // units of one combination
+    int s_run;                   // state tiles of a unit
+    int n_bufs;                  // vector buffers of a CTA
+    int64_t buf_doubles;
+    const int32_t* active;       // [n_active] combined (candidate, category) indices
+    int n_active;
+    int group;                   // combinations interleaved unit by unit
+    int n_slots;                 // combinations whose tables exist at a time
+    int64_t slot_doubles, slot_rows;
+    double* table;               // [n_slots][slot_doubles]
+    int32_t* expo;               // [n_slots][slot_rows] power-of-two exponents of the rows
+    int32_t* done;               // [n_active][n_desc] finished units, zeroed
+    unsigned long long* next;    // unit counter, zeroed
+    int32_t* status;             // nonzero when a bounded wait gave up
+    const int32_t* child;        // child indices (launch_pat_write)
+    const int32_t* leaf_counts;  // the counts that occur at a leaf
+    const int64_t* perm;
+    const double* const* mats;   // [K][n_nodes]
+    int ld_mat;
+    const double* prior;
+    int n_prior;
+    const double* err;
+    int err_rows, err_ndev;
+    const int32_t* fam_R;
+    int scaled, model;
+    double* out;                 // [F][K]
+    int K;
+    const double* cat_probs;
+};
+constexpr int kPat64RootRows = 8;   // families of a root unit
+constexpr int kPat64Rows = 8;       // rows of any other
+constexpr int kPat64States = 16;    // states of a state tile
+// lp: pitch of the longest vectors in shared memory (whole 32-state chunks,
+// plus 2)
+int pat64_bufs(int lp, int max_R);
+int64_t pat64_buf_doubles(int lp, int max_R);
+cudaError_t pat64_init();
+cudaError_t launch_pat64(const Pat64Args& a, int n_ctas, cudaStream_t s);
+int pat64_ctas_per_sm(size_t smem);
+
 struct Prune64Args {
     TreePlan plan;
     const PruneTile* tiles;
@@ -99,14 +192,6 @@ struct Prune64Args {
 
 cudaError_t launch_prune64(const Prune64Args& a, int n_ctas, cudaStream_t s);
 
-// The same walk with one family per tile (count 1) and a thread-block
-// cluster of `cl` CTAs per family (rows split across the cluster); W is the
-// vector length of the launch's bin. `n_clusters` clusters loop over the tiles.
-size_t prune64_cluster_smem(int n_slots, int W);
-size_t prune64_cluster_max_smem();
-cudaError_t prune64_cluster_init();
-cudaError_t launch_prune64_cluster(const Prune64Args& a, int cl, int n_clusters, cudaStream_t s);
-
 struct FinishArgs {
     int64_t F;
     int K;                       // categories per candidate (1 for the base model)
@@ -114,7 +199,6 @@ struct FinishArgs {
     int model;
     int scaled;
     const double* cat;           // [F][n_cand][K]: gamma terms (linear if !scaled, log if scaled); base: lnl
-    const int64_t* ref;          // dedupe reference per family, or null
     double* family_lnl;          // [n_cand][F] out, or null
     double* total;               // [n_cand] out, or null
     int32_t* n_failed;           // [n_cand] out

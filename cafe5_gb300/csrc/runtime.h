@@ -53,6 +53,8 @@ struct TreeHost {
     std::vector<std::vector<int>> children;
     // plan (internal nodes in post-order) and its device copy
     std::vector<int32_t> internal, cstart, child, slot;
+    std::vector<int32_t> internal_index;      // post-order index of a node, -1 for leaves
+    std::vector<int32_t> height;              // per post-order index: internal nodes on the longest way to a leaf
     int n_slots = 0, max_children = 0;
     DevBuf d_plan;
     TreePlan plan{};
@@ -68,6 +70,19 @@ struct BinPlan {
     int W_max = 0;
 };
 
+// Distinct count patterns below every internal node, per group of families
+// (k_patterns.cu): the rows the pruning kernels contract.
+struct PatternPlan {
+    int n_groups = 0, n_internal = 0;
+    std::vector<int64_t> group_first, group_count;   // items (families in group order)
+    std::vector<int> group_max;       // largest count
+    std::vector<int64_t> rows;        // [group][internal]: distinct patterns; the root: the group's families
+    std::vector<int64_t> child_off;   // [group][internal]: first child index in d_child
+    std::vector<int64_t> leaf_off;    // [group][leaf]: first of the counts that occur there, in d_counts; then the end
+    DevBuf d_child, d_counts;
+    int64_t row_count(int g, int ii) const { return rows[(size_t)g * n_internal + ii]; }
+};
+
 struct FamSet {
     int tree_id = 0;
     int64_t F = 0;
@@ -75,10 +90,9 @@ struct FamSet {
     DevBuf d_counts;
     std::vector<int32_t> h_counts;
     std::vector<int32_t> max_count;
-    // dedupe: unique families and reference per family
-    std::vector<int64_t> unique;
-    DevBuf d_unique, d_ref, d_identity;
+    DevBuf d_identity;                // 0..F-1
     BinPlan bins;
+    PatternPlan pat_bins, pat_all;    // grouped by S-bin (bins.d_perm order), and all families together
 };
 
 struct MatKey {
@@ -164,13 +178,14 @@ struct Workspace {
     DevBuf scratch, tiles, mats, cat, fam_lnl, total, nfail, jobs, catp;
     PinnedBuf h_tiles, h_mats, h_jobs, h_out, h_catp;
     // tensor-core path
-    DevBuf term_flags, fb_bins, tile_ctr, tc_hi, tc_tr, tc_mi, tc_vec, conv, flags, fb_perm, tiles64, tiles_fb, parts, fb_count, phase,
+    DevBuf term_flags, fb_bins, tile_ctr, tc_hi, tc_tr, tc_mi, tc_vec, conv, flags, fb_perm, tiles_fb, parts, fb_count, phase,
         catids, cerr;
-    PinnedBuf h_conv, h_mi, h_flags, h_tiles64, h_tiles_fb, h_tail, h_catids;
-    // FP64 bins walked one family per cluster
-    DevBuf tiles_cl;
-    PinnedBuf h_tiles_cl;
-    std::vector<PruneTile> cl_tile_vec;
+    PinnedBuf h_conv, h_mi, h_flags, h_tiles_fb, h_tail, h_catids;
+    // FP64 over distinct rows (k_pat64): per width class, factor tables and
+    // exponents; node descriptors, active combinations, counters
+    static constexpr int kPatClasses = 4;
+    DevBuf pat_table[kPatClasses], pat_expo[kPatClasses], pat_desc, pat_ctr;
+    PinnedBuf h_pat_desc;
     // reconstruction
     DevBuf rc_c, rc_state, rc_rmax, rc_mean, rc_count, rc_nfail, rc_parent, rc_bp, rc_lm, rc_lptr;
     PinnedBuf h_sim, h_simperm;        // p-values: simulated families staged for the device

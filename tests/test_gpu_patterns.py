@@ -1,0 +1,95 @@
+"""FP64 scores over distinct subtree patterns (k_patterns, k_pat64): row,
+state and chunk counts at the edges of a unit (8 rows, 16-state tiles,
+32-column chunks), repeated and distinct rows, polytomies, a unary node, an
+error model, and batches. Against the FP64 oracle; tolerance 1e-12 relative
+per family (the oracle's own sums round differently, by a few 1e-16 per node
+and at most a few dozen nodes)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+BINARY = "((A:3.2,B:3.2):4.5,((C:2.5,D:2.5):1.25,E:3.75):3.95);"
+POLY = "((A:3.2,B:3.2,C:3.2):4.5,(D:2.5,(E:1.5):1.0,F:2.5):5.2,G:7.7);"
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    from cafe5_gb300.engine import Context
+    c = Context()
+    yield c
+    c.close()
+
+
+def _oracle():
+    import os
+    import sys
+    sys.path.insert(0, os.path.join(os.path.dirname(__file__), "..", "oracle"))
+    import oracle
+    return oracle
+
+
+def _counts(rng, F, n_leaves, hi, distinct):
+    """`distinct` different rows among F."""
+    base = rng.integers(0, hi + 1, (max(distinct, 1), n_leaves))
+    base[:, 0] = np.maximum(base[:, 0], 1)
+    return np.ascontiguousarray(base[rng.integers(0, len(base), F)], dtype=np.int32)
+
+
+@pytest.mark.parametrize("newick", [BINARY, POLY], ids=["binary", "polytomy"])
+@pytest.mark.parametrize("F,distinct,hi,S,R", [
+    (1, 1, 3, 15, 10),        # one row, one tile
+    (7, 7, 5, 16, 16),        # a tile and one state over
+    (8, 3, 5, 30, 31),        # root sizes past the states
+    (9, 9, 9, 31, 20),        # one row over; a whole chunk
+    (65, 40, 12, 32, 40),     # a chunk and one column over
+    (300, 40, 20, 130, 100),  # chunks that leave every partial sum unchanged
+    (40, 40, 120, 170, 150),  # large counts at the reference's bounds
+])
+@pytest.mark.parametrize("eps", [0.0, 0.07])
+def test_fp64_ref_rows(ctx, newick, F, distinct, hi, S, R, eps):
+    oracle = _oracle()
+    from cafe5_gb300.inputs import ErrorModel, RootPrior
+    from cafe5_gb300.tree import parse_newick
+    tree = parse_newick(newick)
+    rng = np.random.default_rng([F, distinct, S])
+    c = _counts(rng, F, len(tree.leaves), min(hi, S), distinct)
+    prior = RootPrior.uniform(R).vector()
+    em = ErrorModel.symmetric(eps, int(c.max())) if eps else None
+    tid = ctx.upload_tree(tree)
+    sid = ctx.upload_families(tid, c)
+    ctx.set_prior(prior)
+    ctx.set_error_model(em.table() if em else None)
+    ta = oracle.TreeArrays.from_tree(tree)
+    lams = [0.004, 0.013]
+    got = ctx.score_batch(tid, sid, [dict(lambdas=[l]) for l in lams], S=S, R=R, use_error_model=em is not None)
+    for l, r in zip(lams, got):
+        _, fam, _ = oracle.score(ta, c, [l], prior=prior, S=S, R=R, err_rows=em.table() if em else None)
+        ok = np.isfinite(fam)
+        assert np.array_equal(ok, np.isfinite(r.family_lnl))
+        assert np.all(np.abs(r.family_lnl[ok] - fam[ok]) <= 1e-12 * np.maximum(1.0, np.abs(fam[ok])))
+        # the same bits alone, and for equal families
+        assert np.array_equal(r.family_lnl, ctx.score(tid, sid, [l], S=S, R=R, use_error_model=em is not None).family_lnl)
+    _, inv = np.unique(c, axis=0, return_inverse=True)
+    for g in range(inv.max() + 1):
+        assert len(set(got[0].family_lnl[inv.reshape(-1) == g])) == 1
+    ctx.free_families(sid)
+    ctx.set_error_model(None)
+
+
+def test_fp64_binned_tables_are_reused_across_combinations(ctx):
+    """More (candidate, category) combinations than factor tables: every table
+    is taken over by later ones; each candidate keeps the bits it has alone."""
+    from cafe5_gb300.inputs import RootPrior
+    from cafe5_gb300.synth import workload
+    w = workload(1, n_families=6000, seed=9)
+    tid = ctx.upload_tree(w.tree)
+    sid = ctx.upload_families(tid, w.families.counts)
+    ctx.set_prior(RootPrior.uniform(150).vector())
+    cands = [dict(lambdas=[0.002 * (1 + 0.01 * b)], multipliers=w.multipliers, cat_probs=w.cat_probs) for b in range(24)]
+    got = ctx.score_batch(tid, sid, cands, model=1, precision="fp64_binned")
+    for b in (0, 11, 23):
+        alone = ctx.score(tid, sid, cands[b]["lambdas"], model=1, precision="fp64_binned", multipliers=w.multipliers,
+                          cat_probs=w.cat_probs)
+        assert np.array_equal(alone.family_lnl, got[b].family_lnl) and alone.total == got[b].total
+    ctx.free_families(sid)
