@@ -1191,60 +1191,24 @@ double tiles_flops(const TreeHost& T, const std::vector<PruneTile>& tiles, bool 
     return fl;
 }
 
-// Launch shape of the tensor-core kernel for bin width W: TMEM columns per
-// CTA, CTAs per SM and pipeline stages. By default the most CTAs per SM that
-// TMEM and shared memory allow, then the deepest pipeline that keeps them;
-// cafe_autotune may have measured a better pair for this width.
-struct TcShape {
-    int tmem_cols = 0, per_sm = 0, stages = 0;
-    size_t smem = 0;
-};
-
-int tc_by_smem(const TreeHost& T, int W, int stages, size_t* smem, int nsplit = 1) {
-    *smem = prune_tc_smem_bytes(W, T.n_slots, stages, (int)T.internal.size());
-    if (*smem > (size_t)prune_tc_max_smem(nsplit)) return 0;
-    return (int)((227 * 1024) / (*smem + 1024));
-}
-
-TcShape tc_shape(cafe_ctx* C, const TreeHost& T, int W) {
-    TcShape sh;
-    sh.tmem_cols = 32;
-    while (sh.tmem_cols < 2 * W) sh.tmem_cols *= 2;
-    const int by_tmem = 512 / sh.tmem_cols;
-    auto it = C->tuned.find(W);
-    if (it != C->tuned.end()) {
-        size_t sm;
-        const int per = it->second.first, st = it->second.second;
-        if (per >= 1 && per <= by_tmem && st >= 1 && st <= 4 && tc_by_smem(T, W, st, &sm) >= per) {
-            sh.per_sm = per;
-            sh.stages = st;
-            sh.smem = sm;
-            return sh;
-        }
-    }
-    for (int st = 4; st >= 1; --st) {
-        size_t sm;
-        const int per = std::min(by_tmem, tc_by_smem(T, W, st, &sm));
-        if (per > sh.per_sm) {
-            sh.per_sm = per;
-            sh.stages = st;
-            sh.smem = sm;
-        }
-    }
-    return sh;
+// CTAs per SM of the tensor-core kernel for bin width W: as many as fit, or
+// what cafe_autotune measured to be faster.
+int tc_per_sm(const cafe_ctx* C, int W) {
+    const int most = pat_tc_ctas_per_sm(W);
+    const auto it = C->tuned.find(W);
+    return it == C->tuned.end() ? most : std::max(1, std::min(most, it->second));
 }
 
 // Share of the 1e-6 per-family budget (|dlnL| / |lnL|) left to FP32 range
 // loss; TF32x3 rounding takes the rest.
 constexpr double kRangeTau = 1e-7;
 
-// Widest bin on the tensor cores: one CTA per tile up to 256 states (both
-// children's factors in 2 W <= 512 TMEM columns), a pair of CTAs (half the
-// states each) for 384 and 512.
+// Widest bin on the tensor cores (the root weighting keeps the prior of its
+// states in shared memory).
 constexpr int kTcMaxW = 512;
 
-// MIXED_TF32X3: tensor-core tiles for bins <= 512 states, FP64 tiles for
-// wider bins and for families the tensor-core pass flags. Caller holds C->mu;
+// MIXED_TF32X3: the tensor cores for bins <= 512 states, FP64 for wider bins
+// and for families the tensor-core pass flags. Caller holds C->mu;
 // hm holds the FP64 matrix of every (category, node).
 int enqueue_mixed(cafe_ctx* C, Workspace& ws, const cafe_request* R, TreeHost& T, FamSet& S, int K, int CT,
                   const std::vector<int32_t>& active, double** hm, double* d_fam, double* d_total, ScoreInfo* info) {
@@ -1296,27 +1260,11 @@ int enqueue_mixed(cafe_ctx* C, Workspace& ws, const cafe_request* R, TreeHost& T
     uint8_t* d_term = ws.term_flags.as<uint8_t>();
     CK(op_memset(ws, ws.term_flags.p, 0, (size_t)std::max<int64_t>(F, 1) * K, ws.stream), "term flags");
 
-    // tiles: 128 families (tensor cores)
-    // grouped by bin (bins ascend in width), so each bin's tiles are contiguous
-    std::vector<PruneTile> tc_tiles;
+    std::vector<int> tc_bins;
     std::vector<PatGroup> wide;      // bins past the tensor cores' width
     for (size_t b = 0; b < B.widths.size(); ++b) {
-        const int w = B.widths[b];
-        if (w > kTcMaxW) {
-            wide.push_back(PatGroup{(int)b, w - 1, w - 1});
-            continue;
-        }
-        for (int k : active) {
-            for (int64_t i = 0; i < B.bin_count[b]; i += 128) {
-                PruneTile t{};
-                t.first = (int)(B.bin_first[b] + i);
-                t.count = (int)std::min<int64_t>(128, B.bin_count[b] - i);
-                t.k = k;
-                t.S = w - 1;
-                t.R = w - 1;
-                tc_tiles.push_back(t);
-            }
-        }
+        if (B.widths[b] > kTcMaxW) wide.push_back(PatGroup{(int)b, B.widths[b] - 1, B.widths[b] - 1});
+        else if (B.bin_count[b] > 0) tc_bins.push_back((int)b);
     }
     const bool prof = ws.sync;
     cudaEvent_t ev;
@@ -1330,7 +1278,7 @@ int enqueue_mixed(cafe_ctx* C, Workspace& ws, const cafe_request* R, TreeHost& T
                                    (int)active.size(), ws.catids.as<int32_t>(), K, msize, true, ws.cat.as<double>(), d_status,
                                    false, 3);
     };
-    if (!tc_tiles.empty()) {
+    if (!tc_bins.empty()) {
         const size_t fl = (size_t)n_mat * Wm * Wm;
         CK(ws.tc_hi.reserve(2 * fl * sizeof(float)), "tc matrices");     // hi, then lo
         CK(ws.tc_tr.reserve(fl * sizeof(float)), "tc matrices");
@@ -1359,109 +1307,129 @@ int enqueue_mixed(cafe_ctx* C, Workspace& ws, const cafe_request* R, TreeHost& T
            "convert");
         if (prof) C->prof.end(3, ws.stream, ev);
 
-        // one launch per S-bin, each sized for its own width, run
-        // concurrently: TMEM (512 columns per SM) and shared memory set how
-        // many tiles of a bin share an SM
+        // range-error bounds of the category terms: zero for every term the
+        // tensor cores do not write (FP64 bins, candidates not pruned)
+        CK(ws.cerr.reserve((size_t)std::max<int64_t>(F, 1) * K * sizeof(float)), "range bounds");
+        CK(op_memset(ws, ws.cerr.p, 0, (size_t)std::max<int64_t>(F, 1) * K * sizeof(float), ws.stream), "range bounds");
+
+        // one persistent launch per S-bin, run concurrently
+        const PatternPlan& P = S.pat_bins;
+        const int ni = P.n_internal, n_act = (int)active.size();
+        int levels = 1;
+        for (int h : T.height) levels = std::max(levels, h);
         struct BinLaunch {
-            int W, tmem_cols, stages, per_sm, n_ctas, nsplit;
-            size_t smem;
-            int64_t first_tile, n_tiles, vrow_base;
+            int b, n_ctas;
+            std::vector<PatTcNode> nodes;
+            std::vector<PatTcSeg> segs;
+            long long units = 0;
+            int64_t slot_rows = 0;
+            int n_slots = 1;
+            size_t o_nodes, o_segs, o_done;
         };
-        // Bins of 128 states or more split each tile over a cluster of
-        // nsplit CTAs (4 or 2; W / nsplit a multiple of 32 and at least 64)
-        // when the bin is sparse enough that every tile still gets SMs of
-        // its own: a lone tile's walk is bound by what one SM can stream.
-        // Bins over 256 states always split (both children's factors, 2 W
-        // columns, would not fit one CTA's TMEM).
-        auto pick_split = [&](int W, int64_t n_tiles) {
-            for (int ns : {4, 2}) {
-                const int wn = W / ns;
-                if (W % ns || wn % 32 || wn < 64 || wn > 256) continue;
-                if (n_tiles * ns <= (int64_t)C->sm_count) return ns;
+        std::vector<BinLaunch> launches(tc_bins.size());
+        size_t blob = 0, ctr = launches.size() * sizeof(unsigned long long);
+        for (size_t q = 0; q < launches.size(); ++q) {
+            BinLaunch& L = launches[q];
+            L.b = tc_bins[q];
+            const int W = B.widths[L.b], Ns = pat_tc_states(W), n_share = W / Ns;
+            std::vector<int> at(T.n_nodes, -1), lvl0(levels + 1, 0);
+            std::vector<int64_t> lvl_units(levels, 0);
+            int64_t units = 0;
+            for (int h = 1; h <= levels; ++h) {
+                lvl0[h - 1] = (int)L.nodes.size();
+                for (int ii = 0; ii < ni; ++ii) {
+                    if (T.height[ii] != h) continue;
+                    const int v = T.internal[ii];
+                    PatTcNode nd;
+                    std::memset(&nd, 0, sizeof nd);
+                    nd.cidx = P.child_off[(size_t)L.b * ni + ii];
+                    nd.perm0 = P.group_first[L.b];
+                    nd.rows = (int32_t)P.row_count(L.b, ii);
+                    nd.node = v;
+                    nd.nch = (int32_t)T.children[v].size();
+                    for (int c = 0; c < nd.nch; ++c) {
+                        nd.child_node[c] = T.children[v][c];
+                        nd.child[c] = at[nd.child_node[c]];
+                    }
+                    const int tiles = (nd.rows + 127) / 128;
+                    nd.unit0 = (int32_t)lvl_units[h - 1];
+                    nd.n_units = v == T.root ? tiles : tiles * n_share;
+                    nd.row0 = (int32_t)L.slot_rows;
+                    if (v != T.root) L.slot_rows += (nd.rows + 31) / 32 * 32;
+                    lvl_units[h - 1] += nd.n_units;
+                    at[v] = (int)L.nodes.size();
+                    L.nodes.push_back(nd);
+                }
+                units += lvl_units[h - 1];
             }
-            return W > 256 ? 2 : 1;
-        };
-        std::vector<BinLaunch> launches;
-        int64_t vrows = 0;
-        for (size_t i = 0; i < tc_tiles.size();) {
-            size_t j = i;
-            while (j < tc_tiles.size() && tc_tiles[j].S == tc_tiles[i].S) ++j;
-            BinLaunch L{};
-            L.W = tc_tiles[i].S + 1;
-            L.first_tile = (int64_t)i;
-            L.n_tiles = (int64_t)(j - i);
-            L.nsplit = pick_split(L.W, L.n_tiles);
-            if (L.nsplit > 1) {
-                // the deepest pipeline of W / nsplit B rows that fits
-                const int wn = L.W / L.nsplit;
-                L.tmem_cols = 32;
-                while (L.tmem_cols < 2 * wn) L.tmem_cols *= 2;
-                L.per_sm = 1;
-                for (int st = 4; st >= 1 && !L.stages; --st)
-                    if (tc_by_smem(T, wn, st, &L.smem, L.nsplit) >= 1) L.stages = st;
-                if (!L.stages) return fail(C, CAFE_ERR_INVALID, "tensor-core tile does not fit shared memory");
-                // over half an SM's shared memory: two cluster CTAs (of this or
-                // another cluster launch) never share an SM, so no CTA holding
-                // TMEM waits on a peer that waits for that SM's TMEM
-                L.smem = std::min(std::max(L.smem, (size_t)120 * 1024), (size_t)prune_tc_max_smem(L.nsplit));
-                const int64_t clusters =
-                    std::max<int64_t>(1, std::min<int64_t>(L.n_tiles, (int64_t)C->sm_count / L.nsplit));
-                L.n_ctas = (int)(L.nsplit * clusters);
-                L.vrow_base = vrows;
-                vrows += clusters * T.n_slots * 128;
-                launches.push_back(L);
-                i = j;
-                continue;
+            lvl0[levels] = (int)L.nodes.size();
+            // Segments: blocks of `g` combinations, a block starting its first
+            // level a step after the block before. A step then holds a unit list's
+            // worth of independent units per combination, and a unit's inputs are
+            // at least a step behind it: two steps' worth of resident CTAs is
+            // enough to find them finished. Few units in all: every combination in
+            // one block (levels in step, as wide as they get).
+            const int64_t ctas = (int64_t)C->sm_count * tc_per_sm(C, W);
+            int64_t g = n_act;
+            if (units * n_act > 2 * levels * ctas) g = std::min<int64_t>(n_act, (2 * ctas + units - 1) / units);
+            // (tables within 4 GB)
+            const int64_t fit = std::max<int64_t>(1, ((int64_t)4 << 30) / std::max<int64_t>(1, L.slot_rows * W * 4));
+            if (g < n_act) g = std::max<int64_t>(1, std::min(g, fit / (levels + 1)));
+            else if (g > fit) g = std::max<int64_t>(1, fit / (levels + 1));
+            L.n_slots = (int)std::min<int64_t>(n_act, (levels + 1) * g);
+            const int64_t blocks = (n_act + g - 1) / g;
+            int64_t widest = 1;
+            for (int64_t t = 0; t < blocks + levels - 1; ++t) {
+                int64_t step = 0;
+                for (int l = levels - 1; l >= 0; --l) {
+                    const int64_t blk = t - l;
+                    if (blk < 0 || blk >= blocks || !lvl_units[l]) continue;
+                    PatTcSeg sg;
+                    std::memset(&sg, 0, sizeof sg);
+                    sg.unit0 = L.units;
+                    sg.q0 = (int32_t)(blk * g);
+                    sg.nq = (int32_t)std::min<int64_t>(g, n_act - blk * g);
+                    sg.node0 = lvl0[l];
+                    sg.node1 = lvl0[l + 1];
+                    L.units += lvl_units[l] * sg.nq;
+                    step += lvl_units[l] * sg.nq;
+                    L.segs.push_back(sg);
+                }
+                widest = std::max(widest, step);
             }
-            L.nsplit = 1;
-            const TcShape shape = tc_shape(C, T, L.W);
-            if (shape.per_sm < 1) return fail(C, CAFE_ERR_INVALID, "tensor-core tile does not fit shared memory");
-            L.tmem_cols = shape.tmem_cols;
-            L.stages = shape.stages;
-            L.smem = shape.smem;
-            L.per_sm = shape.per_sm;
-            // pad shared memory so no more CTAs of this launch than TMEM allows share an SM
-            L.smem = std::max(L.smem, (size_t)((227 * 1024) / L.per_sm) - 2048);
-            L.smem = std::min(L.smem, (size_t)prune_tc_max_smem());
-            L.n_ctas = (int)std::max<int64_t>(1, std::min<int64_t>(L.n_tiles, (int64_t)C->sm_count * L.per_sm));
-            L.vrow_base = vrows;
-            vrows += (int64_t)L.n_ctas * T.n_slots * 128;
-            launches.push_back(L);
-            i = j;
+            L.n_ctas = (int)std::min<int64_t>(ctas, widest);
+            if (L.slot_rows * L.n_slots >= ((int64_t)1 << 31)) return fail(C, CAFE_ERR_INVALID, "too many factor rows");
+            const int64_t rows = std::max<int64_t>(128, L.slot_rows * L.n_slots);
+            CK(ws.tcp_table[L.b].reserve((size_t)rows * W * sizeof(float)), "factor tables");
+            CK(ws.tcp_meta[L.b].reserve((size_t)rows * sizeof(int4)), "factor tables");
+            L.o_nodes = blob;
+            blob += L.nodes.size() * sizeof(PatTcNode);
+            L.o_segs = blob;
+            blob += L.segs.size() * sizeof(PatTcSeg);
+            L.o_done = ctr;
+            ctr += L.nodes.size() * n_act * sizeof(int32_t);
         }
-        CK(ws.tc_vec.reserve((size_t)vrows * Wm * sizeof(float)), "tc vectors");
-        // node vectors move in boxes of one tile's 128 rows; each launch's
-        // matrix maps have boxes of its Ws rows (one TMA instruction per
-        // operand and chunk)
-        TcMaps maps;
-        const int kbox = prune_tc_kchunk();
-        int rc = cached_map(C, ws, 2, &maps.vec, ws.tc_vec.as<float>(), vrows, Wm, kbox, 128);
-        if (!rc) rc = cached_map(C, ws, 3, &maps.vst, ws.tc_vec.as<float>(), vrows, Wm, 32, 128);
-        if (rc) return rc;
-        auto launch_maps = [&](int Ws, TcMaps* m) {
-            *m = maps;
-            const int q = 4 + (Ws / 32 - 1);      // Ws: a multiple of 32 up to 256
-            const int64_t fl = (int64_t)n_mat * Wm * Wm;
-            int r = cached_map(C, ws, q, &m->mat, ws.tc_hi.as<float>(), (int64_t)n_mat * Wm, Wm, kbox, Ws, fl);
-            // leaf blocks: W x W (read only where W <= 64, one CTA per tile)
-            if (!r) r = cached_map(C, ws, 12 + (Ws / 32 - 1), &m->tr, ws.tc_tr.as<float>(), (int64_t)n_mat * Wm, Wm, 32, Ws);
-            return r;
-        };
-        const int n_tc = (int)tc_tiles.size();
-        CK(ws.tiles.reserve(n_tc * sizeof(PruneTile)), "tiles");
-        CK(ws.h_tiles.reserve(n_tc * sizeof(PruneTile)), "tiles");
-        std::memcpy(ws.h_tiles.p, tc_tiles.data(), n_tc * sizeof(PruneTile));
-        CK(op_h2d(ws, ws.tiles.p, ws.h_tiles.p, n_tc * sizeof(PruneTile), ws.stream), "tiles");
-        PruneTcArgs a;
+        CK(ws.h_tcp_desc.reserve(blob), "pattern nodes");
+        CK(ws.tcp_desc.reserve(blob), "pattern nodes");
+        CK(ws.tcp_ctr.reserve(ctr), "pattern counters");
+        char* hd = ws.h_tcp_desc.as<char>();
+        for (const BinLaunch& L : launches) {
+            std::memcpy(hd + L.o_nodes, L.nodes.data(), L.nodes.size() * sizeof(PatTcNode));
+            std::memcpy(hd + L.o_segs, L.segs.data(), L.segs.size() * sizeof(PatTcSeg));
+        }
+        CK(op_h2d(ws, ws.tcp_desc.p, hd, blob, ws.stream), "pattern nodes");
+        CK(op_memset(ws, ws.tcp_ctr.p, 0, ctr, ws.stream), "pattern counters");
+        PatTcArgs a;
         std::memset(&a, 0, sizeof a);
-        a.plan = T.plan;
-        a.counts = S.d_counts.as<int32_t>();
+        a.active = ws.catids.as<int32_t>();
+        a.status = d_status;
+        a.any_flag = d_status + 3;
+        a.child = P.d_child.as<int32_t>();
         a.perm = B.d_perm.as<int64_t>();
         a.mat_index = ws.tc_mi.as<int32_t>();
+        a.n_nodes = T.n_nodes;
         a.Wm = Wm;
         a.mat_tr = ws.tc_tr.as<float>();
-        a.vec = ws.tc_vec.as<float>();
-        a.n_slots = T.n_slots;
         a.prior = C->d_prior.as<double>();
         a.n_prior = (int)C->prior.size();
         a.err = R->use_error_model ? C->d_err.as<double>() : nullptr;
@@ -1469,59 +1437,59 @@ int enqueue_mixed(cafe_ctx* C, Workspace& ws, const cafe_request* R, TreeHost& T
         a.err_ndev = C->err_ndev;
         a.fam_R = B.d_famR.as<int32_t>();
         a.out = ws.cat.as<double>();
+        a.out_err = ws.cerr.as<float>();
         a.K = K;
         a.model = gamma ? 1 : 0;
         a.cat_probs = ws.catp.as<double>();
         a.flags = d_flags;
         a.term_flags = d_term;
-        a.status = d_status;
         a.debug_wait_limit = C->debug_wait_limit;
-        // range-error bounds of the category terms: zero for every term the
-        // tensor cores do not write (FP64 bins, candidates not pruned)
-        CK(ws.cerr.reserve((size_t)std::max<int64_t>(F, 1) * K * sizeof(float)), "range bounds");
-        CK(op_memset(ws, ws.cerr.p, 0, (size_t)std::max<int64_t>(F, 1) * K * sizeof(float), ws.stream), "range bounds");
-        a.out_err = ws.cerr.as<float>();
-        a.phase_clocks = nullptr;
-        static const bool phase_env = getenv("CAFE_TC_PHASES") != nullptr;
-        if (phase_env) {
-            CK(ws.phase.reserve(kPhases * sizeof(unsigned long long)), "phase clocks");
-            CK(cudaMemsetAsync(ws.phase.p, 0, kPhases * sizeof(unsigned long long), ws.stream), "phase clocks");
-            a.phase_clocks = ws.phase.as<unsigned long long>();
-        }
         if (prof) {
             C->prof.begin(1, ws.stream, &ev);
-            C->prof.acc.prune_flops += tiles_flops(T, tc_tiles, R->use_error_model);
+            for (int b : tc_bins)
+                C->prof.acc.prune_flops += family_flops(T, B.widths[b] - 1, B.widths[b] - 1, R->use_error_model) *
+                                           (double)B.bin_count[b] * n_act;
         }
-        // tile counters of the one-CTA-per-tile launches, zeroed before the fork
-        CK(ws.tile_ctr.reserve(std::max<size_t>(launches.size(), 1) * sizeof(int)), "tile counters");
-        CK(op_memset(ws, ws.tile_ctr.p, 0, std::max<size_t>(launches.size(), 1) * sizeof(int), ws.stream), "tile counters");
         // fork: bins run on the auxiliary streams after everything queued so far
         const bool fork = launches.size() > 1;
         if (fork) {
             CK(op_record(ws, ws.ev_fork, ws.stream), "fork");
             for (int q = 0; q < Workspace::kAux; ++q) CK(op_wait(ws, ws.aux[q], ws.ev_fork), "fork");
         }
-        // widest bins (the longest walks) first, each on its own stream
+        // widest bins (the longest units) first, each on its own stream
         for (size_t q = 0; q < launches.size(); ++q) {
             const size_t li = launches.size() - 1 - q;
             const BinLaunch& L = launches[li];
-            PruneTcArgs b;
+            const int W = B.widths[L.b];
+            PatTcArgs b;
             std::memcpy(&b, &a, sizeof b);     // padding included: the bytes are a graph signature
-            b.tiles = ws.tiles.as<PruneTile>() + L.first_tile;
-            b.n_tiles = (int)L.n_tiles;
-            b.tmem_cols = L.tmem_cols;
-            b.nsplit = L.nsplit;
-            b.Ws = L.W / L.nsplit;
-            b.stages = L.stages;
-            b.vrow_base = L.vrow_base;
-            b.tile_counter = L.nsplit == 1 ? ws.tile_ctr.as<int>() + li : nullptr;
-            cudaStream_t st = fork ? ws.aux[q % Workspace::kAux] : ws.stream;
-            if (b.Ws % 32 || b.Ws < 32 || b.Ws > 256) return fail(C, CAFE_ERR_INVALID, "tensor-core tile of %d rows", b.Ws);
-            TcMaps lm;
-            const int rcm = launch_maps(b.Ws, &lm);
+            const char* dd = ws.tcp_desc.as<char>();
+            b.nodes = reinterpret_cast<const PatTcNode*>(dd + L.o_nodes);
+            b.segs = reinterpret_cast<const PatTcSeg*>(dd + L.o_segs);
+            b.n_desc = (int)L.nodes.size();
+            b.n_segs = (int)L.segs.size();
+            b.total_units = L.units;
+            b.n_slots = L.n_slots;
+            b.slot_rows = L.slot_rows;
+            b.table = ws.tcp_table[L.b].as<float>();
+            b.meta = ws.tcp_meta[L.b].as<int4>();
+            b.next = ws.tcp_ctr.as<unsigned long long>() + li;
+            b.done = reinterpret_cast<int32_t*>(ws.tcp_ctr.as<char>() + L.o_done);
+            b.W = W;
+            b.Ns = pat_tc_states(W);
+            b.n_share = W / b.Ns;
+            b.tmem_cols = 32;
+            while (b.tmem_cols < b.Ns) b.tmem_cols *= 2;
+            const int64_t rows = std::max<int64_t>(128, L.slot_rows * L.n_slots);
+            PatTcMaps maps;
+            std::memset(&maps, 0, sizeof maps);
+            int rcm = cached_map(C, ws, b.Ns / 32 - 1, &maps.mat, ws.tc_hi.as<float>(), (int64_t)n_mat * Wm, Wm, 32, b.Ns,
+                                 (int64_t)n_mat * Wm * Wm);
+            if (!rcm) rcm = cached_map(C, ws, 4 + L.b, &maps.vst, b.table, rows, W, 32, 128);
+            if (!rcm) rcm = cached_map(C, ws, 4 + kMaxGroups + L.b, &maps.vst32, b.table, rows, W, 32, 32);
             if (rcm) return rcm;
-            CK(op_launch(ws, 5, [&] { return launch_prune_tc(lm, b, L.n_ctas, L.smem, st); }, lm, b, L.n_ctas, L.smem,
-                         st),
+            const cudaStream_t st = fork ? ws.aux[q % Workspace::kAux] : ws.stream;
+            CK(op_launch(ws, 5, [&] { return launch_pat_tc(maps, b, L.n_ctas, st); }, maps, b, L.n_ctas, st),
                "prune tc");
         }
         if (fork && !prof) {
@@ -1535,21 +1503,6 @@ int enqueue_mixed(cafe_ctx* C, Workspace& ws, const cafe_request* R, TreeHost& T
             }
         }
 
-        if (phase_env) {
-            unsigned long long h[kPhases];
-            CK(cudaMemcpyAsync(h, ws.phase.p, sizeof(h), cudaMemcpyDeviceToHost, ws.stream), "phase clocks");
-            CK(cudaStreamSynchronize(ws.stream), "phase clocks");
-            const double n = (double)h[5] + 1e-9;
-            fprintf(stderr, "k_prune_tc clocks per tile-node: setup %.0f gemm %.0f epilogue %.0f root %.0f sync %.0f (%llu tile-nodes)\n",
-                    h[0] / n, h[1] / n, h[2] / n, h[3] / n, h[4] / n, h[5]);
-            fprintf(stderr, "  per tile-node: store wait %.0f leaf gather %.0f; per chunk (%.2f per tile-node): stage wait %.0f "
-                    "TMA wait %.0f split %.0f MMA issue %.0f (of which the stage's wait %.0f); last-MMA wait per tile-node %.0f\n",
-                    h[12] / n, h[13] / n, h[11] / n, h[6] / (h[11] + 1e-9), h[7] / (h[11] + 1e-9), h[8] / (h[11] + 1e-9),
-                    h[9] / (h[11] + 1e-9), h[14] / (h[11] + 1e-9), h[10] / n);
-            fprintf(stderr, "  TMA issue per chunk %.0f; barriers per tile-node: after the chunks %.0f, after the last MMAs %.0f\n",
-                    h[15] / (h[11] + 1e-9), h[16] / n, h[17] / n);
-        }
-
         if (prof) C->prof.end(1, ws.stream, ev);
     }
     if (!wide_done) {
@@ -1560,7 +1513,7 @@ int enqueue_mixed(cafe_ctx* C, Workspace& ws, const cafe_request* R, TreeHost& T
     // families the tensor-core pass could not represent, or whose result FP32's
     // range may have cost accuracy: planned on the device and recomputed in
     // FP64 without a host round trip
-    if (!tc_tiles.empty()) {
+    if (!tc_bins.empty()) {
         RangeFlagArgs rf;
         std::memset(&rf, 0, sizeof rf);
         rf.cat = ws.cat.as<double>();
@@ -1680,9 +1633,9 @@ int enqueue_mixed(cafe_ctx* C, Workspace& ws, const cafe_request* R, TreeHost& T
 int enqueue_mixed_graph(cafe_ctx* C, Workspace& ws, const cafe_request* R, TreeHost& T, FamSet& S, int K, int CT,
                         const std::vector<int32_t>& active, double** hm, double* d_fam, double* d_total,
                         ScoreInfo* info) {
-    static const bool phase_env = getenv("CAFE_TC_PHASES") != nullptr || getenv("CAFE_DEBUG_FLAGS") != nullptr;
+    static const bool flag_env = getenv("CAFE_DEBUG_FLAGS") != nullptr;
     ws.oplog.clear();
-    if (C->prof.on || phase_env) {
+    if (C->prof.on || flag_env) {
         ws.op_mode = Workspace::kOpRun;
         return enqueue_mixed(C, ws, R, T, S, K, CT, active, hm, d_fam, d_total, info);
     }
@@ -2955,7 +2908,7 @@ int cafe_ctx_create(const cafe_config* cfg, cafe_ctx** out) {
     cudaDeviceProp prop;
     cudaGetDeviceProperties(&prop, dev);
     C->sm_count = prop.multiProcessorCount;
-    if (tc_kernels_init() != cudaSuccess || pat64_init() != cudaSuccess || pvalue_kernels_init() != cudaSuccess ||
+    if (pat_tc_init() != cudaSuccess || pat64_init() != cudaSuccess || pvalue_kernels_init() != cudaSuccess ||
         cudaEventCreateWithFlags(&C->gate, cudaEventDisableTiming) != cudaSuccess) {
         delete C;
         return CAFE_ERR_CUDA;
@@ -3247,7 +3200,6 @@ int cafe_autotune(cafe_ctx* C, const cafe_request* reqs, int n, int reps, cafe_t
     auto si = C->sets.find(reqs[0].set_id);
     auto ti = C->trees.find(reqs[0].tree_id);
     if (si == C->sets.end() || ti == C->trees.end()) return fail(C, CAFE_ERR_NOT_FOUND, "unknown tree or family set");
-    const TreeHost& T = *ti->second;
     reps = std::max(1, reps);
     std::vector<cafe_result> res(n);
     // mean device time of the request with the current shapes (one untimed run first)
@@ -3267,32 +3219,29 @@ int cafe_autotune(cafe_ctx* C, const cafe_request* reqs, int n, int reps, cafe_t
         if (B.widths[b] <= 256 && B.bin_count[b] > 0) widths.push_back(B.widths[b]);
     int k = 0;
     for (int W : widths) {
-        // candidates: the three largest feasible CTA counts per SM, each with every stage count that fits
+        // candidates: the three largest feasible CTA counts per SM
         C->tuned.erase(W);
-        const TcShape def = tc_shape(C, T, W);
+        const int most = tc_per_sm(C, W);
         double best_ms;
         int rc = timed(&best_ms);
         if (rc) return rc;
-        std::pair<int, int> best{def.per_sm, def.stages};
-        const int by_tmem = 512 / def.tmem_cols;
-        for (int per = by_tmem; per >= 1 && per > by_tmem - 3; --per)
-            for (int st = 1; st <= 4; ++st) {
-                size_t sm;
-                if (tc_by_smem(T, W, st, &sm) < per || (per == def.per_sm && st == def.stages)) continue;
-                C->tuned[W] = {per, st};
-                double ms;
-                rc = timed(&ms);
-                if (rc) {
-                    C->tuned.erase(W);
-                    return rc;
-                }
-                if (ms < best_ms) {
-                    best_ms = ms;
-                    best = {per, st};
-                }
+        int best = most;
+        for (int per = most - 1; per >= 1 && per > most - 3; --per) {
+            C->tuned[W] = per;
+            double ms;
+            rc = timed(&ms);
+            if (rc) {
+                C->tuned.erase(W);
+                return rc;
             }
+            if (ms < best_ms) {
+                best_ms = ms;
+                best = per;
+            }
+        }
         C->tuned[W] = best;
-        if (k < max_out) out[k] = cafe_tune_result{W, best.first, best.second, best_ms};
+        // (operand stages follow the width: every chunk of a row up to 64 states, else two)
+        if (k < max_out) out[k] = cafe_tune_result{W, best, W == 32 ? 1 : 2, best_ms};
         ++k;
     }
     if (n_out) *n_out = k;

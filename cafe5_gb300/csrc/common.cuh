@@ -64,9 +64,6 @@ namespace cafe {
 
 cudaError_t launch_matrix_build(const MatrixJob* d_jobs, int n_jobs, int max_size, cudaStream_t s);
 
-// One-time per-device kernel attributes (shared-memory limits).
-cudaError_t tc_kernels_init();
-
 // ---- distinct count patterns per subtree (k_patterns.cu) ----
 constexpr int kMaxGroups = 16;
 struct PatBuildArgs {
@@ -235,63 +232,66 @@ constexpr int kMaxErrHalf = 8;   // deviations up to +-8 fold into the transpose
 
 cudaError_t launch_convert_tc(const ConvertJob* d_jobs, int n_jobs, TcBuffers b, cudaStream_t s);
 
-constexpr int kPhases = 18;   // k_prune_tc phase counters (CAFE_TC_PHASES)
-
-struct PruneTcArgs {
-    TreePlan plan;
-    const PruneTile* tiles;      // 128-family tiles; S = W - 1 of the tile's bin
-    int n_tiles;
-    const int32_t* counts;
+// ---- tensor-core pruning over distinct rows (k_pat_tc.cu) ----
+struct PatTcNode {               // an internal node of the bin, by height; the root last
+    int64_t cidx, perm0;         // first child index of its rows; root: first item
+    int32_t unit0, n_units;      // first unit in its level, units
+    int32_t rows, row0;          // rows (root: families), first row in a combination's table (a multiple of 32)
+    int32_t node, nch;           // tree node, children (1 or 2)
+    int32_t child[2], child_node[2];   // the children's PatTcNode (-1: a leaf) and tree nodes
+};
+// The units of one level of combinations q0 .. q0 + nq - 1, the combinations
+// interleaved.
+struct PatTcSeg {
+    long long unit0;             // first unit in the launch's order
+    int32_t q0, nq;
+    int32_t node0, node1;        // the level's nodes
+};
+struct PatTcArgs {
+    const PatTcNode* nodes;
+    const PatTcSeg* segs;
+    int n_desc, n_segs;
+    long long total_units;
+    const int32_t* active;       // combined (candidate, category) indices
+    int n_slots;                 // combinations whose tables exist at a time
+    int64_t slot_rows;           // table rows per combination
+    float* table;                // [n_slots][slot_rows][W] factor rows
+    int4* meta;                  // [n_slots][slot_rows] exponent, flags, error bound
+    int32_t* done;               // [n_active][n_desc] finished units, zeroed
+    unsigned long long* next;    // unit counter, zeroed
+    int32_t* status;             // nonzero when a bounded wait gave up
+    int32_t* any_flag;           // set when a family is left to FP64
+    const int32_t* child;        // child indices (launch_pat_write)
     const int64_t* perm;
-    const int32_t* mat_index;    // [K][n_nodes] converted-matrix index (-1 for the root); bit 30 set
-                                 // when the key is saturated
-    int Wm;                      // pitch of matrices and node vectors (elements)
+    const int32_t* mat_index;    // [K][n_nodes] converted-matrix index; bit 30: the key is saturated
+    int n_nodes;
+    int W, Wm;                   // bin width; pitch of the converted matrices
+    int Ns, n_share;             // states of a unit, units along the states
+    int tmem_cols;
     const float* mat_tr;         // [n_mat][Wm][Wm] FP32 transposed matrices (row c = column c of M)
-    float* vec;                  // node vectors (FP32), rows = CTA x slot x 128 families
-    int n_slots;
     const double* prior;
     int n_prior;
     const double* err;
-    int err_rows;
-    int err_ndev;
+    int err_rows, err_ndev;
     const int32_t* fam_R;
     double* out;                 // [F][K] natural log of each category term
-    int K;
-    int model;                   // 0 base (a zero family is -inf), 1 gamma (a zero family is NaN: failed)
+    float* out_err;              // [F][K] bound on its relative error from FP32 range loss
+    int K, model;                // model 0 base (a zero family is -inf), 1 gamma (a zero family is NaN: failed)
     const double* cat_probs;
     int32_t* flags;              // [F] set when a family must be recomputed in FP64
     uint8_t* term_flags;         // [F][K] set with it for the category term that needs the recompute
-    float* out_err;              // [F][K] bound on the relative error of each category term from FP32
-                                 // range loss (values below 2^-126 flushed), or null
-    int32_t* status;             // [1] nonzero when a bounded wait gave up
-    int tmem_cols;
-    int nsplit;                  // 1: one CTA per tile; 2 or 4: a cluster of nsplit CTAs per tile, CTA h
-                                 // computing states [h W/nsplit, (h + 1) W/nsplit) of every node
-    int Ws;                      // B rows per stage: the launch's bin width / nsplit
-    int stages;                  // pipeline stages (1 to 4)
-    int64_t vrow_base;           // first node-vector row of this launch
-    unsigned long long* phase_clocks;   // optional [kPhases]: SM clocks of thread 0 in child setup, GEMMs,
-                                        // epilogue, root bookkeeping, end-of-node barrier; tile-nodes;
-                                        // then the GEMM chain's parts (k_prune_tc.cu)
-    int* tile_counter;           // one CTA per tile (nsplit 1): zeroed tile counter the CTAs take
-                                 // tiles from; null: a fixed stride
-    int debug_wait_limit;        // > 0: the wait for a node's GEMMs gives up after this many polls
-                                 // minus one (tests of the time-out path); 0: the default bound
+    int debug_wait_limit;        // > 0: the wait for a unit's GEMM gives up after this many polls minus one
 };
-
-// Tensor maps travel by value (__grid_constant__); the host encodes them.
-// Operand loads use prune_tc_kchunk()-column boxes (mat, vec; 128-byte
-// swizzle for 32 columns, 64-byte for 16); the epilogue stores node vectors
-// in 32-column boxes in the 128-byte swizzle (vst). Vector boxes are one
-// tile's 128 rows. mat is 3D: the TF32 hi and lo matrices, one buffer
-// [2][n_mat Wm][Wm], in boxes of the launch's Ws rows x both halves. tr:
-// the FP32 transposed matrices in boxes of 32 columns x the launch's W
-// rows (leaf blocks of bins up to 64 states).
-struct TcMaps {
-    CUtensorMap mat, vec, vst, tr;
+int pat_tc_states(int W);
+cudaError_t pat_tc_init();
+int pat_tc_ctas_per_sm(int W);
+// mat: the TF32 hi and lo matrices [2][n_mat Wm][Wm] in boxes of 32 columns x
+// Ns rows x both; vst, vst32: the factor tables [n_slots slot_rows][W] in boxes
+// of 32 columns x 128 or 32 rows (all 128-byte swizzled)
+struct PatTcMaps {
+    CUtensorMap mat, vst, vst32;
 };
-
-cudaError_t launch_prune_tc(const TcMaps& maps, const PruneTcArgs& a, int n_ctas, size_t smem, cudaStream_t s);
+cudaError_t launch_pat_tc(const PatTcMaps& m, const PatTcArgs& a, int n_ctas, cudaStream_t s);
 
 // ---- device-sampled p-value simulations (k_pvalue.cu) ----
 struct SimDrawArgs {
@@ -353,9 +353,6 @@ struct RangeFlagArgs {
     int32_t* any_flag;           // set to 1 when a family is flagged
 };
 cudaError_t launch_range_flags(const RangeFlagArgs& a, cudaStream_t s);
-size_t prune_tc_smem_bytes(int Ws, int n_slots, int stages, int n_internal);
-int prune_tc_kchunk();   // K columns per operand box of k_prune_tc (its load maps' box width)
-int prune_tc_max_smem(int nsplit = 1);   // dynamic shared memory one k_prune_tc CTA may use (per split)
 
 // Device-side plan of the FP64 recompute of flagged category terms:
 // k_fallback_plan compacts the flagged families of each listed bin (in

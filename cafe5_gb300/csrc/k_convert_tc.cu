@@ -1,0 +1,247 @@
+// Around the tensor-core pruning (k_pat_tc.cu): conversion of the FP64
+// matrices into its operands, and the plan of the FP64 recompute of the
+// category terms it could not represent or whose range bound is too large.
+#include "common.cuh"
+#include "tc_ptx.cuh"
+
+#include <math.h>
+
+#include <algorithm>
+
+namespace cafe {
+namespace {
+
+// FP64 matrix -> TF32 hi/lo operands (row-major, pitch Wm) and the FP32
+// transpose tr[c][s] = M[s][c] (a leaf factor, column c of M, as one row).
+// With an error model the transpose's row c is already the leaf factor of
+// an observed count c: sum_d w_d(c) M[s][c - h + d] over the model's 2h + 1
+// deviations, in deviation order, as FP32 products and sums (the walk then
+// reads one row per leaf, whatever the model's width). A block converts a
+// band of 32 rows of one matrix, 32 columns (plus h on either side) at a
+// time through a shared-memory tile, so the row-major and the transposed
+// stores both write whole 128-byte lines. Wm is a multiple of 32.
+__global__ void __launch_bounds__(256) k_convert_tc(const ConvertJob* __restrict__ jobs, TcBuffers b) {
+    constexpr int TW = 32 + 2 * kMaxErrHalf;
+    __shared__ float tile[32][TW + 1];
+    __shared__ float wsh[32][2 * kMaxErrHalf + 1];   // the band's rows' deviation weights (0: skipped)
+    const int Wm = b.Wm;
+    const int bands = Wm / 32;
+    const ConvertJob J = jobs[blockIdx.x / bands];
+    const int s0 = (int)(blockIdx.x % bands) * 32;
+    const size_t base = (size_t)J.mat * Wm * Wm;
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const int h = b.err ? (b.err_ndev - 1) / 2 : 0;
+    // only what the walk reads: hi/lo for internal children's branches, the
+    // transpose for leaves' (block-uniform)
+    const bool want_hl = (J.what & 1) != 0, want_tr = (J.what & 2) != 0;
+    // the deviations' columns either side of a 32-column step (within
+    // 0 .. Wm - 1): lane tx < 2h loads column c0 + hoff into tile column hcol
+    const bool halo = want_tr && tx < 2 * h;
+    const int hoff = tx < h ? tx - h : 32 + (tx - h);
+    const int hcol = tx < h ? tx : 32 + tx;
+    for (int c0 = 0; c0 < Wm; c0 += 32) {
+        // the thread's four rows (ty + 8 i) of this step, and their halo
+        // entries, are loaded before any store (the stores might alias the
+        // source as far as the compiler knows), so the loads overlap
+        const int c = c0 + tx, cc = c0 + hoff;
+        float x[4], xh[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) x[i] = (float)J.src[(size_t)(s0 + ty + 8 * i) * J.ld + c];
+        if (halo) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                xh[i] = (cc >= 0 && cc < Wm) ? (float)J.src[(size_t)(s0 + ty + 8 * i) * J.ld + cc] : 0.0f;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int r = ty + 8 * i, s = s0 + r;
+            if (want_hl) {
+                const float hi = tc::round_tf32(x[i]);
+                b.hi[base + (size_t)s * Wm + c] = hi;
+                b.lo[base + (size_t)s * Wm + c] = tc::round_tf32(x[i] - hi);
+            }
+            if (!want_tr) continue;
+            tile[r][h + tx] = x[i];
+            if (halo) tile[r][hcol] = xh[i];
+        }
+        if (!want_tr) continue;
+        if (b.err)
+            for (int q = threadIdx.x; q < 32 * b.err_ndev; q += blockDim.x) {
+                const int r = q / b.err_ndev, d = q % b.err_ndev, c = c0 + r, col = c - h + d;
+                const double w = b.err[(size_t)(c < b.err_rows ? c : b.err_rows - 1) * b.err_ndev + d];
+                wsh[r][d] = (col >= 0 && col < Wm && w > 0) ? (float)w : 0.0f;
+            }
+        __syncthreads();
+        for (int r = ty; r < 32; r += 8) {
+            const int c = c0 + r;      // the count (row of tr); tx: the state s0 + tx
+            float v;
+            if (!b.err) {
+                v = tile[tx][r];
+            } else {
+                // a skipped deviation has weight 0 here: fmaf(0, x, v) = v
+                v = 0.0f;
+                for (int d = 0; d < b.err_ndev; ++d) v = fmaf(wsh[r][d], tile[tx][r + d], v);
+            }
+            b.tr[base + (size_t)c * Wm + s0 + tx] = v;
+        }
+        __syncthreads();
+    }
+}
+
+// One block: flagged families of each bin, compacted in permutation order
+// (a block-wide prefix sum per 256-family chunk); each bin's range of
+// fb_perm goes to fb_bins for k_fallback_tiles.
+__global__ void __launch_bounds__(256) k_fallback_plan(FallbackPlanArgs a) {
+    __shared__ int scan[256];
+    __shared__ int64_t base_sh;
+    if (a.any_flag && *a.any_flag == 0) {     // nothing flagged: no work
+        if (threadIdx.x == 0) {
+            a.out_counts[0] = 0;
+            a.out_counts[1] = 0;
+        }
+        return;
+    }
+    if (threadIdx.x == 0) base_sh = 0;
+    __syncthreads();
+    for (int b = 0; b < a.n_bins; ++b) {
+        const int64_t start = base_sh;
+        for (int64_t i0 = 0; i0 < a.bin_count[b]; i0 += 256) {
+            const int64_t i = i0 + threadIdx.x;
+            int64_t fam = -1;
+            int f = 0;
+            if (i < a.bin_count[b]) {
+                fam = a.perm[a.bin_first[b] + i];
+                f = a.flags[fam] != 0;
+            }
+            scan[threadIdx.x] = f;
+            __syncthreads();
+            for (int off = 1; off < 256; off <<= 1) {
+                const int add = threadIdx.x >= off ? scan[threadIdx.x - off] : 0;
+                __syncthreads();
+                scan[threadIdx.x] += add;
+                __syncthreads();
+            }
+            if (f) a.fb_perm[base_sh + scan[threadIdx.x] - 1] = fam;
+            const int total = scan[255];
+            __syncthreads();
+            if (threadIdx.x == 0) base_sh += total;
+            __syncthreads();
+        }
+        if (threadIdx.x == 0) {
+            a.fb_bins[2 * b] = start;
+            a.fb_bins[2 * b + 1] = base_sh - start;
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        a.out_counts[0] = (int32_t)base_sh;
+        a.out_counts[1] = 0;      // k_fallback_tiles counts the tiles
+    }
+}
+
+// A tile for every (32-family chunk of a bin's compacted families, listed
+// category) in which some family has that term flagged: one warp per chunk,
+// one block per category in turn. Tiles are appended in any order.
+__global__ void __launch_bounds__(256) k_fallback_tiles(FallbackPlanArgs a) {
+    if (a.any_flag && *a.any_flag == 0) return;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int q = blockIdx.x; q < a.n_cats; q += gridDim.x) {
+        const int k = a.cats[q];
+        for (int b = 0; b < a.n_bins; ++b) {
+            const int64_t start = a.fb_bins[2 * b], cnt = a.fb_bins[2 * b + 1];
+            for (int64_t c0 = (int64_t)warp * 32; c0 < cnt; c0 += 8 * 32) {
+                const int64_t i = c0 + lane;
+                const bool need = i < cnt && a.term_flags[(size_t)a.fb_perm[start + i] * a.K + k] != 0;
+                if (__any_sync(0xffffffffu, need) && lane == 0) {
+                    PruneTile t;
+                    t.first = (int)(start + c0);
+                    t.count = (int)(cnt - c0 < 32 ? cnt - c0 : 32);
+                    t.k = k;
+                    t.S = a.bin_width[b] - 1;
+                    t.R = a.bin_width[b] - 1;
+                    t.root_lo = t.pad[0] = t.pad[1] = 0;
+                    a.fb_tiles[atomicAdd(&a.out_counts[1], 1)] = t;
+                }
+            }
+        }
+    }
+}
+
+// One thread per (family, candidate): the category terms' range-error
+// bounds weighted by their shares of the family likelihood; a family over
+// tau |lnL| is flagged for the FP64 recompute. Terms that are not finite
+// (a dead or failed category) carry no weight; a family none of whose
+// terms is finite is left to the finish.
+__global__ void __launch_bounds__(256) k_range_flags(RangeFlagArgs a) {
+    const int n_cand = a.K / a.KC;
+    const int64_t n = a.F * n_cand;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t f = i / n_cand;
+        const int b = (int)(i % n_cand);
+        const double* c = a.cat + (size_t)f * a.K + (size_t)b * a.KC;
+        const float* e = a.err + (size_t)f * a.K + (size_t)b * a.KC;
+        double m = -INFINITY;
+        for (int k = 0; k < a.KC; ++k)
+            if (isfinite(c[k])) m = fmax(m, c[k]);
+        if (!(m > -INFINITY)) continue;
+        double w = 0.0, we = 0.0;
+        for (int k = 0; k < a.KC; ++k) {
+            if (!isfinite(c[k])) continue;
+            const double x = exp(c[k] - m);
+            w += x;
+            we += x * (double)e[k];
+        }
+        uint8_t* tf = a.term_flags + (size_t)f * a.K + (size_t)b * a.KC;
+        // a term the walk left to the FP64 pass carries no weight here, so the
+        // others' shares are unknown: every term of the candidate is recomputed
+        bool walk = false;
+        for (int k = 0; k < a.KC; ++k) walk |= tf[k] != 0;
+        if (walk) {
+            for (int k = 0; k < a.KC; ++k) tf[k] = 1;
+            continue;      // (the family is flagged already)
+        }
+        if (!(we != 0.0)) continue;      // no range loss in any term (or a candidate that was not pruned)
+        const double lnl = m + log(w);
+        const double bound = we / w;
+        const double lim = a.tau * fabs(lnl);
+        if (!(bound <= lim)) {
+            // recompute the terms whose share of the bound is over lim / (2 KC):
+            // the others' shares add up to at most lim / 2
+            const double each = lim * w / (2.0 * a.KC);
+            for (int k = 0; k < a.KC; ++k) {
+                const bool fin = isfinite(c[k]);
+                const double share = fin ? exp(c[k] - m) * (double)e[k] : 0.0;
+                if (!(share <= each) || !(lim > 0.0)) tf[k] = 1;
+            }
+            atomicOr(&a.flags[f], 2);
+            atomicOr(a.any_flag, 1);
+        }
+    }
+}
+
+}  // namespace
+
+cudaError_t launch_range_flags(const RangeFlagArgs& a, cudaStream_t s) {
+    const int64_t n = a.F * (a.K / a.KC);
+    if (n <= 0) return cudaSuccess;
+    const int blocks = (int)std::min<int64_t>((n + 255) / 256, 4096);
+    k_range_flags<<<blocks, 256, 0, s>>>(a);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_fallback_plan(const FallbackPlanArgs& a, cudaStream_t s) {
+    k_fallback_plan<<<1, 256, 0, s>>>(a);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess || a.n_cats <= 0) return e;
+    k_fallback_tiles<<<a.n_cats < 1024 ? a.n_cats : 1024, 256, 0, s>>>(a);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_convert_tc(const ConvertJob* d_jobs, int n_jobs, TcBuffers b, cudaStream_t s) {
+    if (n_jobs <= 0) return cudaSuccess;
+    if (b.Wm % 32) return cudaErrorInvalidValue;
+    k_convert_tc<<<(unsigned)(n_jobs * (b.Wm / 32)), 256, 0, s>>>(d_jobs, b);
+    return cudaGetLastError();
+}
+
+}  // namespace cafe

@@ -173,12 +173,12 @@ struct Workspace {
         int box_rows = 0;
         int64_t depth = 0;
         CUtensorMap map;
-    } map_cache[20];   // [2] vector loads, [3] vector stores, [4 + Ws/32 - 1] matrices (hi and lo planes),
-                       // [12 + Ws/32 - 1] transposed matrices
+    } map_cache[4 + 2 * kMaxGroups];   // [Ns/32 - 1] matrices (hi and lo planes), then per bin the
+                                       // factor tables in boxes of 128 rows, and of 32
     DevBuf scratch, tiles, mats, cat, fam_lnl, total, nfail, jobs, catp;
     PinnedBuf h_tiles, h_mats, h_jobs, h_out, h_catp;
     // tensor-core path
-    DevBuf term_flags, fb_bins, tile_ctr, tc_hi, tc_tr, tc_mi, tc_vec, conv, flags, fb_perm, tiles_fb, parts, fb_count, phase,
+    DevBuf term_flags, fb_bins, tc_hi, tc_tr, tc_mi, conv, flags, fb_perm, tiles_fb, parts, fb_count,
         catids, cerr;
     PinnedBuf h_conv, h_mi, h_flags, h_tiles_fb, h_tail, h_catids;
     // FP64 over distinct rows (k_pat64): per width class, factor tables and
@@ -186,6 +186,10 @@ struct Workspace {
     static constexpr int kPatClasses = 4;
     DevBuf pat_table[kPatClasses], pat_expo[kPatClasses], pat_desc, pat_ctr;
     PinnedBuf h_pat_desc;
+    // tensor cores over distinct rows (k_pat_tc): per bin, factor tables and row
+    // records; node and segment descriptors, counters
+    DevBuf tcp_table[kMaxGroups], tcp_meta[kMaxGroups], tcp_desc, tcp_ctr;
+    PinnedBuf h_tcp_desc;
     // reconstruction
     DevBuf rc_c, rc_state, rc_rmax, rc_mean, rc_count, rc_nfail, rc_parent, rc_bp, rc_lm, rc_lptr;
     PinnedBuf h_sim, h_simperm;        // p-values: simulated families staged for the device
@@ -255,7 +259,7 @@ struct cafe_ctx {
     std::vector<cudaEvent_t> batch_events;
     size_t cache_bytes = 0, cache_cap = 0;      // bytes of the current generation, cap of one
     uint64_t request_stamp = 0;
-    std::map<int, std::pair<int, int>> tuned;   // bin width -> (CTAs per SM, stages) chosen by cafe_autotune
+    std::map<int, int> tuned;    // bin width -> CTAs per SM chosen by cafe_autotune
     int debug_wait_limit = 0;    // cafe_debug_set: polls before the tensor-core wait for a node's GEMMs gives up
     // workspaces: [0] for synchronous calls, [1..] for the serving loop
     std::vector<std::unique_ptr<cafe::Workspace>> ws;

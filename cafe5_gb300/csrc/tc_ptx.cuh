@@ -35,15 +35,6 @@ CAFE_DEV bool mbar_wait(uint64_t* b, uint32_t parity, int limit = (1 << 24)) {
     return false;
 }
 
-// 2D TMA tile load (box given by the tensor map) into shared memory,
-// completion counted in bytes on `bar`.
-CAFE_DEV void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-            smem_u32(dst)),
-        "l"((uint64_t)map), "r"(x), "r"(y), "r"(smem_u32(bar))
-        : "memory");
-}
 // 3D TMA tile load (box given by the tensor map) into shared memory,
 // completion counted in bytes on `bar`.
 CAFE_DEV void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
@@ -62,8 +53,6 @@ CAFE_DEV void tma_store_2d(const CUtensorMap* map, int x, int y, const void* src
 CAFE_DEV void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // The shared-memory sources of this thread's bulk stores may be reused.
 CAFE_DEV void bulk_wait_read0() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-// At most one of this thread's bulk store groups still reads shared memory.
-CAFE_DEV void bulk_wait_read1() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
 // This thread's bulk stores are complete in global memory.
 CAFE_DEV void bulk_wait0() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 CAFE_DEV void fence_proxy_async_global() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
@@ -76,12 +65,6 @@ CAFE_DEV void fence_proxy_async_shared() { asm volatile("fence.proxy.async.share
 CAFE_DEV uint64_t desc_sw128(const void* p) {
     const uint64_t a = (uint64_t)(smem_u32(p) & 0x3FFFF) >> 4;
     return a | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
-}
-// Shared-memory matrix descriptor: K-major, 64-byte swizzle, 8-row groups
-// 512 bytes apart (stride byte offset), descriptor version 1.
-CAFE_DEV uint64_t desc_sw64(const void* p) {
-    const uint64_t a = (uint64_t)(smem_u32(p) & 0x3FFFF) >> 4;
-    return a | (1ull << 16) | (32ull << 32) | (1ull << 46) | (4ull << 61);
 }
 // Instruction descriptor, kind::tf32: D = F32, A = B = TF32, both K-major.
 CAFE_DEV uint32_t idesc_tf32(int M, int N) {
@@ -125,51 +108,6 @@ CAFE_DEV void tmem_ld32(uint32_t taddr, float (&v)[32]) {
     for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
 }
 
-// 32 lanes x 16 consecutive columns.
-CAFE_DEV void tmem_ld16(uint32_t taddr, float (&v)[16]) {
-    uint32_t r[16];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
-}
-
-// Issue-only variant: the registers are valid after tmem_wait().
-CAFE_DEV void tmem_ld16_issue(uint32_t taddr, uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr));
-}
-CAFE_DEV void tmem_ld_issue(uint32_t taddr, uint32_t (&r)[16]) { tmem_ld16_issue(taddr, r); }
-// 32 lanes x 8 consecutive columns, issue only.
-CAFE_DEV void tmem_ld_issue(uint32_t taddr, uint32_t (&r)[8]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                 : "r"(taddr));
-}
-CAFE_DEV void tmem_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
-// 32 lanes x 16 consecutive columns from registers (thread t of the warp
-// writes row lane base + t); complete after tmem_wait_st().
-CAFE_DEV void tmem_st16(uint32_t taddr, const float (&v)[16]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(
-            taddr),
-        "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])), "r"(__float_as_uint(v[3])),
-        "r"(__float_as_uint(v[4])), "r"(__float_as_uint(v[5])), "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7])),
-        "r"(__float_as_uint(v[8])), "r"(__float_as_uint(v[9])), "r"(__float_as_uint(v[10])),
-        "r"(__float_as_uint(v[11])), "r"(__float_as_uint(v[12])), "r"(__float_as_uint(v[13])),
-        "r"(__float_as_uint(v[14])), "r"(__float_as_uint(v[15]))
-        : "memory");
-}
-CAFE_DEV void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-
 // Round to the nearest TF32 value (10 mantissa bits, ties away from zero):
 // the result is exact for the tensor core's TF32 input conversion.
 CAFE_DEV float round_tf32(float x) {
@@ -184,48 +122,6 @@ CAFE_DEV float round_tf32(float x) {
 // either sign (sign-magnitude encoding). Cheaper than the conversion
 // instruction where a whole operand tile is split.
 CAFE_DEV float round_tf32_bits(float x) { return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xFFFFE000u); }
-
-// ---- a pair of CTAs in one thread-block cluster ----
-CAFE_DEV uint32_t cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-// Every thread of every CTA of the cluster; orders shared-memory accesses
-// (release / acquire at cluster scope). Waits without a limit: only used
-// where every CTA is known to arrive (after bounded waits only).
-CAFE_DEV void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// The address of this shared-memory location in CTA `rank` of the cluster.
-CAFE_DEV uint32_t mapa(const void* p, uint32_t rank) {
-    uint32_t ra;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(smem_u32(p)), "r"(rank));
-    return ra;
-}
-CAFE_DEV void st_cluster_f32(uint32_t ra, float v) {
-    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(ra), "f"(v) : "memory");
-}
-// One arrival on an mbarrier of another CTA of the cluster, releasing this
-// thread's earlier writes (its remote stores included) at cluster scope.
-CAFE_DEV void mbar_arrive_remote(uint32_t ra_bar) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(ra_bar) : "memory");
-}
-// Bounded wait on this CTA's mbarrier, acquiring at cluster scope what the
-// arrivals (possibly remote) released.
-CAFE_DEV bool mbar_wait_cluster(uint64_t* b, uint32_t parity, int limit = (1 << 24)) {
-    for (int i = 0; i < limit; ++i) {
-        uint32_t ok;
-        asm volatile(
-            "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, "
-            "1, 0, p;\n}\n"
-            : "=r"(ok)
-            : "r"(smem_u32(b)), "r"(parity)
-            : "memory");
-        if (ok) return true;
-    }
-    return false;
-}
 
 }  // namespace tc
 }  // namespace cafe
