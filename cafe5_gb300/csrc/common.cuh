@@ -268,12 +268,12 @@ struct PatTcArgs {
     int W, Wm;                   // bin width; pitch of the converted matrices
     int Ns, n_share;             // states of a unit, units along the states
     int tmem_cols;
+    const int32_t* item_R;       // [F] root bound of each item
     const float* mat_tr;         // [n_mat][Wm][Wm] FP32 transposed matrices (row c = column c of M)
     const double* prior;
     int n_prior;
     const double* err;
     int err_rows, err_ndev;
-    const int32_t* fam_R;
     double* out;                 // [F][K] natural log of each category term
     float* out_err;              // [F][K] bound on its relative error from FP32 range loss
     int K, model;                // model 0 base (a zero family is -inf), 1 gamma (a zero family is NaN: failed)

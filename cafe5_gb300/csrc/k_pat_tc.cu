@@ -50,9 +50,9 @@
 // Factor tables exist for n_slots combinations at a time; a combination's
 // units wait for the root of the one whose table they take over.
 //
-// Roles in a CTA: a control warp (units, waits, child indices, TMA, MMA issue,
-// completion) and 4 or 8 data warps (gather, product, split; epilogue). All
-// waits are bounded; on time-out the kernel records a status, drains its own
+// Roles in a CTA: a scheduler warp (units, their inputs' completion, child
+// indices), an issuer (TMA, MMA, completion) and 4 or 8 data warps (rows:
+// copies, product, split; epilogue). All waits are bounded; on time-out the kernel records a status, drains its own
 // copies and MMAs, frees TMEM and returns.
 #include "common.cuh"
 #include "tc_ptx.cuh"
@@ -68,9 +68,10 @@ namespace {
 constexpr int TM = 128;      // rows per unit = MMA M = TMEM lanes
 constexpr int KC = 32;       // columns per chunk: one 128-byte swizzle row
 constexpr int kChunkA = TM * KC;         // floats of one A chunk (hi or lo)
-constexpr int kPolls = 1 << 26;
-constexpr int kSegSh = 128;  // segments whose first units are kept in shared memory
-constexpr int kNodeSh = 64;  // and nodes kept there
+constexpr int kPolls = 1 << 26;          // of a count in global memory
+constexpr int kBarPolls = 1 << 20;       // of a barrier in shared memory
+constexpr int kSegSh = 64;   // segments whose first units are kept in shared memory
+constexpr int kNodeSh = 32;  // and nodes kept there
 constexpr float kTiny = 0x1p-126f;       // smallest normal FP32 value
 constexpr int32_t kSatBit = 1 << 30;     // of a matrix index: the key is saturated
 enum { kFlag = 1, kDead = 2 };           // row flags
@@ -87,17 +88,20 @@ __device__ __forceinline__ float pow2f(int a) {
     return __uint_as_float((uint32_t)(a + 127) << 23);
 }
 
-__device__ __align__(16) float g_zero_row[512];        // the factor of a padding row or a count outside the bin
+__device__ __align__(16) float g_one_row[512];      // the factor of an absent second child (1; pat_tc_init fills it)
 
-// What the control warp hands to the data warps for one unit.
+constexpr int NB = 3;         // units in hand: one done with, one worked on, one prepared
+
+// One unit, as the scheduler hands it to the issuer and the data warps.
 struct Info {
     const float* tab[2];      // the children's factor rows
     const int4* meta[2];      // an internal child's row records; null: a leaf
     int pitch[2];
     int nch, np, is_root, sat, k, stop;
+    int q, di, row_out, s_off, mat;      // combination, node, first table row, first state, matrix
     int4* meta_out;           // the unit's own row records
+    int64_t item0;            // root: first item
     int idx[2][TM];           // child indices of the rows
-    int fam[TM], Rf[TM];      // root: the rows' families and root bounds
 };
 
 // Record of a factor row: x = exponent << 2 | flags, y = error bound, and
@@ -135,10 +139,10 @@ __device__ __forceinline__ void stat_add4(RowStat& t, const float4& a, const flo
     t.fmn0 = fminf(t.fmn0, min4(a));
     t.fmn1 = fminf(t.fmn1, min4(b));
 }
-// A row's sources: its children's factors, and whether a leaf's count was
-// outside the bin.
+// A row's sources: its children's factor rows, and whether a leaf's count was
+// outside the bin (FP64 recomputes such a family: any row serves).
 struct Row {
-    const float *p0, *p1;
+    int n0, n1;
     int fl;
 };
 // What an internal child's record adds.
@@ -164,54 +168,58 @@ __device__ __forceinline__ bool leaf_ok(const PatTcArgs& a, int n) {
 }
 
 __device__ __forceinline__ Row make_row(const PatTcArgs& a, const Info& I, int r) {
-    Row w;
-    w.p0 = w.p1 = g_zero_row;
-    w.fl = 0;
-    if (r >= I.np) return w;
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-        if (c >= I.nch) continue;
-        const int n = I.idx[c][r];
-        if (!I.meta[c] && !leaf_ok(a, n)) w.fl = kFlag;
-        else (c ? w.p1 : w.p0) = I.tab[c] + (size_t)n * I.pitch[c];
+    Row w{0, 0, 0};
+    if (r >= I.np) return w;      // (a padding row: nothing reads what comes of it)
+    w.n0 = I.idx[0][r];
+    w.n1 = I.idx[1][r];
+    if (!I.meta[0] && !leaf_ok(a, w.n0)) {
+        w.fl = kFlag;
+        w.n0 = 0;
+    }
+    if (!I.meta[1] && !leaf_ok(a, w.n1)) {
+        w.fl = kFlag;
+        w.n1 = 0;
     }
     return w;
 }
-__device__ __forceinline__ const float* shfl_ptr(const float* p, int src) {
-    return reinterpret_cast<const float*>(__shfl_sync(0xffffffffu, (unsigned long long)p, src));
-}
 
-__device__ __forceinline__ RowMeta row_meta(const PatTcArgs& a, const Info& I, int r, const Row& w) {
+// (issued with the first loads, decoded once the rows are done)
+struct RawMeta {
+    int4 q0, q1;
+};
+__device__ __forceinline__ RawMeta load_meta(const Info& I, int r, const Row& w) {
+    RawMeta q{make_int4(0, 0, 0, 0), make_int4(0, 0, 0, 0)};
+    if (r >= I.np) return q;
+    if (I.meta[0]) q.q0 = __ldcg(I.meta[0] + w.n0);
+    if (I.nch > 1 && I.meta[1]) q.q1 = __ldcg(I.meta[1] + w.n1);
+    return q;
+}
+__device__ __forceinline__ RowMeta row_meta(const PatTcArgs& a, const Info& I, const Row& w, const RawMeta& q) {
     RowMeta m;
-    const bool on = r < I.np;
     const float leaf_u = (a.err ? 8.0f : 2.0f) * kTiny;
     m.E = 0;
     m.fl = w.fl;
     m.er0 = leaf_u;
     m.er1 = I.nch > 1 ? leaf_u : 0.0f;
     m.fm0 = m.fm1 = 0.0f;
-    int4 q0 = make_int4(0, 0, 0, 0), q1 = q0;
-    if (I.meta[0] && on) q0 = __ldcg(I.meta[0] + I.idx[0][r]);
-    if (I.nch > 1 && I.meta[1] && on) q1 = __ldcg(I.meta[1] + I.idx[1][r]);
     if (I.meta[0]) {
-        m.E += q0.x >> 2;
-        m.fl |= q0.x & 3;
-        m.er0 = __int_as_float(q0.y) + (float)(8 * a.W) * kTiny;
-        m.fm0 = fmaxf(__int_as_float(q0.z), __int_as_float(q0.w));
+        m.E += q.q0.x >> 2;
+        m.fl |= q.q0.x & 3;
+        m.er0 = __int_as_float(q.q0.y) + (float)(8 * a.W) * kTiny;
+        m.fm0 = fmaxf(__int_as_float(q.q0.z), __int_as_float(q.q0.w));
     }
     if (I.nch > 1 && I.meta[1]) {
-        m.E += q1.x >> 2;
-        m.fl |= q1.x & 3;
-        m.er1 = __int_as_float(q1.y) + (float)(8 * a.W) * kTiny;
-        m.fm1 = fmaxf(__int_as_float(q1.z), __int_as_float(q1.w));
+        m.E += q.q1.x >> 2;
+        m.fl |= q.q1.x & 3;
+        m.er1 = __int_as_float(q.q1.y) + (float)(8 * a.W) * kTiny;
+        m.fm1 = fmaxf(__int_as_float(q.q1.z), __int_as_float(q.q1.w));
     }
     return m;
 }
 
 __device__ __forceinline__ float4 load4(const float* p, int col) { return __ldcg(reinterpret_cast<const float4*>(p + col)); }
-// the second factor of a node with one child is 1
-__device__ __forceinline__ float4 load4b(const Info& I, const float* p, int col) {
-    return I.nch > 1 ? load4(p, col) : make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+__device__ __forceinline__ void cp16(float* dst, const float* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(tc::smem_u32(dst)), "l"(src) : "memory");
 }
 
 // How a row is scaled, from its statistics: the factors of both children
@@ -257,10 +265,11 @@ __device__ __forceinline__ void split_store(float* hi, float* lo, int r, int l, 
     a.y = tc::round_tf32_bits(v.y);
     a.z = tc::round_tf32_bits(v.z);
     a.w = tc::round_tf32_bits(v.w);
-    b.x = tc::round_tf32_bits(v.x - a.x);
-    b.y = tc::round_tf32_bits(v.y - a.y);
-    b.z = tc::round_tf32_bits(v.z - a.z);
-    b.w = tc::round_tf32_bits(v.w - a.w);
+    // (the operand's 13 low bits are ignored: the rounding needs no mask here)
+    b.x = __uint_as_float(__float_as_uint(v.x - a.x) + 0x1000u);
+    b.y = __uint_as_float(__float_as_uint(v.y - a.y) + 0x1000u);
+    b.z = __uint_as_float(__float_as_uint(v.z - a.z) + 0x1000u);
+    b.w = __uint_as_float(__float_as_uint(v.w - a.w) + 0x1000u);
     const int at = r * KC + ((l ^ (r & 7)) << 2);
     *reinterpret_cast<float4*>(hi + at) = a;
     *reinterpret_cast<float4*>(lo + at) = b;
@@ -294,26 +303,31 @@ struct RootRow {
     float s0, s1, er0, er1;   // the factors' scales and error bounds
     int Rf;
 };
+template <bool SC>
 __device__ __forceinline__ void best_add(Best& b, const RootRow& w, bool leaf0, bool leaf1, float q, int s, float r0,
                                          float r1) {
     if (s > w.Rf) q = 0.0f;
-    const float f0 = r0 * w.s0, f1 = r1 * w.s1;
+    const float f0 = SC ? r0 * w.s0 : r0, f1 = SC ? r1 * w.s1 : r1;
     const float v = (f0 * f1) * q;
     if (v > b.f) {
         b.f = v;
         b.s = s;
     }
-    const float u0 = (leaf0 && !(r0 < 0x1p-100f) ? 0.0f : w.er0) * w.s0;
-    const float u1 = (leaf1 && !(r1 < 0x1p-100f) ? 0.0f : w.er1) * w.s1;
+    float u0 = leaf0 && !(r0 < 0x1p-100f) ? 0.0f : w.er0, u1 = leaf1 && !(r1 < 0x1p-100f) ? 0.0f : w.er1;
+    if (SC) {
+        u0 *= w.s0;
+        u1 *= w.s1;
+    }
     b.err = fmaxf(b.err, (u0 * (f1 + u1) + u1 * f0) * q);
 }
+template <bool SC>
 __device__ __forceinline__ void best_add4(Best& b, const RootRow& w, bool leaf0, bool leaf1, const float* prior_s, int s,
                                           const float4& x, const float4& y) {
     const float4 q = *reinterpret_cast<const float4*>(prior_s + s);
-    best_add(b, w, leaf0, leaf1, q.x, s, x.x, y.x);
-    best_add(b, w, leaf0, leaf1, q.y, s + 1, x.y, y.y);
-    best_add(b, w, leaf0, leaf1, q.z, s + 2, x.z, y.z);
-    best_add(b, w, leaf0, leaf1, q.w, s + 3, x.w, y.w);
+    best_add<SC>(b, w, leaf0, leaf1, q.x, s, x.x, y.x);
+    best_add<SC>(b, w, leaf0, leaf1, q.y, s + 1, x.y, y.y);
+    best_add<SC>(b, w, leaf0, leaf1, q.z, s + 2, x.z, y.z);
+    best_add<SC>(b, w, leaf0, leaf1, q.w, s + 3, x.w, y.w);
 }
 __device__ __forceinline__ void best_reduce(Best& b) {
 #pragma unroll
@@ -343,27 +357,32 @@ __device__ __forceinline__ int root_exp4(int m, int s, int Rf, const float4& x, 
     return m;
 }
 
-// NCH: 32-column chunks of the bin (1 or 2: a row stays in registers between
-// its statistics and its operands, and every chunk is resident), or 0: any
-// width, two passes over the rows and a ring of two stages.
+// NCH: 32-column chunks of the bin (1 or 2: every chunk of a unit is
+// resident), or 0: any width, two passes over the rows and a ring of two
+// stages.
 template <int NCH>
 struct Shape {
     static constexpr int kDataWarps = NCH == 1 ? 4 : 8;
     static constexpr int kData = 32 * kDataWarps;
-    static constexpr int kThreads = kData + 32;
+    static constexpr int kThreads = kData + 64;
     static constexpr int kStages = NCH ? NCH : 2;
     static constexpr int kPerSm = NCH == 1 ? 4 : NCH == 2 ? 2 : 1;
 };
 
-// Floats of one stage: A hi, A lo, B hi, B lo.
-__host__ __device__ inline int stage_floats(int Ns) { return 2 * kChunkA + 2 * Ns * KC; }
+// Floats of one stage: A hi, A lo, B hi, B lo. With resident chunks the B
+// area is also the home of the epilogue's 128-row staging tile, so that A is
+// free for the next unit's rows as soon as the MMAs are done.
+__host__ __device__ inline int stage_floats(int W, int Ns) {
+    const int b = 2 * Ns * KC;
+    return 2 * kChunkA + (W <= 64 && b < kChunkA ? kChunkA : b);
+}
 
 template <int NCH>
 struct alignas(16) Shared {
-    uint64_t ready[2], a_full[2], b_full[2], empty[2], mma, stored, a_free, drain;
+    uint64_t ready[NB], freed[NB], a_full[2], b_full[2], empty[2], mma, stored, a_free, drain;
     uint32_t tmem;
     int abort;
-    Info info[2];
+    Info info[NB];
     alignas(16) float prior_s[NCH ? NCH * KC : 512];      // prior of the root size that state s stands for (0 at s = 0)
     long long seg0[kSegSh];
     PatTcNode nodes[kNodeSh];
@@ -371,16 +390,33 @@ struct alignas(16) Shared {
 
 // A wait that gives up when the CTA does. The data warps use the warp-wide
 // form below: a warp's lanes go on or give up together.
+// Each poll may suspend the thread for up to 10 us (spinning instead would take
+// issue slots from the warps that work).
 template <class Sh>
-__device__ __forceinline__ bool wait_bar(Sh& sh, uint64_t* b, uint32_t parity, int limit = kPolls) {
+__device__ __forceinline__ bool wait_bar(Sh& sh, uint64_t* b, uint32_t parity, int limit = kBarPolls) {
     for (int i = 0; i < limit; ++i) {
-        if (tc::mbar_try_wait(b, parity)) return true;
+        uint32_t ok;
+        asm volatile(
+            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n selp.u32 %0, 1, 0, p;\n}\n"
+            : "=r"(ok)
+            : "r"(tc::smem_u32(b)), "r"(parity), "r"(10000u)
+            : "memory");
+        if (ok) return true;
         if (*(volatile int*)&sh.abort) return false;
     }
     return false;
 }
+__device__ __forceinline__ bool test_bar(uint64_t* b, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(ok)
+        : "r"(tc::smem_u32(b)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
 template <class Sh>
-__device__ __forceinline__ bool wait_warp(Sh& sh, uint64_t* b, uint32_t parity, int limit = kPolls) {
+__device__ __forceinline__ bool wait_warp(Sh& sh, uint64_t* b, uint32_t parity, int limit = kBarPolls) {
     const bool ok = __all_sync(0xffffffffu, wait_bar(sh, b, parity, limit));
     if (!ok) *(volatile int*)&sh.abort = 1;
     return ok;
@@ -422,47 +458,48 @@ __device__ __forceinline__ int last_at_most(int lo, int hi, long long x, int lan
     return lo;
 }
 
-// A unit as the control warp sees it.
-struct UnitRef {
-    bool valid, is_root;
-    int q, di, nch, np, row_out, s_off, mat;
-};
-
 // Takes the next unit and fills in its Info (no waits: indices and pointers
-// only). Collective over the control warp.
+// only). Collective over the scheduler warp; false when there is none left.
 template <class Sh>
-__device__ __forceinline__ UnitRef prepare(const PatTcArgs& a, Sh& sh, Info& I, unsigned long long& next, int lane) {
-    UnitRef u;
+__device__ __forceinline__ bool prepare(const PatTcArgs& a, Sh& sh, Info& I, unsigned long long& next, int lane) {
     const long long idx = (long long)__shfl_sync(0xffffffffu, next, 0);
-    u.valid = idx < a.total_units;
-    if (!u.valid) return u;
+    if (idx >= a.total_units) return false;
     if (lane == 0) next = atomicAdd(a.next, 1ull);
     const PatTcSeg sg = a.segs[last_at_most(0, a.n_segs, idx, lane, [&](int i) {
         return i < kSegSh ? sh.seg0[i] : a.segs[i].unit0;
     })];
     const int rem = (int)(idx - sg.unit0);
     const int ul = rem / sg.nq;
-    u.q = sg.q0 + rem % sg.nq;
-    u.di = last_at_most(sg.node0, sg.node1, ul, lane, [&](int i) {
+    const int q = sg.q0 + rem % sg.nq;
+    const int k = __ldg(a.active + q), slot = q % a.n_slots;
+    const int di = last_at_most(sg.node0, sg.node1, ul, lane, [&](int i) {
         return (long long)(i < kNodeSh ? sh.nodes[i].unit0 : a.nodes[i].unit0);
     });
-    const PatTcNode nd = get_node(a, sh, u.di);
+    const PatTcNode nd = get_node(a, sh, di);
     const int un = ul - nd.unit0;
-    const int k = a.active[u.q], slot = u.q % a.n_slots;
-    const int32_t* mi = a.mat_index + (size_t)k * a.n_nodes;
-    u.is_root = u.di == a.n_desc - 1;
-    u.nch = nd.nch;
-    const int share = u.is_root ? 0 : un % a.n_share, p0 = (u.is_root ? un : un / a.n_share) * TM;
-    u.s_off = share * a.Ns;
-    u.mat = u.is_root ? 0 : mi[nd.node] & ~kSatBit;
-    const int64_t slot_row = (int64_t)slot * a.slot_rows;
-    u.row_out = (int)(slot_row + nd.row0 + p0);
+    const bool is_root = di == a.n_desc - 1;
+    const int share = is_root ? 0 : un % a.n_share, p0 = (is_root ? un : un / a.n_share) * TM;
     const int np = min(TM, nd.rows - p0);
-    u.np = np;
-    if (lane < 2 && lane < nd.nch) {
-        const int d = nd.child[lane];
-        const int m = mi[nd.child_node[lane]];
-        if (d >= 0) {
+    // the rows' child indices
+    int i0[TM / 32], i1[TM / 32];
+#pragma unroll
+    for (int i = 0; i < TM / 32; ++i) {
+        const int32_t* ci = a.child + nd.cidx + (int64_t)(p0 + min(lane + 32 * i, np - 1)) * nd.nch;
+        i0[i] = __ldg(ci);
+        i1[i] = nd.nch > 1 ? __ldg(ci + 1) : 0;
+    }
+    const int32_t* mi = a.mat_index + (size_t)k * a.n_nodes;
+    const int64_t slot_row = (int64_t)slot * a.slot_rows;
+    const int m_own = is_root ? 0 : __ldg(mi + nd.node);
+    const int m0 = __ldg(mi + nd.child_node[0]), m1 = nd.nch > 1 ? __ldg(mi + nd.child_node[1]) : 0;
+    if (lane < 2) {
+        const int d = lane < nd.nch ? nd.child[lane] : -1;
+        const int m = lane ? m1 : m0;
+        if (lane >= nd.nch) {      // no second child: a factor of 1 (and not a leaf)
+            I.tab[lane] = g_one_row;
+            I.meta[lane] = a.meta;
+            I.pitch[lane] = 0;
+        } else if (d >= 0) {
             const int64_t r = slot_row + get_node(a, sh, d).row0;
             I.tab[lane] = a.table + r * a.W;
             I.meta[lane] = a.meta + r;
@@ -476,195 +513,171 @@ __device__ __forceinline__ UnitRef prepare(const PatTcArgs& a, Sh& sh, Info& I, 
     if (lane == 0) {
         I.nch = nd.nch;
         I.np = np;
-        I.is_root = u.is_root;
-        int sat = 0;
-        for (int c = 0; c < nd.nch; ++c) sat |= (mi[nd.child_node[c]] & kSatBit) != 0;
-        I.sat = sat;
+        I.is_root = is_root;
+        I.sat = ((m0 | m1) & kSatBit) != 0;
         I.k = k;
         I.stop = 0;
+        I.q = q;
+        I.di = di;
+        I.row_out = (int)(slot_row + nd.row0 + p0);
+        I.s_off = share * a.Ns;
+        I.mat = m_own & ~kSatBit;
         // (only the unit of a row's first states writes its record)
-        I.meta_out = u.is_root || share ? nullptr : a.meta + u.row_out;
-        if (nd.nch < 2) I.meta[1] = a.meta;      // (no second child: not a leaf either)
+        I.meta_out = is_root || share ? nullptr : a.meta + slot_row + nd.row0 + p0;
+        I.item0 = nd.perm0 + p0;
     }
 #pragma unroll
     for (int i = 0; i < TM / 32; ++i) {
-        const int r = lane + 32 * i;
-        if (r >= np) break;
-        const int32_t* ci = a.child + nd.cidx + (int64_t)(p0 + r) * nd.nch;
-        I.idx[0][r] = __ldg(ci);
-        if (nd.nch > 1) I.idx[1][r] = __ldg(ci + 1);
-        if (u.is_root) {
-            const int64_t f = __ldg(a.perm + nd.perm0 + p0 + r);
-            I.fam[r] = (int)f;
-            I.Rf[r] = __ldg(a.fam_R + f);
-        }
+        I.idx[0][lane + 32 * i] = i0[i];
+        I.idx[1][lane + 32 * i] = i1[i];
     }
     __syncwarp();
-    return u;
+    return true;
 }
 
-// Whether (or until) everything the unit reads is complete.
+// Waits until everything the unit reads is complete.
 template <class Sh>
-__device__ __forceinline__ bool inputs_done(const PatTcArgs& a, const Sh& sh, const UnitRef& u, int lane, bool wait) {
+__device__ __forceinline__ bool wait_inputs(const PatTcArgs& a, const Sh& sh, const Info& I, int lane) {
     bool ok = true;
     const int32_t* p = nullptr;
     int n = 0;
-    if (lane < 2 && lane < u.nch) {
-        const int d = get_node(a, sh, u.di).child[lane];
+    if (lane < 2 && lane < I.nch) {
+        const int d = get_node(a, sh, I.di).child[lane];
         if (d >= 0) {
-            p = a.done + (size_t)u.q * a.n_desc + d;
+            p = a.done + (size_t)I.q * a.n_desc + d;
             n = get_node(a, sh, d).n_units;
         }
-    } else if (lane == 2 && u.q >= a.n_slots) {      // the table's last user
-        p = a.done + (size_t)(u.q - a.n_slots) * a.n_desc + a.n_desc - 1;
+    } else if (lane == 2 && I.q >= a.n_slots) {      // the table's last user
+        p = a.done + (size_t)(I.q - a.n_slots) * a.n_desc + a.n_desc - 1;
         n = get_node(a, sh, a.n_desc - 1).n_units;
     }
-    if (p) ok = wait ? wait_count(p, n, a.status, &sh.abort) : count_now(p) >= n;
+    if (p) ok = wait_count(p, n, a.status, &sh.abort);
     ok = __all_sync(0xffffffffu, ok);
     __syncwarp();
     return ok;
 }
 
+// The scheduler warp: units into the Info buffers, each handed on once its
+// inputs are complete.
 template <int NCH>
-__device__ void control(const PatTcArgs& a, const CUtensorMap* map_mat, const CUtensorMap* map_vst,
-                        const CUtensorMap* map_vst32, Shared<NCH>& sh,
-                        float* stages, int lane) {
-    constexpr int NST = Shape<NCH>::kStages;
-    const int n_chunks = a.W / KC;
-    const int sf = stage_floats(a.Ns);
-    const uint32_t idesc = tc::idesc_tf32(TM, a.Ns);
+__device__ void schedule(const PatTcArgs& a, Shared<NCH>& sh, int lane) {
     unsigned long long next = 0;
     if (lane == 0) next = atomicAdd(a.next, 1ull);
-    UnitRef u = prepare(a, sh, sh.info[0], next, lane);
-    bool told = false;           // this unit's Info is already with the data warps
-    uint32_t g = 0;              // chunks so far
-    int pending_b = 0;           // lane 0: B loads not yet waited for (bit per stage)
-    uint32_t par_b[2] = {0, 0};
-    for (int n = 0;; ++n) {
-        const int b = n & 1;
-        bool ok = u.valid && (told || inputs_done(a, sh, u, lane, true));
-        if (u.valid && !ok && lane == 0) atomicCAS(a.status, 0, 1);
-        if (!ok) {
-            if (lane == 0) {
-                sh.info[b].stop = 1;
-                mbar_arrive(&sh.ready[b]);
+    uint32_t use = 0;            // uses of the buffers so far
+    for (int buf = 0;; buf = buf + 1 == NB ? 0 : buf + 1, ++use) {
+        bool ok = use < NB || wait_warp(sh, &sh.freed[buf], (use / NB - 1) & 1);
+        Info& I = sh.info[buf];
+        bool more = false;
+        if (ok) {
+            more = prepare(a, sh, I, next, lane);
+            if (more && !(ok = wait_inputs(a, sh, I, lane)) && lane == 0) {
+                atomicCAS(a.status, 0, 1);
+                *(volatile int*)&sh.abort = 1;
             }
-            break;
         }
-        if (lane == 0 && !told) mbar_arrive(&sh.ready[b]);
-        told = false;
-        UnitRef nu;
-        if (!u.is_root) {
-            // matrix chunks into the stages (their last readers are done: the
-            // previous GEMM's completion was waited for below)
+        if (lane == 0) {
+            if (!ok || !more) I.stop = 1;
+            mbar_arrive(&sh.ready[buf]);
+        }
+        if (!ok || !more) return;
+    }
+}
+
+// The issuer warp (lane 0): matrix chunks by TMA, MMAs, factor tables by TMA,
+// and the count of finished units.
+template <int NCH>
+__device__ void issue(const PatTcArgs& a, const CUtensorMap* map_mat, const CUtensorMap* map_vst,
+                      const CUtensorMap* map_vst32, Shared<NCH>& sh, float* stages) {
+    constexpr int NST = Shape<NCH>::kStages;
+    const int n_chunks = a.W / KC;
+    const int sf = stage_floats(a.W, a.Ns);
+    const uint32_t idesc = tc::idesc_tf32(TM, a.Ns);
+    uint32_t g = 0;              // chunks so far
+    int pending_b = 0;           // B loads not yet waited for (bit per stage)
+    uint32_t par_b[2] = {0, 0};
+    uint32_t use = 0;
+    bool ok = true;
+    for (int buf = 0; ok; buf = buf + 1 == NB ? 0 : buf + 1, ++use) {
+        ok = wait_bar(sh, &sh.ready[buf], (use / NB) & 1);
+        if (!ok) break;
+        const Info& I = sh.info[buf];
+        if (I.stop) break;
+        const int np = I.np, q = I.q, di = I.di, row_out = I.row_out, s_off = I.s_off, mat_row = I.mat * a.Wm + s_off;
+        const bool is_root = I.is_root;
+        if (!is_root) {
+            // matrix chunks into the stages: the previous unit's MMAs are done, and
+            // its stores have read their staging tiles (waited for below)
             auto load_b = [&](int c) {
                 const int st = (int)((g + (uint32_t)c) % NST);
                 tc::mbar_expect_tx(&sh.b_full[st], (uint32_t)(2 * a.Ns * KC * sizeof(float)));
-                tc::tma_load_3d(stages + (size_t)st * sf + 2 * kChunkA, map_mat, c * KC, u.mat * a.Wm + u.s_off, 0,
-                                &sh.b_full[st]);
+                tc::tma_load_3d(stages + (size_t)st * sf + 2 * kChunkA, map_mat, c * KC, mat_row, 0, &sh.b_full[st]);
                 pending_b |= 1 << st;
                 par_b[st] = ((g + (uint32_t)c) / NST) & 1;
             };
-            if (lane == 0)
-                for (int c = 0; c < NST && c < n_chunks; ++c) load_b(c);
-            // the next unit, while the data warps work on this one's rows (its Info
-            // buffer's last readers passed `stored` a unit ago)
-            nu = prepare(a, sh, sh.info[b ^ 1], next, lane);
+            for (int c = 0; c < NST && c < n_chunks; ++c) load_b(c);
             for (int c = 0; c < n_chunks && ok; ++c) {
                 const uint32_t cg = g + (uint32_t)c;
                 const int st = (int)(cg % NST);
                 const uint32_t par = (cg / NST) & 1;
-                if (lane == 0) {
-                    ok = wait_bar(sh, &sh.a_full[st], par) && wait_bar(sh, &sh.b_full[st], par);
-                    if (ok) {
-                        pending_b &= ~(1 << st);
-                        tc::fence_after();
-                        const float* Ah = stages + (size_t)st * sf;
-                        const float* Al = Ah + kChunkA;
-                        const float* Bh = Al + kChunkA;
-                        const float* Bl = Bh + a.Ns * KC;
+                ok = wait_bar(sh, &sh.a_full[st], par) && wait_bar(sh, &sh.b_full[st], par);
+                if (!ok) break;
+                pending_b &= ~(1 << st);
+                tc::fence_after();
+                const float* Ah = stages + (size_t)st * sf;
+                const float* Al = Ah + kChunkA;
+                const float* Bh = Al + kChunkA;
+                const float* Bl = Bh + a.Ns * KC;
 #pragma unroll
-                        for (int ks = 0; ks < KC / 8; ++ks) {
-                            const uint64_t ah = tc::desc_sw128(Ah + ks * 8), al = tc::desc_sw128(Al + ks * 8);
-                            const uint64_t bh = tc::desc_sw128(Bh + ks * 8), bl = tc::desc_sw128(Bl + ks * 8);
-                            tc::mma_tf32(sh.tmem, ah, bh, idesc, (c == 0 && ks == 0) ? 0u : 1u);
-                            tc::mma_tf32(sh.tmem, ah, bl, idesc, 1);
-                            tc::mma_tf32(sh.tmem, al, bh, idesc, 1);
-                        }
-                        if (NCH == 0) tc::mma_commit(&sh.empty[st]);
-                        if (c + 1 == n_chunks) tc::mma_commit(&sh.mma);
-                        // the stage of the chunk before is free when its MMAs are done
-                        if (NCH == 0 && c >= 1 && c - 1 + NST < n_chunks) {
-                            const uint32_t pg = cg - 1;
-                            ok = wait_bar(sh, &sh.empty[pg % NST], (pg / NST) & 1);
-                            if (ok) load_b(c - 1 + NST);
-                        }
-                    }
+                for (int ks = 0; ks < KC / 8; ++ks) {
+                    const uint64_t ah = tc::desc_sw128(Ah + ks * 8), al = tc::desc_sw128(Al + ks * 8);
+                    const uint64_t bh = tc::desc_sw128(Bh + ks * 8), bl = tc::desc_sw128(Bl + ks * 8);
+                    tc::mma_tf32(sh.tmem, ah, bh, idesc, (c == 0 && ks == 0) ? 0u : 1u);
+                    tc::mma_tf32(sh.tmem, ah, bl, idesc, 1);
+                    tc::mma_tf32(sh.tmem, al, bh, idesc, 1);
                 }
-                ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
+                if (NCH == 0) tc::mma_commit(&sh.empty[st]);
+                if (c + 1 == n_chunks) tc::mma_commit(&sh.mma);
+                // the stage of the chunk before is free when its MMAs are done
+                if (NCH == 0 && c >= 1 && c - 1 + NST < n_chunks) {
+                    const uint32_t pg = cg - 1;
+                    ok = wait_bar(sh, &sh.empty[pg % NST], (pg / NST) & 1);
+                    if (ok) load_b(c - 1 + NST);
+                }
             }
             g += (uint32_t)n_chunks;
-        } else {
-            nu = prepare(a, sh, sh.info[b ^ 1], next, lane);
         }
-        if (ok && nu.valid && inputs_done(a, sh, nu, lane, false)) {
-            told = true;
-            if (lane == 0) mbar_arrive(&sh.ready[b ^ 1]);
-        }
-        if (lane == 0 && ok) {
-            ok = wait_bar(sh, &sh.stored, n & 1);
-            if (ok && !u.is_root) {
-                for (int c = 0; c < a.Ns / KC; ++c) {
-                    float* t = stages + (size_t)c * kChunkA;
-                    if (u.np > TM - 32) {
-                        tc::tma_store_2d(map_vst, u.s_off + c * KC, u.row_out, t);
-                    } else {
-                        for (int r = 0; r < u.np; r += 32)
-                            tc::tma_store_2d(map_vst32, u.s_off + c * KC, u.row_out + r, t + r * KC);
-                    }
-                }
-                tc::bulk_commit();
-                tc::bulk_wait_read0();
-                mbar_arrive(&sh.a_free);
-                tc::bulk_wait0();
-                tc::fence_proxy_async_global();
-            }
-            if (ok) {
-                __threadfence();
-                atomicAdd(a.done + (size_t)u.q * a.n_desc + u.di, 1);
-            }
-        }
-        ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
-        if (!ok) {
-            // some wait of this CTA gave up
-            if (lane == 0) {
-                atomicCAS(a.status, 0, 1);
-                *(volatile int*)&sh.abort = 1;
-                if (!told) {
-                    sh.info[b ^ 1].stop = 1;
-                    mbar_arrive(&sh.ready[b ^ 1]);
+        ok = ok && wait_bar(sh, &sh.stored, use & 1);
+        if (!ok) break;
+        mbar_arrive(&sh.freed[buf]);       // nobody reads this unit's Info any more
+        if (!is_root) {
+            for (int c = 0; c < a.Ns / KC; ++c) {
+                float* t = NCH ? stages + (size_t)c * sf + 2 * kChunkA : stages + (size_t)c * kChunkA;
+                if (np > TM - 32) {
+                    tc::tma_store_2d(map_vst, s_off + c * KC, row_out, t);
+                } else {
+                    for (int r = 0; r < np; r += 32) tc::tma_store_2d(map_vst32, s_off + c * KC, row_out + r, t + r * KC);
                 }
             }
-            break;
+            tc::bulk_commit();
+            tc::bulk_wait_read0();
+            if (NCH == 0) mbar_arrive(&sh.a_free);
+            tc::bulk_wait0();
+            tc::fence_proxy_async_global();
         }
-        u = nu;
-        if (!u.valid && !told) {
-            if (lane == 0) {
-                sh.info[b ^ 1].stop = 1;
-                mbar_arrive(&sh.ready[b ^ 1]);
-            }
-            break;
-        }
+        __threadfence();
+        atomicAdd(a.done + (size_t)q * a.n_desc + di, 1);
+    }
+    if (!ok) {
+        // some wait of this CTA gave up
+        atomicCAS(a.status, 0, 1);
+        *(volatile int*)&sh.abort = 1;
     }
     // drain: loads of ours still landing, MMAs still running
-    if (lane == 0) {
-        for (int q = 0; q < NST; ++q)
-            if (pending_b >> q & 1) tc::mbar_wait(&sh.b_full[q], par_b[q], 1 << 20);
-        tc::mma_commit(&sh.drain);
-        tc::mbar_wait(&sh.drain, 0, 1 << 24);
-        tc::bulk_wait0();
-    }
-    __syncwarp();
+    for (int q = 0; q < NST; ++q)
+        if (pending_b >> q & 1) tc::mbar_wait(&sh.b_full[q], par_b[q], 1 << 20);
+    tc::mma_commit(&sh.drain);
+    tc::mbar_wait(&sh.drain, 0, 1 << 24);
+    tc::bulk_wait0();
 }
 
 // Rows of a unit go to the data warps in groups of four, eight lanes a row:
@@ -677,77 +690,108 @@ __device__ void data(const PatTcArgs& a, Shared<NCH>& sh, float* stages, int tid
     constexpr int DW = Shape<NCH>::kDataWarps, NST = Shape<NCH>::kStages;
     constexpr int GPW = TM / 4 / DW;      // groups per warp
     constexpr int VC = NCH ? NCH : 1;
-    constexpr int BT = NCH == 1 ? 4 : NCH == 2 ? 2 : 1;
     const int warp = tid >> 5, lane = tid & 31, l = lane & 7, sub = lane >> 3;
     const int n_chunks = NCH ? NCH : a.W / KC;
-    const int sf = stage_floats(a.Ns);
+    const int sf = stage_floats(a.W, a.Ns);
     const bool fused = a.W <= 64;         // rows of up to 64 states are scaled after the product
     const int own = lane < 4 * GPW ? 4 * ((lane >> 2) * DW + warp) + (lane & 3) : TM;   // the row this lane owns
     const int from = (lane & 3) * 8;      // a lane of the eight that work on it (in its group's turn)
     uint32_t g = 0, gu = 0;               // chunks and GEMM units so far
-    for (int n = 0;; ++n) {
-        const int b = n & 1;
-        if (!wait_warp(sh, &sh.ready[b], (n >> 1) & 1)) return;
-        const Info& I = sh.info[b];
-        if (I.stop) return;
-        const bool leaf0 = !I.meta[0], leaf1 = !I.meta[1];
-        const int np = I.np;
-        const int groups = max(0, min(GPW, ((np + 3) / 4 - warp + DW - 1) / DW));   // this warp's (warp-uniform)
-        const Row w = make_row(a, I, own);
-        // resident chunks: the factors of BT groups in flight at a time
-        float4 x[BT][VC], y[BT][VC];
-        auto load_groups = [&](int i0) {
+    // the unit being worked on; the next one's is set up (and its first loads
+    // issued) while this one's GEMM runs
+    const Info* Ip = nullptr;
+    bool leaf0 = false, leaf1 = false;
+    int np = 0, groups = 0;
+    Row w{0, 0, 0};
+    RawMeta raw;
+    const float *t0 = nullptr, *t1 = nullptr;      // this lane's columns of the children's row 0
+    unsigned pitch0 = 0, pitch1 = 0;
+    auto row0 = [&](int src) { return t0 + (size_t)pitch0 * (unsigned)__shfl_sync(0xffffffffu, w.n0, src); };
+    auto row1 = [&](int src) { return t1 + (size_t)pitch1 * (unsigned)__shfl_sync(0xffffffffu, w.n1, src); };
+    // Resident chunks: all of a unit's factors are copied into the operand
+    // area, a lane's 16-byte pieces of the first child where their product's hi
+    // part will be, of the second where its lo part will be. A lane reads back
+    // only what it copied.
+    auto piece = [&](int i, int c) {
+        const int r = 4 * (i * DW + warp) + sub;
+        return stages + (size_t)c * sf + r * KC + ((l ^ (r & 7)) << 2);
+    };
+    auto copy_rows = [&]() {
+        for (int i = 0; i < groups; ++i) {
+            const float* p0 = row0(4 * i + sub);
+            const float* p1 = row1(4 * i + sub);
 #pragma unroll
-            for (int j = 0; j < BT; ++j) {
-                if (i0 + j >= groups) continue;
-                const float* p0 = shfl_ptr(w.p0, 4 * (i0 + j) + sub) + 4 * l;
-                const float* p1 = shfl_ptr(w.p1, 4 * (i0 + j) + sub) + 4 * l;
-#pragma unroll
-                for (int c = 0; c < VC; ++c) {
-                    x[j][c] = load4(p0, c * KC);
-                    y[j][c] = load4b(I, p1, c * KC);
-                }
+            for (int c = 0; c < VC; ++c) {
+                cp16(piece(i, c), p0 + c * KC);
+                cp16(piece(i, c) + kChunkA, p1 + c * KC);
             }
-        };
-        if (NCH) load_groups(0);
-        const RowMeta m = row_meta(a, I, own, w);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    float4 x[VC], y[VC];      // the group's factors
+    auto get_rows = [&](int i) {
+#pragma unroll
+        for (int c = 0; c < VC; ++c) {
+            x[c] = *reinterpret_cast<const float4*>(piece(i, c));
+            y[c] = *reinterpret_cast<const float4*>(piece(i, c) + kChunkA);
+        }
+    };
+    auto begin = [&](const Info& I) {
+        Ip = &I;
+        leaf0 = !I.meta[0];
+        leaf1 = !I.meta[1];
+        np = I.np;
+        groups = max(0, min(GPW, ((np + 3) / 4 - warp + DW - 1) / DW));   // this warp's (warp-uniform)
+        w = make_row(a, I, own);
+        t0 = I.tab[0] + 4 * l;
+        t1 = I.tab[1] + 4 * l;
+        pitch0 = (unsigned)I.pitch[0];
+        pitch1 = (unsigned)I.pitch[1];
+        if (NCH) copy_rows();
+        raw = load_meta(I, own, w);
+    };
+    bool begun = false;
+    uint32_t use = 0;
+    for (int buf = 0;; buf = buf + 1 == NB ? 0 : buf + 1, ++use) {
+        if (!begun) {
+            if (!wait_warp(sh, &sh.ready[buf], (use / NB) & 1)) return;
+            if (sh.info[buf].stop) return;
+            begin(sh.info[buf]);
+        }
+        begun = false;
+        const Info& I = *Ip;
+        if (NCH) asm volatile("cp.async.wait_group 0;" ::: "memory");
         if (I.is_root) {
-            const int Rf_own = own < np ? I.Rf[own] : 0;
+            const RowMeta m = row_meta(a, I, w, raw);
+            const int64_t fam = own < np ? __ldg(a.perm + I.item0 + own) : 0;
+            const int Rf_own = own < np ? __ldg(a.item_R + I.item0 + own) : 0;
             const bool check_dead = I.sat && !a.err;
             Best mine{0.0f, 0.0f, 1 << 30};
             float my_s0 = 1.0f, my_s1 = 1.0f, my_max = 1.0f;
             int my_E = m.E;
             bool my_nflag = false;
 #pragma unroll 1
-            for (int i0 = 0; i0 < groups; i0 += BT) {
-            if (NCH && i0) load_groups(i0);
-#pragma unroll
-            for (int j = 0; j < BT; ++j) {
-                const int i = i0 + j;
-                if (i >= groups) continue;
+            for (int i = 0; i < groups; ++i) {
                 const int src = 4 * i + sub;
+                if (NCH) get_rows(i);
                 RootRow rr;
                 rr.s0 = rr.s1 = 1.0f;
                 rr.er0 = __shfl_sync(0xffffffffu, m.er0, src);
                 rr.er1 = __shfl_sync(0xffffffffu, m.er1, src);
                 rr.Rf = __shfl_sync(0xffffffffu, Rf_own, src);
-                const float* p0 = shfl_ptr(w.p0, src) + 4 * l;
-                const float* p1 = shfl_ptr(w.p1, src) + 4 * l;
-                Best best;
-                auto scan = [&]() {
-                    best = Best{0.0f, 0.0f, 1 << 30};
+                const float* p0 = row0(src);
+                const float* p1 = row1(src);
+                Best best{0.0f, 0.0f, 1 << 30};
 #pragma unroll(NCH ? NCH : 1)
-                    for (int c = 0; c < n_chunks; ++c)
-                        best_add4(best, rr, leaf0, leaf1, sh.prior_s, c * KC + 4 * l, NCH ? x[j][NCH ? c : 0] : load4(p0, c * KC),
-                                  NCH ? y[j][NCH ? c : 0] : load4b(I, p1, c * KC));
-                    best_reduce(best);
-                };
-                scan();
+                for (int c = 0; c < n_chunks; ++c)
+                    best_add4<false>(best, rr, leaf0, leaf1, sh.prior_s, c * KC + 4 * l,
+                                     NCH ? x[NCH ? c : 0] : load4(p0, c * KC), NCH ? y[NCH ? c : 0] : load4(p1, c * KC));
+                best_reduce(best);
                 const bool mine_now = (lane >> 2) == i;
                 if (check_dead) {
                     float mp = 0.0f;
                     for (int c = 0; c < n_chunks; ++c)
-                        mp = root_max4(mp, c * KC + 4 * l, rr.Rf, load4(p0, c * KC), load4b(I, p1, c * KC));
+                        mp = root_max4(mp, c * KC + 4 * l, rr.Rf, load4(p0, c * KC), load4(p1, c * KC));
                     mp = __shfl_sync(0xffffffffu, lane8_max(mp), from);
                     if (mine_now) my_max = mp;
                 }
@@ -756,14 +800,17 @@ __device__ void data(const PatTcArgs& a, Shared<NCH>& sh, float* stages, int tid
                     // the product underflows at every root row: the factors scaled apart
                     int maxe = -100000;
                     for (int c = 0; c < n_chunks; ++c)
-                        maxe = root_exp4(maxe, c * KC + 4 * l, rr.Rf, load4(p0, c * KC), load4b(I, p1, c * KC));
+                        maxe = root_exp4(maxe, c * KC + 4 * l, rr.Rf, load4(p0, c * KC), load4(p1, c * KC));
 #pragma unroll
                     for (int o = 1; o < 8; o <<= 1) maxe = max(maxe, __shfl_xor_sync(0xffffffffu, maxe, o));
                     Scale sc{1.0f, 1.0f, 1.0f, 0, need, false};
                     if (need) scale_apart(sc, maxe, 0);
                     rr.s0 = sc.s0;
                     rr.s1 = sc.s1;
-                    scan();
+                    best = Best{0.0f, 0.0f, 1 << 30};
+                    for (int c = 0; c < n_chunks; ++c)
+                        best_add4<true>(best, rr, leaf0, leaf1, sh.prior_s, c * KC + 4 * l, load4(p0, c * KC), load4(p1, c * KC));
+                    best_reduce(best);
                     const float t0 = __shfl_sync(0xffffffffu, sc.s0, from), t1 = __shfl_sync(0xffffffffu, sc.s1, from);
                     const int tE = __shfl_sync(0xffffffffu, sc.E, from), tn = __shfl_sync(0xffffffffu, (int)sc.nflag, from);
                     if (mine_now) {
@@ -777,15 +824,14 @@ __device__ void data(const PatTcArgs& a, Shared<NCH>& sh, float* stages, int tid
                 const int s = __shfl_sync(0xffffffffu, best.s, from);
                 if (mine_now) mine = Best{f, e, s};
             }
-            }
             if (own < np) {
-                const int64_t fam = I.fam[own];
                 const bool dead = (m.fl & kDead) || (check_dead && !(my_max > 0.0f));
                 bool flag = ((m.fl & kFlag) || my_nflag) && !dead;
                 double o = NAN;
                 float p = 0.0f, q = 0.0f;
                 if (mine.f > 0.0f) {
-                    p = (__ldcg(w.p0 + mine.s) * my_s0) * ((I.nch > 1 ? __ldcg(w.p1 + mine.s) : 1.0f) * my_s1);
+                    p = (__ldcg(I.tab[0] + (size_t)pitch0 * (unsigned)w.n0 + mine.s) * my_s0) *
+                        (__ldcg(I.tab[1] + (size_t)pitch1 * (unsigned)w.n1 + mine.s) * my_s1);
                     q = sh.prior_s[mine.s];
                 }
                 const double best = (double)p * (double)q;
@@ -809,9 +855,8 @@ __device__ void data(const PatTcArgs& a, Shared<NCH>& sh, float* stages, int tid
         // ---- rows: product, scaling, TF32 operands ----
         RowStat st;                    // of the row this lane owns
         stat_init(st);
+        st.maxp = 1.0f;
         Scale ms{1.0f, 1.0f, 1.0f, 0, false, false};
-        st.fmx0 = m.fm0;
-        st.fmx1 = I.nch > 1 ? m.fm1 : 1.0f;
         // the scales of group i's rows, from their statistics (warp-collective;
         // X, Y give a lane's columns of chunk c)
         auto scales = [&](int i, RowStat t, auto X, auto Y) {
@@ -829,6 +874,7 @@ __device__ void data(const PatTcArgs& a, Shared<NCH>& sh, float* stages, int tid
                 }
                 if (__any_sync(0xffffffffu, sc.need)) {
                     int maxe = -100000;
+                    #pragma unroll(NCH ? NCH : 1)
                     for (int c = 0; c < n_chunks; ++c) maxe = maxexp4(maxe, X(c), Y(c));
 #pragma unroll
                     for (int o = 1; o < 8; o <<= 1) maxe = max(maxe, __shfl_xor_sync(0xffffffffu, maxe, o));
@@ -854,53 +900,52 @@ __device__ void data(const PatTcArgs& a, Shared<NCH>& sh, float* stages, int tid
             }
         };
         if (NCH) {
-            // the last unit's stores have read the stages
-            if (gu && !wait_warp(sh, &sh.a_free, (gu - 1) & 1)) return;
-#pragma unroll 1
-            for (int i0 = 0; i0 < groups; i0 += BT) {
-            if (i0) load_groups(i0);
-#pragma unroll
-            for (int j = 0; j < BT; ++j) {
-                const int i = i0 + j;
-                if (i >= groups) continue;
+#pragma unroll 2
+            for (int i = 0; i < groups; ++i) {
+                get_rows(i);
                 const int r = 4 * (i * DW + warp) + sub;
                 float4 pr[VC];
                 RowStat t;
                 t.maxp = 0.0f;
 #pragma unroll
                 for (int c = 0; c < VC; ++c) {
-                    pr[c] = make_float4(x[j][c].x * y[j][c].x, x[j][c].y * y[j][c].y, x[j][c].z * y[j][c].z,
-                                        x[j][c].w * y[j][c].w);
+                    pr[c] = make_float4(x[c].x * y[c].x, x[c].y * y[c].y, x[c].z * y[c].z,
+                                        x[c].w * y[c].w);
                     t.maxp = fmaxf(t.maxp, max4(pr[c]));
                 }
-                t.maxp = lane8_max(t.maxp);
                 if (leaf0) {
-                    float mx = max4(x[j][0]), mn = min4(x[j][0]);
+                    float mx = max4(x[0]), mn = min4(x[0]);
 #pragma unroll
                     for (int c = 1; c < VC; ++c) {
-                        mx = fmaxf(mx, max4(x[j][c]));
-                        mn = fminf(mn, min4(x[j][c]));
+                        mx = fmaxf(mx, max4(x[c]));
+                        mn = fminf(mn, min4(x[c]));
                     }
                     leaf_stat(i, false, mx, mn);
                 }
                 if (leaf1) {
-                    float mx = max4(y[j][0]), mn = min4(y[j][0]);
+                    float mx = max4(y[0]), mn = min4(y[0]);
 #pragma unroll
                     for (int c = 1; c < VC; ++c) {
-                        mx = fmaxf(mx, max4(y[j][c]));
-                        mn = fminf(mn, min4(y[j][c]));
+                        mx = fmaxf(mx, max4(y[c]));
+                        mn = fminf(mn, min4(y[c]));
                     }
                     leaf_stat(i, true, mx, mn);
                 }
-                const Scale sc = scales(i, t, [&](int c) { return x[j][c]; }, [&](int c) { return y[j][c]; });
-                if (__any_sync(0xffffffffu, sc.s0 != 1.0f || sc.s1 != 1.0f || sc.post != 1.0f)) {
+                // rows whose maximum is at least 2^-32 keep their scale: one of a row's
+                // eight lanes saw it
+                unsigned big = __ballot_sync(0xffffffffu, t.maxp >= 0x1p-32f || r >= np);
+                big |= big >> 1;
+                big |= big >> 2;
+                big |= big >> 4;
+                if ((big & 0x01010101u) != 0x01010101u) {
+                    t.maxp = lane8_max(t.maxp);
+                    const Scale sc = scales(i, t, [&](int c) { return x[c]; }, [&](int c) { return y[c]; });
 #pragma unroll
-                    for (int c = 0; c < VC; ++c) pr[c] = scaled4(sc, x[j][c], y[j][c]);
+                    for (int c = 0; c < VC; ++c) pr[c] = scaled4(sc, x[c], y[c]);
                 }
 #pragma unroll
                 for (int c = 0; c < VC; ++c)
                     split_store(stages + (size_t)c * sf, stages + (size_t)c * sf + kChunkA, r, l, pr[c]);
-            }
             }
             tc::fence_proxy_async_shared();
             for (int c = 0; c < NCH; ++c) mbar_arrive(&sh.a_full[c]);
@@ -911,17 +956,17 @@ __device__ void data(const PatTcArgs& a, Shared<NCH>& sh, float* stages, int tid
             Scale sc[GPW];
 #pragma unroll
             for (int i = 0; i < GPW; ++i) {
-                q0[i] = shfl_ptr(w.p0, 4 * i + sub) + 4 * l;
-                q1[i] = shfl_ptr(w.p1, 4 * i + sub) + 4 * l;
+                q0[i] = row0(4 * i + sub);
+                q1[i] = row1(4 * i + sub);
                 if (i >= groups) continue;
                 RowStat t;
                 stat_init(t);
 #pragma unroll 4
-                for (int c = 0; c < n_chunks; ++c) stat_add4(t, load4(q0[i], c * KC), load4b(I, q1[i], c * KC));
+                for (int c = 0; c < n_chunks; ++c) stat_add4(t, load4(q0[i], c * KC), load4(q1[i], c * KC));
                 t.maxp = lane8_max(t.maxp);
                 leaf_stat(i, false, t.fmx0, t.fmn0);
                 leaf_stat(i, true, t.fmx1, t.fmn1);
-                sc[i] = scales(i, t, [&](int c) { return load4(q0[i], c * KC); }, [&](int c) { return load4b(I, q1[i], c * KC); });
+                sc[i] = scales(i, t, [&](int c) { return load4(q0[i], c * KC); }, [&](int c) { return load4(q1[i], c * KC); });
             }
             if (gu && !wait_warp(sh, &sh.a_free, (gu - 1) & 1)) return;
             for (int c = 0; c < n_chunks; ++c) {
@@ -932,7 +977,7 @@ __device__ void data(const PatTcArgs& a, Shared<NCH>& sh, float* stages, int tid
                 for (int i = 0; i < GPW; ++i) {
                     if (i >= groups) continue;
                     u[i] = load4(q0[i], c * KC);
-                    v[i] = load4b(I, q1[i], c * KC);
+                    v[i] = load4(q1[i], c * KC);
                 }
                 if (c >= NST && !wait_warp(sh, &sh.empty[stg], (cg / NST - 1) & 1)) return;
                 float* Ah = stages + (size_t)stg * sf;
@@ -948,41 +993,54 @@ __device__ void data(const PatTcArgs& a, Shared<NCH>& sh, float* stages, int tid
         }
         // the owned row's record
         if (I.meta_out && own < np) {
+            const RowMeta m = row_meta(a, I, w, raw);
             ms.E += m.E;
+            if (NCH && !leaf0) st.fmx0 = m.fm0;
+            if (NCH && !leaf1) st.fmx1 = I.nch > 1 ? m.fm1 : 1.0f;
             const bool dead = I.sat && !a.err && !(st.maxp > 0.0f);
             *reinterpret_cast<int2*>(I.meta_out + own) = row_record(I, m, st, ms, fused, dead);
         }
 
+        int4* const out = I.meta_out;
+        const int np_out = np;
+
         // ---- epilogue: factors from TMEM into the staging tiles ----
         // (a test hook can make this wait give up after limit - 1 polls)
-        if (!wait_warp(sh, &sh.mma, gu & 1, a.debug_wait_limit > 0 ? a.debug_wait_limit - 1 : kPolls)) {
+        if (!wait_warp(sh, &sh.mma, gu & 1, a.debug_wait_limit > 0 ? a.debug_wait_limit - 1 : kBarPolls)) {
             if (lane == 0) atomicCAS(a.status, 0, 2);
             return;
         }
         tc::fence_after();
-        if (32 * (warp & 3) < np) {
+        // the operand area is free: the next unit's rows, if its inputs are complete
+        const int nb = buf + 1 == NB ? 0 : buf + 1;
+        if (NCH && __all_sync(0xffffffffu, test_bar(&sh.ready[nb], ((use + 1) / NB) & 1)) && !sh.info[nb].stop) {
+            begin(sh.info[nb]);
+            begun = true;
+        }
+        if (32 * (warp & 3) < np_out) {
             const int row = 32 * (warp & 3) + lane;
             const uint32_t base = sh.tmem + ((uint32_t)(32 * (warp & 3)) << 16);
             for (int c = warp >> 2; c < a.Ns / KC; c += DW / 4) {
-                float v[32];
-                tc::tmem_ld32(base + (uint32_t)(c * KC), v);
-                if (NCH) {
+                float mx = 0.0f;
+                float* t = (NCH ? stages + (size_t)c * sf + 2 * kChunkA : stages + (size_t)c * kChunkA) + row * KC;
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    uint32_t v[16];
+                    tc::tmem_ld16(base + (uint32_t)(c * KC + 16 * h), v);
+#pragma unroll
+                    for (int q = 0; q < 16; ++q) mx = fmaxf(mx, __uint_as_float(v[q]));
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                        *reinterpret_cast<uint4*>(t + (((4 * h + q) ^ (row & 7)) << 2)) =
+                            make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+                }
+                if (NCH && row < np_out) {
                     // the factor row's largest value over these columns, for its readers'
                     // error bounds
-                    float mx = 0.0f;
-#pragma unroll
-                    for (int q = 0; q < 32; ++q) mx = fmaxf(mx, v[q]);
-                    if (row < np) {
-                        int* o = reinterpret_cast<int*>(I.meta_out + row) + 2;
-                        o[c] = __float_as_int(mx);
-                        if (NCH == 1) o[1] = 0;
-                    }
+                    int* o = reinterpret_cast<int*>(out + row) + 2;
+                    o[c] = __float_as_int(mx);
+                    if (NCH == 1) o[1] = 0;
                 }
-                float* t = stages + (size_t)c * kChunkA + row * KC;
-#pragma unroll
-                for (int q = 0; q < 8; ++q)
-                    *reinterpret_cast<float4*>(t + ((q ^ (row & 7)) << 2)) =
-                        make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
             }
         }
         tc::fence_before();
@@ -1001,14 +1059,17 @@ __global__ void __launch_bounds__(Shape<NCH>::kThreads, Shape<NCH>::kPerSm)
     __shared__ Shared<NCH> sh;
     constexpr int ND = Shape<NCH>::kData;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    for (int j = tid; j < (NCH ? NCH * KC : 512); j += ND + 32)
+    for (int j = tid; j < (NCH ? NCH * KC : 512); j += ND + 64)
         sh.prior_s[j] = j > 0 && j <= a.n_prior ? (float)a.prior[j - 1] : 0.0f;
-    for (int j = tid; j < min(a.n_segs, kSegSh); j += ND + 32) sh.seg0[j] = a.segs[j].unit0;
-    for (int j = tid; j < min(a.n_desc, kNodeSh); j += ND + 32) sh.nodes[j] = a.nodes[j];
-    if (warp == ND / 32) tc::tmem_alloc(&sh.tmem, (uint32_t)a.tmem_cols);
+    for (int j = tid; j < min(a.n_segs, kSegSh); j += ND + 64) sh.seg0[j] = a.segs[j].unit0;
+    for (int j = tid; j < min(a.n_desc, kNodeSh); j += ND + 64) sh.nodes[j] = a.nodes[j];
+    if (warp == ND / 32 + 1) tc::tmem_alloc(&sh.tmem, (uint32_t)a.tmem_cols);
     if (tid == 0) {
-        for (int q = 0; q < 2; ++q) {
+        for (int q = 0; q < NB; ++q) {
             tc::mbar_init(&sh.ready[q], 1);
+            tc::mbar_init(&sh.freed[q], 1);
+        }
+        for (int q = 0; q < 2; ++q) {
             tc::mbar_init(&sh.a_full[q], ND);
             tc::mbar_init(&sh.b_full[q], 1);
             tc::mbar_init(&sh.empty[q], 1);
@@ -1023,10 +1084,16 @@ __global__ void __launch_bounds__(Shape<NCH>::kThreads, Shape<NCH>::kPerSm)
     tc::fence_before();
     __syncthreads();
     tc::fence_after();
-    if (warp == ND / 32) control<NCH>(a, &map_mat, &map_vst, &map_vst32, sh, stages, lane);
-    else data<NCH>(a, sh, stages, tid);
+    if (warp == ND / 32) {
+        schedule<NCH>(a, sh, lane);
+    } else if (warp == ND / 32 + 1) {
+        if (lane == 0) issue<NCH>(a, &map_mat, &map_vst, &map_vst32, sh, stages);
+        __syncwarp();
+    } else {
+        data<NCH>(a, sh, stages, tid);
+    }
     __syncthreads();
-    if (warp == ND / 32) tc::tmem_dealloc(sh.tmem, (uint32_t)a.tmem_cols);
+    if (warp == ND / 32 + 1) tc::tmem_dealloc(sh.tmem, (uint32_t)a.tmem_cols);
 }
 
 template <int NCH>
@@ -1036,8 +1103,8 @@ cudaError_t init_one() {
 
 size_t dyn_smem(int W, int Ns) {
     const int stages = W == 32 ? 1 : 2;
-    // (the stages are also home of the epilogue's staging tiles)
-    return sizeof(float) * std::max<size_t>((size_t)stages * stage_floats(Ns), (size_t)(Ns / KC) * kChunkA) + 1024;
+    // (wide bins: the stages are also home of the epilogue's staging tiles)
+    return sizeof(float) * std::max<size_t>((size_t)stages * stage_floats(W, Ns), (size_t)(Ns / KC) * kChunkA) + 1024;
 }
 
 }  // namespace
@@ -1047,7 +1114,10 @@ size_t dyn_smem(int W, int Ns) {
 int pat_tc_states(int W) { return W <= 128 ? W : W == 192 ? 96 : 128; }
 
 cudaError_t pat_tc_init() {
-    cudaError_t e = init_one<0>();
+    float ones[512];
+    for (float& x : ones) x = 1.0f;
+    cudaError_t e = cudaMemcpyToSymbol(g_one_row, ones, sizeof ones);
+    if (e == cudaSuccess) e = init_one<0>();
     if (e == cudaSuccess) e = init_one<1>();
     return e == cudaSuccess ? init_one<2>() : e;
 }
