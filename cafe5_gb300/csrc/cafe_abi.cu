@@ -53,8 +53,10 @@ void MatCache::grow(size_t cap) {
     vals_.assign(cap, MatEntry());
     mask_ = cap - 1;
     n_ = 0;
+    const uint32_t was = epoch_;
+    epoch_ = 1;
     for (size_t i = 0; i < old_s.size(); ++i)
-        if (old_s[i].used) {
+        if (old_s[i].epoch == was) {
             auto r = try_emplace(old_s[i].key);
             *r.first = old_v[i];
         }
@@ -75,15 +77,15 @@ void MatCache::prefetch(const MatKey& k) const {
 MatEntry* MatCache::find(const MatKey& k) {
     if (slots_.empty()) return nullptr;
     for (size_t i = home(k);; i = (i + 1) & mask_) {
-        if (!slots_[i].used) return nullptr;
+        if (!used(i)) return nullptr;
         if (slots_[i].key == k) return &vals_[i];
     }
 }
 std::pair<MatEntry*, bool> MatCache::try_emplace(const MatKey& k) {
     if (2 * (n_ + 1) > slots_.size()) reserve(n_ + 1);
     for (size_t i = home(k);; i = (i + 1) & mask_) {
-        if (!slots_[i].used) {
-            slots_[i].used = true;
+        if (!used(i)) {
+            slots_[i].epoch = epoch_;
             slots_[i].key = k;
             vals_[i] = MatEntry();
             ++n_;
@@ -96,11 +98,11 @@ void MatCache::erase(const MatKey& k) {
     if (slots_.empty()) return;
     size_t i = home(k);
     for (;; i = (i + 1) & mask_) {
-        if (!slots_[i].used) return;
+        if (!used(i)) return;
         if (slots_[i].key == k) break;
     }
     // backward shift: pull later members of the probe run into the hole
-    for (size_t j = (i + 1) & mask_; slots_[j].used; j = (j + 1) & mask_) {
+    for (size_t j = (i + 1) & mask_; used(j); j = (j + 1) & mask_) {
         const size_t h = home(slots_[j].key);
         const bool movable = (i <= j) ? (h <= i || h > j) : (h <= i && h > j);
         if (movable) {
@@ -109,12 +111,15 @@ void MatCache::erase(const MatKey& k) {
             i = j;
         }
     }
-    slots_[i].used = false;
+    slots_[i].epoch = 0;
     --n_;
 }
 void MatCache::clear() {
     // keep the table's size (a reset cache refills to about the same size)
-    for (Slot& sl : slots_) sl.used = false;
+    if (++epoch_ == 0) {      // (after four billion of them, the slots' own epochs start over)
+        for (Slot& sl : slots_) sl.epoch = 0;
+        epoch_ = 1;
+    }
     n_ = 0;
 }
 
