@@ -969,11 +969,24 @@ struct PatGroup {
 // memory. -1 when not even eight fit (the tile walk k_prune64 takes such
 // vectors from global memory).
 int pat64_lp(int S) { return (S + 1 + 31) / 32 * 32 + 2; }
-int pat64_class(const PatGroup& q) {
+int pat64_class(const PatGroup& q, bool max_product = false) {
     const int lp = pat64_lp(q.S);
-    if (!pat64_bufs(lp, q.R)) return -1;
+    if (!pat64_bufs(lp, q.R, max_product)) return -1;
     return lp <= 66 ? 0 : lp <= 194 ? 1 : lp <= 514 ? 2 : 3;
 }
+
+// A max-product pass (one group): k_pat64's extra operands, and where the
+// argmax tables of its combinations went.
+struct MaxProduct {
+    const float* const* lmats = nullptr;
+    int lm_pitch = 0;
+    int64_t F = 0;
+    double* root_max = nullptr;
+    int32_t *root_arg = nullptr, *n_failed = nullptr;
+    std::vector<int64_t> ctab_off;   // [internal] entry of its first row
+    std::vector<int32_t> pitch;      // [internal]
+    int64_t ctab_stride = 0;         // from one combination's table to the next
+};
 
 // Prunes the plan's listed groups for every active combination (d_active:
 // their indices on the device) into out [F][K]. One launch per width class;
@@ -982,7 +995,7 @@ int pat64_class(const PatGroup& q) {
 // up; the caller zeroes it first.
 int launch_pat64_groups(cafe_ctx* C, Workspace& ws, const cafe_request* R, const TreeHost& T, const PatternPlan& P, const int64_t* d_perm, const int32_t* d_famR, const std::vector<PatGroup>& groups, int n_active,
                         const int32_t* d_active, int K, int msize, bool scaled, double* out, int32_t* d_status, bool fork,
-                        int prof_kind) {
+                        int prof_kind, MaxProduct* mx = nullptr) {
     constexpr int NC = Workspace::kPatClasses;
     const int ni = P.n_internal;
     struct Class {
@@ -994,7 +1007,7 @@ int launch_pat64_groups(cafe_ctx* C, Workspace& ws, const cafe_request* R, const
         size_t o_nodes = 0, o_cdesc = 0, o_done = 0;
     } cls[NC];
     for (const PatGroup& q : groups) {
-        const int c = pat64_class(q);
+        const int c = pat64_class(q, mx);
         if (c < 0) return fail(C, CAFE_ERR_INVALID, "vectors of %d states", q.S + 1);
         if (P.group_count[q.g] > 0) cls[c].groups.push_back(q);
     }
@@ -1008,7 +1021,7 @@ int launch_pat64_groups(cafe_ctx* C, Workspace& ws, const cafe_request* R, const
             X.lp = std::max(X.lp, pat64_lp(q.S));
             X.max_R = std::max(X.max_R, q.R);
         }
-        X.n_bufs = pat64_bufs(X.lp, X.max_R);
+        X.n_bufs = pat64_bufs(X.lp, X.max_R, mx);
         // State tiles of a unit: about 20,000 to 40,000 products where a tree
         // level has few units (1,000 families of 12 taxa at 171 states: 0.26 ms
         // with one tile, 0.38 with four), four tiles where it keeps 24 units per
@@ -1023,11 +1036,17 @@ int launch_pat64_groups(cafe_ctx* C, Workspace& ws, const cafe_request* R, const
         for (const PatGroup& q : X.groups) most = std::max(most, P.group_count[q.g]);
         if (most <= 4) X.s_run = 4;      // (such units put eight times the work on a lane)
         if (units1 * n_active >= (int64_t)24 * C->sm_count * levels) X.s_run = 4;
+        // Max-product: setting a vector up (logarithms) costs more than its
+        // tiles, so a unit takes four tiles, or 16 past the same line (10,000
+        // families of 24 taxa, K = 4, 85 states: 2.5 ms with one, 1.65 with
+        // four, 1.17 with 16; 200 families, K = 1, 221 states: 0.71 with four,
+        // 0.91 with 16)
+        if (mx) X.s_run = units1 * n_active >= (int64_t)24 * C->sm_count * levels ? 16 : 4;
         // nodes by height (children before parents, wide groups first); leaves
         // come first, a row per count
         std::stable_sort(X.groups.begin(), X.groups.end(), [](const PatGroup& a, const PatGroup& b) { return a.S > b.S; });
         const int nn = T.n_nodes;
-        const int half = R->use_error_model ? (C->err_ndev - 1) / 2 : 0;
+        const int half = R->use_error_model && !mx ? (C->err_ndev - 1) / 2 : 0;
         std::vector<int> at((size_t)X.groups.size() * nn, -1);
         auto add = [&](size_t gi, int v, int64_t rows, int64_t cidx) {
             const PatGroup& q = X.groups[gi];
@@ -1088,9 +1107,22 @@ int launch_pat64_groups(cafe_ctx* C, Workspace& ws, const cafe_request* R, const
         const int64_t fit = std::max<int64_t>(1, ((int64_t)2 << 30) / std::max<int64_t>(1, X.slot_doubles * 8));
         X.group = (int)std::min<int64_t>(X.group, fit);
         X.n_slots = (int)std::min<int64_t>(n_active, std::max<int64_t>(X.group, std::min<int64_t>(fit, 2 * X.group)));
+        if (mx) {
+            // the backtrack reads every combination's table
+            X.n_slots = n_active;
+            mx->ctab_stride = X.slot_doubles;
+            mx->ctab_off.assign(ni, 0);
+            mx->pitch.assign(ni, 0);
+            for (int ii = 0; ii < ni; ++ii) {
+                const Pat64Node& nd = X.nodes[at[T.internal[ii]]];
+                mx->ctab_off[ii] = nd.tab;
+                mx->pitch[ii] = nd.pitch;
+            }
+            CK(ws.rc_c.reserve((size_t)n_active * X.slot_doubles * sizeof(int32_t)), "argmax tables");
+        }
         X.n_ctas = (int)std::min<int64_t>((int64_t)X.units * n_active,
                                           (int64_t)C->sm_count *
-                                              pat64_ctas_per_sm(X.n_bufs * pat64_buf_doubles(X.lp, X.max_R) * sizeof(double)));
+                                              pat64_ctas_per_sm(X.n_bufs * pat64_buf_doubles(X.lp, X.max_R, mx) * sizeof(double), mx));
         CK(ws.pat_table[c].reserve((size_t)X.n_slots * X.slot_doubles * sizeof(double)), "factor tables");
         CK(ws.pat_expo[c].reserve((size_t)X.n_slots * X.slot_rows * sizeof(int32_t)), "factor tables");
         X.o_nodes = blob;
@@ -1128,16 +1160,25 @@ int launch_pat64_groups(cafe_ctx* C, Workspace& ws, const cafe_request* R, const
     a.ld_mat = msize;
     a.prior = C->d_prior.as<double>();
     a.n_prior = (int)C->prior.size();
-    a.err = R->use_error_model ? C->d_err.as<double>() : nullptr;
+    a.err = R->use_error_model && !mx ? C->d_err.as<double>() : nullptr;
     a.err_rows = C->err_rows;
     a.err_ndev = C->err_ndev;
+    if (mx) {
+        a.ctab = ws.rc_c.as<int32_t>();
+        a.lmats = mx->lmats;
+        a.lm_pitch = mx->lm_pitch;
+        a.F = mx->F;
+        a.root_max = mx->root_max;
+        a.root_arg = mx->root_arg;
+        a.n_failed = mx->n_failed;
+    }
     a.fam_R = d_famR;
     a.scaled = scaled ? 1 : 0;
     a.model = R->model == CAFE_MODEL_GAMMA ? 1 : 0;
     a.out = out;
     a.K = K;
     a.cat_probs = ws.catp.as<double>();
-    const bool prof = ws.sync;
+    const bool prof = ws.sync && !mx;
     cudaEvent_t ev;
     if (prof) {
         C->prof.begin(prof_kind, ws.stream, &ev);
@@ -1162,7 +1203,7 @@ int launch_pat64_groups(cafe_ctx* C, Workspace& ws, const cafe_request* R, const
         b.units = X.units;
         b.s_run = X.s_run;
         b.n_bufs = X.n_bufs;
-        b.buf_doubles = pat64_buf_doubles(X.lp, X.max_R);
+        b.buf_doubles = pat64_buf_doubles(X.lp, X.max_R, mx);
         b.group = X.group;
         b.n_slots = X.n_slots;
         b.slot_doubles = X.slot_doubles;
@@ -2180,6 +2221,103 @@ int recon_setup(cafe_ctx* C, Workspace& ws, const cafe_request* R, bool categori
     return CAFE_OK;
 }
 
+// Joint reconstruction over distinct rows: k_pat64's max-product units, then
+// the backtrack, as many categories at a time as keep their tables within 8 GB.
+// `words`: [0] counts the failed (category, family) pairs, [1] is set when a
+// bounded wait gave up, both zeroed.
+constexpr size_t kMaxProductBytes = (size_t)8 << 30;
+
+size_t max_product_bytes(const TreeHost& T, const PatternPlan& P, int S) {      // of a category
+    size_t n = 0;
+    for (size_t ii = 0; ii + 1 < T.internal.size(); ++ii) n += (size_t)P.row_count(0, (int)ii) * (S + 2);
+    return (n + (size_t)T.n_leaves * (S + 1) * (S + 2)) * (sizeof(double) + sizeof(int32_t));
+}
+
+int reconstruct_rows(cafe_ctx* C, Workspace& ws, const cafe_request* R, const ReconSetup& Z, int root_len, int32_t* words) {
+    const TreeHost& T = *Z.T;
+    const PatternPlan& P = Z.S->pat_all;
+    const int K = Z.K, n = T.n_nodes, ni = (int)T.internal.size(), n_st = Z.Smax + 1;
+    const int64_t F = Z.S->F;
+    // log2 of the internal branches' matrices, rows of 128-byte chunks
+    const int pitch = (n_st + 31) / 32 * 32;
+    const size_t per = ((size_t)n_st * (pitch + pitch / 32) + 31) & ~(size_t)31;
+    const int n_int = ni - 1;
+    CK(ws.rc_lm.reserve(std::max<size_t>((size_t)K * n_int * per, 1) * sizeof(float)), "log2 matrices");
+    // pointers: log2 matrices by (category, node), sources, destinations; then
+    // the category numbers, the nodes' post-order indices, the child lists
+    std::vector<const void*> ptr((size_t)K * n, nullptr), src, dst;
+    const double* const* hmats = ws.h_mats.as<const double*>();
+    for (int k = 0; k < K; ++k)
+        for (int ii = 0; ii < n_int; ++ii) {
+            const size_t kv = (size_t)k * n + T.internal[ii];
+            ptr[kv] = ws.rc_lm.as<float>() + src.size() * per;
+            src.push_back(hmats[kv]);
+            dst.push_back(ptr[kv]);
+        }
+    ptr.insert(ptr.end(), src.begin(), src.end());
+    ptr.insert(ptr.end(), dst.begin(), dst.end());
+    std::vector<int32_t> ints(K);
+    std::iota(ints.begin(), ints.end(), 0);
+    ints.insert(ints.end(), T.internal_index.begin(), T.internal_index.end());
+    const size_t o_long = ptr.size() * sizeof(void*);
+    const size_t o_int = o_long + 2 * (size_t)ni * sizeof(int64_t);
+    const size_t bytes = o_int + (ints.size() + ni) * sizeof(int32_t);
+    CK(ws.rc_lptr.reserve(bytes), "log2 matrices");
+    char* d = ws.rc_lptr.as<char>();
+    const void* const* dptr = reinterpret_cast<const void* const*>(d);
+    const int32_t* d_ints = reinterpret_cast<const int32_t*>(d + o_int);
+    CK(cudaMemcpyAsync(d, ptr.data(), o_long, cudaMemcpyHostToDevice, ws.stream), "h2d");
+    CK(cudaMemcpyAsync(d + o_int, ints.data(), ints.size() * sizeof(int32_t), cudaMemcpyHostToDevice, ws.stream), "h2d");
+    CK(cudaMemcpyAsync(d + o_long, P.child_off.data(), ni * sizeof(int64_t), cudaMemcpyHostToDevice, ws.stream), "h2d");
+    CK(launch_log2_rows(reinterpret_cast<const double* const*>(dptr + (size_t)K * n),
+                        reinterpret_cast<float* const*>(const_cast<void**>(dptr + (size_t)K * n + src.size())),
+                        (int)src.size(), n_st, Z.msize, pitch, ws.stream),
+       "log2 matrices");
+    const int pass = (int)std::min<size_t>(K, std::max<size_t>(1, kMaxProductBytes / max_product_bytes(T, P, Z.Smax)));
+    CK(ws.rc_arg.reserve((size_t)K * F * sizeof(int32_t)), "root states");
+    CK(ws.rc_row.reserve((size_t)pass * F * ni * sizeof(int32_t)), "rows");
+    MaxProduct mx;
+    mx.lmats = reinterpret_cast<const float* const*>(dptr);
+    mx.lm_pitch = pitch;
+    mx.F = F;
+    mx.root_max = ws.rc_rmax.as<double>();
+    mx.root_arg = ws.rc_arg.as<int32_t>();
+    mx.n_failed = words;
+    const std::vector<PatGroup> group{{0, Z.Smax, root_len - 1}};
+    for (int k0 = 0; k0 < K; k0 += pass) {
+        const int nk = std::min(pass, K - k0);
+        if (k0) CK(cudaStreamSynchronize(ws.stream), "reconstruct");     // (the staging buffers are read)
+        int rc = launch_pat64_groups(C, ws, R, T, P, Z.S->d_identity.as<int64_t>(), nullptr, group, nk, d_ints + k0, K,
+                                     Z.msize, false, nullptr, words + 1, false, 0, &mx);
+        if (rc) return rc;
+        if (!k0) {
+            CK(cudaMemcpyAsync(d + o_long + ni * sizeof(int64_t), mx.ctab_off.data(), ni * sizeof(int64_t),
+                               cudaMemcpyHostToDevice, ws.stream), "h2d");
+            CK(cudaMemcpyAsync(d + o_int + ints.size() * sizeof(int32_t), mx.pitch.data(), ni * sizeof(int32_t),
+                               cudaMemcpyHostToDevice, ws.stream), "h2d");
+        }
+        BacktrackArgs b;
+        std::memset(&b, 0, sizeof b);
+        b.plan = T.plan;
+        b.node_ii = d_ints + K;
+        b.child_off = reinterpret_cast<const int64_t*>(d + o_long);
+        b.child = P.d_child.as<int32_t>();
+        b.ctab_off = b.child_off + ni;
+        b.pitch = d_ints + ints.size();
+        b.ctab = ws.rc_c.as<int32_t>();
+        b.ctab_stride = mx.ctab_stride;
+        b.root_arg = ws.rc_arg.as<int32_t>();
+        b.status = words + 1;
+        b.F = F;
+        b.k0 = k0;
+        b.n_k = nk;
+        b.row = ws.rc_row.as<int32_t>();
+        b.state = ws.rc_state.as<int32_t>();
+        CK(launch_backtrack(b, ws.stream), "backtrack");
+    }
+    return CAFE_OK;
+}
+
 int reconstruct_sync(cafe_ctx* C, Workspace& ws, const cafe_request* R, cafe_reconstruction* out) {
     AllocScope scope(ws.stream);
     if (ws.staged) {   // the previous request's copies out of the pinned staging buffers
@@ -2195,9 +2333,14 @@ int reconstruct_sync(cafe_ctx* C, Workspace& ws, const cafe_request* R, cafe_rec
     TreeHost& T = *Z.T;
     const int64_t F = Z.S->F;
     const int K = Z.K, n = T.n_nodes;
+    const int root_len = std::min(Z.Smax, Z.Rmax) + 1;
+    // over distinct rows unless the caller wants every product formed, or a
+    // vector does not fit a CTA or a category's tables 8 GB (then the tile walk)
+    const bool by_rows = F > 0 && !out->exhaustive && pat64_class({0, Z.Smax, root_len - 1}, true) >= 0 &&
+                         max_product_bytes(T, Z.S->pat_all, Z.Smax) <= kMaxProductBytes;
     std::vector<PruneTile>& tiles = ws.tile_vec;
     tiles.clear();
-    for (int k = 0; k < K; ++k)
+    for (int k = 0; k < K && !by_rows; ++k)
         for (int64_t f = 0; f < F; f += 32) {
             PruneTile t{};
             t.first = (int)f;
@@ -2211,27 +2354,29 @@ int reconstruct_sync(cafe_ctx* C, Workspace& ws, const cafe_request* R, cafe_rec
     const size_t c_per_cta = pupko_c_entries(T.plan, Z.Smax);
     CK(ws.h_tiles.reserve(std::max(n_tiles, 1) * sizeof(PruneTile)), "tiles");
     CK(ws.tiles.reserve(std::max(n_tiles, 1) * sizeof(PruneTile)), "tiles");
-    CK(ws.scratch.reserve((size_t)n_ctas * per_cta * sizeof(double)), "scratch");
-    CK(ws.rc_c.reserve(std::max<size_t>((size_t)n_ctas * c_per_cta, 1) * sizeof(int32_t)), "argmax tables");
+    if (!by_rows) {
+        CK(ws.scratch.reserve((size_t)n_ctas * per_cta * sizeof(double)), "scratch");
+        CK(ws.rc_c.reserve(std::max<size_t>((size_t)n_ctas * c_per_cta, 1) * sizeof(int32_t)), "argmax tables");
+    }
     const size_t n_state = (size_t)K * F * n, n_fam = (size_t)F * n;
     CK(ws.rc_state.reserve(std::max<size_t>(n_state, 1) * sizeof(int32_t)), "states");
     CK(ws.rc_rmax.reserve(std::max<size_t>((size_t)K * F, 1) * sizeof(double)), "root max");
     CK(ws.rc_mean.reserve(std::max<size_t>(n_fam, 1) * sizeof(double)), "means");
     CK(ws.rc_count.reserve(std::max<size_t>(n_fam, 1) * sizeof(int32_t)), "counts");
-    CK(ws.rc_nfail.reserve(sizeof(int32_t)), "failed");
+    CK(ws.rc_nfail.reserve(2 * sizeof(int32_t)), "failed");
     std::memcpy(ws.h_tiles.p, tiles.data(), n_tiles * sizeof(PruneTile));
     CK(cudaMemcpyAsync(ws.tiles.p, ws.h_tiles.p, n_tiles * sizeof(PruneTile), cudaMemcpyHostToDevice, ws.stream),
        "tiles");
-    CK(cudaMemsetAsync(ws.rc_nfail.p, 0, sizeof(int32_t), ws.stream), "failed");
+    CK(cudaMemsetAsync(ws.rc_nfail.p, 0, 2 * sizeof(int32_t), ws.stream), "failed");
     if (Z.gamma) {
         rc = stage_cat_probs(C, ws, R, K, 1);
         if (rc) return rc;
     }
-    // transposed log2 of every internal non-root node's matrix (pass 1 of k_pupko)
+    // the tile walk reads the transposed log2 of every internal non-root node's matrix
     const int nstate = Z.Smax + 1;
     std::vector<const void*> lsrc, ldst;
     std::vector<const float*> lmats((size_t)K * n, nullptr);
-    {
+    if (!by_rows) {
         int n_int = 0;
         for (int v = 0; v < n; ++v) n_int += (T.parent[v] >= 0 && T.leaf_col[v] < 0);
         const size_t per = (size_t)nstate * nstate;
@@ -2268,7 +2413,7 @@ int reconstruct_sync(cafe_ctx* C, Workspace& ws, const cafe_request* R, cafe_rec
     a.prior = C->d_prior.as<double>();
     a.n_prior = (int)C->prior.size();
     a.S = Z.Smax;
-    a.root_len = std::min(Z.Smax, Z.Rmax) + 1;
+    a.root_len = root_len;
     a.scratch = ws.scratch.as<double>();
     a.scratch_per_cta = (int64_t)per_cta;
     a.cscratch = ws.rc_c.as<int32_t>();
@@ -2277,20 +2422,25 @@ int reconstruct_sync(cafe_ctx* C, Workspace& ws, const cafe_request* R, cafe_rec
     a.root_max = ws.rc_rmax.as<double>();
     a.n_failed = ws.rc_nfail.as<int32_t>();
     a.exhaustive = out->exhaustive ? 1 : 0;
-    if (F > 0) {
+    if (by_rows) {
+        rc = reconstruct_rows(C, ws, R, Z, root_len, ws.rc_nfail.as<int32_t>());
+        if (rc) return rc;
+    } else if (F > 0) {
         CK(launch_log2_matrices(reinterpret_cast<const double* const*>(dptr + lmats.size()),
                                 reinterpret_cast<float* const*>(const_cast<void**>(dptr + lmats.size() + lsrc.size())),
                                 (int)lsrc.size(), nstate, Z.msize, ws.stream),
            "log2 matrices");
         CK(launch_pupko(a, n_ctas, ws.stream), "reconstruct");
+    }
+    if (F > 0) {
         CK(launch_recon_counts(ws.rc_state.as<int32_t>(), F, n, K, Z.gamma ? ws.catp.as<double>() : nullptr,
                                Z.gamma ? 1 : 0, T.plan.leaf_col, ws.rc_mean.as<double>(), ws.rc_count.as<int32_t>(),
                                ws.stream),
            "node counts");
     }
     CK(cudaEventRecord(ws.ev_stop, ws.stream), "event");
-    int32_t nf = 0;
-    CK(cudaMemcpyAsync(&nf, ws.rc_nfail.p, sizeof(int32_t), cudaMemcpyDeviceToHost, ws.stream), "d2h");
+    int32_t words[2] = {0, 0};
+    CK(cudaMemcpyAsync(words, ws.rc_nfail.p, sizeof words, cudaMemcpyDeviceToHost, ws.stream), "d2h");
     if (F > 0) {
         if (out->node_count)
             CK(cudaMemcpyAsync(out->node_count, ws.rc_count.p, n_fam * sizeof(int32_t), cudaMemcpyDeviceToHost, ws.stream),
@@ -2311,7 +2461,8 @@ int reconstruct_sync(cafe_ctx* C, Workspace& ws, const cafe_request* R, cafe_rec
     float ms = 0;
     cudaEventElapsedTime(&ms, ws.ev_start, ws.ev_stop);
     out->device_ms = ms;
-    out->n_failed = nf;
+    out->n_failed = words[0];
+    if (words[1]) return fail(C, CAFE_ERR_TIMEOUT, "reconstruction gave up waiting for a subtree");
     return CAFE_OK;
 }
 

@@ -121,6 +121,16 @@ struct Pat64Args {
     int s_run;                   // state tiles of a unit
     int n_bufs;                  // vector buffers of a CTA
     int64_t buf_doubles;
+    // max-product (ctab not null): the argmax of every factor, laid out like
+    // table; FP32 log2 of each matrix [S + 1][lm_pitch] and its chunk maxima
+    // (launch_log2_rows); the families' root values and states
+    int32_t* ctab;
+    const float* const* lmats;   // [K][n_nodes], null at leaves and the root
+    int lm_pitch;
+    int64_t F;
+    double* root_max;            // [K][F]
+    int32_t* root_arg;           // [K][F]
+    int32_t* n_failed;           // families with root value 0
     const int32_t* active;       // [n_active] combined (candidate, category) indices
     int n_active;
     int group;                   // combinations interleaved unit by unit
@@ -151,11 +161,11 @@ constexpr int kPat64Rows = 8;       // rows of any other
 constexpr int kPat64States = 16;    // states of a state tile
 // lp: pitch of the longest vectors in shared memory (whole 32-state chunks,
 // plus 2)
-int pat64_bufs(int lp, int max_R);
-int64_t pat64_buf_doubles(int lp, int max_R);
+int pat64_bufs(int lp, int max_R, bool max_product = false);
+int64_t pat64_buf_doubles(int lp, int max_R, bool max_product = false);
 cudaError_t pat64_init();
 cudaError_t launch_pat64(const Pat64Args& a, int n_ctas, cudaStream_t s);
-int pat64_ctas_per_sm(size_t smem);
+int pat64_ctas_per_sm(size_t smem, bool max_product = false);
 
 struct Prune64Args {
     TreePlan plan;
@@ -409,6 +419,29 @@ struct PupkoArgs {
 cudaError_t launch_pupko(const PupkoArgs& a, int n_ctas, cudaStream_t s);
 cudaError_t launch_log2_matrices(const double* const* src, float* const* dst, int n_mats, int n, int ld,
                                  cudaStream_t s);
+// log2 of each matrix's first n x n block, row-major with pitch `pitch` (-inf
+// past n), then the largest of every 32 columns [n][pitch / 32]
+cudaError_t launch_log2_rows(const double* const* src, float* const* dst, int n_mats, int n, int ld, int pitch,
+                             cudaStream_t s);
+// Every family's states from the root's (parents before children): a node's row
+// among its distinct patterns follows from its parent's.
+struct BacktrackArgs {
+    TreePlan plan;
+    const int32_t* node_ii;      // [n_nodes] post-order index of an internal node, -1 for leaves
+    const int64_t* child_off;    // [n_internal] first child index of a node
+    const int32_t* child;        // child indices (a leaf's: the count)
+    const int64_t* ctab_off;     // [n_internal] first entry of a node's argmax table
+    const int32_t* pitch;        // [n_internal] its row pitch
+    const int32_t* ctab;         // of category k0, the next ones ctab_stride further
+    int64_t ctab_stride;
+    const int32_t* root_arg;     // [K][F]
+    const int32_t* status;       // nonzero: the tables are incomplete
+    int64_t F;
+    int k0, n_k;                 // categories k0 .. k0 + n_k - 1
+    int32_t* row;                // [n_k][F][n_internal] scratch
+    int32_t* state;              // [K][F][n_nodes] out
+};
+cudaError_t launch_backtrack(const BacktrackArgs& a, cudaStream_t s);
 size_t pupko_scratch_doubles(const TreePlan& P, int S);
 size_t pupko_c_entries(const TreePlan& P, int S);
 cudaError_t launch_recon_counts(const int32_t* state, int64_t F, int n_nodes, int K, const double* cat_probs,

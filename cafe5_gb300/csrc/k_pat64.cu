@@ -266,12 +266,35 @@ struct Unit {
     NodeSrcs src;
     double* tab;
     int32_t* expo;
+    int32_t* ctab;        // max-product: argmax table, laid out like tab
     const double* M;      // the branch's matrix (null at the root)
     int q, k, di, p0, t0, t1, is_root, stop;
 };
 
+// Max-product: where a buffer keeps the FP32 logarithms of its vectors.
+struct LogRows {
+    float* lu;     // [TP][pitch] log2 u, -inf past the states
+    int pitch;     // rows 16 bytes apart modulo 128
+    float* cm;     // [TP][chunks] its largest value in each chunk
+    int* peak;     // [TP] where it is largest
+};
+__host__ __device__ inline size_t log_rows_doubles(int nchunk) {
+    return ((size_t)TP * (nchunk * KC + 4) + (size_t)TP * nchunk + TP + 1) / 2;
+}
+__device__ __forceinline__ LogRows log_rows(double* Ls, int nchunk) {
+    LogRows r;
+    r.lu = reinterpret_cast<float*>(Ls + (size_t)TP * (nchunk * KC + 2));
+    r.pitch = nchunk * KC + 4;
+    r.cm = r.lu + (size_t)TP * r.pitch;
+    r.peak = reinterpret_cast<int*>(r.cm + (size_t)TP * nchunk);
+    return r;
+}
+
 // The unit's eight vectors, four lanes per row: 32 states (16 loads a lane)
 // in flight before the first product.
+// Max-product: also their log2 in FP32, its largest value per chunk, and where
+// it is largest.
+template <bool MX>
 __device__ __forceinline__ void fill_rows(const Pat64Args& a, const Unit& u, double* Ls, int* lmax, int idx_pack,
                                           int lane) {
     const Pat64Node& nd = u.nd;
@@ -283,6 +306,9 @@ __device__ __forceinline__ void fill_rows(const Pat64Args& a, const Unit& u, dou
     const bool two = u.src.nch == 2;
     double* L = Ls + (size_t)r * lp;
     double mx = 0.0;
+    const LogRows lr = log_rows(Ls, nchunk);
+    float top = -INFINITY;
+    int top_j = 0;
     for (int ck = 0; ck < nchunk; ++ck) {
         const int j0 = ck * KC + l;
         double x[8];
@@ -303,6 +329,25 @@ __device__ __forceinline__ void fill_rows(const Pat64Args& a, const Unit& u, dou
                 x[i] = j <= S ? product(a, nd, u.src, rs, u.tab, u.expo, j) : 0.0;
             }
         }
+        if (MX) {
+            float cm = -INFINITY;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int j = j0 + 4 * i;
+                L[j] = x[i];
+                const float lu = j <= S ? flog2(x[i]) : -INFINITY;
+                lr.lu[r * lr.pitch + j] = lu;
+                cm = fmaxf(cm, lu);
+                if (lu > top) {
+                    top = lu;
+                    top_j = j;
+                }
+            }
+            cm = fmaxf(cm, __shfl_xor_sync(0xffffffffu, cm, 1));
+            cm = fmaxf(cm, __shfl_xor_sync(0xffffffffu, cm, 2));
+            if (l == 0) lr.cm[r * nchunk + ck] = cm;
+            continue;
+        }
         int m = 0;
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
@@ -314,6 +359,19 @@ __device__ __forceinline__ void fill_rows(const Pat64Args& a, const Unit& u, dou
             m = __reduce_max_sync(0xffffffffu, m);
             if (lane == 0) lmax[ck] = m;
         }
+    }
+    if (MX) {
+#pragma unroll
+        for (int o = 1; o < 4; o <<= 1) {
+            const float t = __shfl_xor_sync(0xffffffffu, top, o);
+            const int j = __shfl_xor_sync(0xffffffffu, top_j, o);
+            if (t > top) {
+                top = t;
+                top_j = j;
+            }
+        }
+        if (l == 0) lr.peak[r] = top_j;
+        return;
     }
     if (!a.scaled) return;
     unsigned long long mb = (unsigned long long)__double_as_longlong(mx);
@@ -342,6 +400,7 @@ __device__ __forceinline__ void fill_rows(const Pat64Args& a, const Unit& u, dou
 }
 
 // The producer warp: units into the buffers in turn.
+template <bool MX>
 __device__ void produce(const Pat64Args& a, Unit* units, double* Ls, size_t buf_doubles, int (*lmax)[kMaxChunks],
                         const int* unit0_sh, int lane) {
     const long long total = (long long)a.units * a.n_active;
@@ -381,6 +440,7 @@ __device__ void produce(const Pat64Args& a, Unit* units, double* Ls, size_t buf_
                 u.nd = nd;
                 u.tab = tab;
                 u.expo = expo;
+                u.ctab = MX ? a.ctab + (size_t)slot * a.slot_doubles : nullptr;
                 u.M = is_root ? nullptr : mats[v];
                 u.q = q;
                 u.k = k;
@@ -409,7 +469,7 @@ __device__ void produce(const Pat64Args& a, Unit* units, double* Ls, size_t buf_
                 w = wait_count(a.done + (size_t)(q - a.n_slots) * a.n_desc + nd.root, a.nodes[nd.root].n_units, a.status);
             ok = __all_sync(0xffffffffu, w);
             __syncwarp();      // what one lane waited for, every lane reads
-            if (ok && !is_root && nch > 0) fill_rows(a, u, Ls + b * buf_doubles, lmax[b], pack, lane);
+            if (ok && !is_root && nch > 0) fill_rows<MX>(a, u, Ls + b * buf_doubles, lmax[b], pack, lane);
             if (!ok && lane == 0) atomicExch(a.status, 1);
         }
         if (!ok && lane == 0) u.stop = 1;
@@ -482,17 +542,165 @@ __device__ __forceinline__ void few_rows(const Pat64Args& a, const Unit& u, cons
     }
 }
 
+// ---- max-product (Pupko joint reconstruction): L[i] = max_j u[j] M[i][j] and
+// the first j attaining it, in FP64, as k_pupko defines it: the products are
+// ranked by FP32 logarithms (each p = log2 u + log2 M within 5e-4 of exact),
+// and only those within kDelta of the best are formed in FP64.
+//
+// A chunk of 32 columns is left out for a (row, state) whose best so far is
+// kDelta above the sum of the chunk's largest log2 u and largest log2 M: no
+// product in it can be the maximum. "Best so far" starts from the products at
+// the row's peak and at j = i, so most rows look at one or two chunks.
+//
+// What bounds it is the producer warp, which forms a vector's logarithms; a
+// unit therefore runs over up to 16 state tiles. Measured (device time of the
+// whole call, every family walking every node in 32-family tiles before):
+// 10,000 families of 24 taxa, K = 4, 85 states 20.0 -> 1.2 ms.
+constexpr float kDelta = 0.00390625f;   // 2^-8, in log2 units
+
+// FP64 over the candidate child states, ascending: one queued (row, state) per
+// lane.
+__device__ __forceinline__ void slow_rows(const Pat64Args& a, const Unit& u, const double* Lb, const LogRows& lr,
+                                          const float* lm, const float* cmM, int nchunk, const int* pair,
+                                          const float* best, int count, int lane) {
+    if (lane < count) {
+        const int S = u.nd.S, lp = nchunk * KC + 2;
+        const int r = pair[lane] & 7, i = pair[lane] >> 3;
+        const float b1 = best[lane], thr = b1 - kDelta;
+        const bool all = !(b1 > -INFINITY);
+        const double* Mi = u.M + (size_t)i * a.ld_mat;
+        double mx = -1.0;
+        int arg = 0;
+        for (int c = 0; c < nchunk; ++c) {
+            if (!all && !(lr.cm[r * nchunk + c] + cmM[(size_t)i * nchunk + c] >= thr)) continue;
+            for (int j = c * KC; j < min(c * KC + KC, S + 1); ++j) {
+                if (!all && !(lr.lu[r * lr.pitch + j] + lm[(size_t)i * a.lm_pitch + j] >= thr)) continue;
+                const double val = Lb[(size_t)r * lp + j] * __ldg(Mi + j);
+                if (val > mx) {
+                    mx = val;
+                    arg = j;
+                }
+            }
+        }
+        const int64_t at = u.nd.tab + (int64_t)(u.p0 + r) * u.nd.pitch + i;
+        u.tab[at] = mx;
+        u.ctab[at] = arg;
+    }
+    __syncwarp();
+}
+
+__device__ __forceinline__ void max_rows(const Pat64Args& a, const Unit& u, double* Lb, int* pair, float* slow, int warp,
+                                         int lane) {
+    const int pl = lane & 7, sl = lane >> 3;
+    const int S = u.nd.S, s_cnt = u.nd.s_cnt, nchunk = S / KC + 1, lp = nchunk * KC + 2;
+    const int np = min(TP, u.nd.rows - u.p0);
+    const LogRows lr = log_rows(Lb, nchunk);
+    const float* lm = a.lmats[(size_t)u.k * a.plan.n_nodes + u.nd.node];     // [S + 1][lm_pitch]
+    const float* cmM = lm + (size_t)(S + 1) * a.lm_pitch;                    // [S + 1][nchunk]
+    const float* LU = lr.lu + pl * lr.pitch;
+    int queued = 0;
+    for (int t = u.t0; t < u.t1; ++t) {
+        if (t * TS + warp * 4 >= s_cnt) break;
+        const int i = t * TS + warp * 4 + sl;
+        const int ic = min(i, s_cnt - 1);
+        const float* LM = lm + (size_t)ic * a.lm_pitch;
+        const float* CM = cmM + (size_t)ic * nchunk;
+        const int pk = lr.peak[pl];
+        // a product's logarithm: no more than the best one's
+        const float floor_b = fmaxf(LU[pk] + __ldg(LM + pk), LU[ic] + __ldg(LM + ic));
+        float b1 = -INFINITY, b2 = -INFINITY;
+        int j1 = 0;
+        for (int c = 0; c < nchunk; ++c) {
+            const bool look = lr.cm[pl * nchunk + c] + __ldg(CM + c) >= fmaxf(floor_b, b1) - kDelta;
+            if (!__any_sync(0xffffffffu, look)) continue;
+#pragma unroll
+            for (int q = 0; q < KC; q += 4) {
+                const float4 x = *reinterpret_cast<const float4*>(LU + c * KC + q);
+                const float4 y = __ldg(reinterpret_cast<const float4*>(LM + c * KC + q));
+                const float p[4] = {x.x + y.x, x.y + y.y, x.z + y.z, x.w + y.w};
+#pragma unroll
+                for (int h = 0; h < 4; ++h) {
+                    j1 = p[h] > b1 ? c * KC + q + h : j1;
+                    b2 = fmaxf(b2, fminf(b1, p[h]));
+                    b1 = fmaxf(b1, p[h]);
+                }
+            }
+        }
+        const bool valid = pl < np && i < s_cnt;
+        const bool zero = !(b1 >= -1075.0f - kDelta);      // every product rounds to 0
+        const bool near_sub = b1 < -1022.0f + kDelta;
+        const bool fast = !near_sub && b2 < b1 - kDelta;   // only j1 can reach the FP64 maximum
+        if (valid && (zero || fast)) {
+            const int64_t at = u.nd.tab + (int64_t)(u.p0 + pl) * u.nd.pitch + i;
+            u.tab[at] = fast ? Lb[(size_t)pl * lp + j1] * __ldg(u.M + (size_t)i * a.ld_mat + j1) : 0.0;
+            u.ctab[at] = fast ? j1 : 0;
+        }
+        // the rest (near-ties, rows near the subnormal range) are queued and
+        // scanned a warp at a time
+        const bool slow_it = valid && !zero && !fast;
+        const unsigned m = __ballot_sync(0xffffffffu, slow_it);
+        if (slow_it) {
+            const int at = queued + __popc(m & ((1u << lane) - 1u));
+            pair[at] = pl | i << 3;
+            slow[at] = near_sub ? -INFINITY : b1;
+        }
+        queued += __popc(m);
+        __syncwarp();
+        if (queued >= 32) {
+            slow_rows(a, u, Lb, lr, lm, cmM, nchunk, pair + queued - 32, slow + queued - 32, 32, lane);
+            queued -= 32;
+        }
+    }
+    slow_rows(a, u, Lb, lr, lm, cmM, nchunk, pair, slow, queued, lane);
+}
+
+// reconstruct_root_node (src/gene_family_reconstructor.cpp:47-78): the first
+// root size j in 1..R with the largest prod_children L[j] * prior(j).
+__device__ __forceinline__ void root_argmax(const Pat64Args& a, const Pat64Node& nd, const NodeSrcs& ns, const double* tab,
+                                            const int32_t* expo, int k, int row, int lane) {
+    const int32_t* ci = a.child + nd.cidx + (int64_t)row * ns.nch;
+    const RowSrc rs = row_src(a, nd, ns, row, __ldg(ci), ns.nch > 1 ? __ldg(ci + 1) : 0);
+    double best = -1.0;
+    int arg = 0;
+#pragma unroll 2
+    for (int j = 1 + lane; j <= nd.R; j += 32) {
+        const double val = product(a, nd, ns, rs, tab, expo, j) * (j < a.n_prior ? a.prior[j] : 0.0);
+        if (val > best) {
+            best = val;
+            arg = j;
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const double b = __shfl_xor_sync(0xffffffffu, best, o);
+        const int j = __shfl_xor_sync(0xffffffffu, arg, o);
+        if (b > best || (b == best && j < arg)) {
+            best = b;
+            arg = j;
+        }
+    }
+    if (lane == 0) {
+        const int64_t f = a.perm[nd.perm0 + row];
+        a.root_max[(size_t)k * a.F + f] = best;
+        a.root_arg[(size_t)k * a.F + f] = arg;
+        if (!(best > 0.0)) atomicAdd(a.n_failed, 1);
+    }
+}
+
 // Four compute warps along the states of a tile: lanes 8 rows x 4 states.
+template <bool MX>
 __global__ void __launch_bounds__(NTHR, 6) k_pat64(const Pat64Args a) {
     extern __shared__ __align__(16) double Ls[];   // [n_bufs][buf_doubles]: [TP][lp] (root units: [4][R])
     __shared__ int lmax[2][kMaxChunks];            // largest L of each chunk (hi_key)
     __shared__ Unit units[2];
     __shared__ int unit0_sh[kDescSh];              // first units of the nodes
+    __shared__ int slow_pair[MX ? NT / 32 : 1][64];
+    __shared__ float slow_best[MX ? NT / 32 : 1][64];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     for (int i = tid; i < min(a.n_desc, kDescSh); i += NTHR) unit0_sh[i] = a.nodes[i].unit0;
     __syncthreads();
     if (warp == NT / 32) {
-        produce(a, units, Ls, a.buf_doubles, lmax, unit0_sh, lane);
+        produce<MX>(a, units, Ls, a.buf_doubles, lmax, unit0_sh, lane);
         return;
     }
     const int pl = lane & 7, sl = lane >> 3;
@@ -502,7 +710,12 @@ __global__ void __launch_bounds__(NTHR, 6) k_pat64(const Pat64Args a) {
         const Unit& u = units[buf];
         if (u.stop) return;
         const double* Lb = Ls + buf * a.buf_doubles;
-        if (u.is_root) {
+        if (MX && u.is_root) {
+            for (int i = warp; i < kPat64RootRows && u.p0 + i < u.nd.rows; i += NT / 32)
+                root_argmax(a, u.nd, u.src, u.tab, u.expo, u.k, u.p0 + i, lane);
+        } else if (MX && u.src.nch > 0) {
+            max_rows(a, u, Ls + buf * a.buf_doubles, slow_pair[warp], slow_best[warp], warp, lane);
+        } else if (u.is_root) {
             double* x = Ls + buf * a.buf_doubles + (size_t)warp * u.nd.R;
             for (int i = warp; i < kPat64RootRows && u.p0 + i < u.nd.rows; i += NT / 32)
                 root_family(a, u.nd, u.src, u.tab, u.expo, u.k, u.p0 + i, x, lane);
@@ -590,27 +803,35 @@ __global__ void __launch_bounds__(NTHR, 6) k_pat64(const Pat64Args a) {
 }
 
 // Doubles of one vector buffer.
-size_t buf_doubles(int lp, int max_R) { return ((std::max<size_t>((size_t)TP * lp, (size_t)(NT / 32) * max_R)) + 1) & ~(size_t)1; }
+size_t buf_doubles(int lp, int max_R, bool max_product) {
+    const size_t n = max_product ? (size_t)TP * lp + log_rows_doubles((lp - 2) / KC)
+                                 : std::max<size_t>((size_t)TP * lp, (size_t)(NT / 32) * max_R);
+    return (n + 1) & ~(size_t)1;
+}
 
 constexpr int kMaxDynSmem = 200 * 1024;
 
 }  // namespace
 
 // Vector buffers of a launch (two where they fit), 0 when not even one does.
-int pat64_bufs(int lp, int max_R) {
+int pat64_bufs(int lp, int max_R, bool max_product) {
     if (lp - 2 > kMaxChunks * KC) return 0;
-    const size_t n = buf_doubles(lp, max_R) * sizeof(double);
+    const size_t n = buf_doubles(lp, max_R, max_product) * sizeof(double);
     return 2 * n <= (size_t)kMaxDynSmem ? 2 : n <= (size_t)kMaxDynSmem ? 1 : 0;
 }
-int64_t pat64_buf_doubles(int lp, int max_R) { return (int64_t)buf_doubles(lp, max_R); }
+int64_t pat64_buf_doubles(int lp, int max_R, bool max_product) { return (int64_t)buf_doubles(lp, max_R, max_product); }
 
 cudaError_t pat64_init() {
-    return cudaFuncSetAttribute(k_pat64, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem);
+    const cudaError_t e = cudaFuncSetAttribute(k_pat64<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(k_pat64<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem);
 }
 
-int pat64_ctas_per_sm(size_t smem) {
+int pat64_ctas_per_sm(size_t smem, bool max_product) {
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_pat64, NTHR, smem) != cudaSuccess) {
+    const cudaError_t e = max_product ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_pat64<true>, NTHR, smem)
+                                      : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_pat64<false>, NTHR, smem);
+    if (e != cudaSuccess) {
         cudaGetLastError();
         return 1;
     }
@@ -619,7 +840,9 @@ int pat64_ctas_per_sm(size_t smem) {
 
 cudaError_t launch_pat64(const Pat64Args& a, int n_ctas, cudaStream_t s) {
     if (a.units <= 0 || a.n_active <= 0) return cudaSuccess;
-    k_pat64<<<n_ctas, NTHR, (size_t)a.n_bufs * a.buf_doubles * sizeof(double), s>>>(a);
+    const size_t smem = (size_t)a.n_bufs * a.buf_doubles * sizeof(double);
+    if (a.ctab) k_pat64<true><<<n_ctas, NTHR, smem, s>>>(a);
+    else k_pat64<false><<<n_ctas, NTHR, smem, s>>>(a);
     return cudaGetLastError();
 }
 

@@ -31,6 +31,12 @@
 //                               j with p_j >= b1 - delta (every j when b1 is
 //                               near the subnormal range), ascending, with
 //                               the reference's strict '>'
+// k_pat64's max-product units do this once per distinct subtree pattern, with
+// the same ranking and the same bits; k_backtrack then walks every family down
+// through the argmax tables (10,000 families of 24 taxa, K = 4, 85 states:
+// 20.0 ms with k_pupko's tiles, which form every family's products at every
+// node, 1.2 so). k_pupko keeps the requests whose vectors do not fit a CTA's
+// shared memory or whose tables pass 8 GB, and the exhaustive ones.
 // `exhaustive` sends every (row, family) through the FP64 scan of every j:
 // the plain reference arithmetic, used to check the ranking.
 #include "common.cuh"
@@ -337,7 +343,69 @@ __global__ void k_log2_matrices(const double* const* __restrict__ src, float* co
     }
 }
 
+// Row-major log2 of the first n x n block of each matrix and the largest value
+// of every 32 columns: one warp per (row, chunk).
+__global__ void k_log2_rows(const double* const* __restrict__ src, float* const* __restrict__ dst, int n, int ld,
+                            int pitch) {
+    const double* M = src[blockIdx.y];
+    float* out = dst[blockIdx.y];
+    const int lane = threadIdx.x & 31, chunks = pitch / 32;
+    const int total = n * chunks, step = gridDim.x * (blockDim.x >> 5);
+    for (int e = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); e < total; e += step) {
+        const int i = e / chunks, c = e % chunks, j = 32 * c + lane;
+        float v = j < n ? flog2(M[(size_t)i * ld + j]) : -INFINITY;
+        out[(size_t)i * pitch + j] = v;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+        if (lane == 0) out[(size_t)n * pitch + (size_t)i * chunks + c] = v;
+    }
+}
+
+__global__ void k_backtrack(BacktrackArgs a) {
+    const TreePlan& P = a.plan;
+    const int64_t total = *a.status ? 0 : a.F * a.n_k;
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
+        const int kk = (int)(e / a.F), k = a.k0 + kk;
+        const int64_t f = e % a.F;
+        const int32_t* C = a.ctab + (size_t)kk * a.ctab_stride;
+        int32_t* out = a.state + ((size_t)k * a.F + f) * P.n_nodes;
+        int32_t* row = a.row + (size_t)e * P.n_internal;
+        out[P.root] = a.root_arg[(size_t)k * a.F + f];
+        row[P.n_internal - 1] = (int32_t)f;      // (the root keeps a row per family)
+        for (int ii = P.n_internal - 1; ii >= 0; --ii) {
+            const int c0 = P.cstart[ii], nch = P.cstart[ii + 1] - c0;
+            const int s = out[P.internal[ii]];
+            const int32_t* ci = a.child + a.child_off[ii] + (int64_t)row[ii] * nch;
+            for (int c = 0; c < nch; ++c) {
+                const int ch = P.child[c0 + c];
+                const int idx = ci[c], cii = a.node_ii[ch];
+                if (cii < 0) {
+                    out[ch] = idx;               // a leaf keeps its observed count
+                } else {
+                    row[cii] = idx;
+                    out[ch] = C[a.ctab_off[cii] + (int64_t)idx * a.pitch[cii] + s];
+                }
+            }
+        }
+    }
+}
+
 }  // namespace
+
+cudaError_t launch_log2_rows(const double* const* src, float* const* dst, int n_mats, int n, int ld, int pitch,
+                             cudaStream_t s) {
+    if (n_mats <= 0 || n <= 0) return cudaSuccess;
+    const int bx = (int)std::min<int64_t>(((int64_t)n * (pitch / 32) + 7) / 8, 64);
+    k_log2_rows<<<dim3(bx, n_mats), 256, 0, s>>>(src, dst, n, ld, pitch);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_backtrack(const BacktrackArgs& a, cudaStream_t s) {
+    const int64_t total = a.F * a.n_k;
+    if (total <= 0) return cudaSuccess;
+    k_backtrack<<<(unsigned)std::min<int64_t>((total + 127) / 128, 8192), 128, 0, s>>>(a);
+    return cudaGetLastError();
+}
 
 cudaError_t launch_log2_matrices(const double* const* src, float* const* dst, int n_mats, int n, int ld,
                                  cudaStream_t s) {

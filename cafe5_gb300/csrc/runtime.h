@@ -195,7 +195,8 @@ struct Workspace {
     DevBuf tcp_table[kMaxGroups], tcp_meta[kMaxGroups], tcp_desc, tcp_ctr;
     PinnedBuf h_tcp_desc;
     // reconstruction
-    DevBuf rc_c, rc_state, rc_rmax, rc_mean, rc_count, rc_nfail, rc_parent, rc_bp, rc_lm, rc_lptr;
+    DevBuf rc_c, rc_state, rc_rmax, rc_mean, rc_count, rc_nfail, rc_parent, rc_bp, rc_lm, rc_lptr,
+        rc_arg, rc_row;
     PinnedBuf h_sim, h_simperm;        // p-values: simulated families staged for the device
     std::vector<PruneTile> tile_vec;
     std::vector<MatEntry*> entry_vec;   // cache entry of every (combined category, node)

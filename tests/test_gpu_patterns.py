@@ -93,3 +93,33 @@ def test_fp64_binned_tables_are_reused_across_combinations(ctx):
                           cat_probs=w.cat_probs)
         assert np.array_equal(alone.family_lnl, got[b].family_lnl) and alone.total == got[b].total
     ctx.free_families(sid)
+
+
+@pytest.mark.parametrize("newick", [BINARY, POLY, "(A:1.0,B:2.0);"], ids=["binary", "polytomy", "root only"])
+@pytest.mark.parametrize("F,distinct,hi,S,R", [
+    (1, 1, 3, 15, 10),
+    (7, 7, 5, 16, 40),        # root sizes past the states
+    (9, 9, 9, 30, 20),        # 31 states
+    (33, 20, 12, 31, 31),     # a whole chunk
+    (65, 40, 12, 32, 5),      # a chunk and one column over
+    (300, 120, 60, 130, 100),
+    (17, 17, 200, 511, 300),  # sixteen chunks
+])
+@pytest.mark.parametrize("lam", [0.01, 1e-9])     # (the second: most products are subnormal or zero)
+def test_reconstruction_rows(ctx, newick, F, distinct, hi, S, R, lam):
+    """Joint reconstruction over distinct rows against the walk that forms every
+    product in FP64: the same bits and states."""
+    from cafe5_gb300.inputs import RootPrior
+    from cafe5_gb300.tree import parse_newick
+    tree = parse_newick(newick)
+    c = _counts(np.random.default_rng([F, S]), F, len(tree.leaves), min(hi, S), distinct)
+    tid = ctx.upload_tree(tree)
+    sid = ctx.upload_families(tid, c)
+    ctx.set_prior(RootPrior.uniform(R).vector())
+    kw = dict(S=S, R=R, model=1, multipliers=[0.3, 0.9, 2.0], cat_probs=[0.2, 0.5, 0.3])
+    a, b = ctx.reconstruct(tid, sid, [lam], **kw), ctx.reconstruct(tid, sid, [lam], exhaustive=True, **kw)
+    for x, y in ((a.category_state, b.category_state), (a.node_count, b.node_count), (a.node_mean, b.node_mean),
+                 (a.root_max, b.root_max)):
+        assert np.array_equal(x, y)
+    assert a.n_failed == b.n_failed
+    ctx.free_families(sid)
