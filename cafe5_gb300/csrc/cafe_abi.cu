@@ -458,6 +458,7 @@ int build_patterns(cafe_ctx* C, const TreeHost& T, FamSet& S, const int64_t* d_p
     const size_t batch = std::max<size_t>(1, std::min(widest, ((size_t)1 << 30) / (slots * sizeof(int32_t))));
     std::vector<int32_t> ints = T.internal_index;
     for (auto& l : level) ints.insert(ints.end(), l.begin(), l.end());
+    ints.push_back(ni - 1);
     TempBuf d_ints(st), d_rep(st), d_num(st), d_base(st), d_tab(st), d_off(st);
     CK(d_ints.get(ints.size() * sizeof(int32_t)), "patterns");
     CK(d_rep.get((size_t)ni * F * sizeof(int32_t)), "patterns");
@@ -474,13 +475,22 @@ int build_patterns(cafe_ctx* C, const TreeHost& T, FamSet& S, const int64_t* d_p
     a.F = F;
     a.n_groups = ng;
     int64_t n_flags = 0;
+    std::vector<int64_t> longs(first);            // the groups' first items, F; their first flags
+    longs.push_back(F);
+    std::vector<int64_t> flag_off;
     for (int g = 0; g < ng; ++g) {
-        a.group_first[g] = first[g];
-        a.group_max[g] = max_count[g];
-        a.flag_off[g] = n_flags;
+        flag_off.push_back(n_flags);
         n_flags += (int64_t)T.n_leaves * (max_count[g] + 1);
     }
-    TempBuf d_flags(st);
+    longs.insert(longs.end(), flag_off.begin(), flag_off.end());
+    TempBuf d_flags(st), d_longs(st), d_max(st);
+    CK(d_longs.get(longs.size() * sizeof(int64_t)), "patterns");
+    CK(d_max.get(ng * sizeof(int32_t)), "patterns");
+    CK(cudaMemcpyAsync(d_longs.p, longs.data(), longs.size() * sizeof(int64_t), cudaMemcpyHostToDevice, st), "patterns");
+    CK(cudaMemcpyAsync(d_max.p, max_count.data(), ng * sizeof(int32_t), cudaMemcpyHostToDevice, st), "patterns");
+    a.group_first = d_longs.as<int64_t>();
+    a.flag_off = a.group_first + ng + 1;
+    a.group_max = d_max.as<int32_t>();
     CK(d_flags.get((size_t)n_flags), "patterns");
     CK(cudaMemsetAsync(d_flags.p, 0, (size_t)n_flags, st), "patterns");
     CK(launch_pat_counts(a, d_flags.as<uint8_t>(), st), "patterns");
@@ -494,7 +504,7 @@ int build_patterns(cafe_ctx* C, const TreeHost& T, FamSet& S, const int64_t* d_p
                "patterns");
         d_nodes += l.size();
     }
-    CK(launch_pat_number(a, st), "patterns");
+    CK(launch_pat_number(a, d_ints.as<int32_t>() + T.n_nodes, ni - 1, st), "patterns");
     std::vector<int32_t> base((size_t)ni * (ng + 1));
     std::vector<uint8_t> flags((size_t)n_flags);
     CK(cudaMemcpyAsync(flags.data(), d_flags.p, flags.size(), cudaMemcpyDeviceToHost, st), "patterns");
@@ -518,14 +528,14 @@ int build_patterns(cafe_ctx* C, const TreeHost& T, FamSet& S, const int64_t* d_p
     for (int g = 0; g < ng; ++g)
         for (int c = 0; c < T.n_leaves; ++c) {
             P.leaf_off.push_back((int64_t)used.size());
-            const uint8_t* f = flags.data() + a.flag_off[g] + (size_t)c * (max_count[g] + 1);
+            const uint8_t* f = flags.data() + flag_off[g] + (size_t)c * (max_count[g] + 1);
             for (int n = 0; n <= max_count[g]; ++n)
                 if (f[n]) used.push_back(n);
         }
     P.leaf_off.push_back((int64_t)used.size());
     CK(P.d_counts.reserve(used.size() * sizeof(int32_t)), "patterns");
     CK(cudaMemcpyAsync(P.d_counts.p, used.data(), used.size() * sizeof(int32_t), cudaMemcpyHostToDevice, st), "patterns");
-    CK(launch_pat_write(a, d_off.as<int64_t>(), P.d_child.as<int32_t>(), st), "patterns");
+    CK(launch_pat_write(a, d_ints.as<int32_t>() + T.n_nodes, ni, d_off.as<int64_t>(), P.d_child.as<int32_t>(), st), "patterns");
     CK(cudaStreamSynchronize(st), "patterns");
     return CAFE_OK;
 }
@@ -2548,6 +2558,226 @@ int host_sampler_init(cafe_ctx* C, Workspace& ws, const cafe_request* R, const T
 
 // ---- p-values
 
+// The simulated families' root values over distinct rows: families of equal
+// state bound (the groups m = 0..S; slots first[m] ..) share the rows of every
+// internal node below the root's children; those children's factors are needed
+// at one state only, the family's root size (k_sim_root). Returns through
+// `done` whether it ran: vectors that do not fit a CTA's shared memory and
+// groups whose tables pass 16 GB are left to the tile walk.
+constexpr size_t kSimTableBytes = (size_t)16 << 30;
+
+int prune_simulated(cafe_ctx* C, Workspace& ws, const TreeHost& T, int S, int RR, int msize, int64_t NS,
+                    const int32_t* d_counts, const int32_t* d_keys, const int64_t* d_perm, const int64_t* d_first,
+                    double* d_out, int32_t* d_status, bool* done) {
+    *done = false;
+    if (pat64_class({0, S, 1}) < 0 || NS > INT32_MAX) return CAFE_OK;
+    const int ni = (int)T.internal.size(), n = T.n_nodes, ng = S + 1;
+    const cudaStream_t st = ws.stream;
+    // the nodes with rows, by height: all but the root and its children
+    std::vector<std::vector<int32_t>> level;
+    size_t widest = 1;
+    int n_dd = 0;
+    for (int ii = 0; ii + 1 < ni; ++ii) {
+        const int v = T.internal[ii], h = T.height[ii];
+        if (T.parent[v] == T.root) continue;
+        if ((int)level.size() <= h) level.resize(h + 1);
+        level[h].push_back(ii);
+        widest = std::max(widest, level[h].size());
+        ++n_dd;
+    }
+    int64_t slots = 1024;
+    while (slots < 2 * NS) slots *= 2;
+    const size_t batch = std::max<size_t>(1, std::min(widest, ((size_t)1 << 30) / (slots * sizeof(int32_t))));
+    std::vector<int32_t> ints = T.internal_index;
+    for (auto& l : level) ints.insert(ints.end(), l.begin(), l.end());
+    // every count may occur at a leaf
+    const size_t o_list = ints.size();
+    for (int c = 0; c <= S; ++c) ints.push_back(c);
+    TempBuf d_ints(st), d_rep(st), d_num(st), d_base(st), d_tab(st), d_off(st), d_child(st), d_table(st), d_desc(st);
+    CK(d_ints.get(ints.size() * sizeof(int32_t)), "patterns");
+    CK(d_rep.get((size_t)ni * NS * sizeof(int32_t)), "patterns");
+    CK(d_num.get((size_t)ni * NS * sizeof(int32_t)), "patterns");
+    CK(d_base.get((size_t)ni * (ng + 1) * sizeof(int32_t)), "patterns");
+    CK(d_tab.get(batch * slots * sizeof(int32_t)), "patterns");
+    CK(cudaMemcpyAsync(d_ints.p, ints.data(), ints.size() * sizeof(int32_t), cudaMemcpyHostToDevice, st), "patterns");
+    PatBuildArgs a;
+    std::memset(&a, 0, sizeof a);
+    a.plan = T.plan;
+    a.counts = d_counts;
+    a.perm = d_perm;
+    a.node_ii = d_ints.as<int32_t>();
+    a.F = NS;
+    a.n_groups = ng;
+    a.group_first = d_first;
+    a.rep = d_rep.as<int32_t>();
+    a.num = d_num.as<int32_t>();
+    a.base = d_base.as<int32_t>();
+    const int32_t* d_dd = d_ints.as<int32_t>() + n;
+    const int32_t* d_nodes = d_dd;
+    for (auto& l : level) {
+        for (size_t b = 0; b < l.size(); b += batch)
+            CK(launch_pat_insert(a, d_nodes + b, (int)std::min(batch, l.size() - b), d_tab.as<int32_t>(), slots, st),
+               "patterns");
+        d_nodes += l.size();
+    }
+    CK(launch_pat_number(a, d_dd, n_dd, st), "patterns");
+    std::vector<int32_t> base((size_t)ni * (ng + 1));
+    std::vector<int64_t> first(ng + 1);
+    CK(cudaMemcpyAsync(base.data(), d_base.p, base.size() * sizeof(int32_t), cudaMemcpyDeviceToHost, st), "patterns");
+    CK(cudaMemcpyAsync(first.data(), d_first, first.size() * sizeof(int64_t), cudaMemcpyDeviceToHost, st), "patterns");
+    CK(cudaStreamSynchronize(st), "patterns");
+    // child lists, and the groups of each pass (tables within the limit)
+    auto rows = [&](int g, int ii) { return (int64_t)base[(size_t)ii * (ng + 1) + g + 1] - base[(size_t)ii * (ng + 1) + g]; };
+    std::vector<int64_t> child_off((size_t)ng * ni, 0), group_doubles(ng, 0);
+    int64_t n_child = 0;
+    const int leaf_pitch = (S + 2) & ~1;
+    const int64_t leaf_doubles = (int64_t)T.n_leaves * (S + 1) * leaf_pitch;
+    const int64_t limit = (int64_t)(kSimTableBytes / sizeof(double)) - leaf_doubles;
+    for (int g = 0; g < ng; ++g) {
+        for (auto& l : level)
+            for (int ii : l) {
+                child_off[(size_t)g * ni + ii] = n_child;
+                n_child += rows(g, ii) * (T.cstart[ii + 1] - T.cstart[ii]);
+                group_doubles[g] += rows(g, ii) * ((g + 2) & ~1);
+            }
+        if (group_doubles[g] > limit) return CAFE_OK;
+    }
+    CK(d_child.get(n_child * sizeof(int32_t)), "patterns");
+    CK(d_off.get(child_off.size() * sizeof(int64_t)), "patterns");
+    CK(cudaMemcpyAsync(d_off.p, child_off.data(), child_off.size() * sizeof(int64_t), cudaMemcpyHostToDevice, st),
+       "patterns");
+    CK(launch_pat_write(a, d_dd, n_dd, d_off.as<int64_t>(), d_child.as<int32_t>(), st), "patterns");
+    struct Pass {
+        int g0, g1;
+        int64_t doubles;
+    };
+    std::vector<Pass> passes;
+    int64_t most = 0;
+    for (int g = 0; g < ng; ++g) {
+        if (passes.empty() || passes.back().doubles + group_doubles[g] > limit) passes.push_back({g, g, 0});
+        passes.back().g1 = g + 1;
+        passes.back().doubles += group_doubles[g];
+        most = std::max(most, passes.back().doubles);
+    }
+    CK(d_table.get((leaf_doubles + most) * sizeof(double)), "factor tables");
+    const int TP = kPat64Rows, TS = kPat64States;
+    const int lp = pat64_lp(S), n_bufs = pat64_bufs(lp, 1);
+    const int32_t active0 = 0;
+    for (const Pass& q : passes) {
+        // leaves first (a row per count, for every group), then by height
+        std::vector<Pat64Node> nodes;
+        std::vector<int32_t> cdesc;
+        std::vector<int32_t> at((size_t)ng * n, -1);
+        std::vector<int64_t> tab((size_t)ng * n, 0);
+        int units = 0;
+        int64_t doubles = 0;
+        const int s_run = 4;
+        auto add = [&](int g, int v, int64_t n_rows, int bound, int64_t cidx) {
+            Pat64Node nd;
+            std::memset(&nd, 0, sizeof nd);
+            nd.tab = doubles;
+            nd.cidx = cidx;
+            nd.rows = (int32_t)n_rows;
+            nd.node = v;
+            nd.nch = (int32_t)T.children[v].size();
+            nd.n_list = nd.nch ? 0 : (int32_t)n_rows;
+            nd.S = bound;
+            nd.s_cnt = bound + 1;
+            nd.pitch = (bound + 2) & ~1;
+            nd.s_tiles = nd.nch ? ((nd.s_cnt + TS - 1) / TS + s_run - 1) / s_run : 1;
+            nd.unit0 = units;
+            nd.n_units = (nd.rows + TP - 1) / TP * nd.s_tiles;
+            nd.child0 = (int32_t)cdesc.size();
+            for (int c : T.children[v]) cdesc.push_back(at[(size_t)g * n + c]);
+            nd.root = -1;
+            doubles += n_rows * nd.pitch;
+            units += nd.n_units;
+            nodes.push_back(nd);
+        };
+        for (int v = 0; v < n; ++v) {
+            if (T.leaf_col[v] < 0 || T.parent[v] == T.root) continue;
+            for (int g = q.g0; g < q.g1; ++g) {
+                at[(size_t)g * n + v] = (int)nodes.size();
+                tab[(size_t)g * n + v] = doubles;
+            }
+            add(q.g0, v, S + 1, S, 0);
+        }
+        for (auto& l : level)
+            for (int g = q.g1 - 1; g >= q.g0; --g)
+                for (int ii : l) {
+                    if (!rows(g, ii)) continue;
+                    const int v = T.internal[ii];
+                    at[(size_t)g * n + v] = (int)nodes.size();
+                    tab[(size_t)g * n + v] = doubles;
+                    add(g, v, rows(g, ii), g, child_off[(size_t)g * ni + ii]);
+                }
+        if (first[q.g1] == first[q.g0]) continue;
+        const size_t o_tab = nodes.size() * sizeof(Pat64Node);
+        const size_t o_cdesc = o_tab + tab.size() * sizeof(int64_t);
+        const size_t o_active = o_cdesc + cdesc.size() * sizeof(int32_t);
+        const size_t o_done = (o_active + sizeof(int32_t) + 15) & ~(size_t)15;       // the counter, then the finished units
+        const size_t bytes = o_done + sizeof(unsigned long long) + nodes.size() * sizeof(int32_t);
+        std::vector<char> blob(o_done, 0);
+        if (!nodes.empty()) std::memcpy(blob.data(), nodes.data(), o_tab);
+        std::memcpy(blob.data() + o_tab, tab.data(), tab.size() * sizeof(int64_t));
+        if (!cdesc.empty()) std::memcpy(blob.data() + o_cdesc, cdesc.data(), cdesc.size() * sizeof(int32_t));
+        std::memcpy(blob.data() + o_active, &active0, sizeof active0);
+        TempBuf d_blob(st);
+        CK(d_blob.get(bytes), "pattern nodes");
+        char* d = d_blob.as<char>();
+        CK(cudaMemcpyAsync(d, blob.data(), o_done, cudaMemcpyHostToDevice, st), "pattern nodes");
+        CK(cudaMemsetAsync(d + o_done, 0, bytes - o_done, st), "pattern nodes");
+        Pat64Args b;
+        std::memset(&b, 0, sizeof b);
+        b.plan = T.plan;
+        b.nodes = reinterpret_cast<const Pat64Node*>(d);
+        b.cdesc = reinterpret_cast<const int32_t*>(d + o_cdesc);
+        b.n_desc = (int)nodes.size();
+        b.units = units;
+        b.s_run = s_run;
+        b.n_bufs = n_bufs;
+        b.buf_doubles = pat64_buf_doubles(lp, 1);
+        b.active = reinterpret_cast<const int32_t*>(d + o_active);
+        b.n_active = b.group = b.n_slots = 1;
+        b.slot_doubles = doubles;
+        b.table = d_table.as<double>();
+        b.done = reinterpret_cast<int32_t*>(d + o_done + sizeof(unsigned long long));
+        b.next = reinterpret_cast<unsigned long long*>(d + o_done);
+        b.status = d_status;
+        b.child = d_child.as<int32_t>();
+        b.leaf_counts = d_ints.as<int32_t>() + o_list;
+        b.mats = ws.mats.as<const double*>();
+        b.ld_mat = msize;
+        const size_t smem = (size_t)n_bufs * b.buf_doubles * sizeof(double);
+        if (units) CK(launch_pat64(b, (int)std::min<int64_t>(units, (int64_t)C->sm_count * pat64_ctas_per_sm(smem)), st),
+                      "prune simulated families");
+        SimRootArgs r;
+        std::memset(&r, 0, sizeof r);
+        r.plan = T.plan;
+        r.node_ii = d_ints.as<int32_t>();
+        r.keys = d_keys;
+        r.R = RR;
+        r.counts = d_counts;
+        r.perm = d_perm;
+        r.i0 = first[q.g0];
+        r.i1 = first[q.g1];
+        r.F = NS;
+        r.n_groups = ng;
+        r.rep = a.rep;
+        r.num = a.num;
+        r.base = a.base;
+        r.tab = reinterpret_cast<const int64_t*>(d + o_tab);
+        r.table = d_table.as<double>();
+        r.leaf_pitch = leaf_pitch;
+        r.mats = ws.mats.as<const double*>();
+        r.ld_mat = msize;
+        r.out = d_out;
+        CK(launch_sim_root(r, st), "root values");
+    }
+    *done = true;
+    return CAFE_OK;
+}
+
 // compute_pvalues with the simulated families drawn on the GPU (k_pvalue.cu:
 // a counter-based generator, one thread per family; the same distributions
 // as the reference's draws, not its stream). Every step runs on the device:
@@ -2574,7 +2804,7 @@ int pvalues_device(cafe_ctx* C, Workspace& ws, const cafe_request* R, cafe_pvalu
     const int64_t max_tiles = NS / 32 + n_keys + 1;
     const int Wmax = std::max(S + 1, RR);
     DevBuf d_cdf, d_sizes, d_sim, d_keys, d_hist, d_cursor, d_perm, d_tiles, d_ntiles, d_simL, d_obsL, d_pv, d_tree,
-        d_otiles;
+        d_otiles, d_first;
     CK(d_cdf.reserve((size_t)n * n_ps * S * sizeof(double)), "row cdfs");
     CK(d_sizes.reserve((size_t)NS * n * sizeof(int32_t)), "simulated families");
     CK(d_sim.reserve(std::max<size_t>((size_t)NS * L, 1) * sizeof(int32_t)), "simulated families");
@@ -2584,6 +2814,7 @@ int pvalues_device(cafe_ctx* C, Workspace& ws, const cafe_request* R, cafe_pvalu
     CK(d_perm.reserve((size_t)NS * sizeof(int64_t)), "simulation plan");
     CK(d_tiles.reserve((size_t)max_tiles * sizeof(PruneTile)), "tiles");
     CK(d_ntiles.reserve(16), "tiles");
+    CK(d_first.reserve((size_t)(S + 2) * sizeof(int64_t)), "simulation plan");
     CK(d_simL.reserve((size_t)NS * sizeof(double)), "simulated likelihoods");
     CK(d_obsL.reserve(std::max<size_t>((size_t)F * RR, 1) * sizeof(double)), "root vectors");
     CK(d_pv.reserve(std::max<size_t>((size_t)F, 1) * sizeof(double)), "p-values");
@@ -2650,6 +2881,7 @@ int pvalues_device(cafe_ctx* C, Workspace& ws, const cafe_request* R, cafe_pvalu
     sd.S = S;
     sd.n_sim = nsim;
     sd.n_families = NS;
+    sd.R = RR;
     sd.key = sim_seed_key(out->seed);
     sd.sizes = d_sizes.as<int32_t>();
     sd.counts = d_sim.as<int32_t>();
@@ -2658,8 +2890,9 @@ int pvalues_device(cafe_ctx* C, Workspace& ws, const cafe_request* R, cafe_pvalu
     CK(launch_sim_draw(sd, ws.stream), "simulation draws");
     SimPlanArgs sp{};
     sp.hist = d_hist.as<int32_t>();
-    sp.n_keys = n_keys;
     sp.S = S;
+    sp.R = RR;
+    sp.bound_first = d_first.as<int64_t>();
     sp.cursor = d_cursor.as<int32_t>();
     sp.tiles = d_tiles.as<PruneTile>();
     sp.max_tiles = max_tiles;
@@ -2667,16 +2900,24 @@ int pvalues_device(cafe_ctx* C, Workspace& ws, const cafe_request* R, cafe_pvalu
     CK(launch_sim_plan(sp, ws.stream), "simulation plan");
     CK(launch_sim_scatter(d_keys.as<int32_t>(), NS, d_cursor.as<int32_t>(), d_perm.as<int64_t>(), ws.stream),
        "simulation plan");
-    Prune64Args p = a;
-    p.tiles = d_tiles.as<PruneTile>();
-    p.n_tiles = 0;
-    p.n_tiles_dev = d_ntiles.as<int32_t>();
-    p.counts = d_sim.as<int32_t>();
-    p.perm = d_perm.as<int64_t>();
-    p.root_out = d_simL.as<double>();
-    p.root_ld = 1;
-    CK(launch_prune64(p, (int)std::max<int64_t>(1, std::min<int64_t>(max_tiles, n_ctas_max)), ws.stream),
-       "prune simulated families");
+    int32_t* d_status = d_ntiles.as<int32_t>() + 1;
+    CK(cudaMemsetAsync(d_status, 0, sizeof(int32_t), ws.stream), "status");
+    bool by_rows = false;
+    rc = prune_simulated(C, ws, T, S, RR, msize, NS, d_sim.as<int32_t>(), d_keys.as<int32_t>(), d_perm.as<int64_t>(),
+                         d_first.as<int64_t>(), d_simL.as<double>(), d_status, &by_rows);
+    if (rc) return rc;
+    if (!by_rows) {
+        Prune64Args p = a;
+        p.tiles = d_tiles.as<PruneTile>();
+        p.n_tiles = 0;
+        p.n_tiles_dev = d_ntiles.as<int32_t>();
+        p.counts = d_sim.as<int32_t>();
+        p.perm = d_perm.as<int64_t>();
+        p.root_out = d_simL.as<double>();
+        p.root_ld = 1;
+        CK(launch_prune64(p, (int)std::max<int64_t>(1, std::min<int64_t>(max_tiles, n_ctas_max)), ws.stream),
+           "prune simulated families");
+    }
     CK(launch_sort_rows(d_simL.as<double>(), RR, nsim, ws.stream), "sort");
     PvalueSearchArgs ps{};
     ps.counts = FS.d_counts.as<int32_t>();
@@ -2697,7 +2938,10 @@ int pvalues_device(cafe_ctx* C, Workspace& ws, const cafe_request* R, cafe_pvalu
         CK(cudaMemcpyAsync(out->root_likelihood, d_obsL.p, (size_t)F * RR * sizeof(double), cudaMemcpyDeviceToHost,
                            ws.stream),
            "d2h");
+    int32_t status = 0;
+    CK(cudaMemcpyAsync(&status, d_status, sizeof status, cudaMemcpyDeviceToHost, ws.stream), "d2h");
     CK(cudaStreamSynchronize(ws.stream), "p-values");
+    if (status) return fail(C, CAFE_ERR_TIMEOUT, "p-values gave up waiting for a subtree");
     float ms = 0;
     cudaEventElapsedTime(&ms, ws.ev_start, ws.ev_stop);
     out->device_ms = ms;

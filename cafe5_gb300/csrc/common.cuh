@@ -73,9 +73,9 @@ struct PatBuildArgs {
     const int32_t* node_ii;      // [n_nodes] post-order index of an internal node, -1 for leaves
     int64_t F;
     int n_groups;
-    int64_t group_first[kMaxGroups];
-    int group_max[kMaxGroups];   // largest count of a group
-    int64_t flag_off[kMaxGroups];   // its first entry in the flags of launch_pat_counts
+    const int64_t* group_first;  // [n_groups + 1] first item of a group; then F
+    const int64_t* flag_off;     // [n_groups] a group's first entry in the flags of launch_pat_counts
+    const int32_t* group_max;    // [n_groups] its largest count
     int32_t* rep;                // [n_internal][F] the item that represents an item's key at a node
     int32_t* num;                // [n_internal][F] representatives before an item
     int32_t* base;               // [n_internal][n_groups + 1] num at each group's first item; then the total
@@ -86,9 +86,12 @@ cudaError_t launch_pat_insert(const PatBuildArgs& a, const int32_t* d_nodes, int
                               cudaStream_t s);
 // flags: [leaf][group_max + 1] per group, zeroed in; 1 where the count occurs
 cudaError_t launch_pat_counts(const PatBuildArgs& a, uint8_t* flags, cudaStream_t s);
-cudaError_t launch_pat_number(const PatBuildArgs& a, cudaStream_t s);
-// child_off [n_groups][n_internal]: first child index of a (group, node) in `child`
-cudaError_t launch_pat_write(const PatBuildArgs& a, const int64_t* d_child_off, int32_t* d_child, cudaStream_t s);
+// nodes: post-order indices of the deduplicated nodes
+cudaError_t launch_pat_number(const PatBuildArgs& a, const int32_t* d_nodes, int n_nodes, cudaStream_t s);
+// child_off [n_groups][n_internal]: first child index of a (group, node) in
+// `child`; nodes may include the root
+cudaError_t launch_pat_write(const PatBuildArgs& a, const int32_t* d_nodes, int n_nodes, const int64_t* d_child_off,
+                             int32_t* d_child, cudaStream_t s);
 
 // ---- FP64 pruning over distinct rows (k_pat64.cu) ----
 // One node of one group. An internal node's `rows` distinct vectors become
@@ -314,17 +317,37 @@ struct SimDrawArgs {
     uint64_t key;                // sim_seed_key(seed)
     int32_t* sizes;              // [n_families][n_nodes] scratch
     int32_t* counts;             // [n_families][n_leaves] out: leaf counts
-    int32_t* keys;               // [n_families] out: root index x (S + 1) + state bound
-    int32_t* hist;               // [R x (S + 1)] zeroed in, families per key out
+    int R;
+    int32_t* keys;               // [n_families] out: state bound x R + root index
+    int32_t* hist;               // [(S + 1) x R] zeroed in, families per key out
 };
 struct SimPlanArgs {
     const int32_t* hist;
-    int n_keys;
-    int S;
+    int S, R;
     int32_t* cursor;             // [n_keys] out: first family slot of each key (the scatter's cursor)
     PruneTile* tiles;            // [max_tiles] out: 32-family tiles of equal (root size, bound)
     int64_t max_tiles;
     int32_t* n_tiles;            // [1] out
+    int64_t* bound_first;        // [S + 2] out: first family slot of each state bound; then the families
+};
+// Root values of the simulated families i0 <= i < i1 (in slot order) from the
+// factor rows of the root's grandchildren (k_pat64).
+struct SimRootArgs {
+    TreePlan plan;
+    const int32_t* node_ii;      // [n_nodes] post-order index of an internal node, -1 for leaves
+    const int32_t* keys;         // state bound x R + root index
+    int R;
+    const int32_t* counts;       // [n_families][n_leaves]
+    const int64_t* perm;
+    int64_t i0, i1, F;
+    int n_groups;
+    const int32_t *rep, *num, *base;   // PatBuildArgs
+    const int64_t* tab;          // [n_groups][n_nodes] a node's factor rows in `table`, pitch (bound + 2) & ~1
+    const double* table;
+    int leaf_pitch;              // (a leaf's rows, by count, serve every group)
+    const double* const* mats;
+    int ld_mat;
+    double* out;                 // [n_families]
 };
 struct PvalueSearchArgs {
     const int32_t* counts;       // [F][n_leaves] observed families
@@ -342,6 +365,7 @@ cudaError_t launch_cdf_build(const double* const* mats, int n_nodes, int msize, 
                              cudaStream_t s);
 cudaError_t launch_sim_draw(const SimDrawArgs& a, cudaStream_t s);
 cudaError_t launch_sim_plan(const SimPlanArgs& a, cudaStream_t s);
+cudaError_t launch_sim_root(const SimRootArgs& a, cudaStream_t s);
 cudaError_t launch_sim_scatter(const int32_t* keys, int64_t n, int32_t* cursor, int64_t* perm, cudaStream_t s);
 cudaError_t launch_sort_rows(double* v, int rows, int n, cudaStream_t s);
 cudaError_t launch_pvalue_search(const PvalueSearchArgs& a, cudaStream_t s);

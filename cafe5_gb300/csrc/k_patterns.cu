@@ -33,9 +33,13 @@ namespace {
 constexpr int kNumberThreads = 1024;
 
 __device__ __forceinline__ int group_of(const PatBuildArgs& a, int64_t i) {
-    int g = 0;
-    while (g + 1 < a.n_groups && i >= a.group_first[g + 1]) ++g;
-    return g;
+    int lo = 0, hi = a.n_groups;      // the last group whose first item is not past i (empty groups precede it)
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (__ldg(a.group_first + mid) <= i) lo = mid;
+        else hi = mid;
+    }
+    return lo;
 }
 
 // The item's key at child `ch`.
@@ -81,12 +85,11 @@ __global__ void __launch_bounds__(256) k_pat_insert(PatBuildArgs a, const int32_
     }
 }
 
-// One block per non-root internal node: exclusive count of representatives
+// One block per node: exclusive count of representatives
 // before each item, and its value at every group's first item.
-__global__ void __launch_bounds__(kNumberThreads) k_pat_number(PatBuildArgs a) {
+__global__ void __launch_bounds__(kNumberThreads) k_pat_number(PatBuildArgs a, const int32_t* __restrict__ nodes) {
     __shared__ int wsum[kNumberThreads / 32];
-    const int ii = blockIdx.x;
-    if (a.plan.internal[ii] == a.plan.root) return;
+    const int ii = nodes[blockIdx.x];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int32_t* rep = a.rep + (size_t)ii * a.F;
     int32_t* num = a.num + (size_t)ii * a.F;
@@ -105,19 +108,19 @@ __global__ void __launch_bounds__(kNumberThreads) k_pat_number(PatBuildArgs a) {
             all += v;
         }
         const int excl = total + before + __popc(m & ((1u << lane) - 1u));
-        if (i < a.F) {
-            num[i] = excl;
-            for (int g = 0; g < a.n_groups; ++g)
-                if (i == a.group_first[g]) base[g] = excl;
-        }
+        if (i < a.F) num[i] = excl;
         total += all;
         __syncthreads();
     }
-    if (tid == 0) base[a.n_groups] = total;
+    for (int g = tid; g <= a.n_groups; g += kNumberThreads) {
+        const int64_t i = a.group_first[g];
+        base[g] = i < a.F ? num[i] : total;
+    }
 }
 
-__global__ void __launch_bounds__(256) k_pat_write(PatBuildArgs a, const int64_t* __restrict__ child_off, int32_t* out) {
-    const int ii = blockIdx.y;
+__global__ void __launch_bounds__(256) k_pat_write(PatBuildArgs a, const int32_t* __restrict__ nodes,
+                                                   const int64_t* __restrict__ child_off, int32_t* out) {
+    const int ii = nodes[blockIdx.y];
     const bool is_root = a.plan.internal[ii] == a.plan.root;
     const int c0 = a.plan.cstart[ii], nch = a.plan.cstart[ii + 1] - c0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < a.F; i += (int64_t)gridDim.x * blockDim.x) {
@@ -172,16 +175,17 @@ cudaError_t launch_pat_insert(const PatBuildArgs& a, const int32_t* d_nodes, int
     return cudaGetLastError();
 }
 
-cudaError_t launch_pat_number(const PatBuildArgs& a, cudaStream_t s) {
-    if (a.F <= 0) return cudaSuccess;
-    k_pat_number<<<a.plan.n_internal, kNumberThreads, 0, s>>>(a);
+cudaError_t launch_pat_number(const PatBuildArgs& a, const int32_t* d_nodes, int n_nodes, cudaStream_t s) {
+    if (a.F <= 0 || n_nodes <= 0) return cudaSuccess;
+    k_pat_number<<<n_nodes, kNumberThreads, 0, s>>>(a, d_nodes);
     return cudaGetLastError();
 }
 
-cudaError_t launch_pat_write(const PatBuildArgs& a, const int64_t* d_child_off, int32_t* d_child, cudaStream_t s) {
-    if (a.F <= 0) return cudaSuccess;
+cudaError_t launch_pat_write(const PatBuildArgs& a, const int32_t* d_nodes, int n_nodes, const int64_t* d_child_off,
+                             int32_t* d_child, cudaStream_t s) {
+    if (a.F <= 0 || n_nodes <= 0) return cudaSuccess;
     const int bx = (int)std::min<int64_t>((a.F + 255) / 256, 4096);
-    k_pat_write<<<dim3(bx, a.plan.n_internal), 256, 0, s>>>(a, d_child_off, d_child);
+    k_pat_write<<<dim3(bx, n_nodes), 256, 0, s>>>(a, d_nodes, d_child_off, d_child);
     return cudaGetLastError();
 }
 

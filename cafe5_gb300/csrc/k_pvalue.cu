@@ -18,10 +18,17 @@
 //    inverse-CDF search, the leaf counts, the family's state bound
 //    m = min(S, largest + max(50, largest / 5)) (compute_family_probabilities)
 //    and its (root size, bound) key.
-//  * k_sim_plan (one block): families per key -> offsets, and 32-family
-//    tiles of equal (root size, bound) with the tile count on the device.
-//  * k_sim_scatter: the family order the tiles read.
-//  * (k_prune64 over the device tile count writes each family's root value.)
+//  * k_sim_plan (one block): families per key -> offsets, grouped by bound;
+//    and 32-family tiles of equal (root size, bound).
+//  * k_sim_scatter: the family order.
+//  * (k_patterns and k_pat64: families of equal bound share the factor rows of
+//    equal subtrees below the root's children.)
+//  * k_sim_root: each family's root value from those rows, one state of the
+//    root's children only. 150,000 families of 12 taxa, bounds 51 to 170: 19.6
+//    ms a call, 75.1 with k_prune64 walking 32-family tiles, which still takes
+//    vectors that do not fit a CTA's shared memory and groups whose tables
+//    would pass 16 GB. The FP64 pipe is the bound: 10 GFMA over distinct rows,
+//    22 without.
 //  * k_sort_rows: each root size's n_sim likelihoods sorted (bitonic sort
 //    in shared memory), the conditional distributions.
 //  * k_pvalue_search: per observed family, the largest share of simulated
@@ -98,7 +105,7 @@ __global__ void __launch_bounds__(128) k_sim_draw(SimDrawArgs a) {
         if (a.leaf_col[v] >= 0) a.counts[(size_t)fi * a.n_leaves + a.leaf_col[v]] = c;
     }
     const int m = min(S, mx + max(50, mx / 5));
-    const int key = r * (S + 1) + m;
+    const int key = m * a.R + r;
     a.keys[fi] = key;
     atomicAdd(&a.hist[key], 1);
 }
@@ -132,17 +139,19 @@ __device__ __forceinline__ int64_t block_scan(int64_t x, int64_t* sh, int64_t* t
 __global__ void __launch_bounds__(1024) k_sim_plan(SimPlanArgs a) {
     __shared__ int64_t sh[32];
     int64_t fam_base = 0, tile_base = 0;
-    for (int k0 = 0; k0 < a.n_keys; k0 += 1024) {
+    const int n_keys = (a.S + 1) * a.R;
+    for (int k0 = 0; k0 < n_keys; k0 += 1024) {
         const int key = k0 + threadIdx.x;
-        const int64_t cnt = key < a.n_keys ? a.hist[key] : 0;
+        const int64_t cnt = key < n_keys ? a.hist[key] : 0;
         const int64_t nt = (cnt + 31) / 32;
         int64_t tf, tt;
         const int64_t fam_inc = block_scan(cnt, sh, &tf);
         const int64_t tile_inc = block_scan(nt, sh, &tt);
-        if (key < a.n_keys) {
+        if (key < n_keys) {
             const int64_t f0 = fam_base + fam_inc - cnt, t0 = tile_base + tile_inc - nt;
             a.cursor[key] = (int32_t)f0;
-            const int r = key / (a.S + 1), m = key % (a.S + 1);
+            const int m = key / a.R, r = key % a.R;
+            if (r == 0) a.bound_first[m] = f0;
             for (int64_t i = 0; i < nt && t0 + i < a.max_tiles; ++i) {
                 PruneTile t{};
                 t.first = (int)(f0 + 32 * i);
@@ -157,6 +166,7 @@ __global__ void __launch_bounds__(1024) k_sim_plan(SimPlanArgs a) {
         fam_base += tf;
         tile_base += tt;
     }
+    if (threadIdx.x == 0) a.bound_first[a.S + 1] = fam_base;
     if (threadIdx.x == 0) *a.n_tiles = (int32_t)(tile_base < a.max_tiles ? tile_base : a.max_tiles);
 }
 
@@ -166,6 +176,53 @@ __global__ void __launch_bounds__(256) k_sim_scatter(const int32_t* __restrict__
     if (fi >= n) return;
     const int pos = atomicAdd(&cursor[keys[fi]], 1);
     perm[pos] = fi;
+}
+
+// Four lanes per family, one FMA chain each (columns 0, 1, 2, 3 mod 4, as
+// every FP64 sum here): the one state of each root child's factor that the
+// family's root size needs.
+__global__ void __launch_bounds__(256) k_sim_root(SimRootArgs a) {
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t i = min(a.i0 + (t >> 2), a.i1 - 1);      // (past the last: the last again)
+    const int h = (int)(t & 3);
+    const TreePlan& P = a.plan;
+    const int64_t f = a.perm[i];
+    const int key = a.keys[f], m = key / a.R, r = key % a.R + 1;
+    const int pitch = (m + 2) & ~1;
+    auto row = [&](int ch) -> const double* {      // the factor row of grandchild ch
+        const int64_t at = a.tab[(size_t)m * P.n_nodes + ch];
+        const int lc = P.leaf_col[ch];
+        if (lc >= 0) return a.table + at + (int64_t)a.counts[(size_t)f * P.n_leaves + lc] * a.leaf_pitch;
+        const int ii = a.node_ii[ch];
+        const int64_t idx = a.num[(size_t)ii * a.F + a.rep[(size_t)ii * a.F + i]] - a.base[(size_t)ii * (a.n_groups + 1) + m];
+        return a.table + at + idx * pitch;
+    };
+    double value = 1.0;
+    const int ri = P.n_internal - 1;               // the root
+    for (int c = P.cstart[ri]; c < P.cstart[ri + 1]; ++c) {
+        const int ch = P.child[c];
+        const double* M = a.mats[ch] + (size_t)r * a.ld_mat;
+        const int lc = P.leaf_col[ch];
+        if (lc >= 0) {
+            value *= M[a.counts[(size_t)f * P.n_leaves + lc]];
+            continue;
+        }
+        const int ii = a.node_ii[ch], g0 = P.cstart[ii], g1 = P.cstart[ii + 1];
+        const double* p0 = row(P.child[g0]);
+        const double* p1 = g1 - g0 > 1 ? row(P.child[g0 + 1]) : nullptr;
+        double acc = 0.0;
+#pragma unroll 4
+        for (int j = h; j <= m; j += 4) {
+            double u = p0[j];
+            if (p1) u *= p1[j];
+            for (int g = g0 + 2; g < g1; ++g) u *= row(P.child[g])[j];
+            acc = fma(M[j], u, acc);
+        }
+        acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+        acc += __shfl_xor_sync(0xffffffffu, acc, 2);
+        value *= acc;
+    }
+    if (h == 0 && a.i0 + (t >> 2) < a.i1) a.out[f] = value;
 }
 
 // One block per row of n values: ascending bitonic sort of the row padded
@@ -246,6 +303,12 @@ cudaError_t launch_sim_draw(const SimDrawArgs& a, cudaStream_t s) {
 
 cudaError_t launch_sim_plan(const SimPlanArgs& a, cudaStream_t s) {
     k_sim_plan<<<1, 1024, 0, s>>>(a);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_sim_root(const SimRootArgs& a, cudaStream_t s) {
+    if (a.i1 <= a.i0) return cudaSuccess;
+    k_sim_root<<<(unsigned)((4 * (a.i1 - a.i0) + 255) / 256), 256, 0, s>>>(a);
     return cudaGetLastError();
 }
 
