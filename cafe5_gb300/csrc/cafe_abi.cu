@@ -2558,6 +2558,26 @@ int host_sampler_init(cafe_ctx* C, Workspace& ws, const cafe_request* R, const T
 
 // ---- p-values
 
+// Whether the device can follow the reference's stream: every draw takes two
+// words (no branch is saturated: those draw a uniform size first, by rejection;
+// at least two sizes to choose from), a start fits k_sim_chase's table, the
+// rows sort on the device, and the stream's words stay within 4 GB.
+bool stream_on_device(const cafe_request* R, const ReconSetup& Z, int nsim) {
+    const TreeHost& T = *Z.T;
+    if (Z.Smax < 2 || nsim > kSortRowsMaxP || T.n_nodes < 2 || std::max(Z.Rmax, Z.Smax) + 1 > Z.msize) return false;
+    const int64_t NS = (int64_t)Z.Rmax * nsim;
+    if (NS > INT32_MAX || NS * (T.n_nodes - 1) > ((int64_t)4 << 30) / 8) return false;
+    if ((int64_t)Z.Rmax * (Z.Smax + 1) > INT32_MAX) return false;
+    if (T.internal.size() > kMaxNodes / 2) return false;      // k_sim_len's shared memory
+    if ((size_t)T.n_nodes * Z.msize * Z.Smax * sizeof(double) > (size_t)4 << 30) return false;      // the rows' cdfs
+    for (int v = 0; v < T.n_nodes; ++v) {
+        if (T.parent[v] < 0) continue;
+        const double lam = R->lambdas[T.lambda_index[v]], t = T.branch_length[v];
+        if (!((1 - 2 * (lam * t / (1 + lam * t))) >= 0)) return false;      // matrix_cache::is_saturated
+    }
+    return true;
+}
+
 // The simulated families' root values over distinct rows: families of equal
 // state bound (the groups m = 0..S; slots first[m] ..) share the rows of every
 // internal node below the root's children; those children's factors are needed
@@ -2785,11 +2805,9 @@ int prune_simulated(cafe_ctx* C, Workspace& ws, const TreeHost& T, int S, int RR
 // 32-family tiles of equal (root size, state bound), their pruning with the
 // root fixed, the per-root-size sort and the p-value search; the host only
 // copies the results back.
-int pvalues_device(cafe_ctx* C, Workspace& ws, const cafe_request* R, cafe_pvalues_out* out) {
+int pvalues_device(cafe_ctx* C, Workspace& ws, const ReconSetup& Z, bool stream, cafe_pvalues_out* out) {
     const auto t_host0 = std::chrono::steady_clock::now();
-    ReconSetup Z;
-    int rc = recon_setup(C, ws, R, false, &Z);
-    if (rc) return rc;
+    int rc = CAFE_OK;
     TreeHost& T = *Z.T;
     FamSet& FS = *Z.S;
     const int S = Z.Smax, RR = Z.Rmax, msize = Z.msize, nsim = out->n_simulations, n = T.n_nodes;
@@ -2820,11 +2838,12 @@ int pvalues_device(cafe_ctx* C, Workspace& ws, const cafe_request* R, cafe_pvalu
     CK(d_pv.reserve(std::max<size_t>((size_t)F, 1) * sizeof(double)), "p-values");
     // prefix order, parents and leaf columns of the tree
     const std::vector<int> prefix = prefix_order(T);
-    std::vector<int32_t> tree_tab(3 * (size_t)n);
+    std::vector<int32_t> tree_tab(4 * (size_t)n);
     for (int i = 0; i < n; ++i) {
         tree_tab[i] = prefix[i];
         tree_tab[n + i] = T.parent[i];
         tree_tab[2 * n + i] = T.leaf_col[i];
+        tree_tab[3 * n + i] = T.internal_index[i];
     }
     CK(d_tree.reserve(tree_tab.size() * sizeof(int32_t)), "tree");
     CK(cudaMemcpy(d_tree.p, tree_tab.data(), tree_tab.size() * sizeof(int32_t), cudaMemcpyHostToDevice), "tree");
@@ -2857,6 +2876,49 @@ int pvalues_device(cafe_ctx* C, Workspace& ws, const cafe_request* R, cafe_pvalu
     a.tile_families = 32;
     a.W = Wmax;
     CK(cudaEventRecord(ws.ev_start, ws.stream), "event");
+    CK(launch_cdf_build(ws.mats.as<const double*>(), n, msize, S, n_ps, stream, d_cdf.as<double>(), ws.stream),
+       "row cdfs");
+    // the reference's stream: its words and where each family's draws start, on
+    // an auxiliary stream while the observed families are pruned
+    DevBuf d_words, d_len, d_starts;
+    struct Join {      // (whatever happens in between, the buffers' stream waits for the other one)
+        Workspace& ws;
+        bool on = false;
+        void now() {
+            if (!on) return;
+            on = false;
+            cudaEventRecord(ws.ev_join[0], ws.aux[0]);
+            cudaStreamWaitEvent(ws.stream, ws.ev_join[0], 0);
+        }
+        ~Join() { now(); }
+    } join{ws};
+    if (stream) {
+        const int64_t draws = NS * (n - 1);
+        CK(d_words.reserve((size_t)draws * sizeof(uint2)), "draws");
+        CK(d_len.reserve(((size_t)(nsim - 1) * (n - 1) + 1) * sizeof(uint16_t)), "draws");
+        CK(d_starts.reserve((size_t)(NS + 1) * sizeof(int64_t)), "draws");
+        CK(cudaMemsetAsync(d_starts.p, 0, sizeof(int64_t), ws.stream), "draws");
+        CK(cudaEventRecord(ws.ev_fork, ws.stream), "fork");
+        CK(cudaStreamWaitEvent(ws.aux[0], ws.ev_fork, 0), "fork");
+        join.on = true;
+        SimStreamArgs st{};
+        st.cdf = d_cdf.as<double>();
+        st.prefix = d_tree.as<int32_t>();
+        st.parent = d_tree.as<int32_t>() + n;
+        st.leaf_col = d_tree.as<int32_t>() + 2 * n;
+        st.node_ii = d_tree.as<int32_t>() + 3 * n;
+        st.n_nodes = n;
+        st.n_internal = (int)T.internal.size();
+        st.root = T.root;
+        st.n_ps = n_ps;
+        st.S = S;
+        st.n_sim = nsim;
+        st.words = d_words.as<uint2>();
+        st.len = d_len.as<uint16_t>();
+        st.starts = d_starts.as<int64_t>();
+        CK(launch_mt_words(out->seed, 2 * draws, d_words.as<uint32_t>(), ws.aux[0]), "draws");
+        CK(launch_sim_starts(st, RR, ws.aux[0]), "draws");
+    }
     if (!otiles.empty()) {
         Prune64Args o = a;
         o.tiles = d_otiles.as<PruneTile>();
@@ -2867,7 +2929,7 @@ int pvalues_device(cafe_ctx* C, Workspace& ws, const cafe_request* R, cafe_pvalu
         o.root_ld = RR;
         CK(launch_prune64(o, std::max(1, std::min((int)otiles.size(), n_ctas_max)), ws.stream), "prune root vectors");
     }
-    CK(launch_cdf_build(ws.mats.as<const double*>(), n, msize, S, n_ps, d_cdf.as<double>(), ws.stream), "row cdfs");
+    join.now();
     CK(cudaMemsetAsync(d_hist.p, 0, (size_t)n_keys * sizeof(int32_t), ws.stream), "simulation plan");
     SimDrawArgs sd{};
     sd.cdf = d_cdf.as<double>();
@@ -2883,6 +2945,8 @@ int pvalues_device(cafe_ctx* C, Workspace& ws, const cafe_request* R, cafe_pvalu
     sd.n_families = NS;
     sd.R = RR;
     sd.key = sim_seed_key(out->seed);
+    sd.words = d_words.as<uint2>();
+    sd.starts = d_starts.as<int64_t>();
     sd.sizes = d_sizes.as<int32_t>();
     sd.counts = d_sim.as<int32_t>();
     sd.keys = d_keys.as<int32_t>();
@@ -2949,13 +3013,15 @@ int pvalues_device(cafe_ctx* C, Workspace& ws, const cafe_request* R, cafe_pvalu
     return CAFE_OK;
 }
 
-// compute_pvalues (src/probability.cpp:376-570). The simulation runs on the
-// host because its random stream is the reference's: one std::mt19937
-// seeded by the caller, drawing in the reference's order (create_family,
-// :351-373, set_weighted_random_family_size, :449-476) through
+// compute_pvalues (src/probability.cpp:376-570). The simulation's random
+// stream is the reference's: one std::mt19937 seeded by the caller, drawing in
+// the reference's order (create_family, :351-373,
+// set_weighted_random_family_size, :449-476) through
 // std::discrete_distribution over the parent's matrix row
 // (matrix::select_random_y, src/matrix_cache.cpp:60-66) -- identical draws
-// for identical rows. The distributions are built once per (matrix, row)
+// for identical rows. The device follows it where it can (stream_on_device:
+// 150,000 families of 12 taxa 131 -> 25 ms a call); the rest is drawn here.
+// The distributions are built once per (matrix, row)
 // instead of once per draw. Both prunings (R x n_sim simulated families
 // with the root fixed, and the observed families) run on the GPU.
 int pvalues_sync(cafe_ctx* C, Workspace& ws, const cafe_request* R, cafe_pvalues_out* out) {
@@ -2965,12 +3031,17 @@ int pvalues_sync(cafe_ctx* C, Workspace& ws, const cafe_request* R, cafe_pvalues
         ws.staged = false;
     }
     if (!out || !out->pvalues || out->n_simulations < 1) return fail(C, CAFE_ERR_INVALID, "bad p-value arguments");
-    if (out->device_sampling) return pvalues_device(C, ws, R, out);
     const auto t_host0 = std::chrono::steady_clock::now();
     double host_ms = 0.0;
     ReconSetup Z;
     int rc = recon_setup(C, ws, R, false, &Z);
     if (rc) return rc;
+    if (out->device_sampling || stream_on_device(R, Z, out->n_simulations)) {
+        host_ms = host_ms_since(t_host0);
+        rc = pvalues_device(C, ws, Z, !out->device_sampling, out);
+        if (!rc) out->host_ms += host_ms;
+        return rc;
+    }
     TreeHost& T = *Z.T;
     FamSet& FS = *Z.S;
     const int S = Z.Smax, RR = Z.Rmax, msize = Z.msize, nsim = out->n_simulations, n = T.n_nodes;

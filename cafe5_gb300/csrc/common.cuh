@@ -315,6 +315,8 @@ struct SimDrawArgs {
     int n_nodes, n_leaves, root, n_ps, S, n_sim;
     int64_t n_families;          // R x n_sim; family fi has root size fi / n_sim + 1
     uint64_t key;                // sim_seed_key(seed)
+    const uint2* words;          // the reference's stream: two words a draw, and each family's
+    const int64_t* starts;       // first draw; null: draws by (family, node)
     int32_t* sizes;              // [n_families][n_nodes] scratch
     int32_t* counts;             // [n_families][n_leaves] out: leaf counts
     int R;
@@ -361,8 +363,23 @@ struct PvalueSearchArgs {
 constexpr int kSortRowsMaxP = 16384;   // simulations per root size the device sort takes
 uint64_t sim_seed_key(uint32_t seed);
 cudaError_t pvalue_kernels_init();
-cudaError_t launch_cdf_build(const double* const* mats, int n_nodes, int msize, int S, int n_ps, double* cdf,
-                             cudaStream_t s);
+// normalised: weights over their sum, as std::discrete_distribution keeps them
+cudaError_t launch_cdf_build(const double* const* mats, int n_nodes, int msize, int S, int n_ps, bool normalised,
+                             double* cdf, cudaStream_t s);
+// Where every family's draws start in one std::mt19937's stream (k_pvalue.cu).
+struct SimStreamArgs {
+    const double* cdf;           // normalised rows
+    const int32_t* prefix;       // as in SimDrawArgs
+    const int32_t* parent;
+    const int32_t* leaf_col;
+    const int32_t* node_ii;      // [n_nodes] index of an internal node, -1 for leaves
+    int n_nodes, n_internal, root, n_ps, S, n_sim;
+    const uint2* words;          // [R n_sim (n_nodes - 1)]
+    uint16_t* len;               // [(n_sim - 1) (n_nodes - 1) + 1] scratch
+    int64_t* starts;             // [R n_sim + 1] out; the first is set
+};
+cudaError_t launch_mt_words(uint32_t seed, int64_t n, uint32_t* out, cudaStream_t s);
+cudaError_t launch_sim_starts(const SimStreamArgs& a, int R, cudaStream_t s);
 cudaError_t launch_sim_draw(const SimDrawArgs& a, cudaStream_t s);
 cudaError_t launch_sim_plan(const SimPlanArgs& a, cudaStream_t s);
 cudaError_t launch_sim_root(const SimRootArgs& a, cudaStream_t s);

@@ -1,4 +1,4 @@
-// K7 (opt-in): the simulations of compute_pvalues drawn on the GPU.
+// K7: the simulations of compute_pvalues drawn on the GPU.
 //
 // compute_pvalues (src/probability.cpp:376-570) simulates n_sim families
 // per root size r = 1..R down the tree (create_family, :351-373, over
@@ -6,12 +6,21 @@
 // from its parent's matrix row restricted to sizes 0..S-1
 // (matrix::select_random_y, src/matrix_cache.cpp:60-66, a
 // std::discrete_distribution over the row's first S entries). The
-// reference draws from one std::mt19937 in a fixed order, which is serial
-// by construction; this mode draws from a counter-based generator instead
-// (the SplitMix64 sequence of Steele, Lea and Flood, OOPSLA 2014, indexed
-// by (family, node)), so every simulated family is one thread. The draws
-// follow the same distributions but are not the reference's stream: the
-// p-values agree in distribution, not bit for bit.
+// reference draws from one std::mt19937 in a fixed order, and a family that
+// dies out below a node takes fewer draws, so where a family starts in the
+// stream hangs on every family before it. Two modes:
+//  * the reference's stream. k_mt_words writes its words (one block; 1.3 ms for
+//    6.6 million). Root size by root size, k_sim_len finds for every draw how
+//    many draws a family that started there would take (all of them in
+//    parallel: about n_nodes times the work of the families themselves, on
+//    internal nodes only), and k_sim_chase follows the chain of starts. Then
+//    every family is one thread. The chain is the bound: 2 launches of 10 to
+//    15 us per root size. 150,000 families of 12 taxa: 5 ms, where one host
+//    thread draws for 115 ms.
+//  * opt-in, a counter-based generator (the SplitMix64 sequence of Steele, Lea
+//    and Flood, OOPSLA 2014, indexed by (family, node)): the same
+//    distributions, not the reference's stream, so the p-values agree in
+//    distribution, not bit for bit.
 //
 //  * k_cdf_build: cumulative weights of every (node, parent size) row.
 //  * k_sim_draw: one thread per simulated family: sizes in prefix order by
@@ -55,6 +64,165 @@ __device__ __forceinline__ double uniform01(uint64_t key, uint64_t c) {
     return (double)(mix64(key + (c + 1) * kGolden) >> 11) * 0x1.0p-53;
 }
 
+// The reference's own draws. std::discrete_distribution<int> over a row takes
+// two words of the std::mt19937 (generate_canonical: (w0 + 2^32 w1) / 2^64, in
+// double) and returns the first size whose cumulative probability, the last
+// set to 1, is not below it.
+__device__ __forceinline__ double canonical(uint2 w) {
+    const double u = ((double)w.x + (double)w.y * 0x1.0p32) * 0x1.0p-64;
+    return u < 1.0 ? u : 0x1.fffffffffffffp-1;
+}
+
+// (a child's size is near its parent's: the search widens from there)
+__device__ __forceinline__ int draw_size(const double* __restrict__ cp, int S, int ps, double u) {
+    int lo = 0, hi = S - 1;
+    const int g = min(ps, S - 1);
+    if (__ldg(cp + g) < u) {
+        lo = g + 1;
+        int w = 4;
+        for (; lo + w < hi && __ldg(cp + lo + w) < u; w *= 2) lo += w + 1;
+        hi = min(hi, lo + w);
+    } else {
+        hi = g;
+        int w = 4;
+        for (; hi - w > 0 && !(__ldg(cp + hi - w) < u); w *= 2) hi -= w;
+        lo = max(0, hi - w);
+    }
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (__ldg(cp + mid) < u) lo = mid + 1;
+        else hi = mid;
+    }
+    return lo;
+}
+
+// MT19937 (Matsumoto and Nishimura, ACM TOMACS 8, 1998), one block: thread i
+// makes words i, i + 227 and i + 454 of each 624, of which the later two need
+// only its own earlier ones and the old state.
+__device__ __forceinline__ uint32_t mt_twist(uint32_t a, uint32_t b, uint32_t m) {
+    const uint32_t y = (a & 0x80000000u) | (b & 0x7fffffffu);
+    return m ^ (y >> 1) ^ ((y & 1u) ? 0x9908b0dfu : 0u);
+}
+__device__ __forceinline__ uint32_t mt_temper(uint32_t y) {
+    y ^= y >> 11;
+    y ^= (y << 7) & 0x9d2c5680u;
+    y ^= (y << 15) & 0xefc60000u;
+    return y ^ (y >> 18);
+}
+__global__ void __launch_bounds__(256) k_mt_words(uint32_t seed, int64_t n, uint32_t* __restrict__ out) {
+    __shared__ uint32_t st[2][624];
+    const int i = threadIdx.x;
+    if (i == 0) {
+        uint32_t x = seed;
+        st[0][0] = x;
+        for (int k = 1; k < 624; ++k) {
+            x = 1812433253u * (x ^ (x >> 30)) + (uint32_t)k;
+            st[0][k] = x;
+        }
+    }
+    __syncthreads();
+    int cur = 0;
+    for (int64_t b = 0; b < n; b += 624, cur ^= 1) {
+        const uint32_t* s = st[cur];
+        uint32_t* t = st[cur ^ 1];
+        if (i < 227) {
+            const uint32_t x0 = mt_twist(s[i], s[i + 1], s[i + 397]);
+            const uint32_t x1 = mt_twist(s[i + 227], s[i + 228], x0);
+            t[i] = x0;
+            t[i + 227] = x1;
+            if (b + i < n) out[b + i] = mt_temper(x0);
+            if (b + i + 227 < n) out[b + i + 227] = mt_temper(x1);
+            if (i < 170) {
+                const uint32_t nx = i == 169 ? mt_twist(s[0], s[1], s[397]) : s[i + 455];
+                const uint32_t x2 = mt_twist(s[i + 454], nx, x1);
+                t[i + 454] = x2;
+                if (b + i + 454 < n) out[b + i + 454] = mt_temper(x2);
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// A family takes a draw for every node whose parent has genes, so where the
+// next one starts depends on its sizes. For root size r + 1: how many draws a
+// family takes, for every draw it might start at (n_sim families of at most
+// n - 1 draws each). Dynamic shared memory: the sizes of the internal nodes.
+constexpr int kLenThreads = 128;
+__global__ void __launch_bounds__(kLenThreads) k_sim_len(SimStreamArgs a, int r) {
+    extern __shared__ int32_t sz[];       // [n_internal][kLenThreads]
+    const int64_t p = (int64_t)blockIdx.x * kLenThreads + threadIdx.x;
+    if (p > (int64_t)(a.n_sim - 1) * (a.n_nodes - 1)) return;
+    const uint2* w = a.words + a.starts[(int64_t)r * a.n_sim] + p;
+    int32_t* my = sz + threadIdx.x;
+    my[a.node_ii[a.root] * kLenThreads] = r + 1;
+    int used = 0;
+    for (int i = 0; i < a.n_nodes; ++i) {
+        const int v = a.prefix[i];
+        if (v == a.root) continue;
+        const int ps = my[a.node_ii[a.parent[v]] * kLenThreads];
+        const int ii = a.node_ii[v];
+        if (ii >= 0) my[ii * kLenThreads] = ps > 0 ? draw_size(a.cdf + ((size_t)v * a.n_ps + ps) * a.S, a.S, ps, canonical(w[used])) : 0;
+        used += ps > 0;
+    }
+    a.len[p] = (uint16_t)used;
+}
+
+// The chain of starts through those lengths, one block: jumps over eight
+// families by doubling, one thread along them, then a thread per eight.
+constexpr int kChasePos = 24576;          // starts in shared memory (at least 32 x (kMaxNodes - 1))
+constexpr int kChaseThreads = 1024;
+static_assert(kChasePos >= 32 * (kMaxNodes - 1), "a segment holds 32 families");
+__global__ void __launch_bounds__(kChaseThreads) k_sim_chase(SimStreamArgs a, int r) {
+    extern __shared__ uint16_t jump[];    // [3][kChasePos]
+    __shared__ int32_t eighth[kChasePos / 8 + 1];
+    uint16_t* one = jump;
+    const int tid = threadIdx.x, most = a.n_nodes - 1;
+    const int seg = (kChasePos / most) & ~31;
+    int64_t* starts = a.starts + (int64_t)r * a.n_sim;
+    int64_t at = 0;                       // relative to the root size's first draw
+    const int64_t first = starts[0];
+    for (int k0 = 0; k0 < a.n_sim; k0 += seg) {
+        const int q = min(seg, a.n_sim - k0), P = (q - 1) * most + 1;
+        for (int p = tid; p < P; p += kChaseThreads) {
+            // (past the last family's last possible start: not on the chain)
+            const int64_t g = at + p;
+            one[p] = g <= (int64_t)(a.n_sim - 1) * most ? a.len[g] : 0;
+        }
+        __syncthreads();
+        const uint16_t* src = one;
+        for (int d = 0; d < 3; ++d) {
+            uint16_t* dst = jump + (1 + (d & 1)) * kChasePos;
+            for (int p = tid; p < P; p += kChaseThreads) {
+                const int j = src[p], n = p + j;
+                dst[p] = n < P ? (uint16_t)(j + src[n]) : 0;
+            }
+            __syncthreads();
+            src = dst;
+        }
+        const int n8 = (q + 7) / 8;
+        if (tid == 0) {
+            int p = 0;
+            for (int g = 0; g < n8; ++g) {
+                eighth[g] = p;
+                if (g + 1 < n8) p += src[p];
+            }
+        }
+        __syncthreads();
+        for (int g = tid; g < n8; g += kChaseThreads) {
+            int p = eighth[g];
+            const int k1 = min(8 * g + 8, q);
+            for (int k = 8 * g; k < k1; ++k) {
+                starts[k0 + k] = first + at + p;
+                p += one[p];
+            }
+            if (g == n8 - 1) starts[k0 + q] = first + at + p;
+        }
+        __syncthreads();
+        at = starts[k0 + q] - first;
+    }
+}
+
+template <bool NORM>
 __global__ void __launch_bounds__(128) k_cdf_build(const double* const* __restrict__ mats, int n_nodes, int msize,
                                                    int S, int n_ps, double* __restrict__ cdf) {
     const int v = blockIdx.x;
@@ -65,12 +233,22 @@ __global__ void __launch_bounds__(128) k_cdf_build(const double* const* __restri
     const double* row = M + (size_t)ps * msize;
     double* out = cdf + ((size_t)v * n_ps + ps) * S;
     double acc = 0.0;
+    if (NORM) {
+        double sum = 0.0;
+        for (int c = 0; c < S; ++c) sum += row[c];
+        for (int c = 0; c < S; ++c) {
+            acc += row[c] / sum;
+            out[c] = c + 1 < S ? acc : 1.0;
+        }
+        return;
+    }
     for (int c = 0; c < S; ++c) {
         acc += row[c];
         out[c] = acc;
     }
 }
 
+template <bool STREAM>
 __global__ void __launch_bounds__(128) k_sim_draw(SimDrawArgs a) {
     const int64_t fi = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (fi >= a.n_families) return;
@@ -79,13 +257,16 @@ __global__ void __launch_bounds__(128) k_sim_draw(SimDrawArgs a) {
     sz[a.root] = r + 1;
     int mx = r + 1;
     const int S = a.S;
+    const uint2* w = STREAM ? a.words + a.starts[fi] : nullptr;
     for (int i = 0; i < a.n_nodes; ++i) {
         const int v = a.prefix[i];
         if (v == a.root) continue;
         const int ps = sz[a.parent[v]];
         int c = 0;
-        if (ps > 0) {
-            const double* cd = a.cdf + ((size_t)v * a.n_ps + ps) * S;
+        const double* cd = a.cdf + ((size_t)v * a.n_ps + ps) * S;
+        if (STREAM && ps > 0) {
+            c = draw_size(cd, S, ps, canonical(*w++));
+        } else if (ps > 0) {
             const double total = cd[S - 1];
             if (total > 0.0) {
                 // first size whose cumulative weight exceeds u * total
@@ -284,20 +465,47 @@ uint64_t sim_seed_key(uint32_t seed) {
 }
 
 cudaError_t pvalue_kernels_init() {
-    return cudaFuncSetAttribute(k_sort_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, kSortRowsMaxP * 8);
+    cudaError_t e = cudaFuncSetAttribute(k_sort_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, kSortRowsMaxP * 8);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_sim_chase, cudaFuncAttributeMaxDynamicSharedMemorySize, 3 * kChasePos * (int)sizeof(uint16_t));
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_sim_len, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 kMaxNodes * kLenThreads / 2 * (int)sizeof(int32_t));
+    return e;
 }
 
-cudaError_t launch_cdf_build(const double* const* mats, int n_nodes, int msize, int S, int n_ps, double* cdf,
-                             cudaStream_t s) {
+cudaError_t launch_cdf_build(const double* const* mats, int n_nodes, int msize, int S, int n_ps, bool normalised,
+                             double* cdf, cudaStream_t s) {
     if (n_nodes <= 0 || n_ps <= 0 || S <= 0) return cudaSuccess;
-    k_cdf_build<<<dim3((unsigned)n_nodes, (unsigned)((n_ps + 127) / 128)), 128, 0, s>>>(mats, n_nodes, msize, S, n_ps,
-                                                                                        cdf);
+    const dim3 grid((unsigned)n_nodes, (unsigned)((n_ps + 127) / 128));
+    if (normalised) k_cdf_build<true><<<grid, 128, 0, s>>>(mats, n_nodes, msize, S, n_ps, cdf);
+    else k_cdf_build<false><<<grid, 128, 0, s>>>(mats, n_nodes, msize, S, n_ps, cdf);
     return cudaGetLastError();
+}
+
+cudaError_t launch_mt_words(uint32_t seed, int64_t n, uint32_t* out, cudaStream_t s) {
+    if (n <= 0) return cudaSuccess;
+    k_mt_words<<<1, 256, 0, s>>>(seed, n, out);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_sim_starts(const SimStreamArgs& a, int R, cudaStream_t s) {
+    const int64_t P = (int64_t)(a.n_sim - 1) * (a.n_nodes - 1) + 1;
+    const size_t smem = (size_t)a.n_internal * kLenThreads * sizeof(int32_t);
+    for (int r = 0; r < R; ++r) {
+        k_sim_len<<<(unsigned)((P + kLenThreads - 1) / kLenThreads), kLenThreads, smem, s>>>(a, r);
+        k_sim_chase<<<1, kChaseThreads, 3 * kChasePos * sizeof(uint16_t), s>>>(a, r);
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 cudaError_t launch_sim_draw(const SimDrawArgs& a, cudaStream_t s) {
     if (a.n_families <= 0) return cudaSuccess;
-    k_sim_draw<<<(unsigned)((a.n_families + 127) / 128), 128, 0, s>>>(a);
+    const unsigned grid = (unsigned)((a.n_families + 127) / 128);
+    if (a.starts) k_sim_draw<true><<<grid, 128, 0, s>>>(a);
+    else k_sim_draw<false><<<grid, 128, 0, s>>>(a);
     return cudaGetLastError();
 }
 

@@ -400,11 +400,12 @@ typedef struct {
     double* conditional;         /* host [R][n_simulations] out, or NULL: sorted simulated likelihoods
                                     of root sizes 1..R */
     double* root_likelihood;     /* host [F][R] out, or NULL: observed root vectors (root sizes 1..R) */
-    double device_ms;            /* out: device span from the first pruning launch to the last (it
-                                    overlaps the host simulation) */
-    double host_ms;              /* out: host time (matrix copies, simulation, sorting, p-values) */
-    int device_sampling;         /* in: 0 = the reference's std::mt19937 stream drawn on the host (the
-                                    reference's families and p-values, bit for bit); 1 = every simulated
+    double device_ms;            /* out: device span from the first launch to the last */
+    double host_ms;              /* out: host time (set-up; where the draws stay on the host, also the
+                                    simulation, sorting and p-values, which overlap the device) */
+    int device_sampling;         /* in: 0 = the reference's std::mt19937 stream (the reference's families
+                                    and p-values, bit for bit), followed on the GPU unless a branch is
+                                    saturated or the stream is very long; 1 = every simulated
                                     family drawn on the GPU from a counter-based generator seeded by
                                     `seed` (the same distributions, not the reference's stream: p-values
                                     agree in distribution only; at most 16,384 simulations per root size) */

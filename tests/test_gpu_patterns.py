@@ -123,3 +123,30 @@ def test_reconstruction_rows(ctx, newick, F, distinct, hi, S, R, lam):
         assert np.array_equal(x, y)
     assert a.n_failed == b.n_failed
     ctx.free_families(sid)
+
+
+@pytest.mark.parametrize("newick", [BINARY, POLY, "(A:1.0,B:2.0);"], ids=["binary", "polytomy", "root only"])
+@pytest.mark.parametrize("n_sim,S,R,lam,seed", [
+    (1, 2, 1, 0.05, 1),          # a draw between two sizes
+    (31, 16, 40, 0.02, 0),       # root sizes past the states
+    (33, 60, 20, 0.05, 7),       # most families die out somewhere: draws are skipped
+    (3201, 40, 3, 0.03, 2**32 - 1),   # more families than one segment of the chain of starts holds
+    (300, 130, 90, 0.004, 10),   # several state bounds
+])
+def test_pvalue_rows_and_stream(ctx, newick, n_sim, S, R, lam, seed):
+    """The reference's stream followed on the device, and the simulated families
+    pruned over distinct rows: the conditional distributions against the
+    oracle's, 1e-10 relative (two orders of summation, as for the p-values'
+    other tests), zeros in the same places."""
+    oracle = _oracle()
+    from cafe5_gb300.tree import parse_newick
+    tree = parse_newick(newick)
+    c = _counts(np.random.default_rng(5), 3, len(tree.leaves), min(S, 12), 3)
+    tid = ctx.upload_tree(tree)
+    sid = ctx.upload_families(tid, c)
+    got = ctx.pvalues(tid, sid, [lam], S=S, R=R, n_simulations=n_sim, seed=seed)
+    _, cd, rv = oracle.pvalues(oracle.TreeArrays.from_tree(tree), c, [lam], S=S, R=R, n_sim=n_sim, seed=seed)
+    for x, y in ((got["conditional"], cd), (got["root_likelihood"], rv)):
+        assert np.array_equal(x > 0, y > 0)
+        assert np.all(np.abs(x - y) <= 1e-10 * y)
+    ctx.free_families(sid)
