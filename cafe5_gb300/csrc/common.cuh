@@ -378,8 +378,11 @@ struct SimStreamArgs {
     uint16_t* len;               // [(n_sim - 1) (n_nodes - 1) + 1] scratch
     int64_t* starts;             // [R n_sim + 1] out; the first is set
 };
-cudaError_t launch_mt_words(uint32_t seed, int64_t n, uint32_t* out, cudaStream_t s);
-cudaError_t launch_sim_starts(const SimStreamArgs& a, int R, cudaStream_t s);
+constexpr int kMtWords = 624;
+// the next n words of the stream whose state [kMtWords] is kept on the device
+// (n a multiple of kMtWords but in the last call); first: seeded here
+cudaError_t launch_mt_words(bool first, uint32_t seed, uint32_t* state, int64_t n, uint32_t* out, cudaStream_t s);
+cudaError_t launch_sim_starts(const SimStreamArgs& a, int r0, int r1, cudaStream_t s);      // root sizes r0 + 1 .. r1
 cudaError_t launch_sim_draw(const SimDrawArgs& a, cudaStream_t s);
 cudaError_t launch_sim_plan(const SimPlanArgs& a, cudaStream_t s);
 cudaError_t launch_sim_root(const SimRootArgs& a, cudaStream_t s);

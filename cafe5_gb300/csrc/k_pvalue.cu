@@ -9,8 +9,8 @@
 // reference draws from one std::mt19937 in a fixed order, and a family that
 // dies out below a node takes fewer draws, so where a family starts in the
 // stream hangs on every family before it. Two modes:
-//  * the reference's stream. k_mt_words writes its words (one block; 1.3 ms for
-//    6.6 million). Root size by root size, k_sim_len finds for every draw how
+//  * the reference's stream. k_mt_words writes its words (one block, ahead of
+//    the rest on a stream of its own). Root size by root size, k_sim_len finds for every draw how
 //    many draws a family that started there would take (all of them in
 //    parallel: about n_nodes times the work of the families themselves, on
 //    internal nodes only), and k_sim_chase follows the chain of starts. Then
@@ -109,20 +109,22 @@ __device__ __forceinline__ uint32_t mt_temper(uint32_t y) {
     y ^= (y << 15) & 0xefc60000u;
     return y ^ (y >> 18);
 }
-__global__ void __launch_bounds__(256) k_mt_words(uint32_t seed, int64_t n, uint32_t* __restrict__ out) {
-    __shared__ uint32_t st[2][624];
+__global__ void __launch_bounds__(256) k_mt_words(bool first, uint32_t seed, uint32_t* __restrict__ state, int64_t n,
+                                                  uint32_t* __restrict__ out) {
+    __shared__ uint32_t st[2][kMtWords];
     const int i = threadIdx.x;
-    if (i == 0) {
+    for (int k = i; !first && k < kMtWords; k += 256) st[0][k] = state[k];
+    if (first && i == 0) {
         uint32_t x = seed;
         st[0][0] = x;
-        for (int k = 1; k < 624; ++k) {
+        for (int k = 1; k < kMtWords; ++k) {
             x = 1812433253u * (x ^ (x >> 30)) + (uint32_t)k;
             st[0][k] = x;
         }
     }
     __syncthreads();
     int cur = 0;
-    for (int64_t b = 0; b < n; b += 624, cur ^= 1) {
+    for (int64_t b = 0; b < n; b += kMtWords, cur ^= 1) {
         const uint32_t* s = st[cur];
         uint32_t* t = st[cur ^ 1];
         if (i < 227) {
@@ -141,6 +143,7 @@ __global__ void __launch_bounds__(256) k_mt_words(uint32_t seed, int64_t n, uint
         }
         __syncthreads();
     }
+    for (int k = i; k < kMtWords; k += 256) state[k] = st[cur][k];
 }
 
 // A family takes a draw for every node whose parent has genes, so where the
@@ -483,16 +486,16 @@ cudaError_t launch_cdf_build(const double* const* mats, int n_nodes, int msize, 
     return cudaGetLastError();
 }
 
-cudaError_t launch_mt_words(uint32_t seed, int64_t n, uint32_t* out, cudaStream_t s) {
+cudaError_t launch_mt_words(bool first, uint32_t seed, uint32_t* state, int64_t n, uint32_t* out, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
-    k_mt_words<<<1, 256, 0, s>>>(seed, n, out);
+    k_mt_words<<<1, 256, 0, s>>>(first, seed, state, n, out);
     return cudaGetLastError();
 }
 
-cudaError_t launch_sim_starts(const SimStreamArgs& a, int R, cudaStream_t s) {
+cudaError_t launch_sim_starts(const SimStreamArgs& a, int r0, int r1, cudaStream_t s) {
     const int64_t P = (int64_t)(a.n_sim - 1) * (a.n_nodes - 1) + 1;
     const size_t smem = (size_t)a.n_internal * kLenThreads * sizeof(int32_t);
-    for (int r = 0; r < R; ++r) {
+    for (int r = r0; r < r1; ++r) {
         k_sim_len<<<(unsigned)((P + kLenThreads - 1) / kLenThreads), kLenThreads, smem, s>>>(a, r);
         k_sim_chase<<<1, kChaseThreads, 3 * kChasePos * sizeof(uint16_t), s>>>(a, r);
         const cudaError_t e = cudaGetLastError();
