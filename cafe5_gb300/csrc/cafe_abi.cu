@@ -1618,65 +1618,53 @@ int enqueue_mixed(cafe_ctx* C, Workspace& ws, const cafe_request* R, TreeHost& T
             for (int k = 0; k < KC; ++k) fprintf(stderr, " %lld", (long long)by_cat[(size_t)k]);
             fprintf(stderr, "\n");
         }
-        FallbackPlanArgs fp;
-        std::memset(&fp, 0, sizeof fp);
-        fp.flags = d_flags;
-        fp.term_flags = d_term;
-        fp.K = K;
-        fp.perm = B.d_perm.as<int64_t>();
-        fp.n_bins = 0;
-        for (size_t b = 0; b < B.widths.size() && fp.n_bins < 16; ++b) {
+        TermTileArgs tt;
+        std::memset(&tt, 0, sizeof tt);
+        tt.flags = d_flags;
+        tt.term_flags = d_term;
+        tt.K = K;
+        tt.perm = B.d_perm.as<int64_t>();
+        int W = 32;
+        for (size_t b = B.widths.size(); b-- > 0 && tt.n_bins < 16;) {      // (the longest walks first)
             if (B.widths[b] > kTcMaxW) continue;
-            fp.bin_width[fp.n_bins] = B.widths[b];
-            fp.bin_first[fp.n_bins] = B.bin_first[b];
-            fp.bin_count[fp.n_bins] = B.bin_count[b];
-            fp.n_bins++;
+            tt.bin_width[tt.n_bins] = B.widths[b];
+            tt.bin_first[tt.n_bins] = B.bin_first[b];
+            tt.bin_count[tt.n_bins] = B.bin_count[b];
+            tt.n_bins++;
+            W = std::max(W, B.widths[b]);
         }
-        fp.cats = ws.catids.as<int32_t>();
-        fp.n_cats = (int)active.size();
-        const int64_t max_tiles = (int64_t)active.size() * (F / 32 + fp.n_bins + 1);
-        CK(ws.fb_perm.reserve((size_t)std::max<int64_t>(F, 1) * sizeof(int64_t)), "fallback");
-        CK(ws.tiles_fb.reserve((size_t)max_tiles * sizeof(PruneTile)), "fallback");
-        CK(ws.fb_bins.reserve(32 * sizeof(int64_t)), "fallback");
-        fp.fb_perm = ws.fb_perm.as<int64_t>();
-        fp.fb_bins = ws.fb_bins.as<int64_t>();
-        fp.fb_tiles = ws.tiles_fb.as<PruneTile>();
-        fp.out_counts = d_status + 1;     // [families, tiles]
-        fp.any_flag = d_status + 3;
+        tt.cats = ws.catids.as<int32_t>();
+        tt.n_cats = (int)active.size();
+        CK(ws.tiles_fb.reserve((size_t)term_tiles_max(F, tt.n_bins, tt.n_cats) * sizeof(TermTile)), "fallback");
+        tt.tiles = ws.tiles_fb.as<TermTile>();
+        tt.out_counts = d_status + 1;     // [families, tiles]
+        tt.any_flag = d_status + 3;
         if (prof) C->prof.begin(3, ws.stream, &ev);
-        CK(op_launch(ws, 6, [&] { return launch_fallback_plan(fp, ws.stream); }, fp, ws.stream), "fallback plan");
+        CK(op_launch(ws, 6, [&] { return launch_term_tiles(tt, C->sm_count, ws.stream); }, tt, C->sm_count, ws.stream),
+           "fallback plan");
         if (prof) C->prof.end(3, ws.stream, ev);
-        const int n_ctas = C->sm_count;
-        const int64_t per_cta = (int64_t)T.n_slots * msize * 32;
-        CK(ws.scratch.reserve((size_t)n_ctas * per_cta * sizeof(double)), "scratch");
-        Prune64Args a;
+        TermArgs a;
         std::memset(&a, 0, sizeof a);
         a.plan = T.plan;
-        a.tiles = fp.fb_tiles;
-        a.n_tiles = 0;
-        a.n_tiles_dev = d_status + 2;
+        a.tiles = tt.tiles;
+        a.n_tiles = d_status + 2;
         a.counts = S.d_counts.as<int32_t>();
-        a.perm = fp.fb_perm;
+        a.perm = tt.perm;
         a.mats = ws.mats.as<const double*>();
         a.ld_mat = msize;
+        a.W = W;
         a.prior = C->d_prior.as<double>();
         a.n_prior = (int)C->prior.size();
         a.err = R->use_error_model ? C->d_err.as<double>() : nullptr;
         a.err_rows = C->err_rows;
         a.err_ndev = C->err_ndev;
         a.fam_R = B.d_famR.as<int32_t>();
-        a.scratch = ws.scratch.as<double>();
-        a.scratch_per_cta = per_cta;
-        a.scaled = 1;
         a.model = gamma ? 1 : 0;
         a.out = ws.cat.as<double>();
         a.K = K;
         a.cat_probs = ws.catp.as<double>();
-        a.tile_families = 32;
-        a.W = msize;
-        a.term_mask = d_term;     // only the flagged terms of each tile are written
         if (prof) C->prof.begin(3, ws.stream, &ev);
-        CK(op_launch(ws, 7, [&] { return launch_prune64(a, n_ctas, ws.stream); }, a, n_ctas, ws.stream),
+        CK(op_launch(ws, 7, [&] { return launch_terms64(a, C->sm_count, ws.stream); }, a, C->sm_count, ws.stream),
            "fallback prune");
         if (prof) C->prof.end(3, ws.stream, ev);
         info->d_tail = d_status;     // [status, fallback families, fallback tiles]
@@ -3405,7 +3393,7 @@ int cafe_ctx_create(const cafe_config* cfg, cafe_ctx** out) {
     cudaDeviceProp prop;
     cudaGetDeviceProperties(&prop, dev);
     C->sm_count = prop.multiProcessorCount;
-    if (pat_tc_init() != cudaSuccess || pat64_init() != cudaSuccess || pvalue_kernels_init() != cudaSuccess ||
+    if (pat_tc_init() != cudaSuccess || pat64_init() != cudaSuccess || terms64_init() != cudaSuccess || pvalue_kernels_init() != cudaSuccess ||
         cudaEventCreateWithFlags(&C->gate, cudaEventDisableTiming) != cudaSuccess) {
         delete C;
         return CAFE_ERR_CUDA;

@@ -194,7 +194,6 @@ struct Prune64Args {
     int tile_families;           // families per tile (<= 32)
     int W;                       // max vector length over tiles (S + 1 or R)
     const int32_t* n_tiles_dev;  // optional: tile count read from device memory
-    const uint8_t* term_mask;    // optional [F][K]: only the terms set here are written
     double* root_out;            // optional (unscaled runs): root vector of every family,
                                  // root_out[f * root_ld + j] = L(root size root_lo + j); no reduction
     int root_ld;
@@ -408,13 +407,13 @@ struct RangeFlagArgs {
 };
 cudaError_t launch_range_flags(const RangeFlagArgs& a, cudaStream_t s);
 
-// Device-side plan of the FP64 recompute of flagged category terms:
-// k_fallback_plan compacts the flagged families of each listed bin (in
-// permutation order) into fb_perm; k_fallback_tiles then writes a 32-family
-// tile for every (chunk of 32 compacted families, listed category) in which
-// some family has that term flagged (tile order is immaterial: each tile
-// writes its own terms). out_counts[0] = families, out_counts[1] = tiles.
-struct FallbackPlanArgs {
+// ---- FP64 recompute of flagged category terms (k_terms64.cu) ----
+struct TermTile {
+    int32_t first;               // a chunk of 32 families (perm order) of a bin
+    uint32_t mask;               // the tile's families among them, at most four
+    int32_t k, W;                // category, bin width
+};
+struct TermTileArgs {
     const int32_t* flags;        // [F]
     const uint8_t* term_flags;   // [F][K]
     int K;                       // combined (candidate, category) indices
@@ -425,13 +424,33 @@ struct FallbackPlanArgs {
     int64_t bin_count[16];
     const int32_t* cats;         // [n_cats] category indices to recompute
     int n_cats;
-    int64_t* fb_perm;            // [F]
-    int64_t* fb_bins;            // [2 * 16]: start and count of each bin's families in fb_perm
-    PruneTile* fb_tiles;         // [n_cats * (F / 32 + n_bins + 1)]
-    int32_t* out_counts;         // [2]
-    const int32_t* any_flag;     // optional: zero means no family is flagged
+    TermTile* tiles;             // [term_tiles_max]
+    int32_t* out_counts;         // [2] flagged families, tiles; zeroed in
+    const int32_t* any_flag;     // zero: no family is flagged
 };
-cudaError_t launch_fallback_plan(const FallbackPlanArgs& a, cudaStream_t s);
+struct TermArgs {
+    TreePlan plan;
+    const TermTile* tiles;
+    const int32_t* n_tiles;
+    const int32_t* counts;
+    const int64_t* perm;
+    const double* const* mats;   // [K][n_nodes]
+    int ld_mat;
+    int W;                       // widest bin
+    const double* prior;
+    int n_prior;
+    const double* err;
+    int err_rows, err_ndev;
+    const int32_t* fam_R;
+    int model;
+    double* out;                 // [F][K]
+    int K;
+    const double* cat_probs;
+};
+int64_t term_tiles_max(int64_t F, int n_bins, int n_cats);
+cudaError_t terms64_init();
+cudaError_t launch_term_tiles(const TermTileArgs& a, int sm_count, cudaStream_t s);
+cudaError_t launch_terms64(const TermArgs& a, int sm_count, cudaStream_t s);
 
 // ---- Pupko joint reconstruction (k_reconstruct.cu) ----
 // One CTA walks 32-family tiles of one category up the tree; node L

@@ -88,85 +88,6 @@ __global__ void __launch_bounds__(256) k_convert_tc(const ConvertJob* __restrict
     }
 }
 
-// One block: flagged families of each bin, compacted in permutation order
-// (a block-wide prefix sum per 256-family chunk); each bin's range of
-// fb_perm goes to fb_bins for k_fallback_tiles.
-__global__ void __launch_bounds__(256) k_fallback_plan(FallbackPlanArgs a) {
-    __shared__ int scan[256];
-    __shared__ int64_t base_sh;
-    if (a.any_flag && *a.any_flag == 0) {     // nothing flagged: no work
-        if (threadIdx.x == 0) {
-            a.out_counts[0] = 0;
-            a.out_counts[1] = 0;
-        }
-        return;
-    }
-    if (threadIdx.x == 0) base_sh = 0;
-    __syncthreads();
-    for (int b = 0; b < a.n_bins; ++b) {
-        const int64_t start = base_sh;
-        for (int64_t i0 = 0; i0 < a.bin_count[b]; i0 += 256) {
-            const int64_t i = i0 + threadIdx.x;
-            int64_t fam = -1;
-            int f = 0;
-            if (i < a.bin_count[b]) {
-                fam = a.perm[a.bin_first[b] + i];
-                f = a.flags[fam] != 0;
-            }
-            scan[threadIdx.x] = f;
-            __syncthreads();
-            for (int off = 1; off < 256; off <<= 1) {
-                const int add = threadIdx.x >= off ? scan[threadIdx.x - off] : 0;
-                __syncthreads();
-                scan[threadIdx.x] += add;
-                __syncthreads();
-            }
-            if (f) a.fb_perm[base_sh + scan[threadIdx.x] - 1] = fam;
-            const int total = scan[255];
-            __syncthreads();
-            if (threadIdx.x == 0) base_sh += total;
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) {
-            a.fb_bins[2 * b] = start;
-            a.fb_bins[2 * b + 1] = base_sh - start;
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        a.out_counts[0] = (int32_t)base_sh;
-        a.out_counts[1] = 0;      // k_fallback_tiles counts the tiles
-    }
-}
-
-// A tile for every (32-family chunk of a bin's compacted families, listed
-// category) in which some family has that term flagged: one warp per chunk,
-// one block per category in turn. Tiles are appended in any order.
-__global__ void __launch_bounds__(256) k_fallback_tiles(FallbackPlanArgs a) {
-    if (a.any_flag && *a.any_flag == 0) return;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int q = blockIdx.x; q < a.n_cats; q += gridDim.x) {
-        const int k = a.cats[q];
-        for (int b = 0; b < a.n_bins; ++b) {
-            const int64_t start = a.fb_bins[2 * b], cnt = a.fb_bins[2 * b + 1];
-            for (int64_t c0 = (int64_t)warp * 32; c0 < cnt; c0 += 8 * 32) {
-                const int64_t i = c0 + lane;
-                const bool need = i < cnt && a.term_flags[(size_t)a.fb_perm[start + i] * a.K + k] != 0;
-                if (__any_sync(0xffffffffu, need) && lane == 0) {
-                    PruneTile t;
-                    t.first = (int)(start + c0);
-                    t.count = (int)(cnt - c0 < 32 ? cnt - c0 : 32);
-                    t.k = k;
-                    t.S = a.bin_width[b] - 1;
-                    t.R = a.bin_width[b] - 1;
-                    t.root_lo = t.pad[0] = t.pad[1] = 0;
-                    a.fb_tiles[atomicAdd(&a.out_counts[1], 1)] = t;
-                }
-            }
-        }
-    }
-}
-
 // One thread per (family, candidate): the category terms' range-error
 // bounds weighted by their shares of the family likelihood; a family over
 // tau |lnL| is flagged for the FP64 recompute. Terms that are not finite
@@ -226,14 +147,6 @@ cudaError_t launch_range_flags(const RangeFlagArgs& a, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
     const int blocks = (int)std::min<int64_t>((n + 255) / 256, 4096);
     k_range_flags<<<blocks, 256, 0, s>>>(a);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_fallback_plan(const FallbackPlanArgs& a, cudaStream_t s) {
-    k_fallback_plan<<<1, 256, 0, s>>>(a);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess || a.n_cats <= 0) return e;
-    k_fallback_tiles<<<a.n_cats < 1024 ? a.n_cats : 1024, 256, 0, s>>>(a);
     return cudaGetLastError();
 }
 

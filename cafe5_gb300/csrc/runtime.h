@@ -182,9 +182,9 @@ struct Workspace {
     DevBuf scratch, tiles, mats, cat, fam_lnl, total, nfail, jobs, catp;
     PinnedBuf h_tiles, h_mats, h_jobs, h_out, h_catp;
     // tensor-core path
-    DevBuf term_flags, fb_bins, tc_hi, tc_tr, tc_mi, conv, flags, fb_perm, tiles_fb, parts, fb_count,
+    DevBuf term_flags, tc_hi, tc_tr, tc_mi, conv, flags, tiles_fb, parts,
         catids, cerr;
-    PinnedBuf h_conv, h_mi, h_flags, h_tiles_fb, h_tail, h_catids;
+    PinnedBuf h_conv, h_mi, h_flags, h_tail, h_catids;
     // FP64 over distinct rows (k_pat64): per width class, factor tables and
     // exponents; node descriptors, active combinations, counters
     static constexpr int kPatClasses = 4;

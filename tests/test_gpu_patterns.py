@@ -150,3 +150,35 @@ def test_pvalue_rows_and_stream(ctx, newick, n_sim, S, R, lam, seed):
         assert np.array_equal(x > 0, y > 0)
         assert np.all(np.abs(x - y) <= 1e-10 * y)
     ctx.free_families(sid)
+
+
+@pytest.mark.parametrize("hi", [10, 40, 120, 420])           # bins of 64, 96, 192 and 512 states
+@pytest.mark.parametrize("eps", [0.0, 0.07])
+def test_flagged_terms(ctx, hi, eps):
+    """The FP64 recompute of flagged terms (k_term_tiles, k_terms64): nearly
+    diagonal matrices and unequal counts put the FP32 range bound over budget.
+    With one category a flagged family's result is its fp64_binned one, bit for
+    bit; the others are within 1e-6."""
+    from cafe5_gb300.inputs import ErrorModel, RootPrior
+    from cafe5_gb300.synth import workload
+    w = workload(1, n_families=10, seed=3)
+    tid = ctx.upload_tree(w.tree)
+    flagged = 0
+    for F in (1, 4, 5, 33, 300):            # one tile; full; one over; a second chunk; many
+        rng = np.random.default_rng([F, hi])
+        c = rng.integers(max(hi - hi // 4, 0), hi + 1, (F, len(w.tree.leaves)), dtype=np.int32)
+        c[:, rng.integers(0, c.shape[1])] = 1
+        em = ErrorModel.symmetric(eps, int(c.max())) if eps else None
+        ctx.set_prior(RootPrior.uniform(int(c.max() * 1.25) + 1).vector())
+        ctx.set_error_model(em.table() if em else None)
+        sid = ctx.upload_families(tid, c)
+        kw = dict(use_error_model=em is not None)
+        b, m = (ctx.score(tid, sid, [1e-5], precision=p, **kw) for p in ("fp64_binned", "mixed_tf32x3"))
+        flagged += m.n_fallback
+        assert np.array_equal(np.isfinite(b.family_lnl), np.isfinite(m.family_lnl))
+        ok = np.isfinite(b.family_lnl)
+        assert np.all(np.abs(m.family_lnl[ok] - b.family_lnl[ok]) <= 1e-6 * np.abs(b.family_lnl[ok]))
+        assert np.sum(m.family_lnl[ok] == b.family_lnl[ok]) >= m.n_fallback - np.sum(~ok)
+        ctx.free_families(sid)
+    ctx.set_error_model(None)
+    assert flagged > 0
