@@ -379,7 +379,9 @@ __host__ __device__ inline int stage_floats(int W, int Ns) {
 
 template <int NCH>
 struct alignas(16) Shared {
-    uint64_t ready[NB], freed[NB], a_full[2], b_full[2], empty[2], mma, stored, a_free, drain;
+    // (stored is per unit in hand: a warp without rows of a root unit may be done
+    // with the next root unit before the others are with this one)
+    uint64_t ready[NB], freed[NB], stored[NB], a_full[2], b_full[2], empty[2], mma, a_free, drain;
     uint32_t tmem;
     int abort;
     Info info[NB];
@@ -646,7 +648,7 @@ __device__ void issue(const PatTcArgs& a, const CUtensorMap* map_mat, const CUte
             }
             g += (uint32_t)n_chunks;
         }
-        ok = ok && wait_bar(sh, &sh.stored, use & 1);
+        ok = ok && wait_bar(sh, &sh.stored[buf], (use / NB) & 1);
         if (!ok) break;
         mbar_arrive(&sh.freed[buf]);       // nobody reads this unit's Info any more
         if (!is_root) {
@@ -848,7 +850,7 @@ __device__ void data(const PatTcArgs& a, Shared<NCH>& sh, float* stages, int tid
                 }
             }
             __syncwarp();
-            mbar_arrive(&sh.stored);
+            mbar_arrive(&sh.stored[buf]);
             continue;
         }
 
@@ -1045,7 +1047,7 @@ __device__ void data(const PatTcArgs& a, Shared<NCH>& sh, float* stages, int tid
         }
         tc::fence_before();
         tc::fence_proxy_async_shared();
-        mbar_arrive(&sh.stored);
+        mbar_arrive(&sh.stored[buf]);
         ++gu;
     }
 }
@@ -1068,6 +1070,7 @@ __global__ void __launch_bounds__(Shape<NCH>::kThreads, Shape<NCH>::kPerSm)
         for (int q = 0; q < NB; ++q) {
             tc::mbar_init(&sh.ready[q], 1);
             tc::mbar_init(&sh.freed[q], 1);
+            tc::mbar_init(&sh.stored[q], ND);
         }
         for (int q = 0; q < 2; ++q) {
             tc::mbar_init(&sh.a_full[q], ND);
@@ -1075,7 +1078,6 @@ __global__ void __launch_bounds__(Shape<NCH>::kThreads, Shape<NCH>::kPerSm)
             tc::mbar_init(&sh.empty[q], 1);
         }
         tc::mbar_init(&sh.mma, 1);
-        tc::mbar_init(&sh.stored, ND);
         tc::mbar_init(&sh.a_free, 1);
         tc::mbar_init(&sh.drain, 1);
         tc::mbar_init_fence();

@@ -182,3 +182,39 @@ def test_flagged_terms(ctx, hi, eps):
         ctx.free_families(sid)
     ctx.set_error_model(None)
     assert flagged > 0
+
+
+@pytest.mark.parametrize("hi", [8, 30, 45, 100, 300])        # bins of 32, 64, 96, 128 / 192 and 512 states
+@pytest.mark.parametrize("newick", [None, "((A:3.2,B:3.2):4.5,((C:2.5,(D:1.5):1.0):1.25,E:3.75):3.95);"],
+                         ids=["48 taxa", "one-child node"])
+def test_tensor_core_rows(ctx, newick, hi):
+    """k_pat_tc at the edges of its row tiles (128 rows, stored 32 at a time, the
+    root's last tile down to one family) with many combinations in flight: the
+    same bits on every call, and within 1e-6 of fp64_binned."""
+    from cafe5_gb300.inputs import RootPrior
+    from cafe5_gb300.synth import workload
+    from cafe5_gb300.tree import parse_newick
+    w = workload(3, n_families=10, seed=3)
+    tree = parse_newick(newick) if newick else w.tree
+    tid = ctx.upload_tree(tree)
+    cands = [dict(lambdas=[0.002 * (1 + 0.05 * b)], multipliers=[0.3, 0.7, 1.1, 1.9], cat_probs=[0.25] * 4)
+             for b in range(24)]
+    for F in (1, 33, 97, 128, 131, 273):
+        rng = np.random.default_rng([F, hi])
+        c = _counts(rng, F, len(tree.leaves), hi, F)
+        c = np.ascontiguousarray(np.maximum(c, hi // 2))
+        ctx.set_prior(RootPrior.uniform(int(c.max() * 1.25) + 1).vector())
+        sid = ctx.upload_families(tid, c)
+        ref = ctx.score_batch(tid, sid, cands, model=1, precision="fp64_binned")
+        first = None
+        for _ in range(3):
+            got = ctx.score_batch(tid, sid, cands, model=1, precision="mixed_tf32x3")
+            for a, b in zip(got, ref):
+                x, y = a.family_lnl, b.family_lnl
+                ok = np.isfinite(y)             # (a saturated candidate is NaN in both)
+                assert a.status == b.status and np.array_equal(np.isfinite(x), ok)
+                assert np.all(np.abs(x[ok] - y[ok]) <= 1e-6 * np.abs(y[ok]))
+            if first:
+                assert all(np.array_equal(a.family_lnl, b.family_lnl, equal_nan=True) for a, b in zip(got, first))
+            first = got
+        ctx.free_families(sid)
