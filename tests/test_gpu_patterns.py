@@ -218,3 +218,20 @@ def test_tensor_core_rows(ctx, newick, hi):
                 assert all(np.array_equal(a.family_lnl, b.family_lnl, equal_nan=True) for a, b in zip(got, first))
             first = got
         ctx.free_families(sid)
+
+
+@pytest.mark.parametrize("size", [1, 2, 3, 8, 9, 10, 31, 32, 33, 63, 64, 65, 66, 72, 97, 129, 171, 258])
+def test_matrix_rows(ctx, size):
+    """k_matrix_build at the edges of its warps (32 row pairs) and tiles (8
+    steps): odd and even sides, rows that underflow at their left end, the
+    rescaled ones, saturated keys. 1e-12 relative to the oracle where it is at
+    least 1e-280, as for the larger builds."""
+    oracle = _oracle()
+    lams, ts = [1e-6, 0.0025, 0.011, 0.6], [0.001, 0.5, 14.25, 40.0]
+    ctx.matrices_build(lams, ts, size)
+    for lam in lams:
+        for t in ts:
+            ours, ref = ctx.matrix_get(lam, t, size), oracle.fill_matrix(lam, t, size)
+            mask = ref >= 1e-280
+            assert np.all(np.abs(ours[mask] - ref[mask]) <= 1e-12 * ref[mask]), (lam, t)
+            assert np.all(ours[~mask] <= 1e-270)
