@@ -1044,7 +1044,8 @@ int launch_pat64_groups(cafe_ctx* C, Workspace& ws, const cafe_request* R, const
         X.s_run = std::max(1, std::min(4, 40000 / (TP * TS * (X.lp - 2))));
         int64_t most = 0;
         for (const PatGroup& q : X.groups) most = std::max(most, P.group_count[q.g]);
-        if (most <= 4) X.s_run = 4;      // (such units put eight times the work on a lane)
+        if (most <= 4) X.s_run = 2;      // (such units take 32 states a pass: 1.15 ms of 4 x 2 families of 768
+                                         // states and 31 nodes with two passes, 0.71 with one, 0.85 with half)
         if (units1 * n_active >= (int64_t)24 * C->sm_count * levels) X.s_run = 4;
         // Max-product: setting a vector up (logarithms) costs more than its
         // tiles, so a unit takes four tiles, or 16 past the same line (10,000

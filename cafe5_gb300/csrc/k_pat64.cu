@@ -399,6 +399,55 @@ __device__ __forceinline__ void fill_rows(const Pat64Args& a, const Unit& u, dou
     if (u.t0 == 0 && l == 0 && u.p0 + r < nd.rows) u.expo[nd.erow0 + row] = e + child_exp(a, nd, u.src, rs, u.tab, u.expo);
 }
 
+// The vectors of a unit of at most four rows (few_rows reads no others): the
+// warp's lanes along the states, four chunks in flight.
+__device__ __forceinline__ void fill_few(const Pat64Args& a, const Unit& u, double* Ls, int* lmax, int idx_pack, int np,
+                                         int lane) {
+    const Pat64Node& nd = u.nd;
+    const int S = nd.S, nchunk = S / KC + 1, lp = nchunk * KC + 2;
+    const bool two = u.src.nch == 2;
+    for (int r = 0; r < np; ++r) {
+        const int i0 = __shfl_sync(0xffffffffu, idx_pack, 2 * r), i1 = __shfl_sync(0xffffffffu, idx_pack, 2 * r + 1);
+        const RowSrc rs = row_src(a, nd, u.src, u.p0 + r, i0, i1);
+        double* L = Ls + (size_t)r * lp;
+        double mx = 0.0;
+        for (int c0 = 0; c0 < nchunk; c0 += 4) {
+            double x[4], y[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int j = (c0 + i) * KC + lane;
+                x[i] = j > S ? 0.0 : two ? __ldcg(rs.s0 + j) : product(a, nd, u.src, rs, u.tab, u.expo, j);
+                y[i] = two && j <= S ? __ldcg(rs.s1 + j) : 1.0;
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                if (c0 + i >= nchunk) break;
+                if (two) x[i] *= y[i];
+                L[(c0 + i) * KC + lane] = x[i];
+                mx = x[i] > mx ? x[i] : mx;
+                if (!a.scaled) {
+                    const int m = __reduce_max_sync(0xffffffffu, hi_key(x[i]));
+                    if (lane == 0) lmax[c0 + i] = r ? max(lmax[c0 + i], m) : m;
+                }
+            }
+        }
+        if (!a.scaled) continue;
+        const int e = scale_exp(warp_max(mx));
+        for (int ck = 0; ck < nchunk; ++ck) {
+            double x = L[ck * KC + lane];
+            if (e != 0) {
+                x = scalbn(x, -e);
+                L[ck * KC + lane] = x;
+            }
+            const int m = __reduce_max_sync(0xffffffffu, hi_key(x));
+            if (lane == 0) lmax[ck] = r ? max(lmax[ck], m) : m;
+        }
+        // the row's exponent, once per row (the unit of its first states)
+        if (u.t0 == 0 && lane == 0)
+            u.expo[nd.erow0 + u.p0 + r] = e + child_exp(a, nd, u.src, rs, u.tab, u.expo);
+    }
+}
+
 // The producer warp: units into the buffers in turn.
 template <bool MX>
 __device__ void produce(const Pat64Args& a, Unit* units, double* Ls, size_t buf_doubles, int (*lmax)[kMaxChunks],
@@ -469,7 +518,11 @@ __device__ void produce(const Pat64Args& a, Unit* units, double* Ls, size_t buf_
                 w = wait_count(a.done + (size_t)(q - a.n_slots) * a.n_desc + nd.root, a.nodes[nd.root].n_units, a.status);
             ok = __all_sync(0xffffffffu, w);
             __syncwarp();      // what one lane waited for, every lane reads
-            if (ok && !is_root && nch > 0) fill_rows<MX>(a, u, Ls + b * buf_doubles, lmax[b], pack, lane);
+            if (ok && !is_root && nch > 0) {
+                const int np = min(TP, nd.rows - p0);
+                if (!MX && np <= kFewRows) fill_few(a, u, Ls + b * buf_doubles, lmax[b], pack, np, lane);
+                else fill_rows<MX>(a, u, Ls + b * buf_doubles, lmax[b], pack, lane);
+            }
             if (!ok && lane == 0) atomicExch(a.status, 1);
         }
         if (!ok && lane == 0) u.stop = 1;
