@@ -425,14 +425,22 @@ struct TempBuf {
     ~TempBuf() {
         if (p) cudaFreeAsync(p, s);
     }
-    cudaError_t get(size_t n) { return cudaMallocAsync(&p, std::max<size_t>(n, 256), s); }
+    size_t bytes = 0;
+    // (again: kept when large enough)
+    cudaError_t get(size_t n) {
+        if (p && n <= bytes) return cudaSuccess;
+        if (p) cudaFreeAsync(p, s);
+        p = nullptr;
+        bytes = std::max<size_t>(n, 256);
+        return cudaMallocAsync(&p, bytes, s);
+    }
     template <class T> T* as() const { return static_cast<T*>(p); }
 };
 
 // The distinct patterns of every subtree, for families grouped as in `first`
 // / `count` over perm: built on the device, one launch per tree level.
 int build_patterns(cafe_ctx* C, const TreeHost& T, FamSet& S, const int64_t* d_perm, const std::vector<int64_t>& first,
-                   const std::vector<int64_t>& count, const std::vector<int>& max_count, PatternPlan& P) {
+                   const std::vector<int64_t>& count, const std::vector<int>& max_count, TempBuf& mem, PatternPlan& P) {
     const int64_t F = S.F;
     const int ni = (int)T.internal.size(), ng = (int)first.size();
     P.n_groups = ng;
@@ -459,21 +467,8 @@ int build_patterns(cafe_ctx* C, const TreeHost& T, FamSet& S, const int64_t* d_p
     std::vector<int32_t> ints = T.internal_index;
     for (auto& l : level) ints.insert(ints.end(), l.begin(), l.end());
     ints.push_back(ni - 1);
-    TempBuf d_ints(st), d_rep(st), d_num(st), d_base(st), d_tab(st), d_off(st);
-    CK(d_ints.get(ints.size() * sizeof(int32_t)), "patterns");
-    CK(d_rep.get((size_t)ni * F * sizeof(int32_t)), "patterns");
-    CK(d_num.get((size_t)ni * F * sizeof(int32_t)), "patterns");
-    CK(d_base.get((size_t)ni * (ng + 1) * sizeof(int32_t)), "patterns");
-    CK(d_tab.get(batch * slots * sizeof(int32_t)), "patterns");
-    CK(cudaMemcpyAsync(d_ints.p, ints.data(), ints.size() * sizeof(int32_t), cudaMemcpyHostToDevice, st), "patterns");
-    PatBuildArgs a;
-    std::memset(&a, 0, sizeof a);
-    a.plan = T.plan;
-    a.counts = S.d_counts.as<int32_t>();
-    a.perm = d_perm;
-    a.node_ii = d_ints.as<int32_t>();
-    a.F = F;
-    a.n_groups = ng;
+    const size_t n_nodes_list = ints.size();
+    ints.insert(ints.end(), max_count.begin(), max_count.end());
     int64_t n_flags = 0;
     std::vector<int64_t> longs(first);            // the groups' first items, F; their first flags
     longs.push_back(F);
@@ -483,32 +478,55 @@ int build_patterns(cafe_ctx* C, const TreeHost& T, FamSet& S, const int64_t* d_p
         n_flags += (int64_t)T.n_leaves * (max_count[g] + 1);
     }
     longs.insert(longs.end(), flag_off.begin(), flag_off.end());
-    TempBuf d_flags(st), d_longs(st), d_max(st);
-    CK(d_longs.get(longs.size() * sizeof(int64_t)), "patterns");
-    CK(d_max.get(ng * sizeof(int32_t)), "patterns");
-    CK(cudaMemcpyAsync(d_longs.p, longs.data(), longs.size() * sizeof(int64_t), cudaMemcpyHostToDevice, st), "patterns");
-    CK(cudaMemcpyAsync(d_max.p, max_count.data(), ng * sizeof(int32_t), cudaMemcpyHostToDevice, st), "patterns");
-    a.group_first = d_longs.as<int64_t>();
+    // one block of device memory for everything temporary
+    size_t total = 0;
+    auto part = [&](size_t bytes) {
+        const size_t at = total;
+        total += (bytes + 255) & ~(size_t)255;
+        return at;
+    };
+    const size_t in_bytes = longs.size() * sizeof(int64_t) + ints.size() * sizeof(int32_t);
+    const size_t o_in = part(in_bytes), o_rep = part((size_t)ni * F * sizeof(int32_t)),
+                 o_num = part((size_t)ni * F * sizeof(int32_t)), o_base = part((size_t)ni * (ng + 1) * sizeof(int32_t)),
+                 o_flags = part((size_t)n_flags), o_tab = part(batch * slots * sizeof(int32_t)),
+                 o_off = part((size_t)ng * ni * sizeof(int64_t));
+    CK(mem.get(total), "patterns");
+    char* d = mem.as<char>();
+    std::vector<char> in(in_bytes);
+    std::memcpy(in.data(), longs.data(), longs.size() * sizeof(int64_t));
+    std::memcpy(in.data() + longs.size() * sizeof(int64_t), ints.data(), ints.size() * sizeof(int32_t));
+    CK(cudaMemcpyAsync(d + o_in, in.data(), in_bytes, cudaMemcpyHostToDevice, st), "patterns");
+    const int32_t* d_ints = reinterpret_cast<const int32_t*>(d + o_in + longs.size() * sizeof(int64_t));
+    PatBuildArgs a;
+    std::memset(&a, 0, sizeof a);
+    a.plan = T.plan;
+    a.counts = S.d_counts.as<int32_t>();
+    a.perm = d_perm;
+    a.node_ii = d_ints;
+    a.F = F;
+    a.n_groups = ng;
+    a.group_first = reinterpret_cast<const int64_t*>(d + o_in);
     a.flag_off = a.group_first + ng + 1;
-    a.group_max = d_max.as<int32_t>();
-    CK(d_flags.get((size_t)n_flags), "patterns");
-    CK(cudaMemsetAsync(d_flags.p, 0, (size_t)n_flags, st), "patterns");
-    CK(launch_pat_counts(a, d_flags.as<uint8_t>(), st), "patterns");
-    a.rep = d_rep.as<int32_t>();
-    a.num = d_num.as<int32_t>();
-    a.base = d_base.as<int32_t>();
-    const int32_t* d_nodes = d_ints.as<int32_t>() + T.n_nodes;
+    a.group_max = d_ints + n_nodes_list;
+    uint8_t* d_flags = reinterpret_cast<uint8_t*>(d + o_flags);
+    CK(cudaMemsetAsync(d_flags, 0, (size_t)n_flags, st), "patterns");
+    CK(launch_pat_counts(a, d_flags, st), "patterns");
+    a.rep = reinterpret_cast<int32_t*>(d + o_rep);
+    a.num = reinterpret_cast<int32_t*>(d + o_num);
+    a.base = reinterpret_cast<int32_t*>(d + o_base);
+    int32_t* d_tab = reinterpret_cast<int32_t*>(d + o_tab);
+    int64_t* d_off = reinterpret_cast<int64_t*>(d + o_off);
+    const int32_t* d_nodes = d_ints + T.n_nodes;
     for (auto& l : level) {
         for (size_t b = 0; b < l.size(); b += batch)
-            CK(launch_pat_insert(a, d_nodes + b, (int)std::min(batch, l.size() - b), d_tab.as<int32_t>(), slots, st),
-               "patterns");
+            CK(launch_pat_insert(a, d_nodes + b, (int)std::min(batch, l.size() - b), d_tab, slots, st), "patterns");
         d_nodes += l.size();
     }
-    CK(launch_pat_number(a, d_ints.as<int32_t>() + T.n_nodes, ni - 1, st), "patterns");
+    CK(launch_pat_number(a, d_ints + T.n_nodes, ni - 1, st), "patterns");
     std::vector<int32_t> base((size_t)ni * (ng + 1));
     std::vector<uint8_t> flags((size_t)n_flags);
-    CK(cudaMemcpyAsync(flags.data(), d_flags.p, flags.size(), cudaMemcpyDeviceToHost, st), "patterns");
-    CK(cudaMemcpyAsync(base.data(), d_base.p, base.size() * sizeof(int32_t), cudaMemcpyDeviceToHost, st), "patterns");
+    CK(cudaMemcpyAsync(flags.data(), d_flags, flags.size(), cudaMemcpyDeviceToHost, st), "patterns");
+    CK(cudaMemcpyAsync(base.data(), a.base, base.size() * sizeof(int32_t), cudaMemcpyDeviceToHost, st), "patterns");
     CK(cudaStreamSynchronize(st), "patterns");
     int64_t off = 0;
     for (int g = 0; g < ng; ++g)
@@ -520,8 +538,7 @@ int build_patterns(cafe_ctx* C, const TreeHost& T, FamSet& S, const int64_t* d_p
             off += r * (T.cstart[ii + 1] - T.cstart[ii]);
         }
     CK(P.d_child.reserve(std::max<int64_t>(off, 1) * sizeof(int32_t)), "patterns");
-    CK(d_off.get(P.child_off.size() * sizeof(int64_t)), "patterns");
-    CK(cudaMemcpyAsync(d_off.p, P.child_off.data(), P.child_off.size() * sizeof(int64_t), cudaMemcpyHostToDevice, st),
+    CK(cudaMemcpyAsync(d_off, P.child_off.data(), P.child_off.size() * sizeof(int64_t), cudaMemcpyHostToDevice, st),
        "patterns");
     std::vector<int32_t> used;
     P.leaf_off.clear();
@@ -535,7 +552,7 @@ int build_patterns(cafe_ctx* C, const TreeHost& T, FamSet& S, const int64_t* d_p
     P.leaf_off.push_back((int64_t)used.size());
     CK(P.d_counts.reserve(used.size() * sizeof(int32_t)), "patterns");
     CK(cudaMemcpyAsync(P.d_counts.p, used.data(), used.size() * sizeof(int32_t), cudaMemcpyHostToDevice, st), "patterns");
-    CK(launch_pat_write(a, d_ints.as<int32_t>() + T.n_nodes, ni, d_off.as<int64_t>(), P.d_child.as<int32_t>(), st), "patterns");
+    CK(launch_pat_write(a, d_ints + T.n_nodes, ni, d_off, P.d_child.as<int32_t>(), st), "patterns");
     CK(cudaStreamSynchronize(st), "patterns");
     return CAFE_OK;
 }
@@ -566,9 +583,10 @@ int prepare_set(cafe_ctx* C, FamSet& S) {
         bin_max[b] = std::max(bin_max[b], m);
         all_max = std::max(all_max, m);
     }
-    rc = build_patterns(C, T, S, S.bins.d_perm.as<int64_t>(), S.bins.bin_first, S.bins.bin_count, bin_max, S.pat_bins);
+    TempBuf mem(C->ws[0]->stream_hi);
+    rc = build_patterns(C, T, S, S.bins.d_perm.as<int64_t>(), S.bins.bin_first, S.bins.bin_count, bin_max, mem, S.pat_bins);
     if (!rc)
-        rc = build_patterns(C, T, S, S.d_identity.as<int64_t>(), {0}, {F}, {all_max}, S.pat_all);
+        rc = build_patterns(C, T, S, S.d_identity.as<int64_t>(), {0}, {F}, {all_max}, mem, S.pat_all);
     return rc;
 }
 
@@ -1021,6 +1039,9 @@ int launch_pat64_groups(cafe_ctx* C, Workspace& ws, const cafe_request* R, const
         if (c < 0) return fail(C, CAFE_ERR_INVALID, "vectors of %d states", q.S + 1);
         if (P.group_count[q.g] > 0) cls[c].groups.push_back(q);
     }
+    int filled = 0;
+    for (const Class& X : cls) filled += !X.groups.empty();
+    const bool several = filled > 1;
     int levels = 1;
     for (int h : T.height) levels = std::max(levels, h);
     size_t blob = 0, ctr = NC * sizeof(unsigned long long);
@@ -1112,10 +1133,11 @@ int launch_pat64_groups(cafe_ctx* C, Workspace& ws, const cafe_request* R, const
         for (size_t gi = 0; gi < X.groups.size(); ++gi)
             for (int v = 0; v < nn; ++v) X.nodes[at[gi * nn + v]].root = at[gi * nn + T.root];
         // combinations interleaved until a level has about eight units per SM;
-        // tables for twice as many, within 2 GB
+        // tables for twice as many, within 2 GB (a class at most 1 GB of them where
+        // there are several)
         const int64_t want = ((int64_t)8 * C->sm_count * levels + X.units - 1) / std::max(1, X.units);
         X.group = (int)std::max<int64_t>(1, std::min<int64_t>(n_active, want));
-        const int64_t fit = std::max<int64_t>(1, ((int64_t)2 << 30) / std::max<int64_t>(1, X.slot_doubles * 8));
+        const int64_t fit = std::max<int64_t>(1, ((int64_t)2 << 30) / (several ? 2 : 1) / std::max<int64_t>(1, X.slot_doubles * 8));
         X.group = (int)std::min<int64_t>(X.group, fit);
         X.n_slots = (int)std::min<int64_t>(n_active, std::max<int64_t>(X.group, std::min<int64_t>(fit, 2 * X.group)));
         if (mx) {
@@ -1434,8 +1456,9 @@ int enqueue_mixed(cafe_ctx* C, Workspace& ws, const cafe_request* R, TreeHost& T
             const int64_t ctas = (int64_t)C->sm_count * tc_per_sm(C, W);
             int64_t g = n_act;
             if (units * n_act > 2 * levels * ctas) g = std::min<int64_t>(n_act, (4 * ctas + units - 1) / units);
-            // (tables within 4 GB)
-            const int64_t fit = std::max<int64_t>(1, ((int64_t)4 << 30) / std::max<int64_t>(1, L.slot_rows * W * 4));
+            // (the bins' tables within 4 GB together)
+            const int64_t fit = std::max<int64_t>(1, ((int64_t)4 << 30) / (int64_t)launches.size() /
+                                                         std::max<int64_t>(1, L.slot_rows * W * 4));
             if (g < n_act) g = std::max<int64_t>(1, std::min(g, fit / (levels + 1)));
             else if (g > fit) g = std::max<int64_t>(1, fit / (levels + 1));
             L.n_slots = (int)std::min<int64_t>(n_act, (levels + 1) * g);
