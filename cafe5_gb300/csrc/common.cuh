@@ -376,12 +376,15 @@ struct SimStreamArgs {
     const uint2* words;          // [R n_sim (n_nodes - 1)]
     uint16_t* len;               // [(n_sim - 1) (n_nodes - 1) + 1] scratch
     int64_t* starts;             // [R n_sim + 1] out; the first is set
+    int32_t* state;              // [4] root sizes done, first one that is not regular (INT_MAX), CTAs
+                                 // done, whether the next one needs every start
 };
 constexpr int kMtWords = 624;
 // the next n words of the stream whose state [kMtWords] is kept on the device
 // (n a multiple of kMtWords but in the last call); first: seeded here
 cudaError_t launch_mt_words(bool first, uint32_t seed, uint32_t* state, int64_t n, uint32_t* out, cudaStream_t s);
-cudaError_t launch_sim_starts(const SimStreamArgs& a, int r0, int r1, cudaStream_t s);      // root sizes r0 + 1 .. r1
+cudaError_t launch_sim_starts(const SimStreamArgs& a, int r0, int r1, cudaStream_t s);      // root sizes up to r1, of
+                                                                                            // which r0 may be open
 cudaError_t launch_sim_draw(const SimDrawArgs& a, cudaStream_t s);
 cudaError_t launch_sim_plan(const SimPlanArgs& a, cudaStream_t s);
 cudaError_t launch_sim_root(const SimRootArgs& a, cudaStream_t s);

@@ -10,13 +10,15 @@
 // dies out below a node takes fewer draws, so where a family starts in the
 // stream hangs on every family before it. Two modes:
 //  * the reference's stream. k_mt_words writes its words (one block, ahead of
-//    the rest on a stream of its own). Root size by root size, k_sim_len finds for every draw how
-//    many draws a family that started there would take (all of them in
-//    parallel: about n_nodes times the work of the families themselves, on
-//    internal nodes only), and k_sim_chase follows the chain of starts. Then
-//    every family is one thread. The chain is the bound: 2 launches of 10 to
-//    15 us per root size. 150,000 families of 12 taxa: 5 ms, where one host
-//    thread draws for 115 ms.
+//    the rest on a stream of its own). k_sim_regular takes 16 root sizes at a
+//    time as if no family died out anywhere, and keeps those where none did.
+//    For the next one k_sim_len finds for every draw how many draws a family
+//    that started there would take (all of them in parallel: about n_nodes times
+//    the work of the families themselves, on internal nodes only), and
+//    k_sim_chase follows the chain of starts. Then every family is one thread.
+//    The words are the bound (0.45 ms a million); 150,000 families of 12 taxa:
+//    a call of 20.5 ms, 22.4 with the chain for every root size, 131 with one
+//    host thread drawing.
 //  * opt-in, a counter-based generator (the SplitMix64 sequence of Steele, Lea
 //    and Flood, OOPSLA 2014, indexed by (family, node)): the same
 //    distributions, not the reference's stream, so the p-values agree in
@@ -44,6 +46,8 @@
 //    likelihoods not above its own over root sizes up to 1.25 x its largest
 //    count (find_best_pvalue / pvalue, :503-528).
 #include "common.cuh"
+
+#include <limits.h>
 
 #include <algorithm>
 
@@ -147,16 +151,11 @@ __global__ void __launch_bounds__(256) k_mt_words(bool first, uint32_t seed, uin
 }
 
 // A family takes a draw for every node whose parent has genes, so where the
-// next one starts depends on its sizes. For root size r + 1: how many draws a
-// family takes, for every draw it might start at (n_sim families of at most
-// n - 1 draws each). Dynamic shared memory: the sizes of the internal nodes.
+// next one starts depends on its sizes. How many draws the family of root size
+// r + 1 that starts at words w takes; sz holds the sizes of the internal nodes
+// ([n_internal][kLenThreads], this thread's column).
 constexpr int kLenThreads = 128;
-__global__ void __launch_bounds__(kLenThreads) k_sim_len(SimStreamArgs a, int r) {
-    extern __shared__ int32_t sz[];       // [n_internal][kLenThreads]
-    const int64_t p = (int64_t)blockIdx.x * kLenThreads + threadIdx.x;
-    if (p > (int64_t)(a.n_sim - 1) * (a.n_nodes - 1)) return;
-    const uint2* w = a.words + a.starts[(int64_t)r * a.n_sim] + p;
-    int32_t* my = sz + threadIdx.x;
+__device__ __forceinline__ int draws_of(const SimStreamArgs& a, int r, const uint2* w, int32_t* my) {
     my[a.node_ii[a.root] * kLenThreads] = r + 1;
     int used = 0;
     for (int i = 0; i < a.n_nodes; ++i) {
@@ -167,7 +166,54 @@ __global__ void __launch_bounds__(kLenThreads) k_sim_len(SimStreamArgs a, int r)
         if (ii >= 0) my[ii * kLenThreads] = ps > 0 ? draw_size(a.cdf + ((size_t)v * a.n_ps + ps) * a.S, a.S, ps, canonical(w[used])) : 0;
         used += ps > 0;
     }
-    a.len[p] = (uint16_t)used;
+    return used;
+}
+
+// Families that never die out take n - 1 draws each, and from some root size on
+// nearly all are such: the families of the next kSpec root sizes (below r_end)
+// at the starts they have if they all are. The root sizes before the first
+// with another length are done; the last block writes their starts.
+constexpr int kSpec = 16;
+__global__ void __launch_bounds__(kLenThreads) k_sim_regular(SimStreamArgs a, int r_end) {
+    extern __shared__ int32_t sz[];
+    __shared__ int last;
+    const int r0 = *(volatile int32_t*)&a.state[0], r1 = min(r0 + kSpec, r_end);
+    if (r0 >= r_end) return;
+    const int most = a.n_nodes - 1;
+    const int64_t first = a.starts[(int64_t)r0 * a.n_sim];
+    const int64_t t = (int64_t)blockIdx.x * kLenThreads + threadIdx.x;
+    if (t < (int64_t)(r1 - r0) * a.n_sim) {
+        const int r = r0 + (int)(t / a.n_sim);
+        if (draws_of(a, r, a.words + first + t * most, sz + threadIdx.x) != most) atomicMin(&a.state[1], r);
+    }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(&a.state[2], 1) == (int)gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    const int r2 = min(r1, *(volatile int32_t*)&a.state[1]);
+    for (int64_t f = threadIdx.x; f <= (int64_t)(r2 - r0) * a.n_sim; f += kLenThreads)
+        a.starts[(int64_t)r0 * a.n_sim + f] = first + f * most;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        a.state[0] = r2;
+        a.state[1] = INT_MAX;
+        a.state[2] = 0;
+        a.state[3] = r2 < r1;
+    }
+}
+
+// The next root size where some family is not regular: how many draws a family
+// takes, for every draw it might start at (n_sim families of at most n - 1 draws
+// each).
+__global__ void __launch_bounds__(kLenThreads) k_sim_len(SimStreamArgs a) {
+    extern __shared__ int32_t sz[];
+    if (!a.state[3]) return;
+    const int r = a.state[0];
+    const int64_t p = (int64_t)blockIdx.x * kLenThreads + threadIdx.x;
+    if (p > (int64_t)(a.n_sim - 1) * (a.n_nodes - 1)) return;
+    a.len[p] = (uint16_t)draws_of(a, r, a.words + a.starts[(int64_t)r * a.n_sim] + p, sz + threadIdx.x);
 }
 
 // The chain of starts through those lengths, one block: jumps over eight
@@ -175,8 +221,10 @@ __global__ void __launch_bounds__(kLenThreads) k_sim_len(SimStreamArgs a, int r)
 constexpr int kChasePos = 24576;          // starts in shared memory (at least 32 x (kMaxNodes - 1))
 constexpr int kChaseThreads = 1024;
 static_assert(kChasePos >= 32 * (kMaxNodes - 1), "a segment holds 32 families");
-__global__ void __launch_bounds__(kChaseThreads) k_sim_chase(SimStreamArgs a, int r) {
+__global__ void __launch_bounds__(kChaseThreads) k_sim_chase(SimStreamArgs a) {
     extern __shared__ uint16_t jump[];    // [3][kChasePos]
+    if (!a.state[3]) return;
+    const int r = a.state[0];
     __shared__ int32_t eighth[kChasePos / 8 + 1];
     uint16_t* one = jump;
     const int tid = threadIdx.x, most = a.n_nodes - 1;
@@ -222,6 +270,10 @@ __global__ void __launch_bounds__(kChaseThreads) k_sim_chase(SimStreamArgs a, in
         }
         __syncthreads();
         at = starts[k0 + q] - first;
+    }
+    if (tid == 0) {
+        a.state[0] = r + 1;
+        a.state[3] = 0;
     }
 }
 
@@ -474,6 +526,9 @@ cudaError_t pvalue_kernels_init() {
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_sim_len, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  kMaxNodes * kLenThreads / 2 * (int)sizeof(int32_t));
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_sim_regular, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 kMaxNodes * kLenThreads / 2 * (int)sizeof(int32_t));
     return e;
 }
 
@@ -495,9 +550,12 @@ cudaError_t launch_mt_words(bool first, uint32_t seed, uint32_t* state, int64_t 
 cudaError_t launch_sim_starts(const SimStreamArgs& a, int r0, int r1, cudaStream_t s) {
     const int64_t P = (int64_t)(a.n_sim - 1) * (a.n_nodes - 1) + 1;
     const size_t smem = (size_t)a.n_internal * kLenThreads * sizeof(int32_t);
+    const auto blocks = [](int64_t n) { return (unsigned)((n + kLenThreads - 1) / kLenThreads); };
+    // (a round does at least one root size; the rounds left over find none)
     for (int r = r0; r < r1; ++r) {
-        k_sim_len<<<(unsigned)((P + kLenThreads - 1) / kLenThreads), kLenThreads, smem, s>>>(a, r);
-        k_sim_chase<<<1, kChaseThreads, 3 * kChasePos * sizeof(uint16_t), s>>>(a, r);
+        k_sim_regular<<<blocks((int64_t)kSpec * a.n_sim), kLenThreads, smem, s>>>(a, r1);
+        k_sim_len<<<blocks(P), kLenThreads, smem, s>>>(a);
+        k_sim_chase<<<1, kChaseThreads, 3 * kChasePos * sizeof(uint16_t), s>>>(a);
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
