@@ -1023,7 +1023,7 @@ struct MaxProduct {
 // up; the caller zeroes it first.
 int launch_pat64_groups(cafe_ctx* C, Workspace& ws, const cafe_request* R, const TreeHost& T, const PatternPlan& P, const int64_t* d_perm, const int32_t* d_famR, const std::vector<PatGroup>& groups, int n_active,
                         const int32_t* d_active, int K, int msize, bool scaled, double* out, int32_t* d_status, bool fork,
-                        int prof_kind, MaxProduct* mx = nullptr) {
+                        int prof_kind, MaxProduct* mx = nullptr, double* root_out = nullptr) {
     constexpr int NC = Workspace::kPatClasses;
     const int ni = P.n_internal;
     struct Class {
@@ -1205,13 +1205,14 @@ int launch_pat64_groups(cafe_ctx* C, Workspace& ws, const cafe_request* R, const
         a.root_arg = mx->root_arg;
         a.n_failed = mx->n_failed;
     }
+    a.root_out = root_out;
     a.fam_R = d_famR;
     a.scaled = scaled ? 1 : 0;
     a.model = R->model == CAFE_MODEL_GAMMA ? 1 : 0;
     a.out = out;
     a.K = K;
     a.cat_probs = ws.catp.as<double>();
-    const bool prof = ws.sync && !mx;
+    const bool prof = ws.sync && !mx && !root_out;
     cudaEvent_t ev;
     if (prof) {
         C->prof.begin(prof_kind, ws.stream, &ev);
@@ -2843,7 +2844,10 @@ int pvalues_device(cafe_ctx* C, Workspace& ws, const ReconSetup& Z, bool stream,
     CK(d_cursor.reserve((size_t)n_keys * sizeof(int32_t)), "simulation plan");
     CK(d_perm.reserve((size_t)NS * sizeof(int64_t)), "simulation plan");
     CK(d_tiles.reserve((size_t)max_tiles * sizeof(PruneTile)), "tiles");
-    CK(d_ntiles.reserve(16), "tiles");
+    CK(d_ntiles.reserve(16), "tiles");       // the tile count, the status, a zero
+    CK(cudaMemsetAsync(d_ntiles.p, 0, 16, ws.stream), "tiles");
+    int32_t* d_status = d_ntiles.as<int32_t>() + 1;
+    const bool obs_rows = F > 0 && pat64_class({0, S, RR}) >= 0;
     CK(d_first.reserve((size_t)(S + 2) * sizeof(int64_t)), "simulation plan");
     CK(d_simL.reserve((size_t)NS * sizeof(double)), "simulated likelihoods");
     CK(d_obsL.reserve(std::max<size_t>((size_t)F * RR, 1) * sizeof(double)), "root vectors");
@@ -2861,7 +2865,7 @@ int pvalues_device(cafe_ctx* C, Workspace& ws, const ReconSetup& Z, bool stream,
     CK(cudaMemcpy(d_tree.p, tree_tab.data(), tree_tab.size() * sizeof(int32_t), cudaMemcpyHostToDevice), "tree");
     // observed families: states 0..S, root sizes 1..R
     std::vector<PruneTile> otiles;
-    for (int64_t f = 0; f < F; f += 32) {
+    for (int64_t f = 0; f < F && !obs_rows; f += 32) {
         PruneTile t{};
         t.first = (int)f;
         t.count = (int)std::min<int64_t>(32, F - f);
@@ -2956,6 +2960,15 @@ int pvalues_device(cafe_ctx* C, Workspace& ws, const ReconSetup& Z, bool stream,
             r = std::max(r, r1);
         }
     }
+    if (obs_rows) {
+        // over the set's distinct rows (vectors that fit a CTA's shared memory)
+        cafe_request rq;
+        std::memset(&rq, 0, sizeof rq);
+        rc = launch_pat64_groups(C, ws, &rq, T, FS.pat_all, FS.d_identity.as<int64_t>(), nullptr, {{0, S, RR}}, 1,
+                                 d_ntiles.as<int32_t>() + 2, 1, msize, false, nullptr, d_status, false, 0, nullptr,
+                                 d_obsL.as<double>());
+        if (rc) return rc;
+    }
     if (!otiles.empty()) {
         Prune64Args o = a;
         o.tiles = d_otiles.as<PruneTile>();
@@ -3001,8 +3014,6 @@ int pvalues_device(cafe_ctx* C, Workspace& ws, const ReconSetup& Z, bool stream,
     CK(launch_sim_plan(sp, ws.stream), "simulation plan");
     CK(launch_sim_scatter(d_keys.as<int32_t>(), NS, d_cursor.as<int32_t>(), d_perm.as<int64_t>(), ws.stream),
        "simulation plan");
-    int32_t* d_status = d_ntiles.as<int32_t>() + 1;
-    CK(cudaMemsetAsync(d_status, 0, sizeof(int32_t), ws.stream), "status");
     bool by_rows = false;
     rc = prune_simulated(C, ws, T, S, RR, msize, NS, d_sim.as<int32_t>(), d_keys.as<int32_t>(), d_perm.as<int64_t>(),
                          d_first.as<int64_t>(), d_simL.as<double>(), d_status, &by_rows);

@@ -134,6 +134,8 @@ struct Pat64Args {
     double* root_max;            // [K][F]
     int32_t* root_arg;           // [K][F]
     int32_t* n_failed;           // families with root value 0
+    double* root_out;            // not null: every family's root vector (root sizes 1..R) instead of
+                                 // the root weighting, [F][R]
     const int32_t* active;       // [n_active] combined (candidate, category) indices
     int n_active;
     int group;                   // combinations interleaved unit by unit

@@ -201,8 +201,14 @@ __device__ void root_family(const Pat64Args& a, const Pat64Node& nd, const NodeS
                             const int32_t* expo, int k, int row, double* x, int lane) {
     const int32_t* ci = a.child + nd.cidx + (int64_t)row * ns.nch;
     const RowSrc rs = row_src(a, nd, ns, row, __ldg(ci), ns.nch > 1 ? __ldg(ci + 1) : 0);
-    int E = a.scaled ? child_exp(a, nd, ns, rs, tab, expo) : 0;
     const int R = nd.R;
+    if (a.root_out) {
+        double* o = a.root_out + (size_t)a.perm[nd.perm0 + row] * R;
+#pragma unroll 4
+        for (int j = lane; j < R; j += 32) o[j] = product(a, nd, ns, rs, tab, expo, 1 + j);
+        return;
+    }
+    int E = a.scaled ? child_exp(a, nd, ns, rs, tab, expo) : 0;
     double mx = 0.0;
 #pragma unroll 4
     for (int j = lane; j < R; j += 32) {
