@@ -16,9 +16,9 @@
 //    that started there would take (all of them in parallel: about n_nodes times
 //    the work of the families themselves, on internal nodes only), and
 //    k_sim_chase follows the chain of starts. Then every family is one thread.
-//    The words are the bound (0.45 ms a million); 150,000 families of 12 taxa:
-//    a call of 20.5 ms, 22.4 with the chain for every root size, 131 with one
-//    host thread drawing.
+//    Words and rounds of launches are the bound; 150,000 families of 12 taxa: a
+//    call of 19.8 ms (20.1 with one warp set making and writing the words, 22.4
+//    with the chain for every root size, 131 with one host thread drawing).
 //  * opt-in, a counter-based generator (the SplitMix64 sequence of Steele, Lea
 //    and Flood, OOPSLA 2014, indexed by (family, node)): the same
 //    distributions, not the reference's stream, so the p-values agree in
@@ -100,9 +100,10 @@ __device__ __forceinline__ int draw_size(const double* __restrict__ cp, int S, i
     return lo;
 }
 
-// MT19937 (Matsumoto and Nishimura, ACM TOMACS 8, 1998), one block: thread i
-// makes words i, i + 227 and i + 454 of each 624, of which the later two need
-// only its own earlier ones and the old state.
+// MT19937 (Matsumoto and Nishimura, ACM TOMACS 8, 1998), one block: thread i of
+// the first half makes words i, i + 227 and i + 454 of each 624, of which the
+// later two need only its own earlier ones and the old state; the second half
+// tempers and writes the words of the round before.
 __device__ __forceinline__ uint32_t mt_twist(uint32_t a, uint32_t b, uint32_t m) {
     const uint32_t y = (a & 0x80000000u) | (b & 0x7fffffffu);
     return m ^ (y >> 1) ^ ((y & 1u) ? 0x9908b0dfu : 0u);
@@ -113,12 +114,14 @@ __device__ __forceinline__ uint32_t mt_temper(uint32_t y) {
     y ^= (y << 15) & 0xefc60000u;
     return y ^ (y >> 18);
 }
-__global__ void __launch_bounds__(256) k_mt_words(bool first, uint32_t seed, uint32_t* __restrict__ state, int64_t n,
-                                                  uint32_t* __restrict__ out) {
+constexpr int kMtHalf = 256;
+__global__ void __launch_bounds__(2 * kMtHalf) k_mt_words(bool first, uint32_t seed, uint32_t* __restrict__ state, int64_t n,
+                                                          uint32_t* __restrict__ out) {
     __shared__ uint32_t st[2][kMtWords];
-    const int i = threadIdx.x;
-    for (int k = i; !first && k < kMtWords; k += 256) st[0][k] = state[k];
-    if (first && i == 0) {
+    const bool writer = threadIdx.x >= kMtHalf;
+    const int i = threadIdx.x % kMtHalf;
+    for (int k = threadIdx.x; !first && k < kMtWords; k += 2 * kMtHalf) st[0][k] = state[k];
+    if (first && threadIdx.x == 0) {
         uint32_t x = seed;
         st[0][0] = x;
         for (int k = 1; k < kMtWords; ++k) {
@@ -127,27 +130,30 @@ __global__ void __launch_bounds__(256) k_mt_words(bool first, uint32_t seed, uin
         }
     }
     __syncthreads();
-    int cur = 0;
-    for (int64_t b = 0; b < n; b += kMtWords, cur ^= 1) {
-        const uint32_t* s = st[cur];
-        uint32_t* t = st[cur ^ 1];
-        if (i < 227) {
+    const int64_t rounds = (n + kMtWords - 1) / kMtWords;
+    for (int64_t q = 0; q <= rounds; ++q) {
+        const uint32_t* s = st[q & 1];
+        uint32_t* t = st[(q & 1) ^ 1];
+        if (!writer && i < 227 && q < rounds) {
             const uint32_t x0 = mt_twist(s[i], s[i + 1], s[i + 397]);
             const uint32_t x1 = mt_twist(s[i + 227], s[i + 228], x0);
             t[i] = x0;
             t[i + 227] = x1;
-            if (b + i < n) out[b + i] = mt_temper(x0);
-            if (b + i + 227 < n) out[b + i + 227] = mt_temper(x1);
             if (i < 170) {
                 const uint32_t nx = i == 169 ? mt_twist(s[0], s[1], s[397]) : s[i + 455];
-                const uint32_t x2 = mt_twist(s[i + 454], nx, x1);
-                t[i + 454] = x2;
-                if (b + i + 454 < n) out[b + i + 454] = mt_temper(x2);
+                t[i + 454] = mt_twist(s[i + 454], nx, x1);
             }
+        } else if (writer && q > 0) {
+            // (the state the others read now)
+            const int64_t left = n - (q - 1) * kMtWords;
+            uint32_t* o = out + (q - 1) * kMtWords;
+#pragma unroll
+            for (int k = i; k < kMtWords; k += kMtHalf)
+                if (k < left) o[k] = mt_temper(s[k]);
         }
         __syncthreads();
     }
-    for (int k = i; k < kMtWords; k += 256) state[k] = st[cur][k];
+    for (int k = threadIdx.x; k < kMtWords; k += 2 * kMtHalf) state[k] = st[rounds & 1][k];
 }
 
 // A family takes a draw for every node whose parent has genes, so where the
@@ -543,7 +549,7 @@ cudaError_t launch_cdf_build(const double* const* mats, int n_nodes, int msize, 
 
 cudaError_t launch_mt_words(bool first, uint32_t seed, uint32_t* state, int64_t n, uint32_t* out, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
-    k_mt_words<<<1, 256, 0, s>>>(first, seed, state, n, out);
+    k_mt_words<<<1, 2 * kMtHalf, 0, s>>>(first, seed, state, n, out);
     return cudaGetLastError();
 }
 
