@@ -747,8 +747,8 @@ def pvalue_phase(ctx, tid, sid, w, fams, S, R, cpu_seconds: float, n_sim: int = 
     out = {"unit": "families pruned/s (simulated + observed)", "value": pruned / (wall / 1e3), "wall_ms": wall,
            "device_ms": r["device_ms"], "host_ms": r["host_ms"], "n_simulations": n_sim, "root_sizes": R,
            "simulated_families": R * n_sim, "observed_families": F, "S": S,
-           "note": "whole cafe_pvalues call; the simulation is sequential on the host (the reference's "
-                   "mt19937 stream), both prunings on the GPU"}
+           "note": "whole cafe_pvalues call; the reference's mt19937 stream followed on the GPU, both "
+                   "prunings over distinct rows"}
     # the opt-in device-sampled mode: every step on the GPU, the same
     # distributions but not the reference's random stream
     ctx.pvalues(tid, sid, lam, S=S, R=R, n_simulations=50, seed=1, device_sampling=True)
@@ -833,7 +833,7 @@ def run_ours(args):
     d_tot = torch.empty(B, dtype=torch.float64, device=dev)
     if args.profile_config2:
         # two batched mixed-precision scores of the config-2 workload (a small
-        # case for ncu captures of the FP64 cluster walk and the wide bins)
+        # case for ncu captures of the wide bins)
         from cafe5_gb300.inputs import ErrorModel
         w2 = workload_cfg(2)
         tid2 = ctx.upload_tree(w2.tree, w2.lambda_of_node)
@@ -972,7 +972,7 @@ def run_ours(args):
         roof = {"bound": "fp64", "achieved": achieved, "peak": fp64_peak, "unit": "TFLOP/s",
                 "peak_source": "cuBLAS DGEMM 4096^3 measured in this run (FP64 pipe)"}
     roof["frac"] = roof["achieved"] / roof["peak"] if roof["peak"] else None
-    kernel = "k_prune64" if not prec.startswith("mixed") else "k_prune_tc"
+    kernel = "k_pat64" if not prec.startswith("mixed") else "k_pat_tc"
     traffic, tsrc = profiled_traffic(kernel, w.name + f"_B{B}")
     roof["traffic"] = traffic
     roof["traffic_source"] = tsrc

@@ -88,7 +88,7 @@ typedef struct {
     int max_family_size;         /* FP64_REF: global S; binned modes: 0 */
     int max_root_family_size;    /* FP64_REF: global R; binned modes: 0 */
     int precision;               /* cafe_precision */
-    int dedupe;                  /* prune identical count rows once (base model) */
+    int dedupe;                  /* accepted; equal count rows of every subtree are pruned once either way */
 } cafe_request;
 
 typedef struct {
@@ -184,12 +184,11 @@ int cafe_score_batch(cafe_ctx* ctx, const cafe_request* reqs, int n, cafe_result
 
 /* Autotuner for the tensor-core launch shapes: for every S-bin width of the
  * requests' family set (<= 256 states), times the batch (cafe_score_batch
- * semantics, MIXED_TF32X3) with the default shape and with the candidate
- * shapes (the three largest feasible CTA counts per SM x 1-4 pipeline
- * stages), one bin at a time, and keeps the fastest per width for every
- * later call on this context. `reps` timed runs per candidate (after one
- * untimed run). Results do not depend on the shape. Writes up to max_out
- * (width, CTAs per SM, stages, ms) entries. */
+ * semantics, MIXED_TF32X3) with the default shape and with fewer CTAs per SM,
+ * one bin at a time, and keeps the fastest per width for every later call on
+ * this context. `reps` timed runs per candidate (after one untimed run).
+ * Results do not depend on the shape. Writes up to max_out (width, CTAs per
+ * SM, operand stages, ms) entries. */
 typedef struct {
     int width;
     int ctas_per_sm;
