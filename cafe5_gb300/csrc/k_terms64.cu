@@ -16,10 +16,11 @@
 // some are flagged, the flagged ones of every category, four at a time, in any
 // order (every tile writes its own terms).
 //
-// Measured (the pass's time a call, planning included; 32-family tiles of
+// Measured (conversion, planning and recompute of a call; 32-family tiles of
 // k_prune64, planned by one block, before): 10,000 families of 24 taxa, 96
-// states, a few terms flagged 2.67 -> 0.15 ms; 20,000 of 48 taxa, 64 states,
-// 512 categories 2.2 -> 0.2; nothing flagged 0.010 -> 0.008.
+// states, a few terms flagged 2.67 -> 0.15 ms; 20,000 of 48 taxa, 64 states, 512
+// categories, the small categories of 264 families flagged 34.3 -> 22.3; nothing
+// flagged 0.021 -> 0.020.
 #include "common.cuh"
 
 #include <cooperative_groups.h>
@@ -87,11 +88,22 @@ __device__ __forceinline__ double warp_max(double x) {
 
 // The power of two the vector with these maxima is scaled by (frexp's exponent).
 __device__ __forceinline__ int scale_of(const double* m) {
-    double x = 0.0;
-    for (int r = 0; r < CL; ++r) x = m[r] > x ? m[r] : x;
+    unsigned long long b = 0;      // values >= 0: the order of the bits
+    for (int r = 0; r < CL; ++r) {
+        const unsigned long long y = (unsigned long long)__double_as_longlong(m[r]);
+        b = y > b ? y : b;
+    }
+    const double x = __longlong_as_double((long long)b);
     int e = 0;
     if (x > 0.0 && isfinite(x)) frexp(x, &e);
     return e;
+}
+
+// scalbn(x, -e), by the exponent field where it stays within the normal range.
+__device__ __forceinline__ double scaled_down(double x, int e) {
+    const int hi = __double2hiint(x), ne = (hi >> 20) - e;
+    if (hi >= 0x00100000 && ne > 0 && ne < 2047) return __hiloint2double(hi - e * 0x100000, __double2loint(x));
+    return x == 0.0 ? x : scalbn(x, -e);
 }
 
 __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(NT) k_terms64(TermArgs a) {
@@ -109,6 +121,8 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(NT) k_terms64(TermA
     double* maxs = full + (size_t)G * a.W;                      // [n_slots][G][CL] largest value of each CTA's states
     int* exps = reinterpret_cast<int*>(maxs + (size_t)P.n_slots * G * CL);  // [n_slots][G] the children's exponents
     const int n_tiles = *a.n_tiles;
+    if ((int)blockIdx.x / CL >= n_tiles) return;
+    cluster.sync();      // the other CTAs run: their shared memory may be written
     for (int t = blockIdx.x / CL; t < n_tiles; t += gridDim.x / CL) {
         const TermTile tile = a.tiles[t];
         const int cnt = __popc(tile.mask), k = tile.k, W = tile.W, S = W - 1, w = W / CL, s0 = rank * w;
@@ -156,37 +170,30 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(NT) k_terms64(TermA
                         const int g = idx / W, j = idx % W, e = e_sh[g];
                         const double* src = cluster.map_shared_rank(part + ((size_t)cs * G + g) * wmax, j / w);
                         const double x = src[j % w];
-                        full[(size_t)g * a.W + j] = e != 0 ? scalbn(x, -e) : x;
+                        full[(size_t)g * a.W + j] = scaled_down(x, e);
                     }
                     __syncthreads();
-                    // four chains per state, over j = 0, 1, 2, 3 (mod 4)
+                    // four chains per state, over j = 0, 1, 2, 3 (mod 4): a warp takes
+                    // eight states of one family (a warp issues an FP64 instruction
+                    // every 64 clocks, so the families go side by side)
                     const int m = lane & 3;
-                    for (int st0 = warp * 8; st0 < w; st0 += NT / 4) {
-                        const int sl = st0 + (lane >> 2), sc = min(sl, w - 1);
-                        const double* Mr = M + (size_t)(s0 + sc) * a.ld_mat + m;
-                        const double* L = full + m;
-                        double acc[G] = {0.0, 0.0, 0.0, 0.0};
+                    for (int it = warp; it < (w + 7) / 8 * cnt; it += NT / 32) {
+                        const int g = it % cnt, sl = it / cnt * 8 + (lane >> 2);
+                        const double* Mr = M + (size_t)(s0 + min(sl, w - 1)) * a.ld_mat + m;
+                        const double* L = full + (size_t)g * a.W + m;
+                        double v = 0.0;
                         for (int j0 = 0; j0 < W; j0 += 32) {
                             double mv[8];
 #pragma unroll
                             for (int h = 0; h < 8; ++h) mv[h] = __ldg(Mr + j0 + 4 * h);
 #pragma unroll
-                            for (int g = 0; g < G; ++g) {
-                                if (g >= cnt) continue;
-#pragma unroll
-                                for (int h = 0; h < 8; ++h) acc[g] = fma(mv[h], L[(size_t)g * a.W + j0 + 4 * h], acc[g]);
-                            }
+                            for (int h = 0; h < 8; ++h) v = fma(mv[h], L[j0 + 4 * h], v);
                         }
-#pragma unroll
-                        for (int g = 0; g < G; ++g) {
-                            if (g >= cnt) continue;
-                            double v = acc[g];
-                            v += __shfl_xor_sync(0xffffffffu, v, 1);
-                            v += __shfl_xor_sync(0xffffffffu, v, 2);
-                            if (m == 0 && sl < w) {
-                                double* o = dst + (size_t)g * wmax + sl;
-                                *o = first ? v : *o * v;
-                            }
+                        v += __shfl_xor_sync(0xffffffffu, v, 1);
+                        v += __shfl_xor_sync(0xffffffffu, v, 2);
+                        if (m == 0 && sl < w) {
+                            double* o = dst + (size_t)g * wmax + sl;
+                            *o = first ? v : *o * v;
                         }
                     }
                 }
@@ -195,10 +202,10 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(NT) k_terms64(TermA
             // the root's rows are the root sizes 1..S
             const int lo = ii == P.n_internal - 1 && rank == 0 ? 1 : 0;
             if (warp < cnt) {
-                double mx = 0.0;
+                double mx = 0.0;      // (values >= 0: the order of the bits)
                 for (int sl = lo + lane; sl < w; sl += 32) {
                     const double x = dst[(size_t)warp * wmax + sl];
-                    mx = x > mx ? x : mx;
+                    mx = __double_as_longlong(x) > __double_as_longlong(mx) ? x : mx;
                 }
                 mx = warp_max(mx);
                 if (lane < CL) cluster.map_shared_rank(maxs + ((size_t)vs * G + warp) * CL, lane)[rank] = mx;
@@ -216,7 +223,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(NT) k_terms64(TermA
                 const int j = s0 + sl - 1;        // root size j + 1
                 if (j < 0 || j >= Rf) continue;
                 double x = part[((size_t)rs * G + warp) * wmax + sl];
-                if (e != 0) x = scalbn(x, -e);
+                x = scaled_down(x, e);
                 const double eq = j < a.n_prior ? a.prior[j] : 0.0;
                 const double v = a.model == 0 ? log(x) + log(eq) : x * eq;
                 best = v > best ? v : best;
@@ -229,6 +236,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(NT) k_terms64(TermA
             }
             nz = __any_sync(0xffffffffu, nz);
             if (lane == 0) {
+                e_sh[warp] = e;      // (the maxima may be the next tile's after the barrier)
                 cluster.map_shared_rank(&root_v[0][0], 0)[warp * CL + rank] = best;
                 cluster.map_shared_rank(&root_nz[0][0], 0)[warp * CL + rank] = nz;
             }
@@ -241,7 +249,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(NT) k_terms64(TermA
                 b = root_v[tid][r] > b ? root_v[tid][r] : b;
                 nz |= root_nz[tid][r];
             }
-            const double E = (double)(exps[rs * G + tid] + scale_of(maxs + ((size_t)rs * G + tid) * CL)) * 0.69314718055994530942;
+            const double E = (double)(exps[rs * G + tid] + e_sh[tid]) * 0.69314718055994530942;
             double o;
             if (a.model == 0) o = b + E;
             else o = nz ? log(b * a.cat_probs[k]) + E : NAN;      // (an all-zero root vector: the family fails)
@@ -278,7 +286,9 @@ cudaError_t launch_term_tiles(const TermTileArgs& a, int sm_count, cudaStream_t 
 
 cudaError_t launch_terms64(const TermArgs& a, int sm_count, cudaStream_t s) {
     const size_t smem = terms_smem(a.W, a.plan.n_slots);
-    const int per_sm = (int)std::max<size_t>(1, std::min<size_t>(4, (size_t)kMaxDynSmem / smem));
+    // (the walks wait on barriers: with four CTAs per SM the 264 families above
+    // take 35 ms, with 12 24, with 20, more than fit at a time, 22)
+    const int per_sm = (int)std::max<size_t>(1, std::min<size_t>(20, (size_t)kMaxDynSmem / smem));
     k_terms64<<<std::max(1, sm_count * per_sm / CL) * CL, NT, smem, s>>>(a);
     return cudaGetLastError();
 }
