@@ -52,8 +52,15 @@
 //
 // Roles in a CTA: a scheduler warp (units, their inputs' completion, child
 // indices), an issuer (TMA, MMA, completion) and 4 or 8 data warps (rows:
-// copies, product, split; epilogue). All waits are bounded; on time-out the kernel records a status, drains its own
-// copies and MMAs, frees TMEM and returns.
+// copies, product, split; epilogue). All waits are bounded; on time-out the
+// kernel records a status, drains its own copies and MMAs, frees TMEM and
+// returns.
+//
+// Measured (each bin alone; families walked up the tree before): 16 x 4
+// combinations of 10,000 families of 24 taxa, W = 64 1,490 -> 547 us, W = 32
+// 645 -> 139, W = 96 399 -> 99; 64 x 8 of 20,000 families of 48 taxa 54 -> 9.7
+// ms. W = 64 moves 0.91 GB of DRAM in its 547 us (25 % of a copy's rate), the
+// tensor pipe is 8 % active; the rest is the latency of gathered rows.
 #include "common.cuh"
 #include "tc_ptx.cuh"
 
