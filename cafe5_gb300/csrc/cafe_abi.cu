@@ -879,10 +879,12 @@ double host_ms_since(std::chrono::steady_clock::time_point t0) {
 }
 
 // ---- op log: the stream operations of the pruning phase. In the dry mode
-// they are only recorded (their parameters form the CUDA-graph signature),
-// in the run and capture modes they are also issued.
+// they are only recorded (their parameters form the CUDA-graph signature), in
+// the capture mode they are also issued, and in the run mode only issued (FP64
+// scores, reconstructions and p-values keep no record of their operations).
 template <class T>
 void oplog(Workspace& ws, const T& v) {
+    if (ws.op_mode == Workspace::kOpRun) return;
     const uint8_t* p = reinterpret_cast<const uint8_t*>(&v);
     ws.oplog.insert(ws.oplog.end(), p, p + sizeof(T));
 }
@@ -1708,11 +1710,8 @@ int enqueue_mixed_graph(cafe_ctx* C, Workspace& ws, const cafe_request* R, TreeH
                         const std::vector<int32_t>& active, double** hm, double* d_fam, double* d_total,
                         ScoreInfo* info) {
     static const bool flag_env = getenv("CAFE_DEBUG_FLAGS") != nullptr;
+    if (C->prof.on || flag_env) return enqueue_mixed(C, ws, R, T, S, K, CT, active, hm, d_fam, d_total, info);
     ws.oplog.clear();
-    if (C->prof.on || flag_env) {
-        ws.op_mode = Workspace::kOpRun;
-        return enqueue_mixed(C, ws, R, T, S, K, CT, active, hm, d_fam, d_total, info);
-    }
     ws.op_mode = Workspace::kOpDry;
     int rc = enqueue_mixed(C, ws, R, T, S, K, CT, active, hm, d_fam, d_total, info);
     ws.op_mode = Workspace::kOpRun;
@@ -1727,8 +1726,6 @@ int enqueue_mixed_graph(cafe_ctx* C, Workspace& ws, const cafe_request* R, TreeH
     sig.swap(ws.oplog);
     auto issue_directly = [&]() {
         cudaGetLastError();
-        ws.oplog.clear();
-        ws.op_mode = Workspace::kOpRun;
         return enqueue_mixed(C, ws, R, T, S, K, CT, active, hm, d_fam, d_total, info);
     };
     // capture into a free slot at once; evict a cached graph only for a
