@@ -35,6 +35,23 @@ thread_local cudaStream_t t_alloc_stream = nullptr;
 AllocScope::AllocScope(cudaStream_t s) : prev(t_alloc_stream) { t_alloc_stream = s; }
 AllocScope::~AllocScope() { t_alloc_stream = prev; }
 
+// (a test hook: device buffers of more than this many bytes are not to be had)
+thread_local size_t t_alloc_limit = 0;
+struct AllocLimit {
+    size_t prev;
+    explicit AllocLimit(size_t n) : prev(t_alloc_limit) { t_alloc_limit = n; }
+    ~AllocLimit() { t_alloc_limit = prev; }
+};
+cudaError_t device_alloc(void** p, size_t n, cudaStream_t s) {
+    if (t_alloc_limit && n > t_alloc_limit) return cudaErrorMemoryAllocation;
+    const cudaError_t e = s ? cudaMallocAsync(p, n, s) : cudaMalloc(p, n);
+    if (e != cudaSuccess) {
+        *p = nullptr;
+        cudaGetLastError();
+    }
+    return e;
+}
+
 // ---- MatCache
 size_t MatCache::home(const MatKey& k) const {
     uint64_t h = (uint64_t)k.size * 0x9E3779B97F4A7C15ull ^ (uint64_t)k.lq * 0xC2B2AE3D27D4EB4Full ^
@@ -138,19 +155,13 @@ cudaError_t DevBuf::reserve(size_t n) {
     // O(log) reallocations
     size_t want = std::max<size_t>(std::max<size_t>(n, bytes + bytes / 2), 256);
     bytes = 0;
-    cudaError_t e = s ? cudaMallocAsync(&p, want, s) : cudaMalloc(&p, want);
+    cudaError_t e = device_alloc(&p, want, s);
     if (e != cudaSuccess && want > n) {
-        cudaGetLastError();
         want = n;
-        e = s ? cudaMallocAsync(&p, want, s) : cudaMalloc(&p, want);
+        e = device_alloc(&p, want, s);
     }
-    if (e != cudaSuccess) {
-        p = nullptr;
-        cudaGetLastError();
-        return e;
-    }
-    bytes = want;
-    return cudaSuccess;
+    if (e == cudaSuccess) bytes = want;
+    return e;
 }
 PinnedBuf::~PinnedBuf() {
     if (p) cudaFreeHost(p);
@@ -280,6 +291,18 @@ int cuda_fail(cafe_ctx* C, cudaError_t e, const char* what) {
         cudaError_t _e = (expr);                              \
         if (_e != cudaSuccess) return cuda_fail(C, _e, what); \
     } while (0)
+
+// A call that fails half way leaves nothing of its own running: its buffers are
+// about to go, and the next call writes the workspace's staging memory.
+struct DrainOnError {
+    Workspace& ws;
+    bool ok = false;
+    ~DrainOnError() {
+        if (ok) return;
+        cudaStreamSynchronize(ws.stream);
+        for (cudaStream_t s : ws.aux) cudaStreamSynchronize(s);
+    }
+};
 
 // Post-order of internal nodes, children with the larger slot need first
 // (Sethi-Ullman), and greedy slot reuse.
@@ -431,8 +454,11 @@ struct TempBuf {
         if (p && n <= bytes) return cudaSuccess;
         if (p) cudaFreeAsync(p, s);
         p = nullptr;
-        bytes = std::max<size_t>(n, 256);
-        return cudaMallocAsync(&p, bytes, s);
+        bytes = 0;
+        const size_t want = std::max<size_t>(n, 256);
+        const cudaError_t e = device_alloc(&p, want, s);
+        if (e == cudaSuccess) bytes = want;
+        return e;
     }
     template <class T> T* as() const { return static_cast<T*>(p); }
 };
@@ -2061,6 +2087,8 @@ cudaError_t gate_leave(cafe_ctx* C, Workspace& ws) {
 // category values [F][NB * K] when any result asks for them.
 int score_enqueue(cafe_ctx* C, Workspace& ws, const cafe_request* R, int NB, cafe_result* res, ScoreInfo* info) {
     AllocScope scope(ws.stream);
+    AllocLimit limit(C->debug_alloc_limit);
+    DrainOnError drain{ws};
     auto si = C->sets.find(R ? R->set_id : -1);
     if (si == C->sets.end()) return fail(C, CAFE_ERR_NOT_FOUND, "unknown family set");
     if (NB < 1) return fail(C, CAFE_ERR_INVALID, "empty batch");
@@ -2095,6 +2123,7 @@ int score_enqueue(cafe_ctx* C, Workspace& ws, const cafe_request* R, int NB, caf
     if (F) CK(cudaMemcpyAsync(h_fam, ws.fam_lnl.p, (size_t)NB * F * sizeof(double), cudaMemcpyDeviceToHost, ws.stream), "d2h");
     if (any_cat && F && !info->rejected)
         CK(cudaMemcpyAsync(h_cat, ws.cat.p, (size_t)F * NB * K * sizeof(double), cudaMemcpyDeviceToHost, ws.stream), "d2h");
+    drain.ok = true;
     return CAFE_OK;
 }
 
@@ -2340,6 +2369,8 @@ int reconstruct_rows(cafe_ctx* C, Workspace& ws, const cafe_request* R, const Re
 
 int reconstruct_sync(cafe_ctx* C, Workspace& ws, const cafe_request* R, cafe_reconstruction* out) {
     AllocScope scope(ws.stream);
+    AllocLimit limit(C->debug_alloc_limit);
+    DrainOnError drain{ws};
     if (ws.staged) {   // the previous request's copies out of the pinned staging buffers
         CK(cudaEventSynchronize(ws.ev_staged), "staging");
         ws.staged = false;
@@ -2478,6 +2509,7 @@ int reconstruct_sync(cafe_ctx* C, Workspace& ws, const cafe_request* R, cafe_rec
                "d2h");
     }
     CK(cudaStreamSynchronize(ws.stream), "reconstruct");
+    drain.ok = true;
     float ms = 0;
     cudaEventElapsedTime(&ms, ws.ev_start, ws.ev_stop);
     out->device_ms = ms;
@@ -2592,14 +2624,22 @@ bool stream_on_device(const cafe_request* R, const ReconSetup& Z, int nsim) {
 // state bound (the groups m = 0..S; slots first[m] ..) share the rows of every
 // internal node below the root's children; those children's factors are needed
 // at one state only, the family's root size (k_sim_root). Returns through
-// `done` whether it ran: vectors that do not fit a CTA's shared memory and
-// groups whose tables pass 16 GB are left to the tile walk.
+// `done` whether it ran: vectors that do not fit a CTA's shared memory,
+// groups whose tables pass 16 GB and tables that there is no memory for are left
+// to the tile walk.
 constexpr size_t kSimTableBytes = (size_t)16 << 30;
 
 int prune_simulated(cafe_ctx* C, Workspace& ws, const TreeHost& T, int S, int RR, int msize, int64_t NS,
                     const int32_t* d_counts, const int32_t* d_keys, const int64_t* d_perm, const int64_t* d_first,
                     double* d_out, int32_t* d_status, bool* done) {
     *done = false;
+    // (a buffer that is not to be had leaves the families to the tile walk)
+#define ROOM(expr)                                                        \
+    do {                                                                  \
+        const cudaError_t _e = (expr);                                    \
+        if (_e == cudaErrorMemoryAllocation) return CAFE_OK;              \
+        if (_e != cudaSuccess) return cuda_fail(C, _e, "pattern tables"); \
+    } while (0)
     if (pat64_class({0, S, 1}) < 0 || NS > INT32_MAX) return CAFE_OK;
     const int ni = (int)T.internal.size(), n = T.n_nodes, ng = S + 1;
     const cudaStream_t st = ws.stream;
@@ -2624,11 +2664,11 @@ int prune_simulated(cafe_ctx* C, Workspace& ws, const TreeHost& T, int S, int RR
     const size_t o_list = ints.size();
     for (int c = 0; c <= S; ++c) ints.push_back(c);
     TempBuf d_ints(st), d_rep(st), d_num(st), d_base(st), d_tab(st), d_off(st), d_child(st), d_table(st), d_desc(st);
-    CK(d_ints.get(ints.size() * sizeof(int32_t)), "patterns");
-    CK(d_rep.get((size_t)ni * NS * sizeof(int32_t)), "patterns");
-    CK(d_num.get((size_t)ni * NS * sizeof(int32_t)), "patterns");
-    CK(d_base.get((size_t)ni * (ng + 1) * sizeof(int32_t)), "patterns");
-    CK(d_tab.get(batch * slots * sizeof(int32_t)), "patterns");
+    ROOM(d_ints.get(ints.size() * sizeof(int32_t)));
+    ROOM(d_rep.get((size_t)ni * NS * sizeof(int32_t)));
+    ROOM(d_num.get((size_t)ni * NS * sizeof(int32_t)));
+    ROOM(d_base.get((size_t)ni * (ng + 1) * sizeof(int32_t)));
+    ROOM(d_tab.get(batch * slots * sizeof(int32_t)));
     CK(cudaMemcpyAsync(d_ints.p, ints.data(), ints.size() * sizeof(int32_t), cudaMemcpyHostToDevice, st), "patterns");
     PatBuildArgs a;
     std::memset(&a, 0, sizeof a);
@@ -2672,8 +2712,8 @@ int prune_simulated(cafe_ctx* C, Workspace& ws, const TreeHost& T, int S, int RR
             }
         if (group_doubles[g] > limit) return CAFE_OK;
     }
-    CK(d_child.get(n_child * sizeof(int32_t)), "patterns");
-    CK(d_off.get(child_off.size() * sizeof(int64_t)), "patterns");
+    ROOM(d_child.get(n_child * sizeof(int32_t)));
+    ROOM(d_off.get(child_off.size() * sizeof(int64_t)));
     CK(cudaMemcpyAsync(d_off.p, child_off.data(), child_off.size() * sizeof(int64_t), cudaMemcpyHostToDevice, st),
        "patterns");
     CK(launch_pat_write(a, d_dd, n_dd, d_off.as<int64_t>(), d_child.as<int32_t>(), st), "patterns");
@@ -2689,7 +2729,7 @@ int prune_simulated(cafe_ctx* C, Workspace& ws, const TreeHost& T, int S, int RR
         passes.back().doubles += group_doubles[g];
         most = std::max(most, passes.back().doubles);
     }
-    CK(d_table.get((leaf_doubles + most) * sizeof(double)), "factor tables");
+    ROOM(d_table.get((leaf_doubles + most) * sizeof(double)));
     const int TP = kPat64Rows, TS = kPat64States;
     const int lp = pat64_lp(S), n_bufs = pat64_bufs(lp, 1);
     const int32_t active0 = 0;
@@ -2753,7 +2793,7 @@ int prune_simulated(cafe_ctx* C, Workspace& ws, const TreeHost& T, int S, int RR
         if (!cdesc.empty()) std::memcpy(blob.data() + o_cdesc, cdesc.data(), cdesc.size() * sizeof(int32_t));
         std::memcpy(blob.data() + o_active, &active0, sizeof active0);
         TempBuf d_blob(st);
-        CK(d_blob.get(bytes), "pattern nodes");
+        ROOM(d_blob.get(bytes));
         char* d = d_blob.as<char>();
         CK(cudaMemcpyAsync(d, blob.data(), o_done, cudaMemcpyHostToDevice, st), "pattern nodes");
         CK(cudaMemsetAsync(d + o_done, 0, bytes - o_done, st), "pattern nodes");
@@ -2806,6 +2846,7 @@ int prune_simulated(cafe_ctx* C, Workspace& ws, const TreeHost& T, int S, int RR
     }
     *done = true;
     return CAFE_OK;
+#undef ROOM
 }
 
 // compute_pvalues with the simulated families drawn on the GPU (k_pvalue.cu:
@@ -2832,7 +2873,8 @@ int pvalues_device(cafe_ctx* C, Workspace& ws, const ReconSetup& Z, bool stream,
     const int64_t max_tiles = NS / 32 + n_keys + 1;
     const int Wmax = std::max(S + 1, RR);
     DevBuf d_cdf, d_sizes, d_sim, d_keys, d_hist, d_cursor, d_perm, d_tiles, d_ntiles, d_simL, d_obsL, d_pv, d_tree,
-        d_otiles, d_first;
+        d_otiles, d_first, d_words, d_len, d_starts, d_mt;
+    DrainOnError drain{ws};      // (before those go)
     CK(d_cdf.reserve((size_t)n * n_ps * S * sizeof(double)), "row cdfs");
     CK(d_sizes.reserve((size_t)NS * n * sizeof(int32_t)), "simulated families");
     CK(d_sim.reserve(std::max<size_t>((size_t)NS * L, 1) * sizeof(int32_t)), "simulated families");
@@ -2859,7 +2901,8 @@ int pvalues_device(cafe_ctx* C, Workspace& ws, const ReconSetup& Z, bool stream,
         tree_tab[3 * n + i] = T.internal_index[i];
     }
     CK(d_tree.reserve(tree_tab.size() * sizeof(int32_t)), "tree");
-    CK(cudaMemcpy(d_tree.p, tree_tab.data(), tree_tab.size() * sizeof(int32_t), cudaMemcpyHostToDevice), "tree");
+    CK(cudaMemcpyAsync(d_tree.p, tree_tab.data(), tree_tab.size() * sizeof(int32_t), cudaMemcpyHostToDevice, ws.stream),
+       "tree");
     // observed families: states 0..S, root sizes 1..R
     std::vector<PruneTile> otiles;
     for (int64_t f = 0; f < F && !obs_rows; f += 32) {
@@ -2873,7 +2916,8 @@ int pvalues_device(cafe_ctx* C, Workspace& ws, const ReconSetup& Z, bool stream,
     }
     if (!otiles.empty()) {
         CK(d_otiles.reserve(otiles.size() * sizeof(PruneTile)), "tiles");
-        CK(cudaMemcpy(d_otiles.p, otiles.data(), otiles.size() * sizeof(PruneTile), cudaMemcpyHostToDevice), "tiles");
+        CK(cudaMemcpyAsync(d_otiles.p, otiles.data(), otiles.size() * sizeof(PruneTile), cudaMemcpyHostToDevice, ws.stream),
+           "tiles");
     }
     const int n_ctas_max = C->n_ctas;
     CK(ws.scratch.reserve((size_t)n_ctas_max * T.n_slots * Wmax * 32 * sizeof(double)), "scratch");
@@ -2893,7 +2937,6 @@ int pvalues_device(cafe_ctx* C, Workspace& ws, const ReconSetup& Z, bool stream,
        "row cdfs");
     // the reference's stream: its words and where each family's draws start, on
     // an auxiliary stream while the observed families are pruned
-    DevBuf d_words, d_len, d_starts, d_mt;
     struct Join {      // (whatever happens in between, the buffers' stream waits for the other one)
         Workspace& ws;
         bool on = false;
@@ -3050,6 +3093,7 @@ int pvalues_device(cafe_ctx* C, Workspace& ws, const ReconSetup& Z, bool stream,
     int32_t status = 0;
     CK(cudaMemcpyAsync(&status, d_status, sizeof status, cudaMemcpyDeviceToHost, ws.stream), "d2h");
     CK(cudaStreamSynchronize(ws.stream), "p-values");
+    drain.ok = true;
     if (status) return fail(C, CAFE_ERR_TIMEOUT, "p-values gave up waiting for a subtree");
     float ms = 0;
     cudaEventElapsedTime(&ms, ws.ev_start, ws.ev_stop);
@@ -3071,6 +3115,7 @@ int pvalues_device(cafe_ctx* C, Workspace& ws, const ReconSetup& Z, bool stream,
 // with the root fixed, and the observed families) run on the GPU.
 int pvalues_sync(cafe_ctx* C, Workspace& ws, const cafe_request* R, cafe_pvalues_out* out) {
     AllocScope scope(ws.stream);
+    AllocLimit limit(C->debug_alloc_limit);
     if (ws.staged) {
         CK(cudaEventSynchronize(ws.ev_staged), "staging");
         ws.staged = false;
@@ -3085,7 +3130,8 @@ int pvalues_sync(cafe_ctx* C, Workspace& ws, const cafe_request* R, cafe_pvalues
         host_ms = host_ms_since(t_host0);
         rc = pvalues_device(C, ws, Z, !out->device_sampling, out);
         if (!rc) out->host_ms += host_ms;
-        return rc;
+        // (drawn on the host, the simulation needs no words, starts and cdfs on the device)
+        if (rc != CAFE_ERR_OOM || out->device_sampling) return rc;
     }
     TreeHost& T = *Z.T;
     FamSet& FS = *Z.S;
@@ -3104,6 +3150,7 @@ int pvalues_sync(cafe_ctx* C, Workspace& ws, const cafe_request* R, cafe_pvalues
     const int Wmax = std::max(S + 1, RR);
     const int64_t max_tiles = NS / 32 + (int64_t)RR * (S + 2) + F / 32 + 2;
     DevBuf d_sim, d_perm, d_simL, d_obsL, d_tiles;
+    DrainOnError drain{ws};      // (before those go)
     CK(d_sim.reserve(std::max<size_t>((size_t)NS * L, 1) * sizeof(int32_t)), "simulated families");
     CK(d_perm.reserve(std::max<int64_t>(NS, 1) * sizeof(int64_t)), "simulated families");
     CK(d_simL.reserve(std::max<int64_t>(NS, 1) * sizeof(double)), "simulated likelihoods");
@@ -3227,6 +3274,7 @@ int pvalues_sync(cafe_ctx* C, Workspace& ws, const cafe_request* R, cafe_pvalues
     if (F) CK(cudaMemcpyAsync(obsL.data(), d_obsL.p, obsL.size() * sizeof(double), cudaMemcpyDeviceToHost, ws.stream),
               "d2h");
     CK(cudaStreamSynchronize(ws.stream), "p-values");
+    drain.ok = true;
     float ms = 0;
     cudaEventElapsedTime(&ms, ws.ev_start, ws.ev_stop);
     const auto t_pv = std::chrono::steady_clock::now();
@@ -3385,6 +3433,11 @@ int cafe_debug_set(cafe_ctx* C, int knob, int64_t value) {
     if (knob == CAFE_DEBUG_TC_WAIT_LIMIT) {
         if (value < 0 || value > ((int64_t)1 << 30)) return fail(C, CAFE_ERR_INVALID, "wait limit out of range");
         C->debug_wait_limit = (int)value;
+        return CAFE_OK;
+    }
+    if (knob == CAFE_DEBUG_ALLOC_LIMIT) {
+        if (value < 0) return fail(C, CAFE_ERR_INVALID, "allocation limit out of range");
+        C->debug_alloc_limit = (size_t)value;
         return CAFE_OK;
     }
     return fail(C, CAFE_ERR_INVALID, "unknown debug knob %d", knob);
@@ -3808,6 +3861,8 @@ int cafe_score_batch_device(cafe_ctx* C, const cafe_request* req, int n, double*
     C->dev_flip ^= 1;
     Workspace& ws = C->dev_flip ? *C->ws_alt : *C->ws[0];
     AllocScope scope(ws.stream);
+    AllocLimit limit(C->debug_alloc_limit);
+    DrainOnError drain{ws};
     cudaStream_t user = static_cast<cudaStream_t>(stream);
     ScoreInfo info;
     auto si = C->sets.find(req ? req->set_id : -1);
@@ -3833,6 +3888,7 @@ int cafe_score_batch_device(cafe_ctx* C, const cafe_request* req, int n, double*
         CK(cudaEventRecord(ws.ev_stop, ws.stream), "event");
         CK(cudaStreamWaitEvent(user, ws.ev_stop, 0), "event");
     }
+    drain.ok = true;
     return CAFE_OK;
 }
 

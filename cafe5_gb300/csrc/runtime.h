@@ -266,6 +266,7 @@ struct cafe_ctx {
     uint64_t request_stamp = 0;
     std::map<int, int> tuned;    // bin width -> CTAs per SM chosen by cafe_autotune
     int debug_wait_limit = 0;    // cafe_debug_set: polls before the tensor-core wait for a node's GEMMs gives up
+    size_t debug_alloc_limit = 0;   // cafe_debug_set: larger device buffers are not to be had (0: no limit)
     // workspaces: [0] for synchronous calls, [1..] for the serving loop
     std::vector<std::unique_ptr<cafe::Workspace>> ws;
     std::unique_ptr<cafe::Workspace> ws_alt;   // second workspace of the device-pointer calls

@@ -113,8 +113,10 @@ int cafe_version(void);
  * up after n - 1 polls (1: at once); 0 restores the default bound of 2^24
  * polls. With 1 a test can check that the kernel drains its own copies and
  * MMAs, frees TMEM, and the call returns CAFE_ERR_TIMEOUT with the context
- * still usable. */
-typedef enum { CAFE_DEBUG_TC_WAIT_LIMIT = 1 } cafe_debug_knob;
+ * still usable. CAFE_DEBUG_ALLOC_LIMIT: value n > 0 makes every device buffer
+ * of more than n bytes that a later call asks for (matrices apart) fail as if
+ * memory had run out; 0 lifts it. */
+typedef enum { CAFE_DEBUG_TC_WAIT_LIMIT = 1, CAFE_DEBUG_ALLOC_LIMIT = 2 } cafe_debug_knob;
 int cafe_debug_set(cafe_ctx* ctx, int knob, int64_t value);
 
 /* ---- inputs ---------------------------------------------------------- */
