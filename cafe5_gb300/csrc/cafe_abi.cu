@@ -584,6 +584,7 @@ int build_patterns(cafe_ctx* C, const TreeHost& T, FamSet& S, const int64_t* d_p
 }
 
 int prepare_set(cafe_ctx* C, FamSet& S) {
+    AllocLimit limit(C->debug_alloc_limit);
     const int64_t F = S.F;
     const int nl = S.n_leaves;
     S.max_count.assign(F, 0);
@@ -1815,6 +1816,7 @@ int enqueue_score(cafe_ctx* C, Workspace& ws, const cafe_request* Rs, int NB, do
     TreeHost& T = *ti->second;
     FamSet& S = *si->second;
     if (S.tree_id != R->tree_id) return fail(C, CAFE_ERR_INVALID, "family set %d belongs to tree %d", R->set_id, S.tree_id);
+    if (!S.ready) return fail(C, CAFE_ERR_INVALID, "family set %d has no counts (its last update failed)", R->set_id);
     const bool gamma = R->model == CAFE_MODEL_GAMMA;
     if (R->model != CAFE_MODEL_BASE && !gamma) return fail(C, CAFE_ERR_INVALID, "bad model %d", R->model);
     const int K = gamma ? R->n_categories : 1;
@@ -2215,6 +2217,7 @@ int recon_setup(cafe_ctx* C, Workspace& ws, const cafe_request* R, bool categori
     TreeHost& T = *ti->second;
     FamSet& S = *si->second;
     if (S.tree_id != R->tree_id) return fail(C, CAFE_ERR_INVALID, "family set %d belongs to tree %d", R->set_id, S.tree_id);
+    if (!S.ready) return fail(C, CAFE_ERR_INVALID, "family set %d has no counts (its last update failed)", R->set_id);
     const bool gamma = categories && R->model == CAFE_MODEL_GAMMA;
     if (R->model != CAFE_MODEL_BASE && R->model != CAFE_MODEL_GAMMA) return fail(C, CAFE_ERR_INVALID, "bad model %d", R->model);
     const int K = gamma ? R->n_categories : 1;
@@ -3621,6 +3624,7 @@ int cafe_families_upload(cafe_ctx* C, int tree_id, const int32_t* counts, int64_
     if (n_families) CK(cudaMemcpy(S->d_counts.p, counts, (size_t)n_families * n_leaves * sizeof(int32_t), cudaMemcpyHostToDevice), "counts");
     int rc = prepare_set(C, *S);
     if (rc) return rc;
+    S->ready = true;
     *set_id = C->next_set++;
     C->sets[*set_id] = std::move(S);
     return CAFE_OK;
@@ -3635,17 +3639,23 @@ int cafe_families_update(cafe_ctx* C, int set_id, const int32_t* counts) {
     FamSet& S = *si->second;
     const size_t n = (size_t)S.F * S.n_leaves;
     if (!counts && n) return fail(C, CAFE_ERR_INVALID, "null counts");
-    // unchanged counts keep their derived tables (maxima, duplicates, bins)
-    const bool same = S.h_counts.size() == n && (n == 0 || std::memcmp(S.h_counts.data(), counts, n * sizeof(int32_t)) == 0);
+    // unchanged counts keep their derived tables (maxima, bins, patterns)
+    const bool same = S.ready && S.h_counts.size() == n &&
+                      (n == 0 || std::memcmp(S.h_counts.data(), counts, n * sizeof(int32_t)) == 0);
     if (!same) {
         for (size_t i = 0; i < n; ++i)
             if (counts[i] < 0) return fail(C, CAFE_ERR_INVALID, "negative count");
+        CK(cudaDeviceSynchronize(), "counts");      // (calls in flight read what is replaced here)
+        S.ready = false;      // until every table is that of the new counts
         S.h_counts.assign(counts, counts + n);
     }
     Workspace& ws = *C->ws[0];
     CK(cudaMemcpyAsync(S.d_counts.p, counts, n * sizeof(int32_t), cudaMemcpyHostToDevice, ws.stream), "counts");
     CK(cudaStreamSynchronize(ws.stream), "counts");
-    return same ? CAFE_OK : prepare_set(C, S);
+    if (same) return CAFE_OK;
+    const int rc = prepare_set(C, S);
+    S.ready = rc == CAFE_OK;
+    return rc;
 }
 
 int cafe_families_free(cafe_ctx* C, int set_id) {

@@ -87,6 +87,7 @@ struct FamSet {
     int tree_id = 0;
     int64_t F = 0;
     int n_leaves = 0;
+    bool ready = false;               // every table below is that of h_counts
     DevBuf d_counts;
     std::vector<int32_t> h_counts;
     std::vector<int32_t> max_count;

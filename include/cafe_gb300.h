@@ -135,8 +135,10 @@ int cafe_tree_upload(cafe_ctx* ctx, int n_nodes, const int32_t* parent, const do
 int cafe_families_upload(cafe_ctx* ctx, int tree_id, const int32_t* counts, int64_t n_families, int n_leaves,
                          int* set_id);
 /* Replace the counts of an existing set in place (same shape): always
- * copied to the device; the derived tables (per-family maxima, duplicate
- * rows, S-bins) are rebuilt only when the counts differ from the set's. */
+ * copied to the device; the derived tables (per-family maxima, S-bins, distinct
+ * subtree patterns) are rebuilt only when the counts differ from the set's.
+ * After an update that failed the set has no counts: calls that use it are
+ * refused until an update succeeds. */
 int cafe_families_update(cafe_ctx* ctx, int set_id, const int32_t* counts);
 int cafe_families_free(cafe_ctx* ctx, int set_id);
 

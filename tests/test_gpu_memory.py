@@ -55,3 +55,40 @@ def test_pvalues_without_room_for_tables(ctx, device_sampling):
     # (every other buffer takes at most 8 MB: the words, 22 draws of 8 bytes of 45,000 families)
     assert done[16]
     assert device_sampling or done[4]
+
+
+@pytest.mark.parametrize("F", [40, 6000])
+def test_update_that_runs_out_of_memory(ctx, F):
+    """A failed cafe_families_update leaves no half-built tables in use: scores are
+    refused (invalid), the same update repeated rebuilds everything, and the
+    results are those of a set uploaded with these counts. From identical
+    families to distinct ones, so that the pattern tables grow."""
+    from cafe5_gb300.inputs import RootPrior
+    from cafe5_gb300.synth import workload
+    w = workload(1, n_families=F, seed=9)
+    b = w.families.counts
+    a = np.ascontiguousarray(np.tile(b[:1], (F, 1)))
+    tid = ctx.upload_tree(w.tree)
+    ctx.set_prior(RootPrior.uniform(150).vector())
+    modes = [dict(precision="fp64_ref", S=170, R=150), dict(precision="fp64_binned"), dict(precision="mixed_tf32x3")]
+
+    def scores(sid):
+        return [ctx.score(tid, sid, [0.002], **m).family_lnl for m in modes]
+
+    fresh = scores(ctx.upload_families(tid, b))
+    failed = 0
+    for k in range(9, 25):
+        sid = ctx.upload_families(tid, a)
+        if _limited(ctx, 1 << k, lambda: ctx.update_families(sid, b) or True) is None:
+            failed += 1
+            for m in modes:
+                with pytest.raises(_lib.CafeError) as e:
+                    ctx.score(tid, sid, [0.002], **m)
+                assert e.value.code == 6
+            with pytest.raises(_lib.CafeError) as e:
+                ctx.reconstruct(tid, sid, [0.002], S=170, R=150)
+            assert e.value.code == 6
+            ctx.update_families(sid, b)
+        assert all(np.array_equal(x, y) for x, y in zip(scores(sid), fresh))
+        ctx.free_families(sid)
+    assert failed > 0
