@@ -393,6 +393,7 @@ int upload_plan(cafe_ctx* C, TreeHost& T) {
 
 // The S-bin of a family with largest count mx.
 int bin_width(int mx) {
+    if (mx > kDefaultBins[kNumDefaultBins - 1]) return kDefaultBins[kNumDefaultBins - 1];
     const int need = (int)std::ceil(1.2 * mx) + 20 + 1;
     for (int i = 0; i < kNumDefaultBins; ++i)
         if (kDefaultBins[i] >= need) return kDefaultBins[i];
@@ -408,9 +409,10 @@ int compute_bins(cafe_ctx* C, FamSet& S) {
         const int w = bin_width(mx);
         wf[f] = w;
         const int Sf = w - 1;
-        rf[f] = std::min(Sf, std::max(30, (int)std::rint(mx * 1.25)));
+        rf[f] = (int)std::min((double)Sf, std::max(30.0, std::rint(mx * 1.25)));
     }
-    std::vector<int64_t> perm(F);
+    std::vector<int64_t>& perm = B.perm;
+    perm.resize(F);
     std::iota(perm.begin(), perm.end(), 0);
     std::stable_sort(perm.begin(), perm.end(), [&](int64_t a, int64_t b) { return wf[a] < wf[b]; });
     B.widths.clear();
@@ -465,8 +467,10 @@ struct TempBuf {
 
 // The distinct patterns of every subtree, for families grouped as in `first`
 // / `count` over perm: built on the device, one launch per tree level.
-int build_patterns(cafe_ctx* C, const TreeHost& T, FamSet& S, const int64_t* d_perm, const std::vector<int64_t>& first,
-                   const std::vector<int64_t>& count, const std::vector<int>& max_count, TempBuf& mem, PatternPlan& P) {
+constexpr int kFlaggedCounts = 1 << 14;
+
+int build_patterns(cafe_ctx* C, const TreeHost& T, FamSet& S, const int64_t* d_perm, const std::vector<int64_t>& perm,
+                   const std::vector<int64_t>& first, const std::vector<int64_t>& count, const std::vector<int>& max_count, TempBuf& mem, PatternPlan& P) {
     const int64_t F = S.F;
     const int ni = (int)T.internal.size(), ng = (int)first.size();
     P.n_groups = ng;
@@ -498,9 +502,12 @@ int build_patterns(cafe_ctx* C, const TreeHost& T, FamSet& S, const int64_t* d_p
     int64_t n_flags = 0;
     std::vector<int64_t> longs(first);            // the groups' first items, F; their first flags
     longs.push_back(F);
-    std::vector<int64_t> flag_off;
-    for (int g = 0; g < ng; ++g) {
-        flag_off.push_back(n_flags);
+    std::vector<int64_t> flag_off(ng, 0);
+    // the counts that occur at a leaf: flagged on the device, a byte for every
+    // possible one, or (counts past kFlaggedCounts) sorted here
+    const bool flagged = *std::max_element(max_count.begin(), max_count.end()) < kFlaggedCounts;
+    for (int g = 0; flagged && g < ng; ++g) {
+        flag_off[g] = n_flags;
         n_flags += (int64_t)T.n_leaves * (max_count[g] + 1);
     }
     longs.insert(longs.end(), flag_off.begin(), flag_off.end());
@@ -535,8 +542,10 @@ int build_patterns(cafe_ctx* C, const TreeHost& T, FamSet& S, const int64_t* d_p
     a.flag_off = a.group_first + ng + 1;
     a.group_max = d_ints + n_nodes_list;
     uint8_t* d_flags = reinterpret_cast<uint8_t*>(d + o_flags);
-    CK(cudaMemsetAsync(d_flags, 0, (size_t)n_flags, st), "patterns");
-    CK(launch_pat_counts(a, d_flags, st), "patterns");
+    if (flagged) {
+        CK(cudaMemsetAsync(d_flags, 0, (size_t)n_flags, st), "patterns");
+        CK(launch_pat_counts(a, d_flags, st), "patterns");
+    }
     a.rep = reinterpret_cast<int32_t*>(d + o_rep);
     a.num = reinterpret_cast<int32_t*>(d + o_num);
     a.base = reinterpret_cast<int32_t*>(d + o_base);
@@ -551,7 +560,7 @@ int build_patterns(cafe_ctx* C, const TreeHost& T, FamSet& S, const int64_t* d_p
     CK(launch_pat_number(a, d_ints + T.n_nodes, ni - 1, st), "patterns");
     std::vector<int32_t> base((size_t)ni * (ng + 1));
     std::vector<uint8_t> flags((size_t)n_flags);
-    CK(cudaMemcpyAsync(flags.data(), d_flags, flags.size(), cudaMemcpyDeviceToHost, st), "patterns");
+    if (flagged) CK(cudaMemcpyAsync(flags.data(), d_flags, flags.size(), cudaMemcpyDeviceToHost, st), "patterns");
     CK(cudaMemcpyAsync(base.data(), a.base, base.size() * sizeof(int32_t), cudaMemcpyDeviceToHost, st), "patterns");
     CK(cudaStreamSynchronize(st), "patterns");
     int64_t off = 0;
@@ -571,6 +580,13 @@ int build_patterns(cafe_ctx* C, const TreeHost& T, FamSet& S, const int64_t* d_p
     for (int g = 0; g < ng; ++g)
         for (int c = 0; c < T.n_leaves; ++c) {
             P.leaf_off.push_back((int64_t)used.size());
+            if (!flagged) {
+                const auto at = used.size();
+                for (int64_t i = first[g]; i < first[g] + count[g]; ++i) used.push_back(S.h_counts[perm[i] * T.n_leaves + c]);
+                std::sort(used.begin() + at, used.end());
+                used.erase(std::unique(used.begin() + at, used.end()), used.end());
+                continue;
+            }
             const uint8_t* f = flags.data() + flag_off[g] + (size_t)c * (max_count[g] + 1);
             for (int n = 0; n <= max_count[g]; ++n)
                 if (f[n]) used.push_back(n);
@@ -611,9 +627,10 @@ int prepare_set(cafe_ctx* C, FamSet& S) {
         all_max = std::max(all_max, m);
     }
     TempBuf mem(C->ws[0]->stream_hi);
-    rc = build_patterns(C, T, S, S.bins.d_perm.as<int64_t>(), S.bins.bin_first, S.bins.bin_count, bin_max, mem, S.pat_bins);
+    rc = build_patterns(C, T, S, S.bins.d_perm.as<int64_t>(), S.bins.perm, S.bins.bin_first, S.bins.bin_count, bin_max, mem,
+                        S.pat_bins);
     if (!rc)
-        rc = build_patterns(C, T, S, S.d_identity.as<int64_t>(), {0}, {F}, {all_max}, mem, S.pat_all);
+        rc = build_patterns(C, T, S, S.d_identity.as<int64_t>(), ident, {0}, {F}, {all_max}, mem, S.pat_all);
     return rc;
 }
 

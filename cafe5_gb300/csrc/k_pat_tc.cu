@@ -167,7 +167,7 @@ __device__ __forceinline__ bool leaf_ok(const PatTcArgs& a, int n) {
     const int S = a.W - 1;
     if (!a.err) return n <= S;
     const int h = (a.err_ndev - 1) / 2;
-    if (n + h > S) return false;
+    if (n > S - h) return false;
     const double* pr = a.err + (size_t)(n < a.err_rows ? n : a.err_rows - 1) * a.err_ndev;
     for (int d = max(0, h - n); d < a.err_ndev; ++d)
         if (__ldg(pr + d) > 0) return true;

@@ -66,6 +66,7 @@ struct BinPlan {
     // families grouped by bin; perm holds family indices bin by bin
     std::vector<int> widths;                 // bin widths used
     std::vector<int64_t> bin_first, bin_count;
+    std::vector<int64_t> perm;
     DevBuf d_perm, d_famR, d_itemR;          // d_itemR: root bounds in perm order
     int W_max = 0;
 };
