@@ -429,15 +429,20 @@ int compute_bins(cafe_ctx* C, FamSet& S) {
         B.bin_count.back()++;
         B.W_max = std::max(B.W_max, w);
     }
-    std::vector<int32_t> rf32(rf.begin(), rf.end());
-    CK(B.d_perm.reserve(std::max<int64_t>(F, 1) * sizeof(int64_t)), "bins");
+    // the families in bin order, then in their own; root bounds by family and in
+    // bin order
+    std::vector<int64_t> items(perm);
+    items.resize(2 * F);
+    std::iota(items.begin() + F, items.end(), 0);
+    std::vector<int32_t> rf32(rf.begin(), rf.end()), item_R(F);
+    for (int64_t i = 0; i < F; ++i) item_R[i] = rf[perm[i]];
+    CK(S.d_items.reserve(std::max<int64_t>(2 * F, 1) * sizeof(int64_t)), "bins");
     CK(B.d_famR.reserve(std::max<int64_t>(F, 1) * sizeof(int32_t)), "bins");
+    CK(B.d_itemR.reserve(std::max<int64_t>(F, 1) * sizeof(int32_t)), "bins");
     if (F) {
-        CK(cudaMemcpy(B.d_perm.p, perm.data(), F * sizeof(int64_t), cudaMemcpyHostToDevice), "bins");
-        CK(cudaMemcpy(B.d_famR.p, rf32.data(), F * sizeof(int32_t), cudaMemcpyHostToDevice), "bins");
-        for (int64_t i = 0; i < F; ++i) rf32[i] = rf[perm[i]];
-        CK(B.d_itemR.reserve(F * sizeof(int32_t)), "bins");
-        CK(cudaMemcpy(B.d_itemR.p, rf32.data(), F * sizeof(int32_t), cudaMemcpyHostToDevice), "bins");
+        CK(cudaMemcpyAsync(S.d_items.p, items.data(), 2 * F * sizeof(int64_t), cudaMemcpyHostToDevice, C->setup), "bins");
+        CK(cudaMemcpyAsync(B.d_famR.p, rf32.data(), F * sizeof(int32_t), cudaMemcpyHostToDevice, C->setup), "bins");
+        CK(cudaMemcpyAsync(B.d_itemR.p, item_R.data(), F * sizeof(int32_t), cudaMemcpyHostToDevice, C->setup), "bins");
     }
     return CAFE_OK;
 }
@@ -465,46 +470,155 @@ struct TempBuf {
     template <class T> T* as() const { return static_cast<T*>(p); }
 };
 
-// The distinct patterns of every subtree, for families grouped as in `first`
-// / `count` over perm: built on the device, one launch per tree level.
 constexpr int kFlaggedCounts = 1 << 14;
 
-int build_patterns(cafe_ctx* C, const TreeHost& T, FamSet& S, const int64_t* d_perm, const std::vector<int64_t>& perm,
-                   const std::vector<int64_t>& first, const std::vector<int64_t>& count, const std::vector<int>& max_count, TempBuf& mem, PatternPlan& P) {
+// ---- the distinct patterns of every subtree, for the families of every S-bin
+// (the plan's groups, in the order of the bins) and for all of them together
+// (its last group). Items are the families in bin order, then in their own.
+
+// Appends the counts that occur at leaf c of group g, from a flag for every
+// count of the group up to kFlaggedCounts; with larger ones they are sorted.
+void list_counts(const FamSet& S, PatternPlan& P, int g, int c, const uint8_t* flag, std::vector<int32_t>& used) {
+    const size_t at = used.size();
+    P.leaf_off.push_back((int64_t)at);
+    if (P.group_max[g] < kFlaggedCounts) {
+        for (int n = 0; n <= P.group_max[g]; ++n)
+            if (flag[n]) used.push_back(n);
+        return;
+    }
+    for (int64_t i = P.group_first[g]; i < P.group_first[g] + P.group_count[g]; ++i)
+        used.push_back(S.h_counts[(i < S.F ? S.bins.perm[i] : i - S.F) * S.n_leaves + c]);
+    std::sort(used.begin() + at, used.end());
+    used.erase(std::unique(used.begin() + at, used.end()), used.end());
+}
+
+// On the host: the rows of all families together, by hashing (a node's key is
+// its children's, two at a time); then those that occur in each group.
+void patterns_on_host(const TreeHost& T, const FamSet& S, PatternPlan& P, std::vector<int32_t>& child,
+                      std::vector<int32_t>& used) {
     const int64_t F = S.F;
-    const int ni = (int)T.internal.size(), ng = (int)first.size();
-    P.n_groups = ng;
-    P.n_internal = ni;
-    P.group_first = first;
-    P.group_count = count;
-    P.group_max = max_count;
-    P.rows.assign((size_t)ng * ni, 0);
-    P.child_off.assign((size_t)ng * ni, 0);
-    if (!F) return CAFE_OK;
-    CK(cudaDeviceSynchronize(), "patterns");      // the counts and the order are on the device, and no call in flight reads the old plan
-    if (ng > kMaxGroups) return fail(C, CAFE_ERR_INVALID, "%d family groups", ng);
-    const cudaStream_t st = C->ws[0]->stream_hi;
+    const int ni = P.n_internal, nl = S.n_leaves;
+    struct Slot {
+        uint64_t key;
+        int32_t row, stamp;
+    };
+    size_t slots = 16;
+    while (slots < 2 * (size_t)F) slots *= 2;
+    std::vector<Slot> table(slots, Slot{0, 0, 0});
+    std::vector<int32_t> col((size_t)nl * F), row((size_t)ni * F);      // the counts by leaf; a family's row at a node
+    for (int64_t f = 0; f < F; ++f)
+        for (int c = 0; c < nl; ++c) col[c * F + f] = S.h_counts[f * nl + c];
+    std::vector<std::vector<int32_t>> kids(ni);      // the rows' counts (leaves) and children's rows
+    std::vector<const int32_t*> key;
+    int32_t stamp = 0;
+    for (int ii = 0; ii < ni; ++ii) {
+        const int c0 = T.cstart[ii], nch = T.cstart[ii + 1] - c0;
+        key.clear();
+        for (int c = 0; c < nch; ++c) {
+            const int ch = T.child[c0 + c], lc = T.leaf_col[ch];
+            key.push_back(lc >= 0 ? &col[(size_t)lc * F] : &row[(size_t)T.internal_index[ch] * F]);
+        }
+        kids[ii].resize(F * nch);
+        int32_t *r = &row[(size_t)ii * F], *k0 = kids[ii].data();
+        if (ii + 1 == ni) {      // (the root keeps a row per family)
+            for (int64_t f = 0; f < F; ++f)
+                for (int c = 0; c < nch; ++c) *k0++ = key[c][f];
+            break;
+        }
+        for (int c = std::min(1, nch - 1); c < nch; ++c) {
+            const int32_t* left = c == 0 ? nullptr : c == 1 ? key[0] : r;
+            ++stamp;
+            int32_t n = 0;
+            for (int64_t f = 0; f < F; ++f) {
+                const uint64_t k = (left ? (uint64_t)(uint32_t)left[f] << 32 : 0) | (uint32_t)key[c][f];
+                size_t s = (size_t)((k * 0x9E3779B97F4A7C15ull) >> 32) & (slots - 1);
+                while (table[s].stamp == stamp && table[s].key != k) s = (s + 1) & (slots - 1);
+                if (table[s].stamp != stamp) {
+                    table[s] = Slot{k, n++, stamp};
+                    if (c + 1 == nch)
+                        for (int x = 0; x < nch; ++x) *k0++ = key[x][f];
+                }
+                r[f] = table[s].row;
+            }
+        }
+        kids[ii].resize(k0 - kids[ii].data());
+    }
+    std::vector<std::vector<int32_t>> id(ni);       // a row's number in the group, -1: does not occur there
+    std::vector<uint8_t> flag;
+    for (int g = 0; g < P.n_groups; ++g) {
+        const bool all = g == P.all();
+        const int64_t i0 = P.group_first[g], n = P.group_count[g];
+        const size_t span = (size_t)std::min(P.group_max[g], kFlaggedCounts) + 1;
+        if (!all) {
+            for (int ii = 0; ii + 1 < ni; ++ii) id[ii].assign(kids[ii].size() / (T.cstart[ii + 1] - T.cstart[ii]), -1);
+            // parents come after their children: mark downwards
+            for (int ii = ni - 1; ii >= 0; --ii) {
+                const int c0 = T.cstart[ii], nch = T.cstart[ii + 1] - c0;
+                const int64_t rows = ii + 1 == ni ? n : (int64_t)id[ii].size();
+                for (int64_t q = 0; q < rows; ++q) {
+                    if (ii + 1 < ni && id[ii][q] < 0) continue;
+                    const int32_t* k = &kids[ii][(ii + 1 == ni ? S.bins.perm[i0 + q] : q) * nch];
+                    for (int c = 0; c < nch; ++c)
+                        if (const int ci = T.internal_index[T.child[c0 + c]]; ci >= 0) id[ci][k[c]] = 0;
+                }
+            }
+        }
+        flag.assign(nl * span, 0);
+        for (int ii = 0; ii < ni; ++ii) {
+            const bool root = ii + 1 == ni;
+            const int c0 = T.cstart[ii], nch = T.cstart[ii + 1] - c0;
+            const int64_t rows = root ? n : (int64_t)kids[ii].size() / nch;
+            int32_t here = 0;
+            P.child_off[(size_t)g * ni + ii] = (int64_t)child.size();
+            for (int64_t q = 0; q < rows; ++q) {
+                if (!all && !root) {
+                    if (id[ii][q] < 0) continue;
+                    id[ii][q] = here;
+                }
+                ++here;
+                const int32_t* k = &kids[ii][(root && !all ? S.bins.perm[i0 + q] : q) * nch];
+                for (int c = 0; c < nch; ++c) {
+                    const int ch = T.child[c0 + c], ci = T.internal_index[ch];
+                    if (ci < 0) flag[T.leaf_col[ch] * span + std::min(k[c], kFlaggedCounts)] = 1;
+                    child.push_back(ci < 0 || all ? k[c] : id[ci][k[c]]);
+                }
+            }
+            P.rows[(size_t)g * ni + ii] = here;
+        }
+        for (int c = 0; c < nl; ++c) list_counts(S, P, g, c, &flag[c * span], used);
+    }
+    P.leaf_off.push_back((int64_t)used.size());
+}
+
+// On the device, one launch per tree level.
+int patterns_on_device(cafe_ctx* C, const TreeHost& T, FamSet& S, PatternPlan& P, std::vector<int32_t>& used) {
+    const cudaStream_t st = C->setup;
+    const int64_t N = 2 * S.F;
+    const int ni = P.n_internal, ng = P.n_groups;
+    const std::vector<int>& max_count = P.group_max;
     int64_t slots = 1024;
-    while (slots < 2 * F) slots *= 2;
+    while (slots < 2 * N) slots *= 2;
     int max_h = 0;
     for (int h : T.height) max_h = std::max(max_h, h);
     std::vector<std::vector<int32_t>> level(max_h + 1);
     size_t widest = 1;
     for (int ii = 0; ii + 1 < ni; ++ii) level[T.height[ii]].push_back(ii);     // (the root, last, keeps a row per family)
     for (auto& l : level) widest = std::max(widest, l.size());
-    // the insertion tables take at most about 1 GB at a time
-    const size_t batch = std::max<size_t>(1, std::min(widest, ((size_t)1 << 30) / (slots * sizeof(int32_t))));
+    // the insertion tables take at most about 1 GB at a time; small ones are
+    // cleared together
+    const size_t fit = std::max<size_t>(1, ((size_t)1 << 30) / (slots * sizeof(int32_t)));
+    const bool together = (size_t)(ni - 1) * slots * sizeof(int32_t) <= (size_t)64 << 20;
+    const size_t batch = together ? (size_t)std::max(1, ni - 1) : std::min(widest, fit);
     std::vector<int32_t> ints = T.internal_index;
     for (auto& l : level) ints.insert(ints.end(), l.begin(), l.end());
     ints.push_back(ni - 1);
     const size_t n_nodes_list = ints.size();
     ints.insert(ints.end(), max_count.begin(), max_count.end());
     int64_t n_flags = 0;
-    std::vector<int64_t> longs(first);            // the groups' first items, F; their first flags
-    longs.push_back(F);
+    std::vector<int64_t> longs(P.group_first);            // the groups' first items, their number; their first flags
+    longs.push_back(N);
     std::vector<int64_t> flag_off(ng, 0);
-    // the counts that occur at a leaf: flagged on the device, a byte for every
-    // possible one, or (counts past kFlaggedCounts) sorted here
+    // the counts that occur at a leaf (list_counts)
     const bool flagged = *std::max_element(max_count.begin(), max_count.end()) < kFlaggedCounts;
     for (int g = 0; flagged && g < ng; ++g) {
         flag_off[g] = n_flags;
@@ -519,10 +633,11 @@ int build_patterns(cafe_ctx* C, const TreeHost& T, FamSet& S, const int64_t* d_p
         return at;
     };
     const size_t in_bytes = longs.size() * sizeof(int64_t) + ints.size() * sizeof(int32_t);
-    const size_t o_in = part(in_bytes), o_rep = part((size_t)ni * F * sizeof(int32_t)),
-                 o_num = part((size_t)ni * F * sizeof(int32_t)), o_base = part((size_t)ni * (ng + 1) * sizeof(int32_t)),
+    const size_t o_in = part(in_bytes), o_rep = part((size_t)ni * N * sizeof(int32_t)),
+                 o_num = part((size_t)ni * N * sizeof(int32_t)), o_base = part((size_t)ni * (ng + 1) * sizeof(int32_t)),
                  o_flags = part((size_t)n_flags), o_tab = part(batch * slots * sizeof(int32_t)),
                  o_off = part((size_t)ng * ni * sizeof(int64_t));
+    TempBuf mem(st);
     CK(mem.get(total), "patterns");
     char* d = mem.as<char>();
     std::vector<char> in(in_bytes);
@@ -534,9 +649,9 @@ int build_patterns(cafe_ctx* C, const TreeHost& T, FamSet& S, const int64_t* d_p
     std::memset(&a, 0, sizeof a);
     a.plan = T.plan;
     a.counts = S.d_counts.as<int32_t>();
-    a.perm = d_perm;
+    a.perm = S.bin_items();
     a.node_ii = d_ints;
-    a.F = F;
+    a.F = N;
     a.n_groups = ng;
     a.group_first = reinterpret_cast<const int64_t*>(d + o_in);
     a.flag_off = a.group_first + ng + 1;
@@ -552,22 +667,28 @@ int build_patterns(cafe_ctx* C, const TreeHost& T, FamSet& S, const int64_t* d_p
     int32_t* d_tab = reinterpret_cast<int32_t*>(d + o_tab);
     int64_t* d_off = reinterpret_cast<int64_t*>(d + o_off);
     const int32_t* d_nodes = d_ints + T.n_nodes;
+    if (together) CK(cudaMemsetAsync(d_tab, 0xff, batch * slots * sizeof(int32_t), st), "patterns");
     for (auto& l : level) {
-        for (size_t b = 0; b < l.size(); b += batch)
-            CK(launch_pat_insert(a, d_nodes + b, (int)std::min(batch, l.size() - b), d_tab, slots, st), "patterns");
+        for (size_t b = 0; b < l.size(); b += batch) {
+            const int m = (int)std::min(batch, l.size() - b);
+            if (!together) CK(cudaMemsetAsync(d_tab, 0xff, m * slots * sizeof(int32_t), st), "patterns");
+            CK(launch_pat_insert(a, d_nodes + b, m, d_tab, slots, st), "patterns");
+            if (together) d_tab += m * slots;
+        }
         d_nodes += l.size();
     }
     CK(launch_pat_number(a, d_ints + T.n_nodes, ni - 1, st), "patterns");
-    std::vector<int32_t> base((size_t)ni * (ng + 1));
-    std::vector<uint8_t> flags((size_t)n_flags);
-    if (flagged) CK(cudaMemcpyAsync(flags.data(), d_flags, flags.size(), cudaMemcpyDeviceToHost, st), "patterns");
-    CK(cudaMemcpyAsync(base.data(), a.base, base.size() * sizeof(int32_t), cudaMemcpyDeviceToHost, st), "patterns");
+    // (the flags lie behind the bases)
+    std::vector<char> back(o_flags - o_base + (size_t)n_flags);
+    CK(cudaMemcpyAsync(back.data(), d + o_base, back.size(), cudaMemcpyDeviceToHost, st), "patterns");
     CK(cudaStreamSynchronize(st), "patterns");
+    const int32_t* base = reinterpret_cast<const int32_t*>(back.data());
+    const uint8_t* flags = reinterpret_cast<const uint8_t*>(back.data() + (o_flags - o_base));
     int64_t off = 0;
     for (int g = 0; g < ng; ++g)
         for (int ii = 0; ii < ni; ++ii) {
-            const bool root = T.internal[ii] == T.root;
-            const int64_t r = root ? count[g] : base[(size_t)ii * (ng + 1) + g + 1] - base[(size_t)ii * (ng + 1) + g];
+            const bool root = ii == ni - 1;
+            const int64_t r = root ? P.group_count[g] : base[(size_t)ii * (ng + 1) + g + 1] - base[(size_t)ii * (ng + 1) + g];
             P.rows[(size_t)g * ni + ii] = r;
             P.child_off[(size_t)g * ni + ii] = off;
             off += r * (T.cstart[ii + 1] - T.cstart[ii]);
@@ -575,27 +696,47 @@ int build_patterns(cafe_ctx* C, const TreeHost& T, FamSet& S, const int64_t* d_p
     CK(P.d_child.reserve(std::max<int64_t>(off, 1) * sizeof(int32_t)), "patterns");
     CK(cudaMemcpyAsync(d_off, P.child_off.data(), P.child_off.size() * sizeof(int64_t), cudaMemcpyHostToDevice, st),
        "patterns");
-    std::vector<int32_t> used;
-    P.leaf_off.clear();
-    for (int g = 0; g < ng; ++g)
-        for (int c = 0; c < T.n_leaves; ++c) {
-            P.leaf_off.push_back((int64_t)used.size());
-            if (!flagged) {
-                const auto at = used.size();
-                for (int64_t i = first[g]; i < first[g] + count[g]; ++i) used.push_back(S.h_counts[perm[i] * T.n_leaves + c]);
-                std::sort(used.begin() + at, used.end());
-                used.erase(std::unique(used.begin() + at, used.end()), used.end());
-                continue;
-            }
-            const uint8_t* f = flags.data() + flag_off[g] + (size_t)c * (max_count[g] + 1);
-            for (int n = 0; n <= max_count[g]; ++n)
-                if (f[n]) used.push_back(n);
-        }
-    P.leaf_off.push_back((int64_t)used.size());
-    CK(P.d_counts.reserve(used.size() * sizeof(int32_t)), "patterns");
-    CK(cudaMemcpyAsync(P.d_counts.p, used.data(), used.size() * sizeof(int32_t), cudaMemcpyHostToDevice, st), "patterns");
     CK(launch_pat_write(a, d_ints + T.n_nodes, ni, d_off, P.d_child.as<int32_t>(), st), "patterns");
-    CK(cudaStreamSynchronize(st), "patterns");
+    for (int g = 0; g < ng; ++g)
+        for (int c = 0; c < T.n_leaves; ++c)
+            list_counts(S, P, g, c, flags + flag_off[g] + (size_t)c * (max_count[g] + 1), used);
+    P.leaf_off.push_back((int64_t)used.size());
+    return CAFE_OK;
+}
+
+// Families x internal nodes up to which the host builds the plan. Uploads, us,
+// host and device: 100 families of 8 taxa 42 and 104, 500 of 12 115 and 142,
+// 1,000 of 12 193 and 157, 10,000 of 24 3,035 and 893.
+constexpr int64_t kHostPatterns = 6000;
+
+int build_patterns(cafe_ctx* C, const TreeHost& T, FamSet& S, const std::vector<int>& bin_max, int all_max) {
+    PatternPlan& P = S.pats;
+    const int ni = (int)T.internal.size(), ng = (int)S.bins.widths.size() + 1;
+    P.n_groups = ng;
+    P.n_internal = ni;
+    P.group_first = S.bins.bin_first;
+    P.group_first.push_back(S.F);
+    P.group_count = S.bins.bin_count;
+    P.group_count.push_back(S.F);
+    P.group_max = bin_max;
+    P.group_max.push_back(all_max);
+    P.rows.assign((size_t)ng * ni, 0);
+    P.child_off.assign((size_t)ng * ni, 0);
+    P.leaf_off.clear();
+    if (!S.F) return CAFE_OK;
+    std::vector<int32_t> used, child;
+    if (S.F * ni <= kHostPatterns) {
+        patterns_on_host(T, S, P, child, used);
+        CK(P.d_child.reserve(child.size() * sizeof(int32_t)), "patterns");
+        CK(cudaMemcpyAsync(P.d_child.p, child.data(), child.size() * sizeof(int32_t), cudaMemcpyHostToDevice, C->setup),
+           "patterns");
+    } else {
+        const int rc = patterns_on_device(C, T, S, P, used);
+        if (rc) return rc;
+    }
+    CK(P.d_counts.reserve(used.size() * sizeof(int32_t)), "patterns");
+    CK(cudaMemcpyAsync(P.d_counts.p, used.data(), used.size() * sizeof(int32_t), cudaMemcpyHostToDevice, C->setup), "patterns");
+    CK(cudaStreamSynchronize(C->setup), "patterns");      // (any stream may read it from here on)
     return CAFE_OK;
 }
 
@@ -610,10 +751,6 @@ int prepare_set(cafe_ctx* C, FamSet& S) {
         S.max_count[f] = m;
     }
     // (families with equal counts are found subtree by subtree, below)
-    std::vector<int64_t> ident(F);
-    std::iota(ident.begin(), ident.end(), 0);
-    CK(S.d_identity.reserve(std::max<int64_t>(F, 1) * sizeof(int64_t)), "families");
-    if (F) CK(cudaMemcpy(S.d_identity.p, ident.data(), F * sizeof(int64_t), cudaMemcpyHostToDevice), "families");
     int rc = compute_bins(C, S);
     if (rc) return rc;
     const TreeHost& T = *C->trees.find(S.tree_id)->second;
@@ -626,11 +763,8 @@ int prepare_set(cafe_ctx* C, FamSet& S) {
         bin_max[b] = std::max(bin_max[b], m);
         all_max = std::max(all_max, m);
     }
-    TempBuf mem(C->ws[0]->stream_hi);
-    rc = build_patterns(C, T, S, S.bins.d_perm.as<int64_t>(), S.bins.perm, S.bins.bin_first, S.bins.bin_count, bin_max, mem,
-                        S.pat_bins);
-    if (!rc)
-        rc = build_patterns(C, T, S, S.d_identity.as<int64_t>(), ident, {0}, {F}, {all_max}, mem, S.pat_all);
+    rc = build_patterns(C, T, S, bin_max, all_max);
+    if (rc) cudaStreamSynchronize(C->setup);      // (nothing of it still reads the set)
     return rc;
 }
 
@@ -1067,10 +1201,12 @@ struct MaxProduct {
 // with `fork` the classes run side by side on the auxiliary streams.
 // Returns through d_status a word the kernel sets when a bounded wait gave
 // up; the caller zeroes it first.
-int launch_pat64_groups(cafe_ctx* C, Workspace& ws, const cafe_request* R, const TreeHost& T, const PatternPlan& P, const int64_t* d_perm, const int32_t* d_famR, const std::vector<PatGroup>& groups, int n_active,
-                        const int32_t* d_active, int K, int msize, bool scaled, double* out, int32_t* d_status, bool fork,
-                        int prof_kind, MaxProduct* mx = nullptr, double* root_out = nullptr) {
+int launch_pat64_groups(cafe_ctx* C, Workspace& ws, const cafe_request* R, const TreeHost& T, const FamSet& FS,
+                        const int32_t* d_famR, const std::vector<PatGroup>& groups, int n_active, const int32_t* d_active,
+                        int K, int msize, bool scaled, double* out, int32_t* d_status, bool fork, int prof_kind,
+                        MaxProduct* mx = nullptr, double* root_out = nullptr) {
     constexpr int NC = Workspace::kPatClasses;
+    const PatternPlan& P = FS.pats;
     const int ni = P.n_internal;
     struct Class {
         std::vector<PatGroup> groups;
@@ -1234,7 +1370,7 @@ int launch_pat64_groups(cafe_ctx* C, Workspace& ws, const cafe_request* R, const
     a.status = d_status;
     a.child = P.d_child.as<int32_t>();
     a.leaf_counts = P.d_counts.as<int32_t>();
-    a.perm = d_perm;
+    a.perm = FS.bin_items();
     a.mats = ws.mats.as<const double*>();
     a.ld_mat = msize;
     a.prior = C->d_prior.as<double>();
@@ -1403,8 +1539,8 @@ int enqueue_mixed(cafe_ctx* C, Workspace& ws, const cafe_request* R, TreeHost& T
     bool wide_done = false;
     auto launch_wide = [&]() -> int {
         wide_done = true;
-        return launch_pat64_groups(C, ws, R, T, S.pat_bins, B.d_perm.as<int64_t>(), B.d_famR.as<int32_t>(), wide,
-                                   (int)active.size(), ws.catids.as<int32_t>(), K, msize, true, ws.cat.as<double>(), d_status,
+        return launch_pat64_groups(C, ws, R, T, S, B.d_famR.as<int32_t>(), wide, (int)active.size(),
+                                   ws.catids.as<int32_t>(), K, msize, true, ws.cat.as<double>(), d_status,
                                    false, 3);
     };
     if (!tc_bins.empty()) {
@@ -1442,7 +1578,7 @@ int enqueue_mixed(cafe_ctx* C, Workspace& ws, const cafe_request* R, TreeHost& T
         CK(op_memset(ws, ws.cerr.p, 0, (size_t)std::max<int64_t>(F, 1) * K * sizeof(float), ws.stream), "range bounds");
 
         // one persistent launch per S-bin, run concurrently
-        const PatternPlan& P = S.pat_bins;
+        const PatternPlan& P = S.pats;
         const int ni = P.n_internal, n_act = (int)active.size();
         int levels = 1;
         for (int h : T.height) levels = std::max(levels, h);
@@ -1557,7 +1693,7 @@ int enqueue_mixed(cafe_ctx* C, Workspace& ws, const cafe_request* R, TreeHost& T
         a.status = d_status;
         a.any_flag = d_status + 3;
         a.child = P.d_child.as<int32_t>();
-        a.perm = B.d_perm.as<int64_t>();
+        a.perm = S.bin_items();
         a.mat_index = ws.tc_mi.as<int32_t>();
         a.n_nodes = T.n_nodes;
         a.Wm = Wm;
@@ -1694,7 +1830,7 @@ int enqueue_mixed(cafe_ctx* C, Workspace& ws, const cafe_request* R, TreeHost& T
         tt.flags = d_flags;
         tt.term_flags = d_term;
         tt.K = K;
-        tt.perm = B.d_perm.as<int64_t>();
+        tt.perm = S.bin_items();
         int W = 32;
         for (size_t b = B.widths.size(); b-- > 0 && tt.n_bins < 16;) {      // (the longest walks first)
             if (B.widths[b] > kTcMaxW) continue;
@@ -1996,12 +2132,11 @@ int enqueue_score(cafe_ctx* C, Workspace& ws, const cafe_request* Rs, int NB, do
     // FP64: every family at the reference's global bounds, or by S-bin
     std::vector<PatGroup> groups;
     if (ref_mode) {
-        groups.push_back(PatGroup{0, Sg, Rg});
+        groups.push_back(PatGroup{S.pats.all(), Sg, Rg});
     } else {
         for (size_t b = 0; b < S.bins.widths.size(); ++b)
             groups.push_back(PatGroup{(int)b, S.bins.widths[b] - 1, S.bins.widths[b] - 1});
     }
-    const int64_t* d_perm = ref_mode ? S.d_identity.as<int64_t>() : S.bins.d_perm.as<int64_t>();
     const int32_t* d_famR = ref_mode ? nullptr : S.bins.d_famR.as<int32_t>();
     CK(cudaMemcpyAsync(ws.mats.p, hm, (size_t)CT * T.n_nodes * sizeof(double*), cudaMemcpyHostToDevice, ws.stream),
        "mats");
@@ -2014,9 +2149,8 @@ int enqueue_score(cafe_ctx* C, Workspace& ws, const cafe_request* Rs, int NB, do
     bool fits = true;
     for (const PatGroup& q : groups) fits &= pat64_class(q) >= 0;
     if (fits) {
-        rc = launch_pat64_groups(C, ws, Rs, T, ref_mode ? S.pat_all : S.pat_bins, d_perm, d_famR, groups,
-                                 (int)active.size(), ws.catids.as<int32_t>(), CT, msize, scaled, ws.cat.as<double>(),
-                                 d_status, true, 1);
+        rc = launch_pat64_groups(C, ws, Rs, T, S, d_famR, groups, (int)active.size(), ws.catids.as<int32_t>(), CT, msize,
+                                 scaled, ws.cat.as<double>(), d_status, true, 1);
         if (rc) return rc;
         info->d_tail = d_status;
         info->tail_counts = false;
@@ -2052,7 +2186,7 @@ int enqueue_score(cafe_ctx* C, Workspace& ws, const cafe_request* Rs, int NB, do
     a.tiles = ws.tiles.as<PruneTile>();
     a.n_tiles = n_tiles;
     a.counts = S.d_counts.as<int32_t>();
-    a.perm = d_perm;
+    a.perm = S.all_items();
     a.mats = ws.mats.as<const double*>();
     a.ld_mat = msize;
     a.prior = C->d_prior.as<double>();
@@ -2298,13 +2432,13 @@ constexpr size_t kMaxProductBytes = (size_t)8 << 30;
 
 size_t max_product_bytes(const TreeHost& T, const PatternPlan& P, int S) {      // of a category
     size_t n = 0;
-    for (size_t ii = 0; ii + 1 < T.internal.size(); ++ii) n += (size_t)P.row_count(0, (int)ii) * (S + 2);
+    for (size_t ii = 0; ii + 1 < T.internal.size(); ++ii) n += (size_t)P.row_count(P.all(), (int)ii) * (S + 2);
     return (n + (size_t)T.n_leaves * (S + 1) * (S + 2)) * (sizeof(double) + sizeof(int32_t));
 }
 
 int reconstruct_rows(cafe_ctx* C, Workspace& ws, const cafe_request* R, const ReconSetup& Z, int root_len, int32_t* words) {
     const TreeHost& T = *Z.T;
-    const PatternPlan& P = Z.S->pat_all;
+    const PatternPlan& P = Z.S->pats;
     const int K = Z.K, n = T.n_nodes, ni = (int)T.internal.size(), n_st = Z.Smax + 1;
     const int64_t F = Z.S->F;
     // log2 of the internal branches' matrices, rows of 128-byte chunks
@@ -2337,7 +2471,8 @@ int reconstruct_rows(cafe_ctx* C, Workspace& ws, const cafe_request* R, const Re
     const int32_t* d_ints = reinterpret_cast<const int32_t*>(d + o_int);
     CK(cudaMemcpyAsync(d, ptr.data(), o_long, cudaMemcpyHostToDevice, ws.stream), "h2d");
     CK(cudaMemcpyAsync(d + o_int, ints.data(), ints.size() * sizeof(int32_t), cudaMemcpyHostToDevice, ws.stream), "h2d");
-    CK(cudaMemcpyAsync(d + o_long, P.child_off.data(), ni * sizeof(int64_t), cudaMemcpyHostToDevice, ws.stream), "h2d");
+    CK(cudaMemcpyAsync(d + o_long, &P.child_off[(size_t)P.all() * ni], ni * sizeof(int64_t), cudaMemcpyHostToDevice, ws.stream),
+       "h2d");
     CK(launch_log2_rows(reinterpret_cast<const double* const*>(dptr + (size_t)K * n),
                         reinterpret_cast<float* const*>(const_cast<void**>(dptr + (size_t)K * n + src.size())),
                         (int)src.size(), n_st, Z.msize, pitch, ws.stream),
@@ -2352,12 +2487,12 @@ int reconstruct_rows(cafe_ctx* C, Workspace& ws, const cafe_request* R, const Re
     mx.root_max = ws.rc_rmax.as<double>();
     mx.root_arg = ws.rc_arg.as<int32_t>();
     mx.n_failed = words;
-    const std::vector<PatGroup> group{{0, Z.Smax, root_len - 1}};
+    const std::vector<PatGroup> group{{P.all(), Z.Smax, root_len - 1}};
     for (int k0 = 0; k0 < K; k0 += pass) {
         const int nk = std::min(pass, K - k0);
         if (k0) CK(cudaStreamSynchronize(ws.stream), "reconstruct");     // (the staging buffers are read)
-        int rc = launch_pat64_groups(C, ws, R, T, P, Z.S->d_identity.as<int64_t>(), nullptr, group, nk, d_ints + k0, K,
-                                     Z.msize, false, nullptr, words + 1, false, 0, &mx);
+        int rc = launch_pat64_groups(C, ws, R, T, *Z.S, nullptr, group, nk, d_ints + k0, K, Z.msize, false,
+                                     nullptr, words + 1, false, 0, &mx);
         if (rc) return rc;
         if (!k0) {
             CK(cudaMemcpyAsync(d + o_long + ni * sizeof(int64_t), mx.ctab_off.data(), ni * sizeof(int64_t),
@@ -2408,7 +2543,7 @@ int reconstruct_sync(cafe_ctx* C, Workspace& ws, const cafe_request* R, cafe_rec
     // over distinct rows unless the caller wants every product formed, or a
     // vector does not fit a CTA or a category's tables 8 GB (then the tile walk)
     const bool by_rows = F > 0 && !out->exhaustive && pat64_class({0, Z.Smax, root_len - 1}, true) >= 0 &&
-                         max_product_bytes(T, Z.S->pat_all, Z.Smax) <= kMaxProductBytes;
+                         max_product_bytes(T, Z.S->pats, Z.Smax) <= kMaxProductBytes;
     std::vector<PruneTile>& tiles = ws.tile_vec;
     tiles.clear();
     for (int k = 0; k < K && !by_rows; ++k)
@@ -2705,9 +2840,11 @@ int prune_simulated(cafe_ctx* C, Workspace& ws, const TreeHost& T, int S, int RR
     const int32_t* d_dd = d_ints.as<int32_t>() + n;
     const int32_t* d_nodes = d_dd;
     for (auto& l : level) {
-        for (size_t b = 0; b < l.size(); b += batch)
-            CK(launch_pat_insert(a, d_nodes + b, (int)std::min(batch, l.size() - b), d_tab.as<int32_t>(), slots, st),
-               "patterns");
+        for (size_t b = 0; b < l.size(); b += batch) {
+            const int m = (int)std::min(batch, l.size() - b);
+            CK(cudaMemsetAsync(d_tab.p, 0xff, m * slots * sizeof(int32_t), st), "patterns");
+            CK(launch_pat_insert(a, d_nodes + b, m, d_tab.as<int32_t>(), slots, st), "patterns");
+        }
         d_nodes += l.size();
     }
     CK(launch_pat_number(a, d_dd, n_dd, st), "patterns");
@@ -3024,8 +3161,7 @@ int pvalues_device(cafe_ctx* C, Workspace& ws, const ReconSetup& Z, bool stream,
         // over the set's distinct rows (vectors that fit a CTA's shared memory)
         cafe_request rq;
         std::memset(&rq, 0, sizeof rq);
-        rc = launch_pat64_groups(C, ws, &rq, T, FS.pat_all, FS.d_identity.as<int64_t>(), nullptr, {{0, S, RR}}, 1,
-                                 d_ntiles.as<int32_t>() + 2, 1, msize, false, nullptr, d_status, false, 0, nullptr,
+        rc = launch_pat64_groups(C, ws, &rq, T, FS, nullptr, {{FS.pats.all(), S, RR}}, 1, d_ntiles.as<int32_t>() + 2, 1, msize, false, nullptr, d_status, false, 0, nullptr,
                                  d_obsL.as<double>());
         if (rc) return rc;
     }
@@ -3034,7 +3170,7 @@ int pvalues_device(cafe_ctx* C, Workspace& ws, const ReconSetup& Z, bool stream,
         o.tiles = d_otiles.as<PruneTile>();
         o.n_tiles = (int)otiles.size();
         o.counts = FS.d_counts.as<int32_t>();
-        o.perm = FS.d_identity.as<int64_t>();
+        o.perm = FS.all_items();
         o.root_out = d_obsL.as<double>();
         o.root_ld = RR;
         CK(launch_prune64(o, std::max(1, std::min((int)otiles.size(), n_ctas_max)), ws.stream), "prune root vectors");
@@ -3224,7 +3360,7 @@ int pvalues_sync(cafe_ctx* C, Workspace& ws, const cafe_request* R, cafe_pvalues
         t.root_lo = 1;
         tiles[n_tiles++] = t;
     }
-    rc = launch_tiles(0, n_tiles, FS.d_counts.as<int32_t>(), FS.d_identity.as<int64_t>(), Wmax,
+    rc = launch_tiles(0, n_tiles, FS.d_counts.as<int32_t>(), FS.all_items(), Wmax,
                       d_obsL.as<double>(), RR);
     if (rc) return rc;
     // simulated families, a group of root sizes at a time: the device prunes
@@ -3503,6 +3639,7 @@ int cafe_ctx_create(const cafe_config* cfg, cafe_ctx** out) {
     cudaGetDeviceProperties(&prop, dev);
     C->sm_count = prop.multiProcessorCount;
     if (pat_tc_init() != cudaSuccess || pat64_init() != cudaSuccess || terms64_init() != cudaSuccess || pvalue_kernels_init() != cudaSuccess ||
+        cudaStreamCreateWithFlags(&C->setup, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&C->gate, cudaEventDisableTiming) != cudaSuccess) {
         delete C;
         return CAFE_ERR_CUDA;
@@ -3558,6 +3695,7 @@ int cafe_ctx_destroy(cafe_ctx* C) {
         for (cudaEvent_t e : g.marks) cudaEventDestroy(e);
     if (C->gate) cudaEventDestroy(C->gate);
     if (C->serve_epoch) cudaEventDestroy(C->serve_epoch);
+    if (C->setup) cudaStreamDestroy(C->setup);
     delete C;
     return CAFE_OK;
 }
@@ -3638,7 +3776,10 @@ int cafe_families_upload(cafe_ctx* C, int tree_id, const int32_t* counts, int64_
     S->h_counts.assign(counts, counts + n_families * n_leaves);
     const size_t bytes = std::max<size_t>((size_t)n_families * n_leaves * sizeof(int32_t), 4);
     CK(S->d_counts.reserve(bytes), "counts");
-    if (n_families) CK(cudaMemcpy(S->d_counts.p, counts, (size_t)n_families * n_leaves * sizeof(int32_t), cudaMemcpyHostToDevice), "counts");
+    if (n_families)
+        CK(cudaMemcpyAsync(S->d_counts.p, counts, (size_t)n_families * n_leaves * sizeof(int32_t), cudaMemcpyHostToDevice,
+                           C->setup),
+           "counts");
     int rc = prepare_set(C, *S);
     if (rc) return rc;
     S->ready = true;
@@ -3666,10 +3807,11 @@ int cafe_families_update(cafe_ctx* C, int set_id, const int32_t* counts) {
         S.ready = false;      // until every table is that of the new counts
         S.h_counts.assign(counts, counts + n);
     }
-    Workspace& ws = *C->ws[0];
-    CK(cudaMemcpyAsync(S.d_counts.p, counts, n * sizeof(int32_t), cudaMemcpyHostToDevice, ws.stream), "counts");
-    CK(cudaStreamSynchronize(ws.stream), "counts");
-    if (same) return CAFE_OK;
+    CK(cudaMemcpyAsync(S.d_counts.p, counts, n * sizeof(int32_t), cudaMemcpyHostToDevice, C->setup), "counts");
+    if (same) {
+        CK(cudaStreamSynchronize(C->setup), "counts");
+        return CAFE_OK;
+    }
     const int rc = prepare_set(C, S);
     S.ready = rc == CAFE_OK;
     return rc;

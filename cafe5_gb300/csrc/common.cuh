@@ -81,7 +81,7 @@ struct PatBuildArgs {
     int32_t* base;               // [n_internal][n_groups + 1] num at each group's first item; then the total
 };
 // nodes: post-order indices of one level; the table holds n_nodes x slots
-// (a power of two, at least 2 F) entries
+// (a power of two, at least 2 F) entries, all -1
 cudaError_t launch_pat_insert(const PatBuildArgs& a, const int32_t* d_nodes, int n_nodes, int32_t* table, int64_t slots,
                               cudaStream_t s);
 // flags: [leaf][group_max + 1] per group, zeroed in; 1 where the count occurs

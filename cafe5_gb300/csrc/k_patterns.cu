@@ -168,8 +168,6 @@ cudaError_t launch_pat_counts(const PatBuildArgs& a, uint8_t* flags, cudaStream_
 cudaError_t launch_pat_insert(const PatBuildArgs& a, const int32_t* d_nodes, int n_nodes, int32_t* table, int64_t slots,
                               cudaStream_t s) {
     if (a.F <= 0 || n_nodes <= 0) return cudaSuccess;
-    cudaError_t e = cudaMemsetAsync(table, 0xff, (size_t)n_nodes * slots * sizeof(int32_t), s);
-    if (e != cudaSuccess) return e;
     const int bx = (int)std::min<int64_t>((a.F + 255) / 256, 4096);
     k_pat_insert<<<dim3(bx, n_nodes), 256, 0, s>>>(a, d_nodes, table, slots - 1);
     return cudaGetLastError();

@@ -67,12 +67,13 @@ struct BinPlan {
     std::vector<int> widths;                 // bin widths used
     std::vector<int64_t> bin_first, bin_count;
     std::vector<int64_t> perm;
-    DevBuf d_perm, d_famR, d_itemR;          // d_itemR: root bounds in perm order
+    DevBuf d_famR, d_itemR;                  // root bounds by family, and in perm order
     int W_max = 0;
 };
 
 // Distinct count patterns below every internal node, per group of families
-// (k_patterns.cu): the rows the pruning kernels contract.
+// (k_patterns.cu): the rows the pruning kernels contract. The groups are the
+// S-bins in order, and all families together.
 struct PatternPlan {
     int n_groups = 0, n_internal = 0;
     std::vector<int64_t> group_first, group_count;   // items (families in group order)
@@ -81,6 +82,7 @@ struct PatternPlan {
     std::vector<int64_t> child_off;   // [group][internal]: first child index in d_child
     std::vector<int64_t> leaf_off;    // [group][leaf]: first of the counts that occur there, in d_counts; then the end
     DevBuf d_child, d_counts;
+    int all() const { return n_groups - 1; }
     int64_t row_count(int g, int ii) const { return rows[(size_t)g * n_internal + ii]; }
 };
 
@@ -92,9 +94,11 @@ struct FamSet {
     DevBuf d_counts;
     std::vector<int32_t> h_counts;
     std::vector<int32_t> max_count;
-    DevBuf d_identity;                // 0..F-1
+    DevBuf d_items;                   // [2 F] the families in bin order (bins.perm), then in their own
     BinPlan bins;
-    PatternPlan pat_bins, pat_all;    // grouped by S-bin (bins.d_perm order), and all families together
+    PatternPlan pats;
+    const int64_t* bin_items() const { return d_items.as<int64_t>(); }
+    const int64_t* all_items() const { return d_items.as<int64_t>() + F; }
 };
 
 struct MatKey {
@@ -251,6 +255,7 @@ struct cafe_ctx {
     std::vector<double> err;
     int err_rows = 0, err_ndev = 0;
     cafe::DevBuf d_err;
+    cudaStream_t setup = nullptr;     // family sets: copies and pattern plans
     // matrix cache
     cafe::MatCache cache;
     // two generations of slabs, used in turn: the cache fills one; past the
