@@ -473,8 +473,21 @@ struct TempBuf {
 constexpr int kFlaggedCounts = 1 << 14;
 
 // ---- the distinct patterns of every subtree, for the families of every S-bin
-// (the plan's groups, in the order of the bins) and for all of them together
-// (its last group). Items are the families in bin order, then in their own.
+// (the plan's groups, in the order of the bins; a bin whose factor rows would
+// take more than kGroupBytes is several groups) and for all of them together (its
+// last group). Items are the families in bin order, then in their own.
+
+constexpr size_t kGroupBytes = (size_t)1 << 30;
+size_t table_limit(const cafe_ctx* C, size_t bytes) {      // (a test hook makes every limit smaller)
+    return C->debug_table_bytes ? std::min(bytes, C->debug_table_bytes) : bytes;
+}
+// FP64 factor rows of one combination at group g's internal nodes, vectors of
+// n states.
+size_t row_bytes(const PatternPlan& P, int g, size_t n) {
+    int64_t rows = 0;
+    for (int ii = 0; ii + 1 < P.n_internal; ++ii) rows += P.row_count(g, ii);
+    return (size_t)rows * (n + 1) * sizeof(double);
+}
 
 // Appends the counts that occur at leaf c of group g, from a flag for every
 // count of the group up to kFlaggedCounts; with larger ones they are sorted.
@@ -709,17 +722,31 @@ int patterns_on_device(cafe_ctx* C, const TreeHost& T, FamSet& S, PatternPlan& P
 // 1,000 of 12 193 and 157, 10,000 of 24 3,035 and 893.
 constexpr int64_t kHostPatterns = 6000;
 
-int build_patterns(cafe_ctx* C, const TreeHost& T, FamSet& S, const std::vector<int>& bin_max, int all_max) {
+// The plan of bins cut into `parts` groups each.
+int build_groups(cafe_ctx* C, const TreeHost& T, FamSet& S, const std::vector<int>& bin_max, int all_max,
+                 const std::vector<int64_t>& parts) {
     PatternPlan& P = S.pats;
-    const int ni = (int)T.internal.size(), ng = (int)S.bins.widths.size() + 1;
+    const BinPlan& B = S.bins;
+    const int ni = (int)T.internal.size();
+    P.group_first.clear();
+    P.group_count.clear();
+    P.group_max.clear();
+    P.bin.clear();
+    auto add = [&](int64_t first, int64_t count, int max, int bin) {
+        P.group_first.push_back(first);
+        P.group_count.push_back(count);
+        P.group_max.push_back(max);
+        P.bin.push_back(bin);
+    };
+    for (size_t b = 0; b < B.widths.size(); ++b)
+        for (int64_t q = 0; q < parts[b]; ++q) {
+            const int64_t i0 = B.bin_count[b] * q / parts[b], i1 = B.bin_count[b] * (q + 1) / parts[b];
+            add(B.bin_first[b] + i0, i1 - i0, bin_max[b], (int)b);
+        }
+    add(S.F, S.F, all_max, -1);
+    const int ng = (int)P.bin.size();
     P.n_groups = ng;
     P.n_internal = ni;
-    P.group_first = S.bins.bin_first;
-    P.group_first.push_back(S.F);
-    P.group_count = S.bins.bin_count;
-    P.group_count.push_back(S.F);
-    P.group_max = bin_max;
-    P.group_max.push_back(all_max);
     P.rows.assign((size_t)ng * ni, 0);
     P.child_off.assign((size_t)ng * ni, 0);
     P.leaf_off.clear();
@@ -738,6 +765,25 @@ int build_patterns(cafe_ctx* C, const TreeHost& T, FamSet& S, const std::vector<
     CK(cudaMemcpyAsync(P.d_counts.p, used.data(), used.size() * sizeof(int32_t), cudaMemcpyHostToDevice, C->setup), "patterns");
     CK(cudaStreamSynchronize(C->setup), "patterns");      // (any stream may read it from here on)
     return CAFE_OK;
+}
+
+int build_patterns(cafe_ctx* C, const TreeHost& T, FamSet& S, const std::vector<int>& bin_max, int all_max) {
+    const BinPlan& B = S.bins;
+    const size_t limit = table_limit(C, kGroupBytes);
+    std::vector<int64_t> parts(B.widths.size(), 1);
+    for (;;) {
+        const int rc = build_groups(C, T, S, bin_max, all_max, parts);
+        if (rc) return rc;
+        // (parts share no rows, so a cut may have to be repeated)
+        std::vector<int64_t> more(parts);
+        for (int g = 0; g < S.pats.all(); ++g) {
+            const int b = S.pats.bin[g];
+            const int64_t need = (int64_t)(row_bytes(S.pats, g, B.widths[b]) / limit);
+            if (need > 0) more[b] = std::min(B.bin_count[b], std::max(more[b], std::max(2 * parts[b], need + need / 4 + 1)));
+        }
+        if (more == parts) return CAFE_OK;
+        parts.swap(more);
+    }
 }
 
 int prepare_set(cafe_ctx* C, FamSet& S) {
@@ -1183,6 +1229,23 @@ int pat64_class(const PatGroup& q, bool max_product = false) {
     return lp <= 66 ? 0 : lp <= 194 ? 1 : lp <= 514 ? 2 : 3;
 }
 
+// Factor tables: of one combination, up to kWaveBytes for groups that run side by
+// side, and up to kRowTableBytes where all families are one group (past it they
+// are left to the tile walks, whose vectors take the same memory whatever their
+// number); of several combinations, kTableBytes.
+constexpr size_t kWaveBytes = (size_t)4 << 30, kRowTableBytes = (size_t)8 << 30, kTableBytes = (size_t)2 << 30;
+
+// All families at states 0..S and root sizes 1..R: whether k_pat64 takes them.
+// Counts past the states and the error model's reach (half deviations) share a
+// leaf's last row.
+bool takes_rows(const cafe_ctx* C, const TreeHost& T, const PatternPlan& P, int S, int R, int half) {
+    const int g = P.all();
+    if (pat64_class({g, S, R}) < 0) return false;
+    const size_t n = (size_t)std::max(S, R) + 1;
+    const size_t leaf = (size_t)T.n_leaves * (size_t)(std::min<int64_t>(P.group_max[g], (int64_t)S + half + 1) + 1);
+    return row_bytes(P, g, n) + leaf * (n + 1) * sizeof(double) <= table_limit(C, kRowTableBytes);
+}
+
 // A max-product pass (one group): k_pat64's extra operands, and where the
 // argmax tables of its combinations went.
 struct MaxProduct {
@@ -1209,27 +1272,41 @@ int launch_pat64_groups(cafe_ctx* C, Workspace& ws, const cafe_request* R, const
     const PatternPlan& P = FS.pats;
     const int ni = P.n_internal;
     struct Class {
+        int c = 0, wave = 0;
         std::vector<PatGroup> groups;
         std::vector<Pat64Node> nodes;
         std::vector<int32_t> cdesc;
         int s_run = 1, lp = 0, max_R = 0, units = 0, n_bufs = 1, group = 1, n_slots = 1, n_ctas = 1;
         int64_t slot_doubles = 0, slot_rows = 0;
         size_t o_nodes = 0, o_cdesc = 0, o_done = 0;
-    } cls[NC];
+    };
+    // groups whose tables (of one combination) stay within kWaveBytes together
+    // run side by side, the next ones after them
+    std::vector<Class> cls;
+    std::vector<size_t> wave_bytes;
+    size_t wave0 = 0;      // first class of the wave
     for (const PatGroup& q : groups) {
         const int c = pat64_class(q, mx);
         if (c < 0) return fail(C, CAFE_ERR_INVALID, "vectors of %d states", q.S + 1);
-        if (P.group_count[q.g] > 0) cls[c].groups.push_back(q);
+        if (!P.group_count[q.g]) continue;
+        const size_t bytes = row_bytes(P, q.g, q.S + 1);
+        if (wave_bytes.empty() || wave_bytes.back() + bytes > table_limit(C, kWaveBytes)) {
+            wave_bytes.push_back(0);
+            wave0 = cls.size();
+        }
+        wave_bytes.back() += bytes;
+        size_t x = wave0;
+        while (x < cls.size() && cls[x].c != c) ++x;
+        if (x == cls.size()) {
+            cls.emplace_back();
+            cls[x].c = c;
+            cls[x].wave = (int)wave_bytes.size() - 1;
+        }
+        cls[x].groups.push_back(q);
     }
-    int filled = 0;
-    for (const Class& X : cls) filled += !X.groups.empty();
-    const bool several = filled > 1;
     int levels = 1;
     for (int h : T.height) levels = std::max(levels, h);
-    size_t blob = 0, ctr = NC * sizeof(unsigned long long);
-    for (int c = 0; c < NC; ++c) {
-        Class& X = cls[c];
-        if (X.groups.empty()) continue;
+    for (Class& X : cls) {
         for (const PatGroup& q : X.groups) {
             X.lp = std::max(X.lp, pat64_lp(q.S));
             X.max_R = std::max(X.max_R, q.R);
@@ -1314,12 +1391,19 @@ int launch_pat64_groups(cafe_ctx* C, Workspace& ws, const cafe_request* R, const
                     }
         for (size_t gi = 0; gi < X.groups.size(); ++gi)
             for (int v = 0; v < nn; ++v) X.nodes[at[gi * nn + v]].root = at[gi * nn + T.root];
+    }
+    if (cls.empty()) return CAFE_OK;
+    std::vector<int64_t> wave_doubles(wave_bytes.size(), 0);      // (the leaves' rows included)
+    for (const Class& X : cls) wave_doubles[X.wave] += X.slot_doubles;
+    size_t blob = 0, ctr = cls.size() * sizeof(unsigned long long);
+    for (Class& X : cls) {
         // combinations interleaved until a level has about eight units per SM;
-        // tables for twice as many, within 2 GB (a class at most 1 GB of them where
-        // there are several)
+        // tables for twice as many, the wave's within kTableBytes (or one
+        // combination's)
         const int64_t want = ((int64_t)8 * C->sm_count * levels + X.units - 1) / std::max(1, X.units);
         X.group = (int)std::max<int64_t>(1, std::min<int64_t>(n_active, want));
-        const int64_t fit = std::max<int64_t>(1, ((int64_t)2 << 30) / (several ? 2 : 1) / std::max<int64_t>(1, X.slot_doubles * 8));
+        const int64_t fit = std::max<int64_t>(1, (int64_t)table_limit(C, kTableBytes) /
+                                                     std::max<int64_t>(1, wave_doubles[X.wave] * (int64_t)sizeof(double)));
         X.group = (int)std::min<int64_t>(X.group, fit);
         X.n_slots = (int)std::min<int64_t>(n_active, std::max<int64_t>(X.group, std::min<int64_t>(fit, 2 * X.group)));
         if (mx) {
@@ -1328,18 +1412,18 @@ int launch_pat64_groups(cafe_ctx* C, Workspace& ws, const cafe_request* R, const
             mx->ctab_stride = X.slot_doubles;
             mx->ctab_off.assign(ni, 0);
             mx->pitch.assign(ni, 0);
-            for (int ii = 0; ii < ni; ++ii) {
-                const Pat64Node& nd = X.nodes[at[T.internal[ii]]];
-                mx->ctab_off[ii] = nd.tab;
-                mx->pitch[ii] = nd.pitch;
-            }
+            for (const Pat64Node& nd : X.nodes)
+                if (const int ii = T.internal_index[nd.node]; ii >= 0) {
+                    mx->ctab_off[ii] = nd.tab;
+                    mx->pitch[ii] = nd.pitch;
+                }
             CK(ws.rc_c.reserve((size_t)n_active * X.slot_doubles * sizeof(int32_t)), "argmax tables");
         }
         X.n_ctas = (int)std::min<int64_t>((int64_t)X.units * n_active,
                                           (int64_t)C->sm_count *
                                               pat64_ctas_per_sm(X.n_bufs * pat64_buf_doubles(X.lp, X.max_R, mx) * sizeof(double), mx));
-        CK(ws.pat_table[c].reserve((size_t)X.n_slots * X.slot_doubles * sizeof(double)), "factor tables");
-        CK(ws.pat_expo[c].reserve((size_t)X.n_slots * X.slot_rows * sizeof(int32_t)), "factor tables");
+        CK(ws.pat_table[X.c].reserve((size_t)X.n_slots * X.slot_doubles * sizeof(double)), "factor tables");
+        CK(ws.pat_expo[X.c].reserve((size_t)X.n_slots * X.slot_rows * sizeof(int32_t)), "factor tables");
         X.o_nodes = blob;
         blob += X.nodes.size() * sizeof(Pat64Node);
         X.o_cdesc = blob;
@@ -1347,18 +1431,14 @@ int launch_pat64_groups(cafe_ctx* C, Workspace& ws, const cafe_request* R, const
         X.o_done = ctr;
         ctr += X.nodes.size() * n_active * sizeof(int32_t);
     }
-    if (!blob) return CAFE_OK;
     CK(ws.h_pat_desc.reserve(blob), "pattern nodes");
     CK(ws.pat_desc.reserve(blob), "pattern nodes");
     CK(ws.pat_ctr.reserve(ctr), "pattern counters");
     char* h = ws.h_pat_desc.as<char>();
     std::memset(h, 0, blob);
-    int n_cls = 0;
     for (const Class& X : cls) {
-        if (X.groups.empty()) continue;
         std::memcpy(h + X.o_nodes, X.nodes.data(), X.nodes.size() * sizeof(Pat64Node));
         std::memcpy(h + X.o_cdesc, X.cdesc.data(), X.cdesc.size() * sizeof(int32_t));
-        ++n_cls;
     }
     CK(op_h2d(ws, ws.pat_desc.p, h, blob, ws.stream), "pattern nodes");
     CK(op_memset(ws, ws.pat_ctr.p, 0, ctr, ws.stream), "pattern counters");
@@ -1402,41 +1482,46 @@ int launch_pat64_groups(cafe_ctx* C, Workspace& ws, const cafe_request* R, const
             C->prof.acc.prune_flops += (prof_kind == 1) * family_flops(T, q.S, q.R, R->use_error_model) *
                                        (double)P.group_count[q.g] * n_active;
     }
-    const bool forked = fork && n_cls > 1;
-    if (forked) {
-        CK(op_record(ws, ws.ev_fork, ws.stream), "fork");
-        for (int c = 0; c < NC; ++c) CK(op_wait(ws, ws.aux[c], ws.ev_fork), "fork");
-    }
-    for (int c = NC - 1; c >= 0; --c) {      // the widest vectors (the longest units) first
-        const Class& X = cls[c];
-        if (X.groups.empty()) continue;
-        Pat64Args b;
-        std::memcpy(&b, &a, sizeof b);       // padding included: the bytes are a graph signature
-        const char* d = ws.pat_desc.as<char>();
-        b.nodes = reinterpret_cast<const Pat64Node*>(d + X.o_nodes);
-        b.cdesc = reinterpret_cast<const int32_t*>(d + X.o_cdesc);
-        b.n_desc = (int)X.nodes.size();
-        b.units = X.units;
-        b.s_run = X.s_run;
-        b.n_bufs = X.n_bufs;
-        b.buf_doubles = pat64_buf_doubles(X.lp, X.max_R, mx);
-        b.group = X.group;
-        b.n_slots = X.n_slots;
-        b.slot_doubles = X.slot_doubles;
-        b.slot_rows = X.slot_rows;
-        b.table = ws.pat_table[c].as<double>();
-        b.expo = ws.pat_expo[c].as<int32_t>();
-        b.next = ws.pat_ctr.as<unsigned long long>() + c;
-        b.done = reinterpret_cast<int32_t*>(ws.pat_ctr.as<char>() + X.o_done);
-        const cudaStream_t st = forked ? ws.aux[c] : ws.stream;
-        CK(op_launch(ws, 3, [&] { return launch_pat64(b, X.n_ctas, st); }, b, X.n_ctas, st),
-           "prune fp64");
-    }
-    if (forked)
-        for (int c = 0; c < NC; ++c) {
-            CK(op_record(ws, ws.ev_join[c], ws.aux[c]), "join");
-            CK(op_wait(ws, ws.stream, ws.ev_join[c]), "join");
+    for (size_t x0 = 0, x1; x0 < cls.size(); x0 = x1) {      // a wave
+        for (x1 = x0 + 1; x1 < cls.size() && cls[x1].wave == cls[x0].wave; ++x1) {}
+        const bool forked = fork && x1 - x0 > 1;
+        if (forked) {
+            CK(op_record(ws, ws.ev_fork, ws.stream), "fork");
+            for (int c = 0; c < NC; ++c) CK(op_wait(ws, ws.aux[c], ws.ev_fork), "fork");
         }
+        for (int c = NC - 1; c >= 0; --c) {      // the widest vectors (the longest units) first
+            size_t x = x0;
+            while (x < x1 && cls[x].c != c) ++x;
+            if (x == x1) continue;
+            const Class& X = cls[x];
+            Pat64Args b;
+            std::memcpy(&b, &a, sizeof b);       // padding included: the bytes are a graph signature
+            const char* d = ws.pat_desc.as<char>();
+            b.nodes = reinterpret_cast<const Pat64Node*>(d + X.o_nodes);
+            b.cdesc = reinterpret_cast<const int32_t*>(d + X.o_cdesc);
+            b.n_desc = (int)X.nodes.size();
+            b.units = X.units;
+            b.s_run = X.s_run;
+            b.n_bufs = X.n_bufs;
+            b.buf_doubles = pat64_buf_doubles(X.lp, X.max_R, mx);
+            b.group = X.group;
+            b.n_slots = X.n_slots;
+            b.slot_doubles = X.slot_doubles;
+            b.slot_rows = X.slot_rows;
+            b.table = ws.pat_table[c].as<double>();
+            b.expo = ws.pat_expo[c].as<int32_t>();
+            b.next = ws.pat_ctr.as<unsigned long long>() + x;
+            b.done = reinterpret_cast<int32_t*>(ws.pat_ctr.as<char>() + X.o_done);
+            const cudaStream_t st = forked ? ws.aux[c] : ws.stream;
+            CK(op_launch(ws, 3, [&] { return launch_pat64(b, X.n_ctas, st); }, b, X.n_ctas, st),
+               "prune fp64");
+        }
+        if (forked)
+            for (int c = 0; c < NC; ++c) {
+                CK(op_record(ws, ws.ev_join[c], ws.aux[c]), "join");
+                CK(op_wait(ws, ws.stream, ws.ev_join[c]), "join");
+            }
+    }
     if (prof) C->prof.end(prof_kind, ws.stream, ev);
     return CAFE_OK;
 }
@@ -1467,6 +1552,10 @@ int tc_per_sm(const cafe_ctx* C, int W) {
 // Share of the 1e-6 per-family budget (|dlnL| / |lnL|) left to FP32 range
 // loss; TF32x3 rounding takes the rest.
 constexpr double kRangeTau = 1e-7;
+
+// The tensor cores' factor tables (of one combination at least), and the list of
+// the terms that FP64 recomputes (of one category at least).
+constexpr size_t kTcTableBytes = (size_t)4 << 30, kTermListBytes = (size_t)256 << 20;
 
 // Widest bin on the tensor cores (the root weighting keeps the prior of its
 // states in shared memory).
@@ -1525,11 +1614,12 @@ int enqueue_mixed(cafe_ctx* C, Workspace& ws, const cafe_request* R, TreeHost& T
     uint8_t* d_term = ws.term_flags.as<uint8_t>();
     CK(op_memset(ws, ws.term_flags.p, 0, (size_t)std::max<int64_t>(F, 1) * K, ws.stream), "term flags");
 
-    std::vector<int> tc_bins;
+    std::vector<int> tc_groups;
     std::vector<PatGroup> wide;      // bins past the tensor cores' width
-    for (size_t b = 0; b < B.widths.size(); ++b) {
-        if (B.widths[b] > kTcMaxW) wide.push_back(PatGroup{(int)b, B.widths[b] - 1, B.widths[b] - 1});
-        else if (B.bin_count[b] > 0) tc_bins.push_back((int)b);
+    for (int g = 0; g < S.pats.all(); ++g) {
+        const int w = B.widths[S.pats.bin[g]];
+        if (w > kTcMaxW) wide.push_back(PatGroup{g, w - 1, w - 1});
+        else if (S.pats.group_count[g] > 0) tc_groups.push_back(g);
     }
     const bool prof = ws.sync;
     cudaEvent_t ev;
@@ -1543,7 +1633,7 @@ int enqueue_mixed(cafe_ctx* C, Workspace& ws, const cafe_request* R, TreeHost& T
                                    ws.catids.as<int32_t>(), K, msize, true, ws.cat.as<double>(), d_status,
                                    false, 3);
     };
-    if (!tc_bins.empty()) {
+    if (!tc_groups.empty()) {
         const size_t fl = (size_t)n_mat * Wm * Wm;
         CK(ws.tc_hi.reserve(2 * fl * sizeof(float)), "tc matrices");     // hi, then lo
         CK(ws.tc_tr.reserve(fl * sizeof(float)), "tc matrices");
@@ -1577,13 +1667,14 @@ int enqueue_mixed(cafe_ctx* C, Workspace& ws, const cafe_request* R, TreeHost& T
         CK(ws.cerr.reserve((size_t)std::max<int64_t>(F, 1) * K * sizeof(float)), "range bounds");
         CK(op_memset(ws, ws.cerr.p, 0, (size_t)std::max<int64_t>(F, 1) * K * sizeof(float), ws.stream), "range bounds");
 
-        // one persistent launch per S-bin, run concurrently
+        // one persistent launch per group (S-bin), run concurrently; groups whose
+        // tables of one combination pass kTcTableBytes together run in waves
         const PatternPlan& P = S.pats;
         const int ni = P.n_internal, n_act = (int)active.size();
         int levels = 1;
         for (int h : T.height) levels = std::max(levels, h);
         struct BinLaunch {
-            int b, n_ctas;
+            int g, b, wave, n_ctas;      // group, bin
             std::vector<PatTcNode> nodes;
             std::vector<PatTcSeg> segs;
             long long units = 0;
@@ -1591,11 +1682,23 @@ int enqueue_mixed(cafe_ctx* C, Workspace& ws, const cafe_request* R, TreeHost& T
             int n_slots = 1;
             size_t o_nodes, o_segs, o_done;
         };
-        std::vector<BinLaunch> launches(tc_bins.size());
-        size_t blob = 0, ctr = launches.size() * sizeof(unsigned long long);
+        std::vector<BinLaunch> launches(tc_groups.size());
+        std::vector<size_t> wave_bytes;
         for (size_t q = 0; q < launches.size(); ++q) {
             BinLaunch& L = launches[q];
-            L.b = tc_bins[q];
+            L.g = tc_groups[q];
+            L.b = P.bin[L.g];
+            int64_t rows = 0;
+            for (int ii = 0; ii + 1 < ni; ++ii) rows += (P.row_count(L.g, ii) + 31) / 32 * 32;
+            const size_t bytes = (size_t)std::max<int64_t>(1, rows) * (B.widths[L.b] * sizeof(float) + sizeof(int4));
+            // (a bin's groups share its table)
+            if (!q || launches[q - 1].b == L.b || wave_bytes.back() + bytes > table_limit(C, kTcTableBytes))
+                wave_bytes.push_back(0);
+            wave_bytes.back() += bytes;
+            L.wave = (int)wave_bytes.size() - 1;
+        }
+        size_t blob = 0, ctr = launches.size() * sizeof(unsigned long long);
+        for (BinLaunch& L : launches) {
             const int W = B.widths[L.b], Ns = pat_tc_states(W), n_share = W / Ns;
             std::vector<int> at(T.n_nodes, -1), lvl0(levels + 1, 0);
             std::vector<int64_t> lvl_units(levels, 0);
@@ -1607,9 +1710,9 @@ int enqueue_mixed(cafe_ctx* C, Workspace& ws, const cafe_request* R, TreeHost& T
                     const int v = T.internal[ii];
                     PatTcNode nd;
                     std::memset(&nd, 0, sizeof nd);
-                    nd.cidx = P.child_off[(size_t)L.b * ni + ii];
-                    nd.perm0 = P.group_first[L.b];
-                    nd.rows = (int32_t)P.row_count(L.b, ii);
+                    nd.cidx = P.child_off[(size_t)L.g * ni + ii];
+                    nd.perm0 = P.group_first[L.g];
+                    nd.rows = (int32_t)P.row_count(L.g, ii);
                     nd.node = v;
                     nd.nch = (int32_t)T.children[v].size();
                     for (int c = 0; c < nd.nch; ++c) {
@@ -1639,19 +1742,28 @@ int enqueue_mixed(cafe_ctx* C, Workspace& ws, const cafe_request* R, TreeHost& T
             const int64_t ctas = (int64_t)C->sm_count * tc_per_sm(C, W);
             int64_t g = n_act;
             if (units * n_act > 2 * levels * ctas) g = std::min<int64_t>(n_act, (4 * ctas + units - 1) / units);
-            // (the bins' tables within 4 GB together)
-            const int64_t fit = std::max<int64_t>(1, ((int64_t)4 << 30) / (int64_t)launches.size() /
-                                                         std::max<int64_t>(1, L.slot_rows * W * 4));
-            if (g < n_act) g = std::max<int64_t>(1, std::min(g, fit / (levels + 1)));
-            else if (g > fit) g = std::max<int64_t>(1, fit / (levels + 1));
-            L.n_slots = (int)std::min<int64_t>(n_act, (levels + 1) * g);
-            const int64_t blocks = (n_act + g - 1) / g;
+            // Tables for `fit` combinations (the wave's within kTcTableBytes): in
+            // skewed order a block's tables live for levels + 1 steps; where not
+            // even that many fit, blocks come one after the other, every level of
+            // one before the next, and a table is free once its combination's root
+            // is done.
+            const int64_t fit = std::max<int64_t>(1, (int64_t)(table_limit(C, kTcTableBytes) / wave_bytes[L.wave]));
+            const bool skewed = (g < n_act || n_act > fit) && fit >= levels + 1;
+            if (skewed) {
+                g = std::max<int64_t>(1, std::min(g, fit / (levels + 1)));
+                L.n_slots = (int)std::min<int64_t>(n_act, (levels + 1) * g);
+            } else {
+                L.n_slots = (int)std::min<int64_t>(n_act, fit);
+                if (n_act > fit) g = std::max<int64_t>(1, std::min<int64_t>(g, fit / 2));
+            }
+            const int64_t blocks = (n_act + g - 1) / g, skew = skewed ? 1 : levels;
             int64_t widest = 1;
-            for (int64_t t = 0; t < blocks + levels - 1; ++t) {
+            for (int64_t t = 0; t <= (blocks - 1) * skew + levels - 1; ++t) {
                 int64_t step = 0;
                 for (int l = levels - 1; l >= 0; --l) {
-                    const int64_t blk = t - l;
-                    if (blk < 0 || blk >= blocks || !lvl_units[l]) continue;
+                    if ((t - l) % skew || !lvl_units[l]) continue;
+                    const int64_t blk = (t - l) / skew;
+                    if (t < l || blk >= blocks) continue;
                     PatTcSeg sg;
                     std::memset(&sg, 0, sizeof sg);
                     sg.unit0 = L.units;
@@ -1665,8 +1777,7 @@ int enqueue_mixed(cafe_ctx* C, Workspace& ws, const cafe_request* R, TreeHost& T
                 }
                 widest = std::max(widest, step);
             }
-            L.n_ctas = (int)std::min<int64_t>(ctas, widest);
-            if (L.slot_rows * L.n_slots >= ((int64_t)1 << 31)) return fail(C, CAFE_ERR_INVALID, "too many factor rows");
+            L.n_ctas = (int)std::min<int64_t>(ctas, skewed || blocks == 1 ? widest : 2 * widest);
             const int64_t rows = std::max<int64_t>(128, L.slot_rows * L.n_slots);
             CK(ws.tcp_table[L.b].reserve((size_t)rows * W * sizeof(float)), "factor tables");
             CK(ws.tcp_meta[L.b].reserve((size_t)rows * sizeof(int4)), "factor tables");
@@ -1714,61 +1825,62 @@ int enqueue_mixed(cafe_ctx* C, Workspace& ws, const cafe_request* R, TreeHost& T
         a.debug_wait_limit = C->debug_wait_limit;
         if (prof) {
             C->prof.begin(1, ws.stream, &ev);
-            for (int b : tc_bins)
-                C->prof.acc.prune_flops += family_flops(T, B.widths[b] - 1, B.widths[b] - 1, R->use_error_model) *
-                                           (double)B.bin_count[b] * n_act;
+            for (const BinLaunch& L : launches)
+                C->prof.acc.prune_flops += family_flops(T, B.widths[L.b] - 1, B.widths[L.b] - 1, R->use_error_model) *
+                                           (double)P.group_count[L.g] * n_act;
         }
-        // fork: bins run on the auxiliary streams after everything queued so far
-        const bool fork = launches.size() > 1;
-        if (fork) {
-            CK(op_record(ws, ws.ev_fork, ws.stream), "fork");
-            for (int q = 0; q < Workspace::kAux; ++q) CK(op_wait(ws, ws.aux[q], ws.ev_fork), "fork");
-        }
-        // widest bins (the longest units) first, each on its own stream
-        for (size_t q = 0; q < launches.size(); ++q) {
-            const size_t li = launches.size() - 1 - q;
-            const BinLaunch& L = launches[li];
-            const int W = B.widths[L.b];
-            PatTcArgs b;
-            std::memcpy(&b, &a, sizeof b);     // padding included: the bytes are a graph signature
-            const char* dd = ws.tcp_desc.as<char>();
-            b.nodes = reinterpret_cast<const PatTcNode*>(dd + L.o_nodes);
-            b.segs = reinterpret_cast<const PatTcSeg*>(dd + L.o_segs);
-            b.n_desc = (int)L.nodes.size();
-            b.n_segs = (int)L.segs.size();
-            b.total_units = L.units;
-            b.n_slots = L.n_slots;
-            b.slot_rows = L.slot_rows;
-            b.table = ws.tcp_table[L.b].as<float>();
-            b.meta = ws.tcp_meta[L.b].as<int4>();
-            b.next = ws.tcp_ctr.as<unsigned long long>() + li;
-            b.done = reinterpret_cast<int32_t*>(ws.tcp_ctr.as<char>() + L.o_done);
-            b.W = W;
-            b.Ns = pat_tc_states(W);
-            b.n_share = W / b.Ns;
-            b.tmem_cols = 32;
-            while (b.tmem_cols < b.Ns) b.tmem_cols *= 2;
-            const int64_t rows = std::max<int64_t>(128, L.slot_rows * L.n_slots);
-            PatTcMaps maps;
-            std::memset(&maps, 0, sizeof maps);
-            int rcm = cached_map(C, ws, b.Ns / 32 - 1, &maps.mat, ws.tc_hi.as<float>(), (int64_t)n_mat * Wm, Wm, 32, b.Ns,
-                                 (int64_t)n_mat * Wm * Wm);
-            if (!rcm) rcm = cached_map(C, ws, 4 + L.b, &maps.vst, b.table, rows, W, 32, 128);
-            if (!rcm) rcm = cached_map(C, ws, 4 + kMaxGroups + L.b, &maps.vst32, b.table, rows, W, 32, 32);
-            if (rcm) return rcm;
-            const cudaStream_t st = fork ? ws.aux[q % Workspace::kAux] : ws.stream;
-            CK(op_launch(ws, 5, [&] { return launch_pat_tc(maps, b, L.n_ctas, st); }, maps, b, L.n_ctas, st),
-               "prune tc");
-        }
-        if (fork && !prof) {
-            const int rcw = launch_wide();
-            if (rcw) return rcw;
-        }
-        if (fork) {
-            for (int q = 0; q < Workspace::kAux; ++q) {
-                CK(op_record(ws, ws.ev_join[q], ws.aux[q]), "join");
-                CK(op_wait(ws, ws.stream, ws.ev_join[q]), "join");
+        for (size_t l0 = 0, l1; l0 < launches.size(); l0 = l1) {      // a wave
+            for (l1 = l0 + 1; l1 < launches.size() && launches[l1].wave == launches[l0].wave; ++l1) {}
+            // fork: bins run on the auxiliary streams after everything queued so far
+            const bool fork = l1 - l0 > 1;
+            if (fork) {
+                CK(op_record(ws, ws.ev_fork, ws.stream), "fork");
+                for (int q = 0; q < Workspace::kAux; ++q) CK(op_wait(ws, ws.aux[q], ws.ev_fork), "fork");
             }
+            // widest bins (the longest units) first, each on its own stream
+            for (size_t li = l1; li-- > l0;) {
+                const BinLaunch& L = launches[li];
+                const int W = B.widths[L.b];
+                PatTcArgs b;
+                std::memcpy(&b, &a, sizeof b);     // padding included: the bytes are a graph signature
+                const char* dd = ws.tcp_desc.as<char>();
+                b.nodes = reinterpret_cast<const PatTcNode*>(dd + L.o_nodes);
+                b.segs = reinterpret_cast<const PatTcSeg*>(dd + L.o_segs);
+                b.n_desc = (int)L.nodes.size();
+                b.n_segs = (int)L.segs.size();
+                b.total_units = L.units;
+                b.n_slots = L.n_slots;
+                b.slot_rows = L.slot_rows;
+                b.table = ws.tcp_table[L.b].as<float>();
+                b.meta = ws.tcp_meta[L.b].as<int4>();
+                b.next = ws.tcp_ctr.as<unsigned long long>() + li;
+                b.done = reinterpret_cast<int32_t*>(ws.tcp_ctr.as<char>() + L.o_done);
+                b.W = W;
+                b.Ns = pat_tc_states(W);
+                b.n_share = W / b.Ns;
+                b.tmem_cols = 32;
+                while (b.tmem_cols < b.Ns) b.tmem_cols *= 2;
+                const int64_t rows = std::max<int64_t>(128, L.slot_rows * L.n_slots);
+                PatTcMaps maps;
+                std::memset(&maps, 0, sizeof maps);
+                int rcm = cached_map(C, ws, b.Ns / 32 - 1, &maps.mat, ws.tc_hi.as<float>(), (int64_t)n_mat * Wm, Wm, 32, b.Ns,
+                                     (int64_t)n_mat * Wm * Wm);
+                if (!rcm) rcm = cached_map(C, ws, 4 + L.b, &maps.vst, b.table, rows, W, 32, 128);
+                if (!rcm) rcm = cached_map(C, ws, 4 + kMaxGroups + L.b, &maps.vst32, b.table, rows, W, 32, 32);
+                if (rcm) return rcm;
+                const cudaStream_t st = fork ? ws.aux[(l1 - 1 - li) % Workspace::kAux] : ws.stream;
+                CK(op_launch(ws, 5, [&] { return launch_pat_tc(maps, b, L.n_ctas, st); }, maps, b, L.n_ctas, st),
+                   "prune tc");
+            }
+            if (fork && !prof && !wide_done) {
+                const int rcw = launch_wide();
+                if (rcw) return rcw;
+            }
+            if (fork)
+                for (int q = 0; q < Workspace::kAux; ++q) {
+                    CK(op_record(ws, ws.ev_join[q], ws.aux[q]), "join");
+                    CK(op_wait(ws, ws.stream, ws.ev_join[q]), "join");
+                }
         }
 
         if (prof) C->prof.end(1, ws.stream, ev);
@@ -1781,7 +1893,7 @@ int enqueue_mixed(cafe_ctx* C, Workspace& ws, const cafe_request* R, TreeHost& T
     // families the tensor-core pass could not represent, or whose result FP32's
     // range may have cost accuracy: planned on the device and recomputed in
     // FP64 without a host round trip
-    if (!tc_bins.empty()) {
+    if (!tc_groups.empty()) {
         RangeFlagArgs rf;
         std::memset(&rf, 0, sizeof rf);
         rf.cat = ws.cat.as<double>();
@@ -1840,21 +1952,9 @@ int enqueue_mixed(cafe_ctx* C, Workspace& ws, const cafe_request* R, TreeHost& T
             tt.n_bins++;
             W = std::max(W, B.widths[b]);
         }
-        tt.cats = ws.catids.as<int32_t>();
-        tt.n_cats = (int)active.size();
-        CK(ws.tiles_fb.reserve((size_t)term_tiles_max(F, tt.n_bins, tt.n_cats) * sizeof(TermTile)), "fallback");
-        tt.tiles = ws.tiles_fb.as<TermTile>();
-        tt.out_counts = d_status + 1;     // [families, tiles]
-        tt.any_flag = d_status + 3;
-        if (prof) C->prof.begin(3, ws.stream, &ev);
-        CK(op_launch(ws, 6, [&] { return launch_term_tiles(tt, C->sm_count, ws.stream); }, tt, C->sm_count, ws.stream),
-           "fallback plan");
-        if (prof) C->prof.end(3, ws.stream, ev);
         TermArgs a;
         std::memset(&a, 0, sizeof a);
         a.plan = T.plan;
-        a.tiles = tt.tiles;
-        a.n_tiles = d_status + 2;
         a.counts = S.d_counts.as<int32_t>();
         a.perm = tt.perm;
         a.mats = ws.mats.as<const double*>();
@@ -1870,10 +1970,29 @@ int enqueue_mixed(cafe_ctx* C, Workspace& ws, const cafe_request* R, TreeHost& T
         a.out = ws.cat.as<double>();
         a.K = K;
         a.cat_probs = ws.catp.as<double>();
-        if (prof) C->prof.begin(3, ws.stream, &ev);
-        CK(op_launch(ws, 7, [&] { return launch_terms64(a, C->sm_count, ws.stream); }, a, C->sm_count, ws.stream),
-           "fallback prune");
-        if (prof) C->prof.end(3, ws.stream, ev);
+        // the list has room for every term of the categories of a pass
+        const int n_cats = (int)active.size();
+        const size_t each = (size_t)term_tiles_max(F, tt.n_bins, 1) * sizeof(TermTile);
+        const int per = (int)std::min<size_t>(n_cats, std::max<size_t>(1, table_limit(C, kTermListBytes) / each));
+        CK(ws.tiles_fb.reserve(per * each), "fallback");
+        a.tiles = tt.tiles = ws.tiles_fb.as<TermTile>();
+        for (int c0 = 0; c0 < n_cats; c0 += per) {
+            tt.cats = ws.catids.as<int32_t>() + c0;
+            tt.n_cats = std::min(per, n_cats - c0);
+            // [families, tiles]: of the first pass, for the caller; of the others
+            tt.out_counts = d_status + (c0 ? 4 : 1);
+            tt.any_flag = d_status + 3;
+            a.n_tiles = tt.out_counts + 1;
+            if (c0) CK(op_memset(ws, tt.out_counts, 0, 2 * sizeof(int32_t), ws.stream), "fallback plan");
+            if (prof) C->prof.begin(3, ws.stream, &ev);
+            CK(op_launch(ws, 6, [&] { return launch_term_tiles(tt, C->sm_count, ws.stream); }, tt, C->sm_count, ws.stream),
+               "fallback plan");
+            if (prof) C->prof.end(3, ws.stream, ev);
+            if (prof) C->prof.begin(3, ws.stream, &ev);
+            CK(op_launch(ws, 7, [&] { return launch_terms64(a, C->sm_count, ws.stream); }, a, C->sm_count, ws.stream),
+               "fallback prune");
+            if (prof) C->prof.end(3, ws.stream, ev);
+        }
         info->d_tail = d_status;     // [status, fallback families, fallback tiles]
     }
 
@@ -2134,8 +2253,10 @@ int enqueue_score(cafe_ctx* C, Workspace& ws, const cafe_request* Rs, int NB, do
     if (ref_mode) {
         groups.push_back(PatGroup{S.pats.all(), Sg, Rg});
     } else {
-        for (size_t b = 0; b < S.bins.widths.size(); ++b)
-            groups.push_back(PatGroup{(int)b, S.bins.widths[b] - 1, S.bins.widths[b] - 1});
+        for (int g = 0; g < S.pats.all(); ++g) {
+            const int w = S.bins.widths[S.pats.bin[g]];
+            groups.push_back(PatGroup{g, w - 1, w - 1});
+        }
     }
     const int32_t* d_famR = ref_mode ? nullptr : S.bins.d_famR.as<int32_t>();
     CK(cudaMemcpyAsync(ws.mats.p, hm, (size_t)CT * T.n_nodes * sizeof(double*), cudaMemcpyHostToDevice, ws.stream),
@@ -2146,31 +2267,35 @@ int enqueue_score(cafe_ctx* C, Workspace& ws, const cafe_request* Rs, int NB, do
     CK(ws.flags.reserve(64), "status");
     int32_t* d_status = ws.flags.as<int32_t>();
     CK(cudaMemsetAsync(d_status, 0, 64, ws.stream), "status");
-    bool fits = true;
-    for (const PatGroup& q : groups) fits &= pat64_class(q) >= 0;
-    if (fits) {
+    if (!ref_mode || takes_rows(C, T, S.pats, Sg, Rg, R->use_error_model ? (C->err_ndev - 1) / 2 : 0)) {
         rc = launch_pat64_groups(C, ws, Rs, T, S, d_famR, groups, (int)active.size(), ws.catids.as<int32_t>(), CT, msize,
                                  scaled, ws.cat.as<double>(), d_status, true, 1);
-        if (rc) return rc;
-        info->d_tail = d_status;
-        info->tail_counts = false;
-        return finish_batch(C, ws, info, gamma, scaled, d_status, d_fam, d_total);
+        if (!rc) {
+            info->d_tail = d_status;
+            info->tail_counts = false;
+            return finish_batch(C, ws, info, gamma, scaled, d_status, d_fam, d_total);
+        }
+        if (rc != CAFE_ERR_OOM) return rc;
     }
 
-    // vectors too long for shared memory (global bounds in the thousands):
-    // 32-family tiles walked up the tree, vectors in global memory
+    // vectors too long for shared memory (global bounds in the thousands), or
+    // tables past their limit or the memory there is: 32-family tiles walked up the
+    // tree, vectors in global memory
     std::vector<PruneTile>& tiles = ws.tile_vec;
     tiles.clear();
     const int TFm = 32;
     for (int c : active)
-        for (int64_t i = 0; i < F; i += TFm) {
-            PruneTile t{};
-            t.first = (int)i;
-            t.count = (int)std::min<int64_t>(TFm, F - i);
-            t.k = c;
-            t.S = Sg;
-            t.R = Rg;
-            tiles.push_back(t);
+        for (const PatGroup& q : groups) {
+            const int64_t first = S.pats.group_first[q.g], n = S.pats.group_count[q.g];
+            for (int64_t i = 0; i < n; i += TFm) {
+                PruneTile t{};
+                t.first = (int)(first + i);
+                t.count = (int)std::min<int64_t>(TFm, n - i);
+                t.k = c;
+                t.S = q.S;
+                t.R = q.R;
+                tiles.push_back(t);
+            }
         }
     const int n_tiles = (int)tiles.size();
     CK(ws.h_tiles.reserve(std::max(n_tiles, 1) * sizeof(PruneTile)), "tiles");
@@ -2186,7 +2311,7 @@ int enqueue_score(cafe_ctx* C, Workspace& ws, const cafe_request* Rs, int NB, do
     a.tiles = ws.tiles.as<PruneTile>();
     a.n_tiles = n_tiles;
     a.counts = S.d_counts.as<int32_t>();
-    a.perm = S.all_items();
+    a.perm = S.bin_items();
     a.mats = ws.mats.as<const double*>();
     a.ld_mat = msize;
     a.prior = C->d_prior.as<double>();
@@ -2194,6 +2319,7 @@ int enqueue_score(cafe_ctx* C, Workspace& ws, const cafe_request* Rs, int NB, do
     a.err = R->use_error_model ? C->d_err.as<double>() : nullptr;
     a.err_rows = C->err_rows;
     a.err_ndev = C->err_ndev;
+    a.fam_R = d_famR;
     a.scratch = ws.scratch.as<double>();
     a.scratch_per_cta = per_cta;
     a.scaled = scaled ? 1 : 0;
@@ -2425,11 +2551,10 @@ int recon_setup(cafe_ctx* C, Workspace& ws, const cafe_request* R, bool categori
 }
 
 // Joint reconstruction over distinct rows: k_pat64's max-product units, then
-// the backtrack, as many categories at a time as keep their tables within 8 GB.
+// the backtrack, as many categories at a time as keep their tables within
+// kRowTableBytes.
 // `words`: [0] counts the failed (category, family) pairs, [1] is set when a
 // bounded wait gave up, both zeroed.
-constexpr size_t kMaxProductBytes = (size_t)8 << 30;
-
 size_t max_product_bytes(const TreeHost& T, const PatternPlan& P, int S) {      // of a category
     size_t n = 0;
     for (size_t ii = 0; ii + 1 < T.internal.size(); ++ii) n += (size_t)P.row_count(P.all(), (int)ii) * (S + 2);
@@ -2477,7 +2602,7 @@ int reconstruct_rows(cafe_ctx* C, Workspace& ws, const cafe_request* R, const Re
                         reinterpret_cast<float* const*>(const_cast<void**>(dptr + (size_t)K * n + src.size())),
                         (int)src.size(), n_st, Z.msize, pitch, ws.stream),
        "log2 matrices");
-    const int pass = (int)std::min<size_t>(K, std::max<size_t>(1, kMaxProductBytes / max_product_bytes(T, P, Z.Smax)));
+    const int pass = (int)std::min<size_t>(K, std::max<size_t>(1, table_limit(C, kRowTableBytes) / max_product_bytes(T, P, Z.Smax)));
     CK(ws.rc_arg.reserve((size_t)K * F * sizeof(int32_t)), "root states");
     CK(ws.rc_row.reserve((size_t)pass * F * ni * sizeof(int32_t)), "rows");
     MaxProduct mx;
@@ -2522,31 +2647,15 @@ int reconstruct_rows(cafe_ctx* C, Workspace& ws, const cafe_request* R, const Re
     return CAFE_OK;
 }
 
-int reconstruct_sync(cafe_ctx* C, Workspace& ws, const cafe_request* R, cafe_reconstruction* out) {
-    AllocScope scope(ws.stream);
-    AllocLimit limit(C->debug_alloc_limit);
-    DrainOnError drain{ws};
-    if (ws.staged) {   // the previous request's copies out of the pinned staging buffers
-        CK(cudaEventSynchronize(ws.ev_staged), "staging");
-        ws.staged = false;
-    }
-    if (!out) return fail(C, CAFE_ERR_INVALID, "null output");
-    if (C->prior.empty()) return fail(C, CAFE_ERR_INVALID, "no prior set (cafe_prior_set)");
-    CK(cudaEventRecord(ws.ev_start, ws.stream), "event");
-    ReconSetup Z;
-    int rc = recon_setup(C, ws, R, true, &Z);
-    if (rc) return rc;
-    TreeHost& T = *Z.T;
-    const int64_t F = Z.S->F;
+// The tile walk (k_pupko): 32 families of a category at a time, vectors and argmax
+// tables per CTA.
+int reconstruct_tiles(cafe_ctx* C, Workspace& ws, const ReconSetup& Z, int root_len, bool exhaustive, int32_t* n_failed) {
+    const TreeHost& T = *Z.T;
     const int K = Z.K, n = T.n_nodes;
-    const int root_len = std::min(Z.Smax, Z.Rmax) + 1;
-    // over distinct rows unless the caller wants every product formed, or a
-    // vector does not fit a CTA or a category's tables 8 GB (then the tile walk)
-    const bool by_rows = F > 0 && !out->exhaustive && pat64_class({0, Z.Smax, root_len - 1}, true) >= 0 &&
-                         max_product_bytes(T, Z.S->pats, Z.Smax) <= kMaxProductBytes;
+    const int64_t F = Z.S->F;
     std::vector<PruneTile>& tiles = ws.tile_vec;
     tiles.clear();
-    for (int k = 0; k < K && !by_rows; ++k)
+    for (int k = 0; k < K; ++k)
         for (int64_t f = 0; f < F; f += 32) {
             PruneTile t{};
             t.first = (int)f;
@@ -2558,54 +2667,39 @@ int reconstruct_sync(cafe_ctx* C, Workspace& ws, const cafe_request* R, cafe_rec
     const int n_ctas = std::max(1, std::min(n_tiles, C->n_ctas));
     const size_t per_cta = pupko_scratch_doubles(T.plan, Z.Smax);
     const size_t c_per_cta = pupko_c_entries(T.plan, Z.Smax);
-    CK(ws.h_tiles.reserve(std::max(n_tiles, 1) * sizeof(PruneTile)), "tiles");
-    CK(ws.tiles.reserve(std::max(n_tiles, 1) * sizeof(PruneTile)), "tiles");
-    if (!by_rows) {
-        CK(ws.scratch.reserve((size_t)n_ctas * per_cta * sizeof(double)), "scratch");
-        CK(ws.rc_c.reserve(std::max<size_t>((size_t)n_ctas * c_per_cta, 1) * sizeof(int32_t)), "argmax tables");
-    }
-    const size_t n_state = (size_t)K * F * n, n_fam = (size_t)F * n;
-    CK(ws.rc_state.reserve(std::max<size_t>(n_state, 1) * sizeof(int32_t)), "states");
-    CK(ws.rc_rmax.reserve(std::max<size_t>((size_t)K * F, 1) * sizeof(double)), "root max");
-    CK(ws.rc_mean.reserve(std::max<size_t>(n_fam, 1) * sizeof(double)), "means");
-    CK(ws.rc_count.reserve(std::max<size_t>(n_fam, 1) * sizeof(int32_t)), "counts");
-    CK(ws.rc_nfail.reserve(2 * sizeof(int32_t)), "failed");
+    CK(ws.h_tiles.reserve(n_tiles * sizeof(PruneTile)), "tiles");
+    CK(ws.tiles.reserve(n_tiles * sizeof(PruneTile)), "tiles");
+    CK(ws.scratch.reserve((size_t)n_ctas * per_cta * sizeof(double)), "scratch");
+    CK(ws.rc_c.reserve(std::max<size_t>((size_t)n_ctas * c_per_cta, 1) * sizeof(int32_t)), "argmax tables");
     std::memcpy(ws.h_tiles.p, tiles.data(), n_tiles * sizeof(PruneTile));
     CK(cudaMemcpyAsync(ws.tiles.p, ws.h_tiles.p, n_tiles * sizeof(PruneTile), cudaMemcpyHostToDevice, ws.stream),
        "tiles");
-    CK(cudaMemsetAsync(ws.rc_nfail.p, 0, 2 * sizeof(int32_t), ws.stream), "failed");
-    if (Z.gamma) {
-        rc = stage_cat_probs(C, ws, R, K, 1);
-        if (rc) return rc;
-    }
-    // the tile walk reads the transposed log2 of every internal non-root node's matrix
+    // it reads the transposed log2 of every internal non-root node's matrix
     const int nstate = Z.Smax + 1;
     std::vector<const void*> lsrc, ldst;
     std::vector<const float*> lmats((size_t)K * n, nullptr);
-    if (!by_rows) {
-        int n_int = 0;
-        for (int v = 0; v < n; ++v) n_int += (T.parent[v] >= 0 && T.leaf_col[v] < 0);
-        const size_t per = (size_t)nstate * nstate;
-        CK(ws.rc_lm.reserve(std::max<size_t>((size_t)K * n_int * per, 1) * sizeof(float)), "log2 matrices");
-        const double* const* hmats = ws.h_mats.as<const double*>();
-        size_t slot = 0;
-        for (int k = 0; k < K; ++k)
-            for (int v = 0; v < n; ++v) {
-                if (T.parent[v] < 0 || T.leaf_col[v] >= 0) continue;
-                float* d = ws.rc_lm.as<float>() + slot++ * per;
-                lmats[(size_t)k * n + v] = d;
-                lsrc.push_back(hmats[(size_t)k * n + v]);
-                ldst.push_back(d);
-            }
-        const size_t np = lmats.size() + 2 * lsrc.size();
-        CK(ws.rc_lptr.reserve(std::max<size_t>(np, 1) * sizeof(void*)), "log2 matrices");
-        std::vector<const void*> all;
-        all.reserve(np);
-        for (const float* p : lmats) all.push_back(p);
-        all.insert(all.end(), lsrc.begin(), lsrc.end());
-        all.insert(all.end(), ldst.begin(), ldst.end());
-        CK(cudaMemcpyAsync(ws.rc_lptr.p, all.data(), np * sizeof(void*), cudaMemcpyHostToDevice, ws.stream), "h2d");
-    }
+    int n_int = 0;
+    for (int v = 0; v < n; ++v) n_int += (T.parent[v] >= 0 && T.leaf_col[v] < 0);
+    const size_t per = (size_t)nstate * nstate;
+    CK(ws.rc_lm.reserve(std::max<size_t>((size_t)K * n_int * per, 1) * sizeof(float)), "log2 matrices");
+    const double* const* hmats = ws.h_mats.as<const double*>();
+    size_t slot = 0;
+    for (int k = 0; k < K; ++k)
+        for (int v = 0; v < n; ++v) {
+            if (T.parent[v] < 0 || T.leaf_col[v] >= 0) continue;
+            float* d = ws.rc_lm.as<float>() + slot++ * per;
+            lmats[(size_t)k * n + v] = d;
+            lsrc.push_back(hmats[(size_t)k * n + v]);
+            ldst.push_back(d);
+        }
+    const size_t np = lmats.size() + 2 * lsrc.size();
+    CK(ws.rc_lptr.reserve(std::max<size_t>(np, 1) * sizeof(void*)), "log2 matrices");
+    std::vector<const void*> all;
+    all.reserve(np);
+    for (const float* p : lmats) all.push_back(p);
+    all.insert(all.end(), lsrc.begin(), lsrc.end());
+    all.insert(all.end(), ldst.begin(), ldst.end());
+    CK(cudaMemcpyAsync(ws.rc_lptr.p, all.data(), np * sizeof(void*), cudaMemcpyHostToDevice, ws.stream), "h2d");
     const void* const* dptr = ws.rc_lptr.as<const void*>();
     PupkoArgs a{};
     a.lmats = reinterpret_cast<const float* const*>(dptr);
@@ -2626,17 +2720,59 @@ int reconstruct_sync(cafe_ctx* C, Workspace& ws, const cafe_request* R, cafe_rec
     a.c_per_cta = (int64_t)c_per_cta;
     a.state = ws.rc_state.as<int32_t>();
     a.root_max = ws.rc_rmax.as<double>();
-    a.n_failed = ws.rc_nfail.as<int32_t>();
-    a.exhaustive = out->exhaustive ? 1 : 0;
+    a.n_failed = n_failed;
+    a.exhaustive = exhaustive ? 1 : 0;
+    CK(launch_log2_matrices(reinterpret_cast<const double* const*>(dptr + lmats.size()),
+                            reinterpret_cast<float* const*>(const_cast<void**>(dptr + lmats.size() + lsrc.size())),
+                            (int)lsrc.size(), nstate, Z.msize, ws.stream),
+       "log2 matrices");
+    CK(launch_pupko(a, n_ctas, ws.stream), "reconstruct");
+    return CAFE_OK;
+}
+
+int reconstruct_sync(cafe_ctx* C, Workspace& ws, const cafe_request* R, cafe_reconstruction* out) {
+    AllocScope scope(ws.stream);
+    AllocLimit limit(C->debug_alloc_limit);
+    DrainOnError drain{ws};
+    if (ws.staged) {   // the previous request's copies out of the pinned staging buffers
+        CK(cudaEventSynchronize(ws.ev_staged), "staging");
+        ws.staged = false;
+    }
+    if (!out) return fail(C, CAFE_ERR_INVALID, "null output");
+    if (C->prior.empty()) return fail(C, CAFE_ERR_INVALID, "no prior set (cafe_prior_set)");
+    CK(cudaEventRecord(ws.ev_start, ws.stream), "event");
+    ReconSetup Z;
+    int rc = recon_setup(C, ws, R, true, &Z);
+    if (rc) return rc;
+    TreeHost& T = *Z.T;
+    const int64_t F = Z.S->F;
+    const int K = Z.K, n = T.n_nodes;
+    const int root_len = std::min(Z.Smax, Z.Rmax) + 1;
+    // over distinct rows unless the caller wants every product formed, a vector
+    // does not fit a CTA or a category's tables their limit or the memory there is
+    // (then the tile walk)
+    bool by_rows = F > 0 && !out->exhaustive && pat64_class({0, Z.Smax, root_len - 1}, true) >= 0 &&
+                   max_product_bytes(T, Z.S->pats, Z.Smax) <= table_limit(C, kRowTableBytes);
+    const size_t n_state = (size_t)K * F * n, n_fam = (size_t)F * n;
+    CK(ws.rc_state.reserve(std::max<size_t>(n_state, 1) * sizeof(int32_t)), "states");
+    CK(ws.rc_rmax.reserve(std::max<size_t>((size_t)K * F, 1) * sizeof(double)), "root max");
+    CK(ws.rc_mean.reserve(std::max<size_t>(n_fam, 1) * sizeof(double)), "means");
+    CK(ws.rc_count.reserve(std::max<size_t>(n_fam, 1) * sizeof(int32_t)), "counts");
+    CK(ws.rc_nfail.reserve(2 * sizeof(int32_t)), "failed");
+    if (Z.gamma) {
+        rc = stage_cat_probs(C, ws, R, K, 1);
+        if (rc) return rc;
+    }
+    CK(cudaMemsetAsync(ws.rc_nfail.p, 0, 2 * sizeof(int32_t), ws.stream), "failed");
     if (by_rows) {
         rc = reconstruct_rows(C, ws, R, Z, root_len, ws.rc_nfail.as<int32_t>());
+        if (rc && rc != CAFE_ERR_OOM) return rc;
+        by_rows = !rc;
+    }
+    if (!by_rows && F > 0) {
+        CK(cudaMemsetAsync(ws.rc_nfail.p, 0, 2 * sizeof(int32_t), ws.stream), "failed");
+        rc = reconstruct_tiles(C, ws, Z, root_len, out->exhaustive != 0, ws.rc_nfail.as<int32_t>());
         if (rc) return rc;
-    } else if (F > 0) {
-        CK(launch_log2_matrices(reinterpret_cast<const double* const*>(dptr + lmats.size()),
-                                reinterpret_cast<float* const*>(const_cast<void**>(dptr + lmats.size() + lsrc.size())),
-                                (int)lsrc.size(), nstate, Z.msize, ws.stream),
-           "log2 matrices");
-        CK(launch_pupko(a, n_ctas, ws.stream), "reconstruct");
     }
     if (F > 0) {
         CK(launch_recon_counts(ws.rc_state.as<int32_t>(), F, n, K, Z.gamma ? ws.catp.as<double>() : nullptr,
@@ -2859,7 +2995,7 @@ int prune_simulated(cafe_ctx* C, Workspace& ws, const TreeHost& T, int S, int RR
     int64_t n_child = 0;
     const int leaf_pitch = (S + 2) & ~1;
     const int64_t leaf_doubles = (int64_t)T.n_leaves * (S + 1) * leaf_pitch;
-    const int64_t limit = (int64_t)(kSimTableBytes / sizeof(double)) - leaf_doubles;
+    const int64_t limit = (int64_t)(table_limit(C, kSimTableBytes) / sizeof(double)) - leaf_doubles;
     for (int g = 0; g < ng; ++g) {
         for (auto& l : level)
             for (int ii : l) {
@@ -3043,7 +3179,6 @@ int pvalues_device(cafe_ctx* C, Workspace& ws, const ReconSetup& Z, bool stream,
     CK(d_ntiles.reserve(16), "tiles");       // the tile count, the status, a zero
     CK(cudaMemsetAsync(d_ntiles.p, 0, 16, ws.stream), "tiles");
     int32_t* d_status = d_ntiles.as<int32_t>() + 1;
-    const bool obs_rows = F > 0 && pat64_class({0, S, RR}) >= 0;
     CK(d_first.reserve((size_t)(S + 2) * sizeof(int64_t)), "simulation plan");
     CK(d_simL.reserve((size_t)NS * sizeof(double)), "simulated likelihoods");
     CK(d_obsL.reserve(std::max<size_t>((size_t)F * RR, 1) * sizeof(double)), "root vectors");
@@ -3060,22 +3195,6 @@ int pvalues_device(cafe_ctx* C, Workspace& ws, const ReconSetup& Z, bool stream,
     CK(d_tree.reserve(tree_tab.size() * sizeof(int32_t)), "tree");
     CK(cudaMemcpyAsync(d_tree.p, tree_tab.data(), tree_tab.size() * sizeof(int32_t), cudaMemcpyHostToDevice, ws.stream),
        "tree");
-    // observed families: states 0..S, root sizes 1..R
-    std::vector<PruneTile> otiles;
-    for (int64_t f = 0; f < F && !obs_rows; f += 32) {
-        PruneTile t{};
-        t.first = (int)f;
-        t.count = (int)std::min<int64_t>(32, F - f);
-        t.S = S;
-        t.R = RR;
-        t.root_lo = 1;
-        otiles.push_back(t);
-    }
-    if (!otiles.empty()) {
-        CK(d_otiles.reserve(otiles.size() * sizeof(PruneTile)), "tiles");
-        CK(cudaMemcpyAsync(d_otiles.p, otiles.data(), otiles.size() * sizeof(PruneTile), cudaMemcpyHostToDevice, ws.stream),
-           "tiles");
-    }
     const int n_ctas_max = C->n_ctas;
     CK(ws.scratch.reserve((size_t)n_ctas_max * T.n_slots * Wmax * 32 * sizeof(double)), "scratch");
     double host_ms = host_ms_since(t_host0);
@@ -3157,15 +3276,30 @@ int pvalues_device(cafe_ctx* C, Workspace& ws, const ReconSetup& Z, bool stream,
             r = std::max(r, r1);
         }
     }
-    if (obs_rows) {
-        // over the set's distinct rows (vectors that fit a CTA's shared memory)
+    // observed families, states 0..S and root sizes 1..R: over the set's distinct
+    // rows, or 32-family tiles
+    rc = CAFE_ERR_OOM;
+    if (F > 0 && takes_rows(C, T, FS.pats, S, RR, 0)) {
         cafe_request rq;
         std::memset(&rq, 0, sizeof rq);
-        rc = launch_pat64_groups(C, ws, &rq, T, FS, nullptr, {{FS.pats.all(), S, RR}}, 1, d_ntiles.as<int32_t>() + 2, 1, msize, false, nullptr, d_status, false, 0, nullptr,
-                                 d_obsL.as<double>());
-        if (rc) return rc;
+        rc = launch_pat64_groups(C, ws, &rq, T, FS, nullptr, {{FS.pats.all(), S, RR}}, 1, d_ntiles.as<int32_t>() + 2, 1, msize,
+                                 false, nullptr, d_status, false, 0, nullptr, d_obsL.as<double>());
+        if (rc && rc != CAFE_ERR_OOM) return rc;
     }
-    if (!otiles.empty()) {
+    if (F > 0 && rc == CAFE_ERR_OOM) {
+        std::vector<PruneTile> otiles;
+        for (int64_t f = 0; f < F; f += 32) {
+            PruneTile t{};
+            t.first = (int)f;
+            t.count = (int)std::min<int64_t>(32, F - f);
+            t.S = S;
+            t.R = RR;
+            t.root_lo = 1;
+            otiles.push_back(t);
+        }
+        CK(d_otiles.reserve(otiles.size() * sizeof(PruneTile)), "tiles");
+        CK(cudaMemcpyAsync(d_otiles.p, otiles.data(), otiles.size() * sizeof(PruneTile), cudaMemcpyHostToDevice, ws.stream),
+           "tiles");
         Prune64Args o = a;
         o.tiles = d_otiles.as<PruneTile>();
         o.n_tiles = (int)otiles.size();
@@ -3591,9 +3725,9 @@ int cafe_debug_set(cafe_ctx* C, int knob, int64_t value) {
         C->debug_wait_limit = (int)value;
         return CAFE_OK;
     }
-    if (knob == CAFE_DEBUG_ALLOC_LIMIT) {
-        if (value < 0) return fail(C, CAFE_ERR_INVALID, "allocation limit out of range");
-        C->debug_alloc_limit = (size_t)value;
+    if (knob == CAFE_DEBUG_ALLOC_LIMIT || knob == CAFE_DEBUG_TABLE_BYTES) {
+        if (value < 0) return fail(C, CAFE_ERR_INVALID, "limit out of range");
+        (knob == CAFE_DEBUG_ALLOC_LIMIT ? C->debug_alloc_limit : C->debug_table_bytes) = (size_t)value;
         return CAFE_OK;
     }
     return fail(C, CAFE_ERR_INVALID, "unknown debug knob %d", knob);

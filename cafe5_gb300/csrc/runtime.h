@@ -73,11 +73,12 @@ struct BinPlan {
 
 // Distinct count patterns below every internal node, per group of families
 // (k_patterns.cu): the rows the pruning kernels contract. The groups are the
-// S-bins in order, and all families together.
+// S-bins in order (a very large one in several), and all families together.
 struct PatternPlan {
     int n_groups = 0, n_internal = 0;
     std::vector<int64_t> group_first, group_count;   // items (families in group order)
     std::vector<int> group_max;       // largest count
+    std::vector<int> bin;             // S-bin, -1 for all families
     std::vector<int64_t> rows;        // [group][internal]: distinct patterns; the root: the group's families
     std::vector<int64_t> child_off;   // [group][internal]: first child index in d_child
     std::vector<int64_t> leaf_off;    // [group][leaf]: first of the counts that occur there, in d_counts; then the end
@@ -274,6 +275,7 @@ struct cafe_ctx {
     std::map<int, int> tuned;    // bin width -> CTAs per SM chosen by cafe_autotune
     int debug_wait_limit = 0;    // cafe_debug_set: polls before the tensor-core wait for a node's GEMMs gives up
     size_t debug_alloc_limit = 0;   // cafe_debug_set: larger device buffers are not to be had (0: no limit)
+    size_t debug_table_bytes = 0;   // cafe_debug_set: factor tables' limits are at most this (0: their own)
     // workspaces: [0] for synchronous calls, [1..] for the serving loop
     std::vector<std::unique_ptr<cafe::Workspace>> ws;
     std::unique_ptr<cafe::Workspace> ws_alt;   // second workspace of the device-pointer calls

@@ -115,8 +115,16 @@ int cafe_version(void);
  * MMAs, frees TMEM, and the call returns CAFE_ERR_TIMEOUT with the context
  * still usable. CAFE_DEBUG_ALLOC_LIMIT: value n > 0 makes every device buffer
  * of more than n bytes that a later call asks for (matrices apart) fail as if
- * memory had run out; 0 lifts it. */
-typedef enum { CAFE_DEBUG_TC_WAIT_LIMIT = 1, CAFE_DEBUG_ALLOC_LIMIT = 2 } cafe_debug_knob;
+ * memory had run out; 0 lifts it. CAFE_DEBUG_TABLE_BYTES: value n > 0 lowers
+ * every limit on the pruning kernels' tables to n bytes (those of family sets
+ * uploaded or changed from then on included), so that small calls take the
+ * routes of very large ones: bins in several parts, tables taken over in turn,
+ * several passes, tile walks. 0 restores the limits. */
+typedef enum {
+    CAFE_DEBUG_TC_WAIT_LIMIT = 1,
+    CAFE_DEBUG_ALLOC_LIMIT = 2,
+    CAFE_DEBUG_TABLE_BYTES = 3
+} cafe_debug_knob;
 int cafe_debug_set(cafe_ctx* ctx, int knob, int64_t value);
 
 /* ---- inputs ---------------------------------------------------------- */

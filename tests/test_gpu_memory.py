@@ -92,3 +92,138 @@ def test_update_that_runs_out_of_memory(ctx, F):
         assert all(np.array_equal(x, y) for x, y in zip(scores(sid), fresh))
         ctx.free_families(sid)
     assert failed > 0
+
+
+def _caterpillar(taxa):
+    """A tree with as many levels as internal nodes."""
+    from cafe5_gb300.tree import parse_newick
+    s = "(T0:1,T1:1)"
+    for i in range(2, taxa):
+        s = f"({s}:1,T{i}:{i})"
+    return parse_newick(s + ";")
+
+
+def test_tables_of_a_deep_tree(ctx):
+    """20,000 families of a tree of 39 levels: a combination's factor table takes
+    0.2 GB, and 64 combinations are in flight for one launch. No buffer passes 4
+    GB, and every candidate keeps the bits it has alone."""
+    from cafe5_gb300.inputs import RootPrior
+    c = np.random.default_rng(7).integers(0, 31, (20000, 40), dtype=np.int32)
+    tid = ctx.upload_tree(_caterpillar(40))
+    sid = ctx.upload_families(tid, c)
+    ctx.set_prior(RootPrior.uniform(40).vector())
+    kw = dict(model=1, precision="mixed_tf32x3")
+    cands = [dict(lambdas=[0.004 * (1 + 0.01 * b)], multipliers=[0.3, 0.7, 1.1, 1.9], cat_probs=[0.25] * 4)
+             for b in range(16)]
+    got = _limited(ctx, 4 << 30, lambda: ctx.score_batch(tid, sid, cands, **kw))
+    assert got is not None
+    for b in (0, 9, 15):
+        alone = ctx.score(tid, sid, cands[b]["lambdas"], multipliers=cands[b]["multipliers"],
+                          cat_probs=cands[b]["cat_probs"], **kw)
+        assert np.array_equal(alone.family_lnl, got[b].family_lnl)
+
+
+def test_fp64_without_room_for_tables(ctx):
+    """FP64 tables of 1 GB (0.4 in bins) where no buffer may pass 256 MB: the tile
+    walk takes the families, with the same bits (the same chains of sums)."""
+    from cafe5_gb300.inputs import RootPrior
+    c = np.random.default_rng(8).integers(0, 31, (20000, 40), dtype=np.int32)
+    tid = ctx.upload_tree(_caterpillar(40))
+    sid = ctx.upload_families(tid, c)
+    ctx.set_prior(RootPrior.uniform(40).vector())
+    for kw in (dict(precision="fp64_ref", S=170, R=150), dict(precision="fp64_binned"),
+               dict(precision="fp64_binned", model=1, multipliers=[0.5, 1.5], cat_probs=[0.4, 0.6])):
+        tiles = _limited(ctx, 256 << 20, lambda: ctx.score(tid, sid, [0.004], **kw))
+        rows = ctx.score(tid, sid, [0.004], **kw)
+        assert tiles is not None
+        assert np.array_equal(tiles.family_lnl, rows.family_lnl) and tiles.total == rows.total
+
+
+@pytest.fixture(params=[1, 100 << 10, 1 << 20], ids=["1 byte", "100 KB", "1 MB"])
+def small_tables(ctx, request):
+    ctx.debug_set(_lib.DEBUG_TABLE_BYTES, request.param)
+    yield ctx
+    ctx.debug_set(_lib.DEBUG_TABLE_BYTES, 0)
+
+
+def _families(F, tree, tail, seed):
+    """Random families: counts up to 30, a few up to each of `tail`."""
+    rng = np.random.default_rng(seed)
+    hi = np.full(F, 30)
+    hi[:len(tail)] = tail
+    c = rng.integers(0, hi[:, None] + 1, (F, len(tree.leaves))).astype(np.int32)
+    c[:, 0] = np.maximum(hi, 1)
+    return np.ascontiguousarray(c[rng.permutation(F)])
+
+
+@pytest.mark.parametrize("F,eps", [(70, 0.0), (70, 0.07), (300, 0.0)])      # (the plan from the host, and the device)
+def test_scores_with_tables_split(small_tables, F, eps):
+    """The routes of very large sets on a small one: bins in parts (at one byte a
+    family each), tables taken over by every next combination, the list of flagged
+    terms in passes, FP64 at global bounds by the tile walk. Bins of 64 to 768
+    states; the same bits as unsplit."""
+    from cafe5_gb300.inputs import ErrorModel, RootPrior
+    from cafe5_gb300.synth import workload
+    ctx = small_tables
+    tree = workload(1, n_families=10, seed=3).tree
+    c = _families(F, tree, [60, 60, 100, 150, 200, 300, 380, 600, 610], 5)
+    ctx.set_prior(RootPrior.uniform(700).vector())
+    ctx.set_error_model(ErrorModel.symmetric(eps, int(c.max())).table() if eps else None)
+    tid = ctx.upload_tree(tree)
+    split = ctx.upload_families(tid, c)
+    limit = {}
+    for p, kw in (("fp64_ref", dict(S=620, R=640)), ("fp64_binned", {}), ("mixed_tf32x3", {})):
+        for model, extra in ((0, [{}] * 9), (1, [dict(multipliers=[0.3, 0.8, 1.9], cat_probs=[0.2, 0.5, 0.3])] * 9)):
+            cands = [dict(e, lambdas=[0.002 * (1 + 0.05 * b)]) for b, e in enumerate(extra)]
+            limit[p, model] = (cands, kw, ctx.score_batch(tid, split, cands, model=model, precision=p,
+                                                          use_error_model=eps > 0, want_categories=True, **kw))
+    ctx.debug_set(_lib.DEBUG_TABLE_BYTES, 0)
+    whole = ctx.upload_families(tid, c)
+    for (p, model), (cands, kw, got) in limit.items():
+        ref = ctx.score_batch(tid, whole, cands, model=model, precision=p, use_error_model=eps > 0, want_categories=True,
+                              **kw)
+        for a, b in zip(got, ref):
+            assert a.status == b.status and a.n_fallback == b.n_fallback, p
+            assert np.array_equal(a.family_lnl, b.family_lnl, equal_nan=True), p
+            assert np.array_equal(a.category_lnl, b.category_lnl, equal_nan=True), p
+            assert a.total == b.total or (np.isnan(a.total) and np.isnan(b.total)), p
+    ctx.set_error_model(None)
+
+
+def test_reconstruction_with_tables_split(small_tables):
+    """Categories in passes, and the tile walk where one category's tables pass the
+    limit: the same states, counts and root values."""
+    from cafe5_gb300.inputs import RootPrior
+    from cafe5_gb300.synth import workload
+    ctx = small_tables
+    tree = workload(1, n_families=10, seed=3).tree
+    c = _families(150, tree, [], 6)
+    ctx.set_prior(RootPrior.uniform(60).vector())
+    tid = ctx.upload_tree(tree)
+    sid = ctx.upload_families(tid, c)
+    kw = dict(S=80, R=60, model=1, multipliers=[0.2, 0.6, 1.1, 2.1], cat_probs=[0.25] * 4)
+    got = ctx.reconstruct(tid, sid, [0.002], **kw)
+    ctx.debug_set(_lib.DEBUG_TABLE_BYTES, 12 << 20)      # (between one category's tables, 5 MB, and all four's)
+    passes = ctx.reconstruct(tid, sid, [0.002], **kw)
+    ctx.debug_set(_lib.DEBUG_TABLE_BYTES, 0)
+    for ref in (ctx.reconstruct(tid, sid, [0.002], **kw), ctx.reconstruct(tid, sid, [0.002], exhaustive=True, **kw)):
+        for a in (got, passes):
+            assert np.array_equal(a.category_state, ref.category_state) and np.array_equal(a.node_count, ref.node_count)
+            assert np.array_equal(a.root_max, ref.root_max) and np.array_equal(a.node_mean, ref.node_mean)
+            assert a.n_failed == ref.n_failed
+
+
+@pytest.mark.parametrize("kb", [1, 4 << 10, 16 << 10])
+def test_pvalues_with_tables_split(ctx, kb):
+    """Simulated families in several passes of state bounds, or by the tile walk
+    where one bound's tables pass the limit; observed ones by the tile walk."""
+    from cafe5_gb300.synth import workload
+    w = workload(0, n_families=300, seed=4)
+    tid = ctx.upload_tree(w.tree)
+    sid = ctx.upload_families(tid, w.families.counts)
+    kw = dict(S=130, R=90, n_simulations=400, seed=3)
+    ref = ctx.pvalues(tid, sid, [0.0025], **kw)
+    ctx.debug_set(_lib.DEBUG_TABLE_BYTES, kb << 10)
+    got = ctx.pvalues(tid, sid, [0.0025], **kw)
+    for k in ("pvalues", "conditional", "root_likelihood"):
+        assert np.array_equal(got[k], ref[k]), k
