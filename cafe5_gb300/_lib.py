@@ -29,7 +29,7 @@ EXPORTS = [
     "cafe_nelder_mead", "cafe_score_batch", "cafe_score_batch_device", "cafe_serving_counters", "cafe_autotune",
     "cafe_reconstruct", "cafe_branch_probabilities", "cafe_pvalues", "cafe_simulate", "cafe_debug_set",
 ]
-DEBUG_TC_WAIT_LIMIT, DEBUG_ALLOC_LIMIT, DEBUG_TABLE_BYTES = 1, 2, 3
+DEBUG_TC_WAIT_LIMIT, DEBUG_ALLOC_LIMIT, DEBUG_TABLE_BYTES, DEBUG_SERVE_BUDGET = 1, 2, 3, 4
 OPT_LAMBDA, OPT_LAMBDA_ALPHA, OPT_LAMBDA_EPSILON, OPT_ALPHA = 0, 1, 2, 3
 
 

@@ -3730,6 +3730,12 @@ int cafe_debug_set(cafe_ctx* C, int knob, int64_t value) {
         (knob == CAFE_DEBUG_ALLOC_LIMIT ? C->debug_alloc_limit : C->debug_table_bytes) = (size_t)value;
         return CAFE_OK;
     }
+    if (knob == CAFE_DEBUG_SERVE_BUDGET) {
+        if (value < 1) return fail(C, CAFE_ERR_INVALID, "budget out of range");
+        std::lock_guard<std::mutex> lq(C->qmu);
+        C->serve_budget = (size_t)value;
+        return CAFE_OK;
+    }
     return fail(C, CAFE_ERR_INVALID, "unknown debug knob %d", knob);
 }
 
@@ -4200,11 +4206,24 @@ int cafe_score_batch_device(cafe_ctx* C, const cafe_request* req, int n, double*
 // ------------------------------------------------------- serving loop
 
 namespace cafe {
+// Device bytes a request holds while admitted: per-family category terms, results
+// and flags, and the factor tables of its combinations (the other buffers of a
+// workspace do not grow with the families). A batch's tables are those of all its
+// combinations, up to `most`.
+struct Footprint {
+    size_t bytes = 0, tables = 0, most = 0;
+    size_t total() const { return bytes + std::min(tables, most); }
+    void add(const Footprint& o) {
+        bytes += o.bytes;
+        tables += o.tables;
+        most = std::max(most, o.most);
+    }
+};
 struct Request {
     cafe_request req{};
     std::vector<double> lambdas, mult, probs;
     cafe_result* res = nullptr;
-    size_t bytes = 0;          // admission footprint
+    Footprint need;            // for admission
     bool small = false;        // too small to fill the device alone (runs beside others)
     int rc = CAFE_OK;
     bool done = false;
@@ -4231,13 +4250,35 @@ bool batchable(const cafe_request& a, const cafe_request& b) {
     return true;
 }
 
-// Device bytes a request holds while admitted: per-family category terms,
-// results and flags (the workspaces' fixed buffers are not counted).
-size_t request_footprint(cafe_ctx* C, const cafe_request& r) {
-    auto it = C->sets.find(r.set_id);
-    const int64_t F = it == C->sets.end() ? 0 : it->second->F;
+Footprint request_footprint(cafe_ctx* C, const cafe_request& r) {
+    Footprint f;
+    f.bytes = 4096;
+    const auto si = C->sets.find(r.set_id);
+    if (si == C->sets.end() || !si->second->ready) return f;
+    const FamSet& S = *si->second;
+    const PatternPlan& P = S.pats;
     const int K = r.model == CAFE_MODEL_GAMMA ? std::max(r.n_categories, 1) : 1;
-    return (size_t)F * ((size_t)K * 8 + 8 + 4) + 4096;
+    f.bytes += (size_t)S.F * ((size_t)K * 8 + 8 + 4);
+    // of one combination: FP64 rows, and the tensor cores'
+    size_t fp64 = 0, tc = 0;
+    auto leaves = [&](int g, size_t n) { return (size_t)S.n_leaves * (std::min<size_t>(P.group_max[g], n) + 1) * (n + 1) * sizeof(double); };
+    if (r.precision == CAFE_PREC_FP64_REF) {
+        const size_t n = (size_t)std::max(0, std::max(r.max_family_size, r.max_root_family_size)) + 1;
+        fp64 = row_bytes(P, P.all(), n) + leaves(P.all(), n);
+        if (fp64 > kRowTableBytes) fp64 = 0;      // (the tile walk's vectors)
+    } else {
+        for (int g = 0; g < P.all(); ++g) {
+            const size_t w = S.bins.widths[P.bin[g]];
+            if (r.precision == CAFE_PREC_MIXED_TF32X3 && w <= (size_t)kTcMaxW)
+                tc += row_bytes(P, g, w) / ((w + 1) * sizeof(double)) * (w * sizeof(float) + sizeof(int4));
+            else
+                fp64 += row_bytes(P, g, w) + leaves(g, w);
+        }
+    }
+    f.tables = K * (fp64 + tc);
+    f.most = (fp64 ? std::max(kTableBytes, r.precision == CAFE_PREC_FP64_REF ? fp64 : std::min(fp64, kWaveBytes)) : 0) +
+             (tc ? kTcTableBytes : 0);
+    return f;
 }
 
 constexpr int kMaxMerge = 32;           // candidates merged into one batched launch
@@ -4248,7 +4289,7 @@ void server_loop(cafe_ctx* C, int wi) {
     Workspace& ws = *C->ws[wi];
     for (;;) {
         std::vector<std::shared_ptr<Request>> batch;
-        size_t bytes = 0;
+        Footprint need;
         bool behind = false;     // another batch is in flight: this one runs at the lower priority
         {
             std::unique_lock<std::mutex> lk(C->qmu);
@@ -4262,17 +4303,19 @@ void server_loop(cafe_ctx* C, int wi) {
                 // small requests run side by side on every server stream
                 const bool small = C->queue.front()->small;
                 if (C->batches_in_flight >= (small ? (int)C->servers.size() : kMaxBatchesInFlight)) return false;
-                return C->in_flight == 0 || C->in_flight_bytes + C->queue.front()->bytes <= C->serve_budget;
+                return C->in_flight == 0 || C->in_flight_bytes + C->queue.front()->need.total() <= C->serve_budget;
             });
             if (C->stop && C->queue.empty()) return;
             batch.push_back(C->queue.front());
             C->queue.pop_front();
-            bytes = batch[0]->bytes;
+            need = batch[0]->need;
             // continuous batching: compatible requests queued behind it join
             // the same launch
             for (auto it = C->queue.begin(); it != C->queue.end() && (int)batch.size() < kMaxMerge;) {
-                if (batchable(batch[0]->req, (*it)->req) && C->in_flight_bytes + bytes + (*it)->bytes <= C->serve_budget) {
-                    bytes += (*it)->bytes;
+                Footprint with = need;
+                with.add((*it)->need);
+                if (batchable(batch[0]->req, (*it)->req) && C->in_flight_bytes + with.total() <= C->serve_budget) {
+                    need = with;
                     batch.push_back(*it);
                     it = C->queue.erase(it);
                 } else {
@@ -4280,7 +4323,7 @@ void server_loop(cafe_ctx* C, int wi) {
                 }
             }
             C->in_flight += (int)batch.size();
-            C->in_flight_bytes += bytes;
+            C->in_flight_bytes += need.total();
             C->batches_in_flight++;
             behind = C->batches_in_flight > 1;
         }
@@ -4346,7 +4389,7 @@ void server_loop(cafe_ctx* C, int wi) {
         {
             std::lock_guard<std::mutex> lk(C->qmu);
             C->in_flight -= n;
-            C->in_flight_bytes -= bytes;
+            C->in_flight_bytes -= need.total();
             C->batches_in_flight--;
             C->completed += n;
             for (auto& r : batch)
@@ -4397,7 +4440,7 @@ int cafe_submit(cafe_ctx* C, const cafe_request* req, cafe_result* res, uint64_t
     r->t_submit = std::chrono::steady_clock::now();
     {
         std::lock_guard<std::mutex> lk(C->mu);
-        r->bytes = request_footprint(C, r->req);
+        r->need = request_footprint(C, r->req);
         auto si = C->sets.find(r->req.set_id);
         r->small = si != C->sets.end() && small_request(C, &r->req, 1, si->second->F);
     }

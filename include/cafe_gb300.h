@@ -119,11 +119,13 @@ int cafe_version(void);
  * every limit on the pruning kernels' tables to n bytes (those of family sets
  * uploaded or changed from then on included), so that small calls take the
  * routes of very large ones: bins in several parts, tables taken over in turn,
- * several passes, tile walks. 0 restores the limits. */
+ * several passes, tile walks. 0 restores the limits. CAFE_DEBUG_SERVE_BUDGET:
+ * value n > 0 is the request loop's budget from then on (cafe_submit). */
 typedef enum {
     CAFE_DEBUG_TC_WAIT_LIMIT = 1,
     CAFE_DEBUG_ALLOC_LIMIT = 2,
-    CAFE_DEBUG_TABLE_BYTES = 3
+    CAFE_DEBUG_TABLE_BYTES = 3,
+    CAFE_DEBUG_SERVE_BUDGET = 4
 } cafe_debug_knob;
 int cafe_debug_set(cafe_ctx* ctx, int knob, int64_t value);
 
@@ -224,8 +226,9 @@ int cafe_score_batch_device(cafe_ctx* ctx, const cafe_request* reqs, int n, doub
 
 /* Continuous-batching request loop for many concurrent optimizers: submit
  * returns at once with a ticket; the request is admitted when a stream is
- * free and its estimated device footprint fits the loop's budget (a quarter
- * of the device memory free at context creation). Compatible requests
+ * free and its estimated device footprint, factor tables included, fits the
+ * loop's budget (a quarter of the device memory free at context creation).
+ * Compatible requests
  * queued at that moment (the batching rules of cafe_score_batch) are merged
  * into one batched launch; admitted batches run concurrently on separate
  * streams. `res` is filled when done (host buffers must stay valid).

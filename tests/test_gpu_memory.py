@@ -227,3 +227,36 @@ def test_pvalues_with_tables_split(ctx, kb):
     got = ctx.pvalues(tid, sid, [0.0025], **kw)
     for k in ("pvalues", "conditional", "root_likelihood"):
         assert np.array_equal(got[k], ref[k]), k
+
+
+@pytest.mark.parametrize("kw", [dict(precision="mixed_tf32x3"), dict(precision="fp64_binned"),
+                                dict(precision="fp64_ref", S=170, R=150)], ids=lambda k: k["precision"])
+def test_serving_counts_the_tables(kw):
+    """The request loop's budget covers the factor tables: 10,000 families of 24
+    taxa take 3 MB of results and over 10 MB of tables a category, so with a budget
+    of 40 MB two requests of four categories (on two sets: they share no launch) never run
+    side by side, which they do without it."""
+    from cafe5_gb300.engine import Context
+    from cafe5_gb300.inputs import RootPrior
+    from cafe5_gb300.synth import workload
+    w = workload(1, n_families=10000, seed=36)
+    ctx = Context()
+    try:
+        ctx.set_prior(RootPrior.uniform(150).vector())
+        tid = ctx.upload_tree(w.tree)
+        sets = [ctx.upload_families(tid, w.families.counts) for _ in range(2)]
+        kw = dict(kw, model=1, multipliers=w.multipliers, cat_probs=w.cat_probs)
+        ref = [ctx.score(tid, s, [0.002], **kw).total for s in sets]
+
+        def overlap():
+            before = ctx.serving_stats()["overlap_ms"]
+            handles = [ctx.submit(tid, sets[i % 2], [0.002], **kw) for i in range(12)]
+            got = np.array([ctx.poll(h).total for h in handles])
+            assert np.all(np.abs(got - ref * 6) <= 1e-6 * got)
+            return ctx.serving_stats()["overlap_ms"] - before
+
+        assert any(overlap() > 0 for _ in range(5))
+        ctx.debug_set(_lib.DEBUG_SERVE_BUDGET, 40 << 20)
+        assert overlap() == 0
+    finally:
+        ctx.close()
