@@ -978,7 +978,7 @@ int cache_build_impl(cafe_ctx* C, Workspace& ws, PendingJobs& P) {
     const bool prof = ws.sync;
     cudaEvent_t ev;
     if (prof) C->prof.begin(0, bs, &ev);
-    CK(launch_matrix_build(ws.jobs.as<MatrixJob>(), (int)n, max_size, bs), "matrix build");
+    CK(launch_matrix_build(ws.jobs.as<MatrixJob>(), (int)n, max_size, C->sm_count, bs), "matrix build");
     if (prof) {
         C->prof.end(0, bs, ev);
         C->prof.acc.matrices_built += (int64_t)n;

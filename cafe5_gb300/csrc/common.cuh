@@ -62,7 +62,7 @@ constexpr int kMaxNodes = 512;
 // Launch wrappers implemented in the .cu files (host side).
 namespace cafe {
 
-cudaError_t launch_matrix_build(const MatrixJob* d_jobs, int n_jobs, int max_size, cudaStream_t s);
+cudaError_t launch_matrix_build(const MatrixJob* d_jobs, int n_jobs, int max_size, int sm_count, cudaStream_t s);
 
 // ---- distinct count patterns per subtree (k_patterns.cu) ----
 constexpr int kMaxGroups = 16;

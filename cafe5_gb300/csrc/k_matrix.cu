@@ -234,14 +234,14 @@ __global__ void __launch_bounds__(128) k_matrix_build(const MatrixJob* __restric
 
 }  // namespace
 
-cudaError_t launch_matrix_build(const MatrixJob* d_jobs, int n_jobs, int max_size, cudaStream_t s) {
+cudaError_t launch_matrix_build(const MatrixJob* d_jobs, int n_jobs, int max_size, int sm_count, cudaStream_t s) {
     if (n_jobs <= 0) return cudaSuccess;
     // one thread per row pair, in whole warps, and as many CTAs per matrix as
     // its pairs need: one warp each while that gives at most four per SM, then
     // two, which share the tables
     const int pairs = max_size / 2;
     const int warps = std::max(1, (pairs + 31) / 32);
-    const int threads = warps == 1 || (int64_t)n_jobs * warps <= 600 ? 32 : 64;
+    const int threads = warps == 1 || (int64_t)n_jobs * warps <= 4 * sm_count ? 32 : 64;
     const int parts = std::max(1, (pairs + threads - 1) / threads);
     size_t smem = sizeof(double) * (3 * (size_t)(max_size + 1) + (size_t)(threads / 32) * kStageCols * kStagePitch);
     if (smem > 48 * 1024) {
