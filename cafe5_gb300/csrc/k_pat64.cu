@@ -227,16 +227,17 @@ __device__ void root_family(const Pat64Args& a, const Pat64Node& nd, const NodeS
     double o;
     if (a.model == 0) {
         // max_j log x + log eq, evaluated only where the FP32 logarithms (each
-        // within 1.3e-4) come within 2^-6 of the best
+        // within 1.3e-4) come within 2^-6 of the best (of priors above 0: others,
+        // NaN among them, have no logarithm)
         float top = -INFINITY;
         for (int j = lane; j < Rf; j += 32)
-            if (j < a.n_prior) top = fmaxf(top, flog2(x[j]) + flog2(a.prior[j]));
+            if (j < a.n_prior && a.prior[j] > 0.0) top = fmaxf(top, flog2(x[j]) + flog2(a.prior[j]));
 #pragma unroll
         for (int q = 16; q > 0; q >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, q));
         double best = -INFINITY;
         if (top > -INFINITY)
             for (int j = lane; j < Rf; j += 32)
-                if (j < a.n_prior && flog2(x[j]) + flog2(a.prior[j]) >= top - 0.015625f) {
+                if (j < a.n_prior && a.prior[j] > 0.0 && flog2(x[j]) + flog2(a.prior[j]) >= top - 0.015625f) {
                     const double v = log(x[j]) + log(a.prior[j]);
                     best = v > best ? v : best;
                 }

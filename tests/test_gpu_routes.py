@@ -120,3 +120,21 @@ def test_pvalues_drawn_on_the_host(ctx, lam, n_sim, R):
     for x, y in ((got["conditional"], cd), (got["root_likelihood"], rv)):
         assert np.array_equal(x > 0, y > 0)
         assert np.all(np.abs(x - y) <= 1e-10 * y)
+
+
+@pytest.mark.parametrize("bad", [np.nan, -1.0])
+def test_prior_entries_that_are_no_probabilities(ctx, bad):
+    """A prior entry that is NaN or negative takes no part in the base model's
+    maximum over root sizes (its logarithm is not above any): as if it were 0."""
+    rng = np.random.default_rng(7)
+    from cafe5_gb300.inputs import RootPrior
+    tree, tid, sid = _upload(ctx, BINARY, rng.integers(1, 25, (37, 5)), 60)
+    p = RootPrior.uniform(60).vector().copy()
+    got = []
+    for v in (0.0, bad):
+        p[20] = v
+        ctx.set_prior(p)
+        got.append([ctx.score(tid, sid, [0.01], **kw).family_lnl for kw in
+                    (dict(S=90, R=60), dict(precision="fp64_binned"), dict(precision="mixed_tf32x3"))])
+    for a, b in zip(*got):
+        assert np.all(np.isfinite(a)) and np.array_equal(a, b)
