@@ -17,7 +17,7 @@
 //    families x nodes on 10,000 families of 24 taxa;
 //  * a warp leaves out a 32-column chunk of the sum when every term in it is
 //    below 2^-55 of every partial sum it would join (exponents of the
-//    chunk's largest M and L against the smallest partial sum): each of
+//    chunk's largest M and |L| against the smallest partial sum): each of
 //    those FMAs would return its addend unchanged, so the bits stay. L
 //    falls off geometrically past the observed counts, and with the
 //    reference's global bound (171 states for counts up to 35) most of the
@@ -75,9 +75,11 @@ __device__ __forceinline__ void bar_arrive(int id, int n) {
     asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory");
 }
 
-// High word of a value >= 0, with 0 only for an exact zero.
+// High word of |x|, with 0 only for an exact zero. (Vectors can hold negative
+// values: a search over an error model's epsilon may try a negative one.)
+__device__ __forceinline__ int hi_abs(double x) { return __double2hiint(x) & 0x7fffffff; }
 __device__ __forceinline__ int hi_key(double x) {
-    const int h = __double2hiint(x);
+    const int h = hi_abs(x);
     return h ? h : (__double2loint(x) ? 1 : 0);
 }
 
@@ -576,7 +578,7 @@ __device__ __forceinline__ void few_rows(const Pat64Args& a, const Unit& u, cons
                 int am = 0x7fffffff;
 #pragma unroll
                 for (int r = 0; r < kFewRows; ++r)
-                    if (r < np) am = min(am, __double2hiint(acc[r]));
+                    if (r < np) am = min(am, hi_abs(acc[r]));
                 const int ea = am >> 20;
                 skip = mk == 0 || lk == 0 || (ea > 0 && (mk >> 20) + (lk >> 20) + 2 <= ea + 968);
                 skip = __all_sync(0xffffffffu, skip);
@@ -814,8 +816,7 @@ __global__ void __launch_bounds__(NTHR, 6) k_pat64(const Pat64Args a) {
                         for (int h = 0; h < KC / 8; ++h) mk = max(mk, hi_key(pf[h]));
 #pragma unroll
                         for (int o = 1; o < 8; o <<= 1) mk = max(mk, __shfl_xor_sync(0xffffffffu, mk, o));
-                        const int am = min(min(__double2hiint(acc[0]), __double2hiint(acc[1])),
-                                           min(__double2hiint(acc[2]), __double2hiint(acc[3])));
+                        const int am = min(min(hi_abs(acc[0]), hi_abs(acc[1])), min(hi_abs(acc[2]), hi_abs(acc[3])));
                         const int ea = am >> 20;
                         skip = mk == 0 || lk == 0 || (ea > 0 && (mk >> 20) + (lk >> 20) + 2 <= ea + 968);
                         skip = __all_sync(0xffffffffu, skip);

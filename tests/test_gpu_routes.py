@@ -138,3 +138,40 @@ def test_prior_entries_that_are_no_probabilities(ctx, bad):
                     (dict(S=90, R=60), dict(precision="fp64_binned"), dict(precision="mixed_tf32x3"))])
     for a, b in zip(*got):
         assert np.all(np.isfinite(a)) and np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("F", [3, 150])           # (units of a few rows, and of eight)
+@pytest.mark.parametrize("eps", [-0.05, -0.2])
+def test_negative_epsilon(ctx, F, eps):
+    """A search over an error model's epsilon may try a negative one: leaf vectors
+    are then negative away from the observed count, whole chunks of columns of
+    them, and every sum still holds all its terms. At global bounds the bits of the
+    tile walk, which forms every product; in bins the oracle's values, 1e-11
+    relative (two orders of summation, of terms that partly cancel)."""
+    import oracle
+    from cafe5_gb300.families import FamilySet, bin_families
+    from cafe5_gb300.inputs import RootPrior
+    rng = np.random.default_rng(8)
+    # C and D pull their parent's vector past state 32, where E's is negative: the
+    # node above has its largest values there
+    c = rng.integers([22, 22, 35, 35, 18], [31, 31, 38, 38, 24], (F, 5)).astype(np.int32)
+    tree, tid, sid = _upload(ctx, BINARY, c, 60)
+    table = np.tile([eps, 1 - 2 * eps, eps], (40, 1))
+    table[0] = [0.0, 1 - eps, eps]
+    ctx.set_error_model(table)
+    kw = dict(model=1, multipliers=[0.4, 1.6], cat_probs=[0.5, 0.5])
+    score = dict(kw, use_error_model=True, want_categories=True)
+    rows = ctx.score(tid, sid, [0.01], S=110, R=60, **score)
+    ctx.debug_set(_lib.DEBUG_TABLE_BYTES, 1)
+    tiles = ctx.score(tid, sid, [0.01], S=110, R=60, **score)
+    ctx.debug_set(_lib.DEBUG_TABLE_BYTES, 0)
+    assert np.any(np.isfinite(rows.category_lnl))
+    assert np.array_equal(rows.category_lnl, tiles.category_lnl, equal_nan=True)
+    assert np.array_equal(rows.family_lnl, tiles.family_lnl, equal_nan=True)
+    _, Sf, Rf = bin_families(FamilySet([str(i) for i in range(F)], c))
+    _, ref, _ = oracle.score(oracle.TreeArrays.from_tree(tree), c, [0.01], fam_S=Sf, fam_R=Rf, scaled=True,
+                             prior=RootPrior.uniform(60).vector(), err_rows=table, **kw)
+    got = ctx.score(tid, sid, [0.01], precision="fp64_binned", **score).family_lnl
+    ok = np.isfinite(ref)          # (the oracle's NaN: a category whose root values are all negative)
+    assert np.all(np.abs(got[ok] - ref[ok]) <= 1e-11 * np.abs(ref[ok]))
+    ctx.set_error_model(None)
