@@ -559,8 +559,8 @@ def config2_phase(ctx, torch, stream, flush, steps: int = 4, B: int = 4):
     """The two-lambda local model with the error model: a 32-taxon tree whose
     10-taxon clade runs at lambda2, epsilon 0.05, 50,000 families from a
     heavy-tailed root (95 % Poisson(4), 5 % geometric(0.02); S-bins 32 to
-    512). Every bin goes into one request on the tensor cores (bins of 384
-    and 512 states in CTA pairs), replayed as one CUDA graph. B candidate
+    512). Every bin goes into one request on the tensor cores, replayed as one
+    CUDA graph. B candidate
     (lambda1, lambda2) vectors per step; device
     time per step, the FP64 path at the same bins, and the largest
     per-family dlnL against it."""
@@ -609,7 +609,7 @@ def config2_phase(ctx, torch, stream, flush, steps: int = 4, B: int = 4):
             "profiled_call_ms": {k: round(v, 3) for k, v in prof.items()
                                  if k in ("matrix_ms", "prune_ms", "other_ms", "finish_ms", "host_total_ms")},
             "note": "profiled_call_ms: one direct (unreplayed) call on new candidates with per-launch events: prune_ms = "
-                    "tensor-core bins (384 and 512 in CTA pairs), other_ms = TF32 conversion"}
+                    "tensor-core bins (32 to 512 states), other_ms = TF32 conversion"}
 
 
 def config0_phase(ctx, cpu_seconds: float, reps: int = 10):

@@ -48,7 +48,9 @@
 // segments are independent, and a unit's inputs were handed out a whole step
 // earlier, to CTAs that are running, so every wait for them (bounded) ends.
 // Factor tables exist for n_slots combinations at a time; a combination's
-// units wait for the root of the one whose table they take over.
+// units wait for the root of the one whose table they take over. The skew keeps
+// levels + 1 blocks of tables alive; where memory has room for fewer, the blocks'
+// segments follow one another unskewed, and one table is enough.
 //
 // Roles in a CTA: a scheduler warp (units, their inputs' completion, child
 // indices), an issuer (TMA, MMA, completion) and 4 or 8 data warps (rows:

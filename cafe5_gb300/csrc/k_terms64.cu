@@ -18,9 +18,10 @@
 //
 // Measured (conversion, planning and recompute of a call; 32-family tiles of
 // k_prune64, planned by one block, before): 10,000 families of 24 taxa, 96
-// states, a few terms flagged 2.67 -> 0.15 ms; 20,000 of 48 taxa, 64 states, 512
-// categories, the small categories of 264 families flagged 34.3 -> 22.3; nothing
-// flagged 0.021 -> 0.020.
+// states, a few terms flagged 2.67 -> 0.15 ms; 20,000 of 48 taxa, 64 states, 64
+// candidates with the eight rates of alpha = 0.5, small categories of 264 families
+// flagged in each 34.3 -> 22.3 (6.0 with alpha from 0.5 to 1.13, where fewer terms
+// are); nothing flagged 0.021 -> 0.020.
 #include "common.cuh"
 
 #include <cooperative_groups.h>
