@@ -213,7 +213,7 @@ def test_reconstruction_with_tables_split(small_tables):
             assert a.n_failed == ref.n_failed
 
 
-@pytest.mark.parametrize("kb", [1, 4 << 10, 16 << 10])
+@pytest.mark.parametrize("kb", [1, 8 << 10, 32 << 10])      # (the tile walk; many passes; a few)
 def test_pvalues_with_tables_split(ctx, kb):
     """Simulated families in several passes of state bounds, or by the tile walk
     where one bound's tables pass the limit; observed ones by the tile walk."""
@@ -221,7 +221,7 @@ def test_pvalues_with_tables_split(ctx, kb):
     w = workload(0, n_families=300, seed=4)
     tid = ctx.upload_tree(w.tree)
     sid = ctx.upload_families(tid, w.families.counts)
-    kw = dict(S=130, R=90, n_simulations=400, seed=3)
+    kw = dict(S=200, R=90, n_simulations=400, seed=3)      # (state bounds 51 to about 150)
     ref = ctx.pvalues(tid, sid, [0.0025], **kw)
     ctx.debug_set(_lib.DEBUG_TABLE_BYTES, kb << 10)
     got = ctx.pvalues(tid, sid, [0.0025], **kw)
