@@ -477,7 +477,7 @@ constexpr int kFlaggedCounts = 1 << 14;
 // take more than kGroupBytes is several groups) and for all of them together (its
 // last group). Items are the families in bin order, then in their own.
 
-constexpr size_t kGroupBytes = (size_t)1 << 30;
+constexpr size_t kGroupBytes = (size_t)8 << 30;
 size_t table_limit(const cafe_ctx* C, size_t bytes) {      // (a test hook makes every limit smaller)
     return C->debug_table_bytes ? std::min(bytes, C->debug_table_bytes) : bytes;
 }
@@ -778,7 +778,8 @@ int build_patterns(cafe_ctx* C, const TreeHost& T, FamSet& S, const std::vector<
         std::vector<int64_t> more(parts);
         for (int g = 0; g < S.pats.all(); ++g) {
             const int b = S.pats.bin[g];
-            const int64_t need = (int64_t)(row_bytes(S.pats, g, B.widths[b]) / limit);
+            // (8 W + 32 bytes a row: twice the tensor cores', more than FP64's)
+            const int64_t need = (int64_t)(row_bytes(S.pats, g, B.widths[b] + 3) / limit);
             if (need > 0) more[b] = std::min(B.bin_count[b], std::max(more[b], std::max(2 * parts[b], need + need / 4 + 1)));
         }
         if (more == parts) return CAFE_OK;
@@ -1233,7 +1234,7 @@ int pat64_class(const PatGroup& q, bool max_product = false) {
 // side, and up to kRowTableBytes where all families are one group (past it they
 // are left to the tile walks, whose vectors take the same memory whatever their
 // number); of several combinations, kTableBytes.
-constexpr size_t kWaveBytes = (size_t)4 << 30, kRowTableBytes = (size_t)8 << 30, kTableBytes = (size_t)2 << 30;
+constexpr size_t kWaveBytes = (size_t)8 << 30, kRowTableBytes = (size_t)8 << 30, kTableBytes = (size_t)2 << 30;
 
 // All families at states 0..S and root sizes 1..R: whether k_pat64 takes them.
 // Counts past the states and the error model's reach (half deviations) share a
