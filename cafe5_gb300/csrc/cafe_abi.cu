@@ -473,9 +473,9 @@ struct TempBuf {
 constexpr int kFlaggedCounts = 1 << 14;
 
 // ---- the distinct patterns of every subtree, for the families of every S-bin
-// (the plan's groups, in the order of the bins; a bin whose factor rows would
-// take more than kGroupBytes is several groups) and for all of them together (its
-// last group). Items are the families in bin order, then in their own.
+// (the plan's groups, in the order of the bins) and for all of them together (its
+// last group). A group whose factor rows would take more than kGroupBytes is cut
+// into several. Items are the families in bin order, then in their own.
 
 constexpr size_t kGroupBytes = (size_t)8 << 30;
 size_t table_limit(const cafe_ctx* C, size_t bytes) {      // (a test hook makes every limit smaller)
@@ -559,8 +559,9 @@ void patterns_on_host(const TreeHost& T, const FamSet& S, PatternPlan& P, std::v
     std::vector<std::vector<int32_t>> id(ni);       // a row's number in the group, -1: does not occur there
     std::vector<uint8_t> flag;
     for (int g = 0; g < P.n_groups; ++g) {
-        const bool all = g == P.all();
         const int64_t i0 = P.group_first[g], n = P.group_count[g];
+        const bool all = i0 == F && n == F;
+        auto fam = [&](int64_t q) { return i0 < F ? S.bins.perm[i0 + q] : i0 - F + q; };
         const size_t span = (size_t)std::min(P.group_max[g], kFlaggedCounts) + 1;
         if (!all) {
             for (int ii = 0; ii + 1 < ni; ++ii) id[ii].assign(kids[ii].size() / (T.cstart[ii + 1] - T.cstart[ii]), -1);
@@ -570,7 +571,7 @@ void patterns_on_host(const TreeHost& T, const FamSet& S, PatternPlan& P, std::v
                 const int64_t rows = ii + 1 == ni ? n : (int64_t)id[ii].size();
                 for (int64_t q = 0; q < rows; ++q) {
                     if (ii + 1 < ni && id[ii][q] < 0) continue;
-                    const int32_t* k = &kids[ii][(ii + 1 == ni ? S.bins.perm[i0 + q] : q) * nch];
+                    const int32_t* k = &kids[ii][(ii + 1 == ni ? fam(q) : q) * nch];
                     for (int c = 0; c < nch; ++c)
                         if (const int ci = T.internal_index[T.child[c0 + c]]; ci >= 0) id[ci][k[c]] = 0;
                 }
@@ -589,7 +590,7 @@ void patterns_on_host(const TreeHost& T, const FamSet& S, PatternPlan& P, std::v
                     id[ii][q] = here;
                 }
                 ++here;
-                const int32_t* k = &kids[ii][(root && !all ? S.bins.perm[i0 + q] : q) * nch];
+                const int32_t* k = &kids[ii][(root ? fam(q) : q) * nch];
                 for (int c = 0; c < nch; ++c) {
                     const int ch = T.child[c0 + c], ci = T.internal_index[ch];
                     if (ci < 0) flag[T.leaf_col[ch] * span + std::min(k[c], kFlaggedCounts)] = 1;
@@ -722,7 +723,7 @@ int patterns_on_device(cafe_ctx* C, const TreeHost& T, FamSet& S, PatternPlan& P
 // 1,000 of 12 193 and 157, 10,000 of 24 3,035 and 893.
 constexpr int64_t kHostPatterns = 6000;
 
-// The plan of bins cut into `parts` groups each.
+// The plan of bins, and of the whole set (last), cut into `parts` groups each.
 int build_groups(cafe_ctx* C, const TreeHost& T, FamSet& S, const std::vector<int>& bin_max, int all_max,
                  const std::vector<int64_t>& parts) {
     PatternPlan& P = S.pats;
@@ -738,12 +739,15 @@ int build_groups(cafe_ctx* C, const TreeHost& T, FamSet& S, const std::vector<in
         P.group_max.push_back(max);
         P.bin.push_back(bin);
     };
-    for (size_t b = 0; b < B.widths.size(); ++b)
+    const size_t nb = B.widths.size();
+    for (size_t b = 0; b <= nb; ++b) {
+        const int64_t first = b < nb ? B.bin_first[b] : S.F, count = b < nb ? B.bin_count[b] : S.F;
+        if (b == nb) P.all0 = (int)P.bin.size();
         for (int64_t q = 0; q < parts[b]; ++q) {
-            const int64_t i0 = B.bin_count[b] * q / parts[b], i1 = B.bin_count[b] * (q + 1) / parts[b];
-            add(B.bin_first[b] + i0, i1 - i0, bin_max[b], (int)b);
+            const int64_t i0 = count * q / parts[b], i1 = count * (q + 1) / parts[b];
+            add(first + i0, i1 - i0, b < nb ? bin_max[b] : all_max, b < nb ? (int)b : -1);
         }
-    add(S.F, S.F, all_max, -1);
+    }
     const int ng = (int)P.bin.size();
     P.n_groups = ng;
     P.n_internal = ni;
@@ -770,17 +774,23 @@ int build_groups(cafe_ctx* C, const TreeHost& T, FamSet& S, const std::vector<in
 int build_patterns(cafe_ctx* C, const TreeHost& T, FamSet& S, const std::vector<int>& bin_max, int all_max) {
     const BinPlan& B = S.bins;
     const size_t limit = table_limit(C, kGroupBytes);
-    std::vector<int64_t> parts(B.widths.size(), 1);
+    const size_t nb = B.widths.size();
+    std::vector<int64_t> parts(nb + 1, 1);
+    // (the whole set at the bounds that the reference takes for it, up to the
+    // longest vectors that k_pat64 takes)
+    const int64_t all_states = std::min<int64_t>((int64_t)all_max + std::max(50, all_max / 5) + 1, 3168);
     for (;;) {
         const int rc = build_groups(C, T, S, bin_max, all_max, parts);
         if (rc) return rc;
         // (parts share no rows, so a cut may have to be repeated)
         std::vector<int64_t> more(parts);
-        for (int g = 0; g < S.pats.all(); ++g) {
-            const int b = S.pats.bin[g];
-            // (8 W + 32 bytes a row: twice the tensor cores', more than FP64's)
-            const int64_t need = (int64_t)(row_bytes(S.pats, g, B.widths[b] + 3) / limit);
-            if (need > 0) more[b] = std::min(B.bin_count[b], std::max(more[b], std::max(2 * parts[b], need + need / 4 + 1)));
+        for (int g = 0; g < S.pats.n_groups; ++g) {
+            const bool bin = S.pats.bin[g] >= 0;
+            const size_t b = bin ? S.pats.bin[g] : nb;
+            // (a bin: 8 W + 32 bytes a row, twice the tensor cores', more than FP64's)
+            const int64_t need = (int64_t)(row_bytes(S.pats, g, bin ? B.widths[b] + 3 : all_states) / limit);
+            if (need > 0)
+                more[b] = std::min(bin ? B.bin_count[b] : S.F, std::max(more[b], std::max(2 * parts[b], need + need / 4 + 1)));
         }
         if (more == parts) return CAFE_OK;
         parts.swap(more);
@@ -1231,7 +1241,7 @@ int pat64_class(const PatGroup& q, bool max_product = false) {
 }
 
 // Factor tables: of one combination, up to kWaveBytes for groups that run side by
-// side, and up to kRowTableBytes where all families are one group (past it they
+// side, and up to kRowTableBytes for a group at global bounds (past it they
 // are left to the tile walks, whose vectors take the same memory whatever their
 // number); of several combinations, kTableBytes.
 constexpr size_t kWaveBytes = (size_t)8 << 30, kRowTableBytes = (size_t)8 << 30, kTableBytes = (size_t)2 << 30;
@@ -1240,11 +1250,19 @@ constexpr size_t kWaveBytes = (size_t)8 << 30, kRowTableBytes = (size_t)8 << 30,
 // Counts past the states and the error model's reach (half deviations) share a
 // leaf's last row.
 bool takes_rows(const cafe_ctx* C, const TreeHost& T, const PatternPlan& P, int S, int R, int half) {
-    const int g = P.all();
-    if (pat64_class({g, S, R}) < 0) return false;
+    if (pat64_class({P.all0, S, R}) < 0) return false;
     const size_t n = (size_t)std::max(S, R) + 1;
-    const size_t leaf = (size_t)T.n_leaves * (size_t)(std::min<int64_t>(P.group_max[g], (int64_t)S + half + 1) + 1);
-    return row_bytes(P, g, n) + leaf * (n + 1) * sizeof(double) <= table_limit(C, kRowTableBytes);
+    for (int g = P.all0; g < P.n_groups; ++g) {
+        const size_t leaf = (size_t)T.n_leaves * (size_t)(std::min<int64_t>(P.group_max[g], (int64_t)S + half + 1) + 1);
+        if (row_bytes(P, g, n) + leaf * (n + 1) * sizeof(double) > table_limit(C, kRowTableBytes)) return false;
+    }
+    return true;
+}
+// All families' groups at those bounds.
+std::vector<PatGroup> all_groups(const PatternPlan& P, int S, int R) {
+    std::vector<PatGroup> v;
+    for (int g = P.all0; g < P.n_groups; ++g) v.push_back({g, S, R});
+    return v;
 }
 
 // A max-product pass (one group): k_pat64's extra operands, and where the
@@ -1617,7 +1635,7 @@ int enqueue_mixed(cafe_ctx* C, Workspace& ws, const cafe_request* R, TreeHost& T
 
     std::vector<int> tc_groups;
     std::vector<PatGroup> wide;      // bins past the tensor cores' width
-    for (int g = 0; g < S.pats.all(); ++g) {
+    for (int g = 0; g < S.pats.all0; ++g) {
         const int w = B.widths[S.pats.bin[g]];
         if (w > kTcMaxW) wide.push_back(PatGroup{g, w - 1, w - 1});
         else if (S.pats.group_count[g] > 0) tc_groups.push_back(g);
@@ -2252,9 +2270,9 @@ int enqueue_score(cafe_ctx* C, Workspace& ws, const cafe_request* Rs, int NB, do
     // FP64: every family at the reference's global bounds, or by S-bin
     std::vector<PatGroup> groups;
     if (ref_mode) {
-        groups.push_back(PatGroup{S.pats.all(), Sg, Rg});
+        groups = all_groups(S.pats, Sg, Rg);
     } else {
-        for (int g = 0; g < S.pats.all(); ++g) {
+        for (int g = 0; g < S.pats.all0; ++g) {
             const int w = S.bins.widths[S.pats.bin[g]];
             groups.push_back(PatGroup{g, w - 1, w - 1});
         }
@@ -2556,10 +2574,15 @@ int recon_setup(cafe_ctx* C, Workspace& ws, const cafe_request* R, bool categori
 // kRowTableBytes.
 // `words`: [0] counts the failed (category, family) pairs, [1] is set when a
 // bounded wait gave up, both zeroed.
-size_t max_product_bytes(const TreeHost& T, const PatternPlan& P, int S) {      // of a category
-    size_t n = 0;
-    for (size_t ii = 0; ii + 1 < T.internal.size(); ++ii) n += (size_t)P.row_count(P.all(), (int)ii) * (S + 2);
-    return (n + (size_t)T.n_leaves * (S + 1) * (S + 2)) * (sizeof(double) + sizeof(int32_t));
+// A category's tables, of its largest group.
+size_t max_product_bytes(const TreeHost& T, const PatternPlan& P, int S) {
+    size_t most = 0;
+    for (int g = P.all0; g < P.n_groups; ++g) {
+        size_t n = (size_t)T.n_leaves * (S + 1);
+        for (int ii = 0; ii + 1 < P.n_internal; ++ii) n += (size_t)P.row_count(g, ii);
+        most = std::max(most, n * (S + 2) * (sizeof(double) + sizeof(int32_t)));
+    }
+    return most;
 }
 
 int reconstruct_rows(cafe_ctx* C, Workspace& ws, const cafe_request* R, const ReconSetup& Z, int root_len, int32_t* words) {
@@ -2597,8 +2620,6 @@ int reconstruct_rows(cafe_ctx* C, Workspace& ws, const cafe_request* R, const Re
     const int32_t* d_ints = reinterpret_cast<const int32_t*>(d + o_int);
     CK(cudaMemcpyAsync(d, ptr.data(), o_long, cudaMemcpyHostToDevice, ws.stream), "h2d");
     CK(cudaMemcpyAsync(d + o_int, ints.data(), ints.size() * sizeof(int32_t), cudaMemcpyHostToDevice, ws.stream), "h2d");
-    CK(cudaMemcpyAsync(d + o_long, &P.child_off[(size_t)P.all() * ni], ni * sizeof(int64_t), cudaMemcpyHostToDevice, ws.stream),
-       "h2d");
     CK(launch_log2_rows(reinterpret_cast<const double* const*>(dptr + (size_t)K * n),
                         reinterpret_cast<float* const*>(const_cast<void**>(dptr + (size_t)K * n + src.size())),
                         (int)src.size(), n_st, Z.msize, pitch, ws.stream),
@@ -2613,38 +2634,42 @@ int reconstruct_rows(cafe_ctx* C, Workspace& ws, const cafe_request* R, const Re
     mx.root_max = ws.rc_rmax.as<double>();
     mx.root_arg = ws.rc_arg.as<int32_t>();
     mx.n_failed = words;
-    const std::vector<PatGroup> group{{P.all(), Z.Smax, root_len - 1}};
-    for (int k0 = 0; k0 < K; k0 += pass) {
-        const int nk = std::min(pass, K - k0);
-        if (k0) CK(cudaStreamSynchronize(ws.stream), "reconstruct");     // (the staging buffers are read)
-        int rc = launch_pat64_groups(C, ws, R, T, *Z.S, nullptr, group, nk, d_ints + k0, K, Z.msize, false,
-                                     nullptr, words + 1, false, 0, &mx);
-        if (rc) return rc;
-        if (!k0) {
-            CK(cudaMemcpyAsync(d + o_long + ni * sizeof(int64_t), mx.ctab_off.data(), ni * sizeof(int64_t),
-                               cudaMemcpyHostToDevice, ws.stream), "h2d");
-            CK(cudaMemcpyAsync(d + o_int + ints.size() * sizeof(int32_t), mx.pitch.data(), ni * sizeof(int32_t),
-                               cudaMemcpyHostToDevice, ws.stream), "h2d");
+    for (int g = P.all0; g < P.n_groups; ++g)
+        for (int k0 = 0; k0 < K; k0 += pass) {
+            const int nk = std::min(pass, K - k0);
+            if (k0 || g > P.all0) CK(cudaStreamSynchronize(ws.stream), "reconstruct");     // (the staging buffers are read)
+            int rc = launch_pat64_groups(C, ws, R, T, *Z.S, nullptr, {{g, Z.Smax, root_len - 1}}, nk, d_ints + k0, K, Z.msize,
+                                         false, nullptr, words + 1, false, 0, &mx);
+            if (rc) return rc;
+            if (!k0) {
+                CK(cudaMemcpyAsync(d + o_long, &P.child_off[(size_t)g * ni], ni * sizeof(int64_t), cudaMemcpyHostToDevice,
+                                   ws.stream), "h2d");
+                CK(cudaMemcpyAsync(d + o_long + ni * sizeof(int64_t), mx.ctab_off.data(), ni * sizeof(int64_t),
+                                   cudaMemcpyHostToDevice, ws.stream), "h2d");
+                CK(cudaMemcpyAsync(d + o_int + ints.size() * sizeof(int32_t), mx.pitch.data(), ni * sizeof(int32_t),
+                                   cudaMemcpyHostToDevice, ws.stream), "h2d");
+            }
+            BacktrackArgs b;
+            std::memset(&b, 0, sizeof b);
+            b.plan = T.plan;
+            b.node_ii = d_ints + K;
+            b.child_off = reinterpret_cast<const int64_t*>(d + o_long);
+            b.child = P.d_child.as<int32_t>();
+            b.ctab_off = b.child_off + ni;
+            b.pitch = d_ints + ints.size();
+            b.ctab = ws.rc_c.as<int32_t>();
+            b.ctab_stride = mx.ctab_stride;
+            b.root_arg = ws.rc_arg.as<int32_t>();
+            b.status = words + 1;
+            b.F = F;
+            b.f0 = P.group_first[g] - F;
+            b.nf = P.group_count[g];
+            b.k0 = k0;
+            b.n_k = nk;
+            b.row = ws.rc_row.as<int32_t>();
+            b.state = ws.rc_state.as<int32_t>();
+            CK(launch_backtrack(b, ws.stream), "backtrack");
         }
-        BacktrackArgs b;
-        std::memset(&b, 0, sizeof b);
-        b.plan = T.plan;
-        b.node_ii = d_ints + K;
-        b.child_off = reinterpret_cast<const int64_t*>(d + o_long);
-        b.child = P.d_child.as<int32_t>();
-        b.ctab_off = b.child_off + ni;
-        b.pitch = d_ints + ints.size();
-        b.ctab = ws.rc_c.as<int32_t>();
-        b.ctab_stride = mx.ctab_stride;
-        b.root_arg = ws.rc_arg.as<int32_t>();
-        b.status = words + 1;
-        b.F = F;
-        b.k0 = k0;
-        b.n_k = nk;
-        b.row = ws.rc_row.as<int32_t>();
-        b.state = ws.rc_state.as<int32_t>();
-        CK(launch_backtrack(b, ws.stream), "backtrack");
-    }
     return CAFE_OK;
 }
 
@@ -3283,7 +3308,7 @@ int pvalues_device(cafe_ctx* C, Workspace& ws, const ReconSetup& Z, bool stream,
     if (F > 0 && takes_rows(C, T, FS.pats, S, RR, 0)) {
         cafe_request rq;
         std::memset(&rq, 0, sizeof rq);
-        rc = launch_pat64_groups(C, ws, &rq, T, FS, nullptr, {{FS.pats.all(), S, RR}}, 1, d_ntiles.as<int32_t>() + 2, 1, msize,
+        rc = launch_pat64_groups(C, ws, &rq, T, FS, nullptr, all_groups(FS.pats, S, RR), 1, d_ntiles.as<int32_t>() + 2, 1, msize,
                                  false, nullptr, d_status, false, 0, nullptr, d_obsL.as<double>());
         if (rc && rc != CAFE_ERR_OOM) return rc;
     }
@@ -4265,10 +4290,12 @@ Footprint request_footprint(cafe_ctx* C, const cafe_request& r) {
     auto leaves = [&](int g, size_t n) { return (size_t)S.n_leaves * (std::min<size_t>(P.group_max[g], n) + 1) * (n + 1) * sizeof(double); };
     if (r.precision == CAFE_PREC_FP64_REF) {
         const size_t n = (size_t)std::max(0, std::max(r.max_family_size, r.max_root_family_size)) + 1;
-        fp64 = row_bytes(P, P.all(), n) + leaves(P.all(), n);
-        if (fp64 > kRowTableBytes) fp64 = 0;      // (the tile walk's vectors)
+        for (int g = P.all0; g < P.n_groups; ++g) {
+            const size_t one = row_bytes(P, g, n) + leaves(g, n);
+            if (one <= kRowTableBytes) fp64 += one;      // (the tile walk's vectors take none)
+        }
     } else {
-        for (int g = 0; g < P.all(); ++g) {
+        for (int g = 0; g < P.all0; ++g) {
             const size_t w = S.bins.widths[P.bin[g]];
             if (r.precision == CAFE_PREC_MIXED_TF32X3 && w <= (size_t)kTcMaxW)
                 tc += row_bytes(P, g, w) / ((w + 1) * sizeof(double)) * (w * sizeof(float) + sizeof(int4));
@@ -4277,7 +4304,7 @@ Footprint request_footprint(cafe_ctx* C, const cafe_request& r) {
         }
     }
     f.tables = K * (fp64 + tc);
-    f.most = (fp64 ? std::max(kTableBytes, r.precision == CAFE_PREC_FP64_REF ? fp64 : std::min(fp64, kWaveBytes)) : 0) +
+    f.most = (fp64 ? std::max(kTableBytes, std::min(fp64, kWaveBytes)) : 0) +
              (tc ? kTcTableBytes : 0);
     return f;
 }

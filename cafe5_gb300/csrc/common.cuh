@@ -505,8 +505,9 @@ struct BacktrackArgs {
     const int32_t* root_arg;     // [K][F]
     const int32_t* status;       // nonzero: the tables are incomplete
     int64_t F;
+    int64_t f0, nf;              // families f0 .. f0 + nf - 1, whose patterns these are
     int k0, n_k;                 // categories k0 .. k0 + n_k - 1
-    int32_t* row;                // [n_k][F][n_internal] scratch
+    int32_t* row;                // [n_k][nf][n_internal] scratch
     int32_t* state;              // [K][F][n_nodes] out
 };
 cudaError_t launch_backtrack(const BacktrackArgs& a, cudaStream_t s);

@@ -363,15 +363,15 @@ __global__ void k_log2_rows(const double* const* __restrict__ src, float* const*
 
 __global__ void k_backtrack(BacktrackArgs a) {
     const TreePlan& P = a.plan;
-    const int64_t total = *a.status ? 0 : a.F * a.n_k;
+    const int64_t total = *a.status ? 0 : a.nf * a.n_k;
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
-        const int kk = (int)(e / a.F), k = a.k0 + kk;
-        const int64_t f = e % a.F;
+        const int kk = (int)(e / a.nf), k = a.k0 + kk;
+        const int64_t f = a.f0 + e % a.nf;
         const int32_t* C = a.ctab + (size_t)kk * a.ctab_stride;
         int32_t* out = a.state + ((size_t)k * a.F + f) * P.n_nodes;
         int32_t* row = a.row + (size_t)e * P.n_internal;
         out[P.root] = a.root_arg[(size_t)k * a.F + f];
-        row[P.n_internal - 1] = (int32_t)f;      // (the root keeps a row per family)
+        row[P.n_internal - 1] = (int32_t)(e % a.nf);      // (the root keeps a row per family)
         for (int ii = P.n_internal - 1; ii >= 0; --ii) {
             const int c0 = P.cstart[ii], nch = P.cstart[ii + 1] - c0;
             const int s = out[P.internal[ii]];
@@ -401,7 +401,7 @@ cudaError_t launch_log2_rows(const double* const* src, float* const* dst, int n_
 }
 
 cudaError_t launch_backtrack(const BacktrackArgs& a, cudaStream_t s) {
-    const int64_t total = a.F * a.n_k;
+    const int64_t total = a.nf * a.n_k;
     if (total <= 0) return cudaSuccess;
     k_backtrack<<<(unsigned)std::min<int64_t>((total + 127) / 128, 8192), 128, 0, s>>>(a);
     return cudaGetLastError();

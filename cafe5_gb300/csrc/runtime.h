@@ -73,9 +73,10 @@ struct BinPlan {
 
 // Distinct count patterns below every internal node, per group of families
 // (k_patterns.cu): the rows the pruning kernels contract. The groups are the
-// S-bins in order (a very large one in several), and all families together.
+// S-bins in order, and from all0 on all families together (a very large one of
+// these is several).
 struct PatternPlan {
-    int n_groups = 0, n_internal = 0;
+    int n_groups = 0, n_internal = 0, all0 = 0;
     std::vector<int64_t> group_first, group_count;   // items (families in group order)
     std::vector<int> group_max;       // largest count
     std::vector<int> bin;             // S-bin, -1 for all families
@@ -83,7 +84,6 @@ struct PatternPlan {
     std::vector<int64_t> child_off;   // [group][internal]: first child index in d_child
     std::vector<int64_t> leaf_off;    // [group][leaf]: first of the counts that occur there, in d_counts; then the end
     DevBuf d_child, d_counts;
-    int all() const { return n_groups - 1; }
     int64_t row_count(int g, int ii) const { return rows[(size_t)g * n_internal + ii]; }
 };
 
