@@ -75,12 +75,21 @@ __device__ __forceinline__ void bar_arrive(int id, int n) {
     asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory");
 }
 
-// High word of |x|, with 0 only for an exact zero. (Vectors can hold negative
-// values: a search over an error model's epsilon may try a negative one.)
-__device__ __forceinline__ int hi_abs(double x) { return __double2hiint(x) & 0x7fffffff; }
+// High word of a value >= 0, with 0 only for an exact zero.
 __device__ __forceinline__ int hi_key(double x) {
-    const int h = hi_abs(x);
+    const int h = __double2hiint(x);
     return h ? h : (__double2loint(x) ? 1 : 0);
+}
+// The same of |x|, for vectors: they can hold negative values (a search over an
+// error model's epsilon may try a negative one). A negative partial sum needs none:
+// its word is below every exponent's, and then no chunk is left out.
+__device__ __forceinline__ int hi_key_abs(double x) {
+    const int h = __double2hiint(x) & 0x7fffffff;
+    return h ? h : (__double2loint(x) ? 1 : 0);
+}
+// 0 < p <= infinity, on the integer pipe.
+__device__ __forceinline__ bool has_log(double p) {
+    return (unsigned long long)(__double_as_longlong(p) - 1) < 0x7ff0000000000000ull;
 }
 
 // One thread: wait until *p has reached n.
@@ -233,13 +242,13 @@ __device__ void root_family(const Pat64Args& a, const Pat64Node& nd, const NodeS
         // NaN among them, have no logarithm)
         float top = -INFINITY;
         for (int j = lane; j < Rf; j += 32)
-            if (j < a.n_prior && a.prior[j] > 0.0) top = fmaxf(top, flog2(x[j]) + flog2(a.prior[j]));
+            if (j < a.n_prior && has_log(a.prior[j])) top = fmaxf(top, flog2(x[j]) + flog2(a.prior[j]));
 #pragma unroll
         for (int q = 16; q > 0; q >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, q));
         double best = -INFINITY;
         if (top > -INFINITY)
             for (int j = lane; j < Rf; j += 32)
-                if (j < a.n_prior && a.prior[j] > 0.0 && flog2(x[j]) + flog2(a.prior[j]) >= top - 0.015625f) {
+                if (j < a.n_prior && has_log(a.prior[j]) && flog2(x[j]) + flog2(a.prior[j]) >= top - 0.015625f) {
                     const double v = log(x[j]) + log(a.prior[j]);
                     best = v > best ? v : best;
                 }
@@ -362,7 +371,7 @@ __device__ __forceinline__ void fill_rows(const Pat64Args& a, const Unit& u, dou
         for (int i = 0; i < 8; ++i) {
             L[j0 + 4 * i] = x[i];
             mx = x[i] > mx ? x[i] : mx;
-            m = max(m, hi_key(x[i]));
+            m = max(m, hi_key_abs(x[i]));
         }
         if (!a.scaled) {
             m = __reduce_max_sync(0xffffffffu, m);
@@ -399,7 +408,7 @@ __device__ __forceinline__ void fill_rows(const Pat64Args& a, const Unit& u, dou
                 x = scalbn(x, -e);
                 L[ck * KC + l + 4 * i] = x;
             }
-            m = max(m, hi_key(x));
+            m = max(m, hi_key_abs(x));
         }
         m = __reduce_max_sync(0xffffffffu, m);
         if (lane == 0) lmax[ck] = m;
@@ -435,7 +444,7 @@ __device__ __forceinline__ void fill_few(const Pat64Args& a, const Unit& u, doub
                 L[(c0 + i) * KC + lane] = x[i];
                 mx = x[i] > mx ? x[i] : mx;
                 if (!a.scaled) {
-                    const int m = __reduce_max_sync(0xffffffffu, hi_key(x[i]));
+                    const int m = __reduce_max_sync(0xffffffffu, hi_key_abs(x[i]));
                     if (lane == 0) lmax[c0 + i] = r ? max(lmax[c0 + i], m) : m;
                 }
             }
@@ -448,7 +457,7 @@ __device__ __forceinline__ void fill_few(const Pat64Args& a, const Unit& u, doub
                 x = scalbn(x, -e);
                 L[ck * KC + lane] = x;
             }
-            const int m = __reduce_max_sync(0xffffffffu, hi_key(x));
+            const int m = __reduce_max_sync(0xffffffffu, hi_key_abs(x));
             if (lane == 0) lmax[ck] = r ? max(lmax[ck], m) : m;
         }
         // the row's exponent, once per row (the unit of its first states)
@@ -578,7 +587,7 @@ __device__ __forceinline__ void few_rows(const Pat64Args& a, const Unit& u, cons
                 int am = 0x7fffffff;
 #pragma unroll
                 for (int r = 0; r < kFewRows; ++r)
-                    if (r < np) am = min(am, hi_abs(acc[r]));
+                    if (r < np) am = min(am, __double2hiint(acc[r]));
                 const int ea = am >> 20;
                 skip = mk == 0 || lk == 0 || (ea > 0 && (mk >> 20) + (lk >> 20) + 2 <= ea + 968);
                 skip = __all_sync(0xffffffffu, skip);
@@ -816,7 +825,8 @@ __global__ void __launch_bounds__(NTHR, 6) k_pat64(const Pat64Args a) {
                         for (int h = 0; h < KC / 8; ++h) mk = max(mk, hi_key(pf[h]));
 #pragma unroll
                         for (int o = 1; o < 8; o <<= 1) mk = max(mk, __shfl_xor_sync(0xffffffffu, mk, o));
-                        const int am = min(min(hi_abs(acc[0]), hi_abs(acc[1])), min(hi_abs(acc[2]), hi_abs(acc[3])));
+                        const int am = min(min(__double2hiint(acc[0]), __double2hiint(acc[1])),
+                                           min(__double2hiint(acc[2]), __double2hiint(acc[3])));
                         const int ea = am >> 20;
                         skip = mk == 0 || lk == 0 || (ea > 0 && (mk >> 20) + (lk >> 20) + 2 <= ea + 968);
                         skip = __all_sync(0xffffffffu, skip);
