@@ -1600,6 +1600,7 @@ int enqueue_mixed(cafe_ctx* C, Workspace& ws, const cafe_request* R, TreeHost& T
     // entry stamped with this request already has its conversion slot)
     std::vector<int32_t> mat_index((size_t)K * T.n_nodes, -1);
     std::vector<ConvertJob> jobs;
+    jobs.reserve(active.size() * T.n_nodes);
     const uint64_t stamp = ++C->request_stamp;
     for (int k = 0; k < K; ++k)
         for (int v = 0; v < T.n_nodes; ++v) {
@@ -1719,6 +1720,7 @@ int enqueue_mixed(cafe_ctx* C, Workspace& ws, const cafe_request* R, TreeHost& T
         size_t blob = 0, ctr = launches.size() * sizeof(unsigned long long);
         for (BinLaunch& L : launches) {
             const int W = B.widths[L.b], Ns = pat_tc_states(W), n_share = W / Ns;
+            L.nodes.reserve(ni);
             std::vector<int> at(T.n_nodes, -1), lvl0(levels + 1, 0);
             std::vector<int64_t> lvl_units(levels, 0);
             int64_t units = 0;
@@ -1777,6 +1779,7 @@ int enqueue_mixed(cafe_ctx* C, Workspace& ws, const cafe_request* R, TreeHost& T
             }
             const int64_t blocks = (n_act + g - 1) / g, skew = skewed ? 1 : levels;
             int64_t widest = 1;
+            L.segs.reserve(blocks * levels);
             for (int64_t t = 0; t <= (blocks - 1) * skew + levels - 1; ++t) {
                 int64_t step = 0;
                 for (int l = levels - 1; l >= 0; --l) {
